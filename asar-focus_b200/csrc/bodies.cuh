@@ -1270,18 +1270,70 @@ ASARF_HD ASARF_INLINE void az_rd_body(const AzRdArgs& a, int tile, int k1, int t
         fft_inverse_pairs<AzRdOut, false>(a.plan2, s + a.hl, a.xt, wt, tid, nthr, AzRdOut{&a, x0, k1});
 }
 
-// ----------------------------------------------------------------------------- ERS level-0 packets
+// ----------------------------------------------------------------------------- level-0 packets
+// Word `w` (0 .. 3) of the 16 bytes that start `sh` bytes into the 32 bytes (lo, hi).
+ASARF_HD ASARF_INLINE uint4 shift_bytes(const uint4& lo, const uint4& hi, unsigned int sh) {
+    const unsigned int bits = 8u * (sh & 3u);
+    const bool two = (sh & 8u) != 0, one = (sh & 4u) != 0;
+    unsigned int v0 = lo.x, v1 = lo.y, v2 = lo.z, v3 = lo.w, v4 = hi.x, v5 = hi.y, v6 = hi.z;
+    const unsigned int v7 = hi.w;
+    if (two) v0 = v2, v1 = v3, v2 = v4, v3 = v5, v4 = v6, v5 = v7;
+    if (one) v0 = v1, v1 = v2, v2 = v3, v3 = v4, v4 = v5;
+    return make_uint4(funnel_r(v0, v1, bits), funnel_r(v1, v2, bits), funnel_r(v2, v3, bits), funnel_r(v3, v4, bits));
+}
+
+// Whole 16-byte units that copy_units may write from n source bytes at src: a unit whose source
+// is not 16-byte aligned is read as the two aligned 16-byte words it lies in, and both words
+// must end inside the n bytes.
+ASARF_HD ASARF_INLINE int copy_units_of(const uint8_t* src, int n) {
+    const int sh = static_cast<int>(reinterpret_cast<uintptr_t>(src) & 15);
+    const int usable = sh ? n - (16 - sh) : n;
+    return usable > 0 ? usable / 16 : 0;
+}
+
+// units 16-byte units from src (any alignment) to dst (16-byte aligned), threads on
+// consecutive units.  The aligned word below src is read too: the callers' sources start
+// inside a packet, past its header.  kBatch units of a thread are loaded before any is stored.
+template <int kBatch>
+ASARF_HD ASARF_INLINE void copy_units(const uint8_t* src, uint8_t* dst, int units, int tid, int nthr) {
+    const unsigned int sh = static_cast<unsigned int>(reinterpret_cast<uintptr_t>(src) & 15);
+    const uint4* a = reinterpret_cast<const uint4*>(src - sh);
+    uint4* d = reinterpret_cast<uint4*>(dst);
+    for (int u0 = tid; u0 < units; u0 += kBatch * nthr) {
+        uint4 lo[kBatch], hi[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            const int u = u0 + k * nthr;
+            if (u < units) {
+                lo[k] = ASARF_LDG(a + u);
+                if (sh) hi[k] = ASARF_LDG(a + u + 1);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            const int u = u0 + k * nthr;
+            if (u < units) d[u] = sh ? shift_bytes(lo[k], hi[k], sh) : lo[k];
+        }
+    }
+}
+
 // Line y of an ERS IM measurement data set: its packet's 11232 measurement bytes go to raw
 // line y, its SWST and PRI codes (big-endian, ISP bytes 38-39 and 40-41 after the 32 bytes of
 // sensing time and FEP annotation) to swst[y] / pri[y]; the FEP ISP length (11465) and the
 // auxiliary section's 0xAA marker are checked as ParseErsLevel0ImPackets checks them
-// (envisat_format/src/ers_im_parse.cc:423-453).  Block y, threads over 2-byte words
-// (packet offsets are even: whole MDSRs of 11498 bytes).
+// (envisat_format/src/ers_im_parse.cc:423-453).  Block y.  Raw lines are multiples of 16 bytes,
+// so a 16-byte aligned raw buffer takes whole 16-byte units; any other one, and the end of a line
+// whose packet is not aligned, 2-byte words (packet offsets are even: whole MDSRs of 11498 bytes).
 ASARF_HD ASARF_INLINE void ers_unpack_line(const ErsUnpackArgs& a, int y, int tid, int nthr) {
     const uint8_t* pk = a.mdsr + ASARF_LDG(a.offset + y);
-    const uint16_t* src = reinterpret_cast<const uint16_t*>(pk + kErsMeasurementOffset);
-    uint16_t* dst = reinterpret_cast<uint16_t*>(a.raw + static_cast<long long>(y) * kErsMeasurementBytes);
-    for (int i = tid; i < kErsMeasurementBytes / 2; i += nthr) dst[i] = src[i];
+    const uint8_t* src = pk + kErsMeasurementOffset;
+    uint8_t* dst = a.raw + static_cast<long long>(y) * kErsMeasurementBytes;
+    const int units =
+        (reinterpret_cast<uintptr_t>(a.raw) & 15) == 0 ? copy_units_of(src, kErsMeasurementBytes) : 0;
+    copy_units<4>(src, dst, units, tid, nthr);
+    const uint16_t* src2 = reinterpret_cast<const uint16_t*>(src);
+    uint16_t* dst2 = reinterpret_cast<uint16_t*>(dst);
+    for (int i = 8 * units + tid; i < kErsMeasurementBytes / 2; i += nthr) dst2[i] = src2[i];
     if (tid == 0) {
         const int isp_len = (pk[24] << 8) | pk[25];
         unsigned e = 0;
@@ -1301,7 +1353,8 @@ ASARF_HD ASARF_INLINE void ers_unpack_line(const ErsUnpackArgs& a, int y, int ti
 // little-endian host), the blocks, zeros up to record_bytes.  SWST and PRI codes are the source
 // packet's.  The packet's data field header length (29) and mode ID (0x54) are checked as the
 // reference checks them (:470-484); a block length beyond the record sets kErrL0Length and the
-// record keeps only what fits.  Block y, threads over the record's bytes.
+// record keeps only what fits.  Block y: the record's 16-byte aligned interior moves by whole
+// units, what lies before and after it (records have any size and any alignment) by bytes.
 ASARF_HD ASARF_INLINE void asar_unpack_line(const AsarUnpackArgs& a, int y, int tid, int nthr) {
     const uint8_t* pk = a.mdsr + ASARF_LDG(a.src + y);
     const int packet_length = (pk[36] << 8) | pk[37];
@@ -1316,13 +1369,18 @@ ASARF_HD ASARF_INLINE void asar_unpack_line(const AsarUnpackArgs& a, int y, int 
     }
     uint8_t* rec = a.records + static_cast<long long>(y) * a.record_bytes;
     const uint8_t* blocks = pk + kAsarPacketHeader;
-    for (int i = tid; i < a.record_bytes; i += nthr) {
-        uint8_t v;
-        if (i == 0) v = static_cast<uint8_t>(len & 0xFF);
-        else if (i == 1) v = static_cast<uint8_t>(len >> 8);
-        else v = (i - 2 < len) ? blocks[i - 2] : static_cast<uint8_t>(0);
-        rec[i] = v;
-    }
+    // record bytes [head, head + 16 units) by units: head is the first aligned byte past the length
+    const int head = 2 + static_cast<int>((16 - (reinterpret_cast<uintptr_t>(rec + 2) & 15)) & 15);
+    const int units = copy_units_of(blocks + (head - 2), len - (head - 2));
+    copy_units<4>(blocks + (head - 2), rec + head, units, tid, nthr);
+    auto byte_at = [&](int i) -> uint8_t {
+        if (i == 0) return static_cast<uint8_t>(len & 0xFF);
+        if (i == 1) return static_cast<uint8_t>(len >> 8);
+        return i - 2 < len ? blocks[i - 2] : static_cast<uint8_t>(0);
+    };
+    const int first = head < a.record_bytes ? head : a.record_bytes;
+    for (int i = tid; i < first; i += nthr) rec[i] = byte_at(i);
+    for (int i = head + 16 * units + tid; i < a.record_bytes; i += nthr) rec[i] = byte_at(i);
     if (tid == 0) {
         if (e) atomic_or_u32(a.errors, e);
         if (a.pri) a.pri[y] = static_cast<uint16_t>((pk[54] << 8) | pk[55]);
