@@ -99,13 +99,13 @@ ASARF_HD inline bool polyfit_qr(const double* x, const double* y, int m, int deg
 // and of CalculateDopplerCentroid (sar/fractional_doppler_centroid.cu:33-69: lag-1
 // azimuth correlation per range block): the IQ correction is affine in the raw bytes,
 // so every sum the reference takes over corrected floats is a closed form of these.
-// Block (bx, by) covers kStatsCols work units and lines [by*L, (by+1)*L).  A unit is either
-// one column (general path) or, when the raw base and line stride are 8-byte aligned, the
-// columns of one Doppler block inside an aligned group of 4 (quad path: columns 4g .. 4g + 3,
-// one aligned 8-byte load per line, byte-lane dot products for all sums; a group that straddles
-// a Doppler block boundary is two units, one per block, each masking the other's columns).
-// Either way every sum a thread keeps belongs to a single Doppler block, and kStatsBatch lines
-// are loaded before any is consumed.
+// Block (bx, by) covers kStatsCols work units and lines [by*L, (by+1)*L).  A unit is the columns
+// of one Doppler block inside an aligned group of 4 (columns 4g .. 4g + 3, one 8-byte window per
+// line, byte-lane dot products for all sums; a group that straddles a Doppler block boundary is
+// two units, one per block, each masking the other's columns), so every sum a thread keeps
+// belongs to a single Doppler block, and kStatsBatch lines are loaded before any is consumed.
+// A window is one aligned 8-byte load when the raw base and line stride are 8-byte aligned,
+// otherwise the three aligned 4-byte words around it, funnelled into place.
 constexpr int kStatsCols = 256;
 constexpr int kStatsBatch = 8;
 constexpr int kStatsMaxLines = 256;
@@ -114,21 +114,24 @@ constexpr int kStatsMaxLines = 256;
 constexpr int kStatsLinesPerBlock = 192;
 constexpr int kStatsBlocksPerSm = 3;  // resident blocks of k_raw_stats (its launch bounds)
 
-// Lines per statistics block for a grid of gx block columns over na lines: kStatsLinesPerBlock,
-// raised in whole batches (at most kStatsMaxLines) when that fits the grid into one wave fewer
-// of the `slots` resident blocks, since the last wave of a grid of equal blocks runs mostly
-// empty (ASAR IM-like 30000 lines, 6 columns, 444 slots: 942 blocks of 192 lines take three
-// waves, 870 of 208 lines two).
+// Lines per statistics block for a grid of gx block columns over na lines.  When blocks of
+// kStatsLinesPerBlock lines fill the `slots` resident blocks more than once, that height, raised
+// in whole batches (at most kStatsMaxLines) when it fits the grid into one wave fewer, since the
+// last wave of a grid of equal blocks runs mostly empty (ASAR IM-like 30000 lines, 6 columns, 444
+// slots: 942 blocks of 192 lines take three waves, 870 of 208 lines two).  Scenes below that
+// get blocks low enough to fill the slots once, at least kStatsMinLines: a block's time is its
+// chain of batches, so blocks of 192 lines left a 768 x 1024 scene to 6 of 148 SMs (kernel time
+// 41 -> 11 us; 2048 x 4096 47 -> 24, 5644 x 9973 101 -> 76 us).
+constexpr int kStatsMinLines = 16;
 inline int stats_lines_per_block(int na, int gx, int slots) {
     const long long rows = (na + kStatsLinesPerBlock - 1) / kStatsLinesPerBlock;
     const long long waves = (rows * gx + slots - 1) / slots;
-    if (waves > 1 && gx > 0) {
-        const long long fit_rows = (waves - 1) * slots / gx;
-        if (fit_rows > 0) {
-            long long l = (na + fit_rows - 1) / fit_rows;
-            l = (l + kStatsBatch - 1) / kStatsBatch * kStatsBatch;
-            if (l <= kStatsMaxLines) return static_cast<int>(l);
-        }
+    const long long fit_rows = gx > 0 ? (waves > 1 ? waves - 1 : 1) * slots / gx : 0;
+    if (fit_rows > 0) {
+        long long l = (na + fit_rows - 1) / fit_rows;
+        l = (l + kStatsBatch - 1) / kStatsBatch * kStatsBatch;
+        if (l < kStatsMinLines) l = kStatsMinLines;
+        if (l <= (waves > 1 ? kStatsMaxLines : kStatsLinesPerBlock)) return static_cast<int>(l);
     }
     return kStatsLinesPerBlock;
 }
@@ -142,8 +145,8 @@ struct RawStatsSmem {
 // Host side: work units and grid width of the statistics kernel for this raw buffer.
 inline int raw_stats_grid_x(RawStatsArgs& a, const void* raw) {
     a.gpb = (a.dc_step + 3) / 4 + 1;  // aligned groups a block's columns touch
-    a.quad = (reinterpret_cast<uintptr_t>(raw) % 8 == 0 && a.line_bytes % 8 == 0) ? 1 : 0;
-    const int units = a.quad ? a.nblk * a.gpb : a.nr;
+    a.aligned = (reinterpret_cast<uintptr_t>(raw) % 8 == 0 && a.line_bytes % 8 == 0) ? 1 : 0;
+    const int units = a.nblk * a.gpb;
     return (units + kStatsCols - 1) / kStatsCols;
 }
 
@@ -217,69 +220,15 @@ ASARF_HD ASARF_INLINE void raw_stats_reduce(RawStatsSmem* sm, bool valid, int bl
 #endif
 }
 
-// General path: one column per unit, one 2-byte load per line.
-ASARF_HD ASARF_INLINE void raw_stats_column(const RawStatsArgs& a, const RawStatsSmem* sm, int x, int y0, int y1,
-                                            int ys, unsigned long long mv[6], unsigned int lv[9]) {
-    unsigned int cnt = 0, si = 0, sq = 0, sii = 0, sqq = 0, siq = 0;
-    unsigned int l0 = 0, l1 = 0, l2 = 0, l3 = 0, l4 = 0, l5 = 0, l6 = 0, l7 = 0, l8 = 0;
-    unsigned int pi = 0, pq = 0;
-    bool pf = false;
-    const uint8_t* col = a.raw + 2ll * x;
-    for (int yg = ys; yg < y1; yg += kStatsBatch) {
-        unsigned int w[kStatsBatch];
-        bool f[kStatsBatch];
-#pragma unroll
-        for (int u = 0; u < kStatsBatch; ++u) {
-            const int y = yg + u;
-            f[u] = false;
-            w[u] = 0u;
-            if (y < y1) {
-                const int off = sm->off[y - ys];
-                const int i = x - off;
-                if (i >= 0 && i < a.spl) {
-                    f[u] = true;
-                    w[u] = *reinterpret_cast<const uint16_t*>(col + static_cast<long long>(y) * a.line_bytes - 2ll * off);
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kStatsBatch; ++u) {
-            const int y = yg + u;
-            if (y >= y1) break;
-            const unsigned int iv = w[u] & 0xffu, qv = w[u] >> 8;
-            if (y >= y0 && f[u]) {
-                cnt += 1;
-                si += iv;
-                sq += qv;
-                sii += iv * iv;
-                sqq += qv * qv;
-                siq += iv * qv;
-                if (y > 0 && pf) {
-                    l0 += 1;
-                    l1 += pi;
-                    l2 += pq;
-                    l3 += iv;
-                    l4 += qv;
-                    l5 += pi * iv;
-                    l6 += pq * qv;
-                    l7 += pi * qv;
-                    l8 += pq * iv;
-                }
-            }
-            pi = iv;
-            pq = qv;
-            pf = f[u];
-        }
-    }
-    mv[0] = cnt, mv[1] = si, mv[2] = sq, mv[3] = sii, mv[4] = sqq, mv[5] = siq;
-    lv[0] = l0, lv[1] = l1, lv[2] = l2, lv[3] = l3, lv[4] = l4, lv[5] = l5, lv[6] = l6, lv[7] = l7, lv[8] = l8;
-}
-
-// Quad path: the columns of `colmask` (bit k: column x0 + k) of the aligned group at x0
-// (x0 % 4 == 0), all in one Doppler block.  A line's four samples are the aligned 8 bytes
-// (I0 Q0 I1 Q1 | I2 Q2 I3 Q3) at raw + y*line_bytes + 2*(x0 - off) (the SWST shift is a
-// multiple of 4 samples, so the window stays aligned on every line).  Samples outside the
-// record or the mask are zero bytes, which drop out of every sum.
+// The columns of `colmask` (bit k: column x0 + k) of the aligned group at x0 (x0 % 4 == 0), all in
+// one Doppler block.  A line's four samples are the 8 bytes (I0 Q0 I1 Q1 | I2 Q2 I3 Q3) at
+// raw + y*line_bytes + 2*(x0 - off) (the SWST shift is a multiple of 4 samples, so with ALIGNED the
+// window stays 8-byte aligned on every line; without, it starts at any even address, and a window
+// at the very start or end of its record is read sample by sample, so that the words around a
+// window never leave the record: 5193 x 17011, 10386-byte lines, 206 us, against 296 one column and
+// one 2-byte load at a time).  Samples outside the record or the mask are zero bytes, which
+// drop out of every sum.
+template <bool ALIGNED>
 ASARF_HD ASARF_INLINE void raw_stats_quad(const RawStatsArgs& a, const RawStatsSmem* sm, int x0, unsigned int colmask,
                                           int y0, int y1, int ys, unsigned long long mv[6], unsigned int lv[9]) {
     constexpr unsigned int kLo = 0x00ff00ffu, kOnes = 0x01010101u;
@@ -310,9 +259,18 @@ ASARF_HD ASARF_INLINE void raw_stats_quad(const RawStatsArgs& a, const RawStatsS
             if (y < ye) {
                 const int off = sm->off[y - ys];
                 const int i = x0 - off;
-                if (i >= 0 && i + 4 <= a.spl) {
+                constexpr int kMargin = ALIGNED ? 0 : 1;  // samples the words around a window reach past it
+                if (i >= kMargin && i + 4 + kMargin <= a.spl) {
                     // the whole 8-byte window is inside the record
-                    w[u] = *reinterpret_cast<const uint2*>(base + static_cast<long long>(y) * a.line_bytes - 2ll * off);
+                    const uint8_t* p = base + static_cast<long long>(y) * a.line_bytes - 2ll * off;
+                    if constexpr (ALIGNED) {
+                        w[u] = *reinterpret_cast<const uint2*>(p);
+                    } else {
+                        const unsigned int odd = static_cast<unsigned int>(reinterpret_cast<uintptr_t>(p) & 2);
+                        const uint32_t* q = reinterpret_cast<const uint32_t*>(p - odd);
+                        const uint32_t q0 = q[0], q1 = q[1], q2 = odd ? q[2] : 0u;
+                        w[u] = make_uint2(funnel_r(q0, q1, 8 * odd), funnel_r(q1, q2, 8 * odd));
+                    }
                     fbv[u] = colbits;
                     vec[u] = true;
                 } else {
@@ -412,6 +370,7 @@ ASARF_HD ASARF_INLINE void raw_stats_quad(const RawStatsArgs& a, const RawStatsS
     lv[0] = l0, lv[1] = l1, lv[2] = l2, lv[3] = l3, lv[4] = l4, lv[5] = l5, lv[6] = l6, lv[7] = l7, lv[8] = l8;
 }
 
+template <bool ALIGNED>
 ASARF_HD ASARF_INLINE void raw_stats_body(const RawStatsArgs& a, int bx, int by, int tid, int nthr,
                                           RawStatsSmem* sm) {
     unsigned long long* flat = &sm->mom[0];
@@ -422,31 +381,22 @@ ASARF_HD ASARF_INLINE void raw_stats_body(const RawStatsArgs& a, int bx, int by,
     const int ys = y0 > 0 ? y0 - 1 : 0;
     for (int y = ys + tid; y < y1; y += nthr) sm->off[y - ys] = a.swst ? 4 * (static_cast<int>(a.swst[y]) - a.min_swst) : 0;
     ASARF_SYNC();
-    const FastDiv dstep = make_fastdiv(static_cast<unsigned int>(a.dc_step));
     const FastDiv dgpb = make_fastdiv(static_cast<unsigned int>(a.gpb));
     for (int c = tid; c < kStatsCols; c += nthr) {
         const int unit = bx * kStatsCols + c;
         unsigned long long mv[6] = {0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
         unsigned int lv[9] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-        bool valid;
-        int blk;
-        if (a.quad) {
-            // group k of Doppler block blk: the aligned group at (block start & ~3) + 4k, the
-            // block's columns [xs, xe) in it
-            blk = static_cast<int>(fdiv_u(static_cast<unsigned int>(unit), dgpb));
-            const int xs = blk * a.dc_step;
-            const int xe = (blk + 1) * a.dc_step < a.nr ? (blk + 1) * a.dc_step : a.nr;
-            const int x0 = (xs & ~3) + 4 * (unit - blk * a.gpb);
-            const int c_lo = xs > x0 ? xs - x0 : 0;
-            const int c_hi = xe - x0 < 4 ? xe - x0 : 4;
-            valid = blk < a.nblk && c_hi > c_lo;
-            const unsigned int colmask = valid ? ((1u << c_hi) - 1u) & ~((1u << c_lo) - 1u) : 0u;
-            if (valid) raw_stats_quad(a, sm, x0, colmask, y0, y1, ys, mv, lv);
-        } else {
-            valid = unit < a.nr;
-            blk = valid ? static_cast<int>(fdiv_u(static_cast<unsigned int>(unit), dstep)) : 0;
-            if (valid) raw_stats_column(a, sm, unit, y0, y1, ys, mv, lv);
-        }
+        // group k of Doppler block blk: the aligned group at (block start & ~3) + 4k, the
+        // block's columns [xs, xe) in it
+        const int blk = static_cast<int>(fdiv_u(static_cast<unsigned int>(unit), dgpb));
+        const int xs = blk * a.dc_step;
+        const int xe = (blk + 1) * a.dc_step < a.nr ? (blk + 1) * a.dc_step : a.nr;
+        const int x0 = (xs & ~3) + 4 * (unit - blk * a.gpb);
+        const int c_lo = xs > x0 ? xs - x0 : 0;
+        const int c_hi = xe - x0 < 4 ? xe - x0 : 4;
+        const bool valid = blk < a.nblk && c_hi > c_lo;
+        const unsigned int colmask = valid ? ((1u << c_hi) - 1u) & ~((1u << c_lo) - 1u) : 0u;
+        if (valid) raw_stats_quad<ALIGNED>(a, sm, x0, colmask, y0, y1, ys, mv, lv);
         raw_stats_reduce(sm, valid, blk, mv, lv);
     }
     ASARF_SYNC();
@@ -655,7 +605,7 @@ ASARF_HD ASARF_INLINE void stats_fold_body(const RawStatsArgs& a, int tiles_y, i
 }
 
 // ----------------------------------------------------------------------------- finalisation
-// Single-threaded: IQ statistics and correction constants exactly as RawDataCorrection
+// IQ statistics and correction constants exactly as RawDataCorrection
 // derives them (sar/iq_correction.cu:200-273, CalcMean/CalcStdDev of
 // cuda_util/device_padded_image.cu:331-414), the Doppler centroid per range block and its
 // quadratic fit (sar/fractional_doppler_centroid.cu:98-139), and the results-window choice
@@ -753,17 +703,11 @@ ASARF_HD inline void finalize_block(const FinalizeArgs& a, const FinalizeMap& m,
     st.dc_blk_hz[b] = hz;
 }
 
-// Doppler polynomial fit over the blocks, the DC-sign variant and the error bits.
-ASARF_HD inline void finalize_fit(const FinalizeArgs& a, FocusState& st, const double* xs, const double* ys,
-                                  unsigned int err) {
-    const int nblk = a.nblk < kMaxDcBlocks ? a.nblk : kMaxDcBlocks;
+// The fitted Doppler polynomial (or the caller's), the DC-sign variant and the error bits.
+ASARF_HD inline void finalize_poly(const FinalizeArgs& a, FocusState& st, double poly[3], unsigned int err) {
     if (a.nblk > kMaxDcBlocks) err |= kErrDcBlocks;
-    st.nblk = nblk;
-    double poly[3] = {0.0, 0.0, 0.0};
-    polyfit_qr<kMaxDcBlocks, 3>(xs, ys, nblk, 2, poly);
-    st.dc_est[0] = poly[0];
-    st.dc_est[1] = poly[1];
-    st.dc_est[2] = poly[2];
+    st.nblk = a.nblk < kMaxDcBlocks ? a.nblk : kMaxDcBlocks;
+    for (int k = 0; k < 3; ++k) st.dc_est[k] = poly[k];
     if (a.dc_given)
         for (int k = 0; k < 3; ++k) poly[k] = a.dc_in[k];
     for (int k = 0; k < 3; ++k) {
@@ -783,7 +727,9 @@ ASARF_HD inline void finalize_body(const FinalizeArgs& a) {
     double xs[kMaxDcBlocks], ys[kMaxDcBlocks];
     const int nblk = a.nblk < kMaxDcBlocks ? a.nblk : kMaxDcBlocks;
     for (int b = 0; b < nblk; ++b) finalize_block(a, m, b, xs, ys, st);
-    finalize_fit(a, st, xs, ys, m.err);
+    double poly[3] = {0.0, 0.0, 0.0};
+    polyfit_qr<kMaxDcBlocks, 3>(xs, ys, nblk, 2, poly);
+    finalize_poly(a, st, poly, m.err);
 }
 
 // ----------------------------------------------------------------------------- range compression

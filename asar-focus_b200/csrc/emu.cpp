@@ -26,7 +26,10 @@ struct TileBuf {
 int backend_raw_stats(const RawStatsArgs& a, int gx, int gy, void*) {
     RawStatsSmem sm;
     for (int by = 0; by < gy; ++by)
-        for (int bx = 0; bx < gx; ++bx) raw_stats_body(a, bx, by, 0, 1, &sm);
+        for (int bx = 0; bx < gx; ++bx) {
+            if (a.aligned) raw_stats_body<true>(a, bx, by, 0, 1, &sm);
+            else raw_stats_body<false>(a, bx, by, 0, 1, &sm);
+        }
     return ASARF_OK;
 }
 
@@ -45,6 +48,7 @@ int backend_stats_fold(const RawStatsArgs& a, int tiles_y, void*) {
 
 int backend_finalize(const FinalizeArgs& a, void*) {
     finalize_body(a);
+    if (!a.facc) *a.acc = StatAccum{};  // as the device finalisation leaves it
     return ASARF_OK;
 }
 

@@ -819,6 +819,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
         rc |= mem_h2d(lut_dev, lut.data(), sizeof(float) * lut.size(), nullptr);
     }
     rc |= mem_zero(p->state, sizeof(FocusState), nullptr);
+    rc |= mem_zero(p->acc, sizeof(StatAccum), nullptr);  // each run's finalisation leaves it zero again
     rc |= stream_sync(nullptr);
     if (rc) {
         delete p;
@@ -1133,8 +1134,10 @@ int asarf_focus(asarf_plan* p, const uint8_t* d_raw, const uint16_t* d_swst, int
         if (ev) event_record(ev[k], stream);
         ++k;
     };
-    int rc = mem_zero(p->acc, sizeof(StatAccum), stream);
+    // the accumulators are zero unless a run ended between its statistics and its finalisation
+    int rc = p->acc_dirty ? mem_zero(p->acc, sizeof(StatAccum), stream) : ASARF_OK;
     if (rc) return rc;
+    p->acc_dirty = true;
     RawStatsArgs st = p->a_stats;
     st.raw = d_raw;
     st.swst = d_swst;
@@ -1151,6 +1154,7 @@ int asarf_focus(asarf_plan* p, const uint8_t* d_raw, const uint16_t* d_swst, int
     mark();
     rc = backend_finalize(p->a_fin, stream);
     if (rc) return rc;
+    p->acc_dirty = false;
     RangeCompressArgs r = p->a_rc;
     r.raw = d_raw;
     r.swst = d_swst;

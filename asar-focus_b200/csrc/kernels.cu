@@ -20,12 +20,16 @@ namespace asarf {
 
 namespace {
 
+constexpr int kFinalizeThreads = 96;
+static_assert(kFinalizeThreads >= kMaxDcBlocks, "one Doppler block per thread");
+
 // Three blocks per SM (80 registers, no spills).  Four blocks at 64 registers spilled 176
 // bytes per thread in the batched loads and measured slower on the ERS-like scene:
 // 0.156 against 0.143 ms.
+template <bool ALIGNED>
 __global__ void __launch_bounds__(kStatsCols, kStatsBlocksPerSm) k_raw_stats(RawStatsArgs a) {
     __shared__ RawStatsSmem sm;
-    raw_stats_body(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, &sm);
+    raw_stats_body<ALIGNED>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, &sm);
 }
 
 __global__ void __launch_bounds__(32 * kFbaqStatsWarps, 3) k_raw_stats_fbaq(RawStatsArgs a) {
@@ -52,16 +56,90 @@ __global__ void __launch_bounds__(256) k_condition(ConditionArgs a) {
     condition_row(a, blockIdx.x, threadIdx.x, blockDim.x);
 }
 
-// One warp: the Doppler blocks' angles (an FP64 atan2 each) lane-parallel, the fit on lane 0.
-__global__ void k_finalize(FinalizeArgs a) {
+// Quadratic least-squares fit through nblk <= kMaxDcBlocks points by one warp: the Householder
+// steps of polyfit_qr with row r on lane r % 32, every sum of a step reduced over the lanes at once
+// (fixed order, the same on every lane).  Coefficients highest power first, on every lane.
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ bool warp_fit_quadratic(const double* xs, const double* ys, int nblk, double out[3]) {
+    constexpr int kRows = (kMaxDcBlocks + 31) / 32;
+    const int lane = threadIdx.x & 31;
+    if (nblk < 3) return false;
+    double A[4][kRows];  // columns 1, x, x^2 and the right-hand side; rows past the last are zero
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+        const int r = lane + 32 * i;
+        const bool ok = r < nblk;
+        const double x = ok ? xs[r] : 0.0;
+        A[0][i] = ok ? 1.0 : 0.0;
+        A[1][i] = x;
+        A[2][i] = x * x;
+        A[3][i] = ok ? ys[r] : 0.0;
+    }
+    double R[3][4];  // rows of the triangular system
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        // sums over rows r > k of column k times each column from k on
+        double dot[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int i = 0; i < kRows; ++i)
+            if (lane + 32 * i > k)
+#pragma unroll
+                for (int c = k; c < 4; ++c) dot[c] += A[k][i] * A[c][i];
+#pragma unroll
+        for (int c = k; c < 4; ++c) dot[c] = warp_sum(dot[c]);
+        double head[4];
+#pragma unroll
+        for (int c = k; c < 4; ++c) head[c] = __shfl_sync(0xffffffffu, A[c][0], k);
+        const double nrm = sqrt(head[k] * head[k] + dot[k]);
+        if (nrm == 0.0) return false;
+        const double alpha = head[k] > 0 ? -nrm : nrm;
+        const double vk = head[k] - alpha;
+        const double vn = vk * vk + dot[k];
+        if (vn == 0.0) return false;
+        R[k][k] = alpha;
+#pragma unroll
+        for (int c = k + 1; c < 4; ++c) {
+            const double f = 2.0 * (vk * head[c] + dot[c]) / vn;
+            R[k][c] = head[c] - f * vk;
+#pragma unroll
+            for (int i = 0; i < kRows; ++i)
+                if (lane + 32 * i > k) A[c][i] -= f * A[k][i];
+        }
+    }
+    const double c2 = R[2][3] / R[2][2];
+    const double c1 = (R[1][3] - R[1][2] * c2) / R[1][1];
+    const double c0 = (R[0][3] - R[0][1] * c1 - R[0][2] * c2) / R[0][0];
+    out[0] = c2, out[1] = c1, out[2] = c0;
+    return true;
+}
+
+// The Doppler blocks' angles (an FP64 atan2 each) one per thread, the statistics' own results on
+// the last warp beside them, the fit over warp 0 (by one thread's serial QR the kernel took 16 us
+// in every focus run, whatever the scene, and now 6; a chain of latencies, not work).  The accumulators are
+// zeroed for the plan's next run once every thread has read them.
+__global__ void __launch_bounds__(kFinalizeThreads) k_finalize(FinalizeArgs a) {
     __shared__ double xs[kMaxDcBlocks], ys[kMaxDcBlocks];
     if (blockIdx.x != 0) return;
     FocusState& st = *a.state;
-    const FinalizeMap m = finalize_stats(a, threadIdx.x == 0 ? &st : nullptr);
+    const int tid = threadIdx.x;
+    const FinalizeMap m = finalize_stats(a, tid == kFinalizeThreads - 1 ? &st : nullptr);
     const int nblk = a.nblk < kMaxDcBlocks ? a.nblk : kMaxDcBlocks;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) finalize_block(a, m, b, xs, ys, st);
+    if (tid < nblk) finalize_block(a, m, tid, xs, ys, st);
     __syncthreads();
-    if (threadIdx.x == 0) finalize_fit(a, st, xs, ys, m.err);
+    if (!a.facc) {
+        unsigned long long* acc = &a.acc->mom[0];
+        for (int i = tid; i < 6 + 9 * nblk; i += kFinalizeThreads) acc[i] = 0ull;
+    }
+    if (tid < 32) {
+        double poly[3] = {0.0, 0.0, 0.0};
+        if (!warp_fit_quadratic(xs, ys, nblk, poly)) poly[0] = poly[1] = poly[2] = 0.0;
+        if (tid == 0) finalize_poly(a, st, poly, m.err);
+    }
 }
 
 // FBAQ4 record into shared memory: its 16-byte-aligned interior with vector loads, the
@@ -409,12 +487,13 @@ cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
 }  // namespace
 
 int backend_raw_stats(const RawStatsArgs& a, int gx, int gy, void* stream) {
-    k_raw_stats<<<dim3(gx, gy), kStatsCols, 0, S(stream)>>>(a);
+    if (a.aligned) k_raw_stats<true><<<dim3(gx, gy), kStatsCols, 0, S(stream)>>>(a);
+    else k_raw_stats<false><<<dim3(gx, gy), kStatsCols, 0, S(stream)>>>(a);
     return check_launch("raw_stats");
 }
 
 int backend_finalize(const FinalizeArgs& a, void* stream) {
-    k_finalize<<<1, 32, 0, S(stream)>>>(a);
+    k_finalize<<<1, kFinalizeThreads, 0, S(stream)>>>(a);
     return check_launch("finalize");
 }
 

@@ -103,9 +103,10 @@ int scratch_address(NoallocScratch** out) {
     return ASARF_OK;
 }
 
+template <bool ALIGNED>
 __global__ void __launch_bounds__(kStatsCols) k_noalloc_raw_stats(RawStatsArgs a) {
     __shared__ RawStatsSmem sm;
-    raw_stats_body(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, &sm);
+    raw_stats_body<ALIGNED>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, &sm);
 }
 
 __global__ void k_noalloc_finalize(FinalizeArgs a, asarf_raw_stats* out) {
@@ -176,7 +177,8 @@ extern "C" int asarf_raw_statistics_noalloc(const uint8_t* d_raw, int32_t raw_li
     st.lines_per_cta = kStatsMaxLines / 4;
     st.acc = &scratch->acc;
     dim3 grid(raw_stats_grid_x(st, d_raw), (azimuth_size + st.lines_per_cta - 1) / st.lines_per_cta);
-    k_noalloc_raw_stats<<<grid, kStatsCols, 0, s>>>(st);
+    if (st.aligned) k_noalloc_raw_stats<true><<<grid, kStatsCols, 0, s>>>(st);
+    else k_noalloc_raw_stats<false><<<grid, kStatsCols, 0, s>>>(st);
 
     FinalizeArgs fin{};
     fin.acc = &scratch->acc;

@@ -64,7 +64,7 @@ enum ErrorBits : unsigned int {
 
 // Everything the statistics finalisation needs besides the accumulators.
 struct FinalizeArgs {
-    const StatAccum* acc;
+    StatAccum* acc;          // device finalisation: zeroed again once read
     FocusState* state;
     long long n_total;       // CorrectionParams::n_total_samples
     long long n_pad;         // range-padding samples entering the gain / phase sums
@@ -92,7 +92,7 @@ struct RawStatsArgs {
     int min_swst;
     int dc_step, nblk;
     int lines_per_cta;    // at most kStatsMaxLines
-    int quad;             // 4-column units (raw base and line stride 8-byte aligned)
+    int aligned;          // raw base and line stride 8-byte aligned
     int gpb;              // 4-column groups per Doppler block: ceil(dc_step / 4)
     StatAccum* acc;
     // ASAR FBAQ4 records (k_raw_stats_fbaq): FP64 partial sums of each 32-column tile

@@ -43,6 +43,7 @@ struct asarf_plan {
     float2* bufA = nullptr;
     float2* bufB = nullptr;
     StatAccum* acc = nullptr;
+    bool acc_dirty = false;       // a run's statistics were enqueued without its finalisation
     FocusState* state = nullptr;
     uint8_t* raw_dev = nullptr;
     uint16_t* swst_dev = nullptr;
