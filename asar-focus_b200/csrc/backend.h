@@ -24,6 +24,8 @@ int backend_range_compress(const RangeCompressArgs& a, int lines, LaunchShape sh
 int backend_az_strided(const AzStridedArgs& a, const void* tmap, int tiles, int nblocks, LaunchShape sh, void* stream);
 int backend_az_rd(const AzRdArgs& a, const void* tmap, int tiles, int nblocks, LaunchShape sh, unsigned int* err,
                   void* stream);
+// interpolation weights of AzRdArgs::rcmc: (kRcmcNodes + 1) rows of kRcmcRowFloats
+int backend_rcmc_table(float* table, void* stream);
 // split-precision range-Doppler block (tensor-core forward transform); device build only
 int backend_az_rd_split(const AzRdArgs& a, const AzRdSplit& sp, const void* tmap, int tiles, int nblocks,
                         LaunchShape sh, unsigned int* err, void* stream);

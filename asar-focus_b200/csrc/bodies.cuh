@@ -865,28 +865,15 @@ ASARF_HD ASARF_INLINE void az_strided_tables(const AzStridedArgs& a, int b, int 
     }
 }
 
-// Store of a column pair (u at column x, v at x + 1) of one output row: one 16-byte store when
-// both columns exist and the address allows it.
-ASARF_HD ASARF_INLINE void store_pair(float2* dst, int x, int nk, float2 u, float2 v) {
-    if (x + 1 < nk && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-        *reinterpret_cast<float4*>(dst) = make_float4(u.x, u.y, v.x, v.y);
-    } else {
-        dst[0] = u;
-        if (x + 1 < nk) dst[1] = v;
-    }
-}
-
-// R0, R1, R2, XT > 0: the transform's radix schedule and tile width as compile-time constants
-// (they must be the plan's: the planner picks this instantiation only when they are).
-template <int R0 = 0, int R1 = 0, int R2 = 0, int XT = 0>
+// XT: the tile width (16 or 32).  R0, R1, R2 > 0: the transform's radix schedule as compile-time
+// constants (it must be the plan's: the planner picks this instantiation only when it is).
+template <int R0, int R1, int R2, int XT>
 ASARF_HD ASARF_INLINE void az_strided_body(const AzStridedArgs& a, int tile, int b, int tid, int nthr, float2* s,
                                            const float2* tw, const int* rowmap, bool preloaded) {
-    constexpr bool kCt = R0 > 0;
-    const int n1 = kCt ? R0 * R1 * R2 : a.n1, xt = kCt ? XT : a.xt;
+    const int n1 = R0 > 0 ? R0 * R1 * R2 : a.n1;
+    constexpr int xt = XT;
     const int x0 = tile * xt;
-    const FastDiv dxt = make_fastdiv(static_cast<unsigned int>(xt));
-    // position t of the tile -> row (t / xt), by a constant when the schedule is compiled
-    auto row_of = [&](int t) { return kCt ? t / XT : static_cast<int>(fdiv_u(t, dxt)); };
+    auto row_of = [](int t) { return t / XT; };
     // tile [r][c] = row r*n2 + b, column x0 + c (natural order; columns >= nk read as 0)
     if (!preloaded) {
         for (int t = tid; t < n1 * xt; t += nthr) {
@@ -909,7 +896,7 @@ ASARF_HD ASARF_INLINE void az_strided_body(const AzStridedArgs& a, int tile, int
         if constexpr (R0 > 0)
             fft_forward_pairs_ct3<R0, R1, R2, XT / 2, XT, true>(s, a.plan1.tw, tid, nthr);
         else
-            fft_forward_pairs<true, true>(a.plan1, s, xt, xt, tid, nthr);
+            fft_forward_pairs_xt<XT / 2, XT>(a.plan1, s, tid, nthr);
         for (int t = tid; t < n1 * xt; t += nthr) {
             const int p = row_of(t), c = t - p * xt;
             const int x = x0 + c;
@@ -920,7 +907,7 @@ ASARF_HD ASARF_INLINE void az_strided_body(const AzStridedArgs& a, int tile, int
         if constexpr (R0 > 0)
             fft_inverse_dif_pairs_ct3<R0, R1, R2, XT / 2, XT, true>(s, a.plan1.tw, tid, nthr, tw);
         else
-            fft_inverse_dif_pairs<true, true>(a.plan1, s, xt, xt, tid, nthr, tw);
+            fft_inverse_dif_pairs_xt<XT / 2, XT>(a.plan1, s, tid, nthr, tw);
         const int lo = a.state ? a.state->first_line : 0;
         const int hi = a.state ? lo + a.state->n_lines : n1 * a.n2;
         for (int t = tid; t < n1 * xt; t += nthr) {
@@ -1069,34 +1056,324 @@ ASARF_HD ASARF_INLINE float2 az_abs_phase(const AzRdArgs& a, const ColParams& cp
     return make_float2(static_cast<float>(cos(ph)), static_cast<float>(sin(ph)));
 }
 
-// Shared-memory tables after the tile: column constants (xt), absolute-phase factors (xt),
-// row bin frequencies (n2).
-ASARF_HD ASARF_INLINE float2* az_rd_phase_table(ColParams* cps, const AzRdArgs& a) {
-    return reinterpret_cast<float2*>(cps + a.xt);
-}
-ASARF_HD ASARF_INLINE float* az_rd_freq_table(ColParams* cps, const AzRdArgs& a) {
-    return reinterpret_cast<float*>(az_rd_phase_table(cps, a) + a.xt);
-}
+// ---- rows that one range walk and one band decision serve
+// A row of the tile is one Doppler bin.  Over its xt <= 64 columns the aliased frequency, the band
+// test and the integer walk nearly always agree, and the fraction dl of the walk moves by a
+// few 1e-4 (lambda^2 f^2 / 8 Vr^2 samples a column).  For such a row the 14 interpolation weights
+// and their derivatives come from a table over the fraction (kRcmcNodes steps, FP64 values
+// rounded once): w + (dl - node) w' is one multiply-add where forming a weight took a
+// multiply-add, a reciprocal and its share of the normaliser, and a lane takes two adjacent
+// columns, whose taps are 15 samples read as eight 16-byte loads instead of 28 8-byte ones.  The
+// first neglected term is (dl - node)^2 w'' / 2 < 4.2e-7 at the limit kRcmcMaxStep (w'' <= 3.4,
+// the sinc's centre), about 1e-8 over a scene, below the 1e-6 the reference's fraction is rounded
+// to.  Every branch-deciding quantity keeps the reference's float32 value: a row is taken as
+// uniform only when the extremes over its columns prove that each of them decides alike, and any
+// other row goes sample by sample (rcmc_mf_sample).  The block is bound by instruction issue and
+// shared-memory wavefronts: on the ERS 5616 x 8990 cut 360 -> 296 million warp instructions, 28000
+// lines 1462 -> 1320 us, ASAR IM 30000 lines 1606 -> 1450 us.  (With one column per lane and the
+// table's weights summed as sum w d + (dl - node) sum w' d, 345 million instructions and 15 % more
+// wavefronts, it took 1537 us; weights read straight from the table 1549 us.)
+constexpr int kRcmcNodes = 4096;
+constexpr int kRcmcRowFloats = 32;                   // per node: (w, w') of taps 1 .. 14, padded to 128 bytes
+constexpr int kRcmcBufFloats = 2 * (kRcmcTaps - 2);  // a warp's copy of one node
+constexpr float kRcmcMaxStep = 5e-4f;
+constexpr int kRowSlow = -1, kRowSkip = -2;          // other codes: rcmc_row_code
 
-// Per-block tables of the range-Doppler block, built while the tile is in flight: column
-// constants of the xt output columns (and their absolute-phase factors when asked for) and
-// the Doppler bin frequency of each of the n2 rows (bin k1 + n1 drev2(p)).
-ASARF_HD ASARF_INLINE void az_rd_tables(const AzRdArgs& a, int tile, int k1, int tid, int nthr, ColParams* cps,
-                                        float* fbf) {
-    const int x0 = tile * a.xt;
-    float2* phs = az_rd_phase_table(cps, a);
-    for (int c = tid; c < a.xt; c += nthr) {
-        cps[c] = az_col_params(a, x0 + c);
-        if (a.absolute_phase) phs[c] = az_abs_phase(a, cps[c], x0 + c);
+// Weights of tap i = 1 .. 14 at fraction dl = n / kRcmcNodes - 1/2 and their derivatives, as the
+// quotients v_i / sum v of v_i = dl (-1)^i W_i / (dl + 8 - i) (v_8 = W_8: finite at dl = 0).
+ASARF_HD inline void rcmc_weight_row(int n, float* row) {
+    constexpr float kWin[kRcmcTaps] = ASARF_BLACKMAN16;
+    const double dl = static_cast<double>(n) / kRcmcNodes - 0.5;
+    double v[kRcmcTaps], dv[kRcmcTaps], sum = 0.0, dsum = 0.0;
+    for (int i = 1; i < kRcmcTaps - 1; ++i) {
+        const double w = (i & 1) ? -static_cast<double>(kWin[i]) : static_cast<double>(kWin[i]);
+        const double m = kRcmcTaps / 2 - i;
+        v[i] = m == 0.0 ? w : dl * w / (dl + m);
+        dv[i] = m == 0.0 ? 0.0 : w * m / ((dl + m) * (dl + m));
+        sum += v[i];
+        dsum += dv[i];
     }
-    for (int p = tid; p < a.n2; p += nthr)
-        fbf[p] = bin_frequency(k1 + a.n1 * ASARF_LDG(a.drev2 + p), a.az_pad, a.bin_step);
+    for (int k = 0; k < kRcmcRowFloats; ++k) row[k] = 0.0f;
+    for (int i = 1; i < kRcmcTaps - 1; ++i) {
+        const double w = v[i] / sum;
+        row[2 * (i - 1)] = static_cast<float>(w);
+        row[2 * (i - 1) + 1] = static_cast<float>((dv[i] - w * dsum) / sum);
+    }
 }
 
-// Shared-memory bytes of the range-Doppler block: tile, column constants, phase factors, row frequencies.
-inline size_t az_rd_smem(int n2, int wt, int xt) {
-    return sizeof(float2) * static_cast<size_t>(n2) * wt + sizeof(ColParams) * static_cast<size_t>(xt) +
-           sizeof(float2) * static_cast<size_t>(xt) + sizeof(float) * static_cast<size_t>(n2) + 16;
+// What a uniform row's samples need of their column.
+struct ColUse {
+    float den, rden;      // 8 Vr^2 and its rounded reciprocal
+    float r0_hi, r0_lo;   // R0 / range spacing as a float pair
+    float dc_off, ka, rka, sh;  // sh = 2 pi (dc_off / Ka), rounded as the reference rounds it
+    ASARF_HD ASARF_INLINE void set(const ColParams& c) {
+        den = c.den, rden = c.rden;
+        r0_hi = static_cast<float>(c.r0_dr);
+        r0_lo = static_cast<float>(c.r0_dr - static_cast<double>(r0_hi));
+        dc_off = c.dc_off, ka = c.ka, rka = c.rka;
+        sh = fmul_rn(fmul_rn(2.0f, 3.14159265358979323846f), c.dc_off_ka);
+    }
+};
+
+// Extremes over a tile's columns of what the row decisions depend on.
+struct RowSpan {
+    float dc_min, dc_max, lo_min, lo_max, hi_min, hi_max, off_min, off_max;
+    float g_min, g_max;  // walk per lambda^2 f^2, widened by the roundings of both sides
+    ASARF_HD ASARF_INLINE void set(const ColParams& c) {
+        dc_min = dc_max = c.dc;
+        lo_min = lo_max = c.cut_lo;
+        hi_min = hi_max = c.cut_hi;
+        off_min = off_max = c.dc_off;
+        const float g = fmul_rn(static_cast<float>(c.r0_dr), c.rden);
+        // quotient, products and casts on either side together round by less than 1e-6
+        g_min = fmul_rn(g, 1.0f - 2e-6f);
+        g_max = fmul_rn(g, 1.0f + 2e-6f);
+    }
+    ASARF_HD ASARF_INLINE void join(const RowSpan& o) {
+        dc_min = o.dc_min < dc_min ? o.dc_min : dc_min;
+        dc_max = o.dc_max > dc_max ? o.dc_max : dc_max;
+        lo_min = o.lo_min < lo_min ? o.lo_min : lo_min;
+        lo_max = o.lo_max > lo_max ? o.lo_max : lo_max;
+        hi_min = o.hi_min < hi_min ? o.hi_min : hi_min;
+        hi_max = o.hi_max > hi_max ? o.hi_max : hi_max;
+        off_min = o.off_min < off_min ? o.off_min : off_min;
+        off_max = o.off_max > off_max ? o.off_max : off_max;
+        g_min = o.g_min < g_min ? o.g_min : g_min;
+        g_max = o.g_max > g_max ? o.g_max : g_max;
+    }
+#if defined(__CUDA_ARCH__)
+    static __device__ __forceinline__ float warp_min(float v) {
+        float r;
+        asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+        return r;
+    }
+    static __device__ __forceinline__ float warp_max(float v) {
+        float r;
+        asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+        return r;
+    }
+    __device__ __forceinline__ void join_warp() {
+        dc_min = warp_min(dc_min), dc_max = warp_max(dc_max);
+        lo_min = warp_min(lo_min), lo_max = warp_max(lo_max);
+        hi_min = warp_min(hi_min), hi_max = warp_max(hi_max);
+        off_min = warp_min(off_min), off_max = warp_max(off_max);
+        g_min = warp_min(g_min), g_max = warp_max(g_max);
+    }
+#endif
+};
+
+// lambda^2 fn^2 as rcmc_mf_sample rounds it.
+ASARF_HD ASARF_INLINE float rcmc_numerator(const AzRdArgs& a, float fn) {
+    return fmul_rn(fmul_rn(fmul_rn(a.lambda, a.lambda), fn), fn);
+}
+
+struct RowRec {
+    float bf;   // Doppler bin frequency
+    float num;  // uniform rows: lambda^2 fn^2
+    int code;   // kRowSlow, kRowSkip or the packed decisions
+};
+
+// Record of the row at bin frequency bf.  Code of a uniform row: table node (from bit 12), wrap + 1
+// (bits 8-9: the filter's frequency is bf - dc_off - wrap PRF), walk (bits 0-7).  All tests are
+// written so that a NaN takes the slow path.
+ASARF_HD ASARF_INLINE RowRec rcmc_row(const AzRdArgs& a, const RowSpan& sp, float bf) {
+    RowRec r{bf, 0.0f, kRowSlow};
+    const float half = a.half_prf;
+    float fn;
+    if (!(sp.dc_min < 0.0f && bf > fadd_rn(half, sp.dc_min)) && !(sp.dc_max > 0.0f && bf < fadd_rn(-half, sp.dc_max)))
+        fn = bf;
+    else if (sp.dc_max < 0.0f && bf > fadd_rn(half, sp.dc_max)) fn = fsub_rn(bf, a.prf);
+    else if (sp.dc_min > 0.0f && bf < fadd_rn(-half, sp.dc_min)) fn = fadd_rn(bf, a.prf);
+    else return r;
+    if (fn < sp.lo_min || fn > sp.hi_max) {
+        r.code = kRowSkip;
+        return r;
+    }
+    if (!(fn >= sp.lo_max && fn <= sp.hi_min)) return r;
+    const float fc_max = fsub_rn(bf, sp.off_min), fc_min = fsub_rn(bf, sp.off_max);
+    int wrap;
+    if (fc_max <= half && fc_min >= -half) wrap = 0;
+    else if (fc_min > half) wrap = 1;
+    else if (fc_max < -half) wrap = -1;
+    else return r;
+    // the walk of every column lies in [lo, hi]
+    r.num = rcmc_numerator(a, fn);
+    const float lo = fmul_rn(r.num, sp.g_min), hi = fmul_rn(r.num, sp.g_max);
+    const float mid = fmul_rn(fadd_rn(lo, hi), 0.5f), walk = floorf(fadd_rn(mid, 0.5f));
+    if (!(walk >= 0.0f && walk < 256.0f && lo - walk >= -0.5f && hi - walk < 0.5f)) return r;
+    int node = static_cast<int>(floorf((mid - walk + 0.5f) * kRcmcNodes + 0.5f));
+    node = node < 0 ? 0 : (node > kRcmcNodes ? kRcmcNodes : node);
+    const float d0 = fma_rn(static_cast<float>(node), 1.0f / kRcmcNodes, -0.5f);
+    if (!(hi - walk - d0 <= kRcmcMaxStep && lo - walk - d0 >= -kRcmcMaxStep)) return r;
+    const int w = static_cast<int>(walk);
+    // every sample the two columns of a lane read, whole 16-byte units, inside the loaded row
+    const int first = a.hl + w - kRcmcTaps / 2;
+    if (first < 0 || first + a.xt + kRcmcTaps - 2 > a.wt) return r;
+    r.code = node << 12 | (wrap + 1) << 8 | w;
+    return r;
+}
+
+// Columns of the tile that the taps of its in-band samples reach: up to 6 right of the largest
+// integer walk in the band.  The loaded halo holds the walk at |f| = PRF and a margin; the forward
+// transform leaves out what no row of this tile reads (ERS: 80 of 82 columns, so that a radix-5 stage's
+// 1000 butterfly pairs take 512 threads two rounds, not 1025 three).
+ASARF_HD ASARF_INLINE int az_rd_used_columns(const AzRdArgs& a, const RowSpan& sp) {
+    const float f = sp.hi_max > -sp.lo_min ? sp.hi_max : -sp.lo_min;  // largest |frequency| in a band
+    const float walk = fmul_rn(rcmc_numerator(a, f), sp.g_max);
+    const float n = static_cast<float>(a.hl + a.xt + kRcmcTaps / 2 - 2) + floorf(walk + 0.5f);
+    if (!(n < static_cast<float>(a.wt))) return a.wt;
+    return (static_cast<int>(n) + 1) & ~1;
+}
+
+// Shared-memory tables after the tile: the columns' constants (xt) and their extremes (two warps'),
+// and in the same memory, once every lane holds its columns' constants, the 16 warps' weight buffers;
+// absolute-phase factors (xt, only when asked for); the rows' records (n2).
+ASARF_HD ASARF_INLINE int az_rd_cols_bytes(int xt) {
+    const int cols = static_cast<int>(sizeof(ColUse)) * xt + 2 * static_cast<int>(sizeof(RowSpan)) + 16;
+    const int bufs = 16 * kRcmcBufFloats * static_cast<int>(sizeof(float));
+    return cols > bufs ? cols : bufs;
+}
+struct AzRdTables {
+    ColUse* cols;
+    RowSpan* span;
+    int* used;  // az_rd_used_columns
+    float* weights;
+    float2* phs;
+    RowRec* rows;
+    ASARF_HD ASARF_INLINE AzRdTables(const AzRdArgs& a, float2* tile) {
+        // the tile is a multiple of 16 bytes (even tile width), and so are the parts before rows
+        cols = reinterpret_cast<ColUse*>(tile + static_cast<size_t>(a.n2) * a.wt);
+        span = reinterpret_cast<RowSpan*>(cols + a.xt);
+        used = reinterpret_cast<int*>(span + 2);
+        weights = reinterpret_cast<float*>(cols);
+        phs = reinterpret_cast<float2*>(reinterpret_cast<unsigned char*>(cols) + az_rd_cols_bytes(a.xt));
+        rows = reinterpret_cast<RowRec*>(phs + (a.absolute_phase ? a.xt : 0));
+    }
+};
+
+// Per-block tables of the range-Doppler block, built while the tile is in flight: constants of
+// the xt output columns (and their absolute-phase factors when asked for), and for each of the n2
+// rows its Doppler bin frequency (bin k1 + n1 drev2(p)) and decisions.
+ASARF_HD ASARF_INLINE void az_rd_tables(const AzRdArgs& a, int tile, int k1, int tid, int nthr, const AzRdTables& t) {
+    const int x0 = tile * a.xt;
+#if defined(__CUDA_ARCH__)
+    if (tid < 64) {
+        const int c = tid < a.xt ? tid : a.xt - 1;
+        const ColParams cp = az_col_params(a, x0 + c);
+        if (tid < a.xt) {
+            t.cols[c].set(cp);
+            if (a.absolute_phase) t.phs[c] = az_abs_phase(a, cp, x0 + c);
+        }
+        RowSpan sp;
+        sp.set(cp);
+        sp.join_warp();
+        if ((tid & 31) == 0) t.span[tid >> 5] = sp;
+    }
+#else
+    for (int c = 0; c < a.xt; ++c) {
+        const ColParams cp = az_col_params(a, x0 + c);
+        t.cols[c].set(cp);
+        if (a.absolute_phase) t.phs[c] = az_abs_phase(a, cp, x0 + c);
+        RowSpan o;
+        o.set(cp);
+        if (c == 0) t.span[0] = t.span[1] = o;
+        t.span[0].join(o);
+    }
+#endif
+    ASARF_SYNC();
+    RowSpan sp = t.span[0];
+    sp.join(t.span[1]);
+    if (tid == 0) *t.used = az_rd_used_columns(a, sp);
+    for (int p = tid; p < a.n2; p += nthr)
+        t.rows[p] = rcmc_row(a, sp, bin_frequency(k1 + a.n1 * ASARF_LDG(a.drev2 + p), a.az_pad, a.bin_step));
+}
+
+// Shared-memory bytes of the range-Doppler block.
+inline size_t az_rd_smem(int n2, int wt, int xt, bool absolute_phase) {
+    return sizeof(float2) * static_cast<size_t>(n2) * wt + static_cast<size_t>(az_rd_cols_bytes(xt)) +
+           sizeof(RowRec) * static_cast<size_t>(n2) +
+           (absolute_phase ? sizeof(float2) * static_cast<size_t>(xt) : 0);
+}
+
+// Table row of a uniform row's weights.
+ASARF_HD ASARF_INLINE const float* rcmc_weights(const AzRdArgs& a, int code) {
+    return a.rcmc + static_cast<size_t>(code >> 12) * kRcmcRowFloats;
+}
+
+// Interpolated samples of two adjacent columns of a uniform row: q holds the 16-byte units from the
+// even tile column at or below tap 1 of the first one (ODD: tap 1 is the unit's second sample), w
+// its weights as (w, w', w, w') of taps (1, 2), (3, 4), ..., step the columns' dl - node.
+template <bool ODD>
+ASARF_HD ASARF_INLINE void rcmc_pair_taps(const float4* q, const float4* w, float2 step, float2* va, float2* vb) {
+    float2 acc_a = make_float2(0.0f, 0.0f), acc_b = acc_a;
+    float4 d = q[0];
+    float2 lo = ODD ? make_float2(d.z, d.w) : make_float2(d.x, d.y);  // first column's next sample
+#pragma unroll
+    for (int i = 0; i < kRcmcTaps - 2; i += 2) {
+        const float4 wv = w[i / 2];
+        float2 mid, hi;
+        if (ODD) {
+            d = q[i / 2 + 1];
+            mid = make_float2(d.x, d.y), hi = make_float2(d.z, d.w);
+        } else {
+            mid = make_float2(d.z, d.w);
+            d = q[i / 2 + 1];
+            hi = make_float2(d.x, d.y);
+        }
+        const float2 w0 = pfma2(step, make_float2(wv.y, wv.y), make_float2(wv.x, wv.x));
+        const float2 w1 = pfma2(step, make_float2(wv.w, wv.w), make_float2(wv.z, wv.z));
+        acc_a = pfma(lo, w0.x, acc_a);
+        acc_b = pfma(mid, w0.y, acc_b);
+        acc_a = pfma(mid, w1.x, acc_a);
+        acc_b = pfma(hi, w1.y, acc_b);
+        lo = hi;
+    }
+    *va = acc_a;
+    *vb = acc_b;
+}
+
+// Fraction of the range walk past the row's integer walk, with the reference's roundings
+// (rcmc_mf_sample): quotient num / den, times R0 / range spacing as a float pair (the product's
+// rounding differs from the FP64 one's only within 2^-45 of a tie), minus the walk, plus 8.
+ASARF_HD ASARF_INLINE float rcmc_offset(const ColUse& c, float num, float walk) {
+    const float q = div_by_recip_rn(num, c.den, c.rden);
+    const float p = fmul_rn(q, c.r0_hi);
+    const float shift = fadd_rn(p, fma_rn(q, c.r0_lo, fma_rn(q, c.r0_hi, -p)));
+    return fadd_rn(fsub_rn(shift, walk), static_cast<float>(kRcmcTaps / 2));
+}
+
+// Two adjacent columns x, x + 1 of a uniform row, interpolated and filtered: srow the tile row, c the
+// first one's column of the output tile (even).  edge: a column whose taps leave [0, nk) is zero.
+ASARF_HD ASARF_INLINE void rcmc_mf_pair(const AzRdArgs& a, const RowRec& r, const float* weights, bool edge,
+                                        const ColUse& ca, const ColUse& cb, int x, const float2* srow, int c,
+                                        float2* va, float2* vb) {
+    const int wk = r.code & 255;
+    const float walk = static_cast<float>(wk);
+    const float wrap = static_cast<float>(((r.code >> 8) & 3) - 1) * a.prf;
+    const float node = fma_rn(static_cast<float>(r.code >> 12), 1.0f / kRcmcNodes, kRcmcTaps / 2 - 0.5f);  // exact
+    const float2 step = make_float2(fsub_rn(rcmc_offset(ca, r.num, walk), node),
+                                    fsub_rn(rcmc_offset(cb, r.num, walk), node));
+    const int tap1 = a.hl + wk - kRcmcTaps / 2 + 1 + c;
+    const float4* q = reinterpret_cast<const float4*>(srow + (tap1 & ~1));
+    const float4* w = reinterpret_cast<const float4*>(weights);
+    float2 v[2];
+    if (tap1 & 1) rcmc_pair_taps<true>(q, w, step, &v[0], &v[1]);
+    else rcmc_pair_taps<false>(q, w, step, &v[0], &v[1]);
+    if (edge) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int cx = x + h + wk;
+            if (cx - kRcmcTaps / 2 < 0 || cx + kRcmcTaps / 2 >= a.nk) v[h] = make_float2(0.0f, 0.0f);
+        }
+    }
+    float2* out[2] = {va, vb};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const ColUse& k = h ? cb : ca;
+        const float fc = fsub_rn(fsub_rn(r.bf, k.dc_off), wrap);
+        const float mf_phase = div_by_recip_rn(fmul_rn(fmul_rn(3.14159265358979323846f, fc), fc), k.ka, k.rka);
+        *out[h] = cmul(v[h], expj_neg_sum(mf_phase, fmul_rn(k.sh, r.bf)));
+    }
 }
 
 // Right range halo of the range-Doppler block: the taps used (1 .. 14 of 16) reach 6 columns
@@ -1108,22 +1385,31 @@ inline int rcmc_right_halo(double max_walk) { return kRcmcTaps / 2 - 1 + static_
 // room for two resident blocks per SM (2 x 512 threads at 64 registers fill the register file;
 // 228 KB of shared memory per SM, 1 KB reserved per block).  With one block per SM the
 // block-wide barriers of the FFT stages leave the SM idle (measured 2.63 -> 1.92 ms at n2 = 168).
-constexpr size_t kAzRdTwoBlockSmem = 228 * 1024 / 2 - 1024 - 256;
-inline int az_rd_tile_width(int n2, int hl, int hr) {
+constexpr size_t kAzRdTwoBlockSmem = 228 * 1024 / 2 - 1024 - 128;
+inline int az_rd_tile_width(int n2, int hl, int hr, bool absolute_phase) {
     int xt = 64;
-    while (xt > 16 && az_rd_smem(n2, xt + hl + hr, xt) > kAzRdTwoBlockSmem) xt -= 2;
+    while (xt > 16 && az_rd_smem(n2, xt + hl + hr, xt, absolute_phase) > kAzRdTwoBlockSmem) xt -= 2;
     return xt;
 }
 
 // Epilogue of the range-Doppler block: row r of the inverse transform, column pair cp.
 struct AzRdOut {
     static constexpr bool kActive = true;
-    const AzRdArgs* a;
-    int x0, k1;
+    float2* out;   // output row 0, column x0
+    long long pitch;
+    int cols;      // columns of the tile inside the line
+    bool aligned;  // every row's pairs lie on 16-byte boundaries
+    ASARF_HD ASARF_INLINE AzRdOut(const AzRdArgs& a, int x0, int k1)
+        : out(a.out + static_cast<long long>(k1) * a.n2 * a.pitch + x0), pitch(a.pitch), cols(a.nk - x0),
+          aligned((a.pitch & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {}
     ASARF_HD ASARF_INLINE void operator()(int r, int cp, float2 u, float2 v) const {
-        const int x = x0 + 2 * cp;
-        if (x >= a->nk) return;
-        store_pair(a->out + static_cast<long long>(k1 * a->n2 + r) * a->pitch + x, x, a->nk, u, v);
+        float2* dst = out + r * pitch + 2 * cp;
+        if (aligned && 2 * cp + 1 < cols) {
+            *reinterpret_cast<float4*>(dst) = make_float4(u.x, u.y, v.x, v.y);
+        } else {
+            if (2 * cp < cols) dst[0] = u;
+            if (2 * cp + 1 < cols) dst[1] = v;
+        }
     }
 };
 
@@ -1142,9 +1428,10 @@ ASARF_HD ASARF_INLINE bool az_rd_packed_twiddles(const FftPlan& p) {
 // transforms' radix schedule as compile-time constants (it must be the plan's).
 template <bool FWD = true, int R0 = 0, int R1 = 0, int R2 = 0>
 ASARF_HD ASARF_INLINE void az_rd_body(const AzRdArgs& a, int tile, int k1, int tid, int nthr, float2* s,
-                                      const ColParams* cps, const float* fbf, unsigned int* err_flag, bool preloaded) {
+                                      const AzRdTables& t, unsigned int* err_flag, bool preloaded) {
     const int x0 = tile * a.xt;
     const int n2 = a.n2, wt = a.wt;
+    const int ncol = *t.used;
     const FastDiv dwt = make_fastdiv(static_cast<unsigned int>(wt));
     if (!preloaded) {
         for (int t = tid; t < n2 * wt; t += nthr) {
@@ -1156,38 +1443,55 @@ ASARF_HD ASARF_INLINE void az_rd_body(const AzRdArgs& a, int tile, int k1, int t
         }
     }
     if constexpr (FWD) {
-        ASARF_SYNC();
+        if (!preloaded) ASARF_SYNC();
         if constexpr (R0 > 0)
-            fft_forward_pairs_cs3<R0, R1, R2, (R0 <= 5 && R1 <= 5 && R2 <= 5)>(s, wt, wt, a.plan2.tw, tid, nthr);
+            fft_forward_pairs_cs3<R0, R1, R2, (R0 <= 5 && R1 <= 5 && R2 <= 5)>(s, ncol, wt, a.plan2.tw, tid, nthr);
         else if (az_rd_packed_twiddles(a.plan2))
-            fft_forward_pairs<false, true>(a.plan2, s, wt, wt, tid, nthr);
+            fft_forward_pairs<true>(a.plan2, s, ncol, wt, tid, nthr);
         else
-            fft_forward_pairs<false, false>(a.plan2, s, wt, wt, tid, nthr);
+            fft_forward_pairs<false>(a.plan2, s, ncol, wt, tid, nthr);
     }
     // RCMC + matched filter.  Every output (row p, column c) reads taps of row p only, so a
-    // row is computed into registers by one warp (lane = column, xt <= 64), the warp
+    // row is computed into registers by one warp (lane = two adjacent columns, xt <= 64), the warp
     // synchronises, and writes it back in place: no block-wide barrier per row.
+    const bool edge = x0 < kRcmcTaps || x0 + a.wt + kRcmcTaps > a.nk;  // tiles where some taps may leave the line
 #if defined(__CUDA_ARCH__)
     {
         const int lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
-        // a lane's two column records stay in registers for all rows (read from shared memory
-        // per sample, the 48-byte records cost 4-way bank conflicts on every field)
-        const ColParams cp0 = cps[lane < a.xt ? lane : 0], cp1 = cps[lane + 32 < a.xt ? lane + 32 : 0];
+        // lanes past the tile repeat its last columns and store nothing
+        const int c = 2 * lane < a.xt ? 2 * lane : a.xt - 2;
+        const int x = x0 + c;
+        // a lane's two column records stay in registers for all rows
+        const ColUse ca = t.cols[c], cb = t.cols[c + 1];
+        ASARF_SYNC();  // the records' memory becomes the warps' weight buffers
+        // a row's weights reach the lanes while the row before it is processed, then the
+        // warp's buffer (read straight from the table, their latency was exposed)
+        float* wbuf = t.weights + warp * kRcmcBufFloats;
+        auto fetch = [&](int p) -> float {
+            const int code = p < n2 ? t.rows[p].code : kRowSkip;
+            return code >= 0 && lane < kRcmcBufFloats ? ASARF_LDG(rcmc_weights(a, code) + lane) : 0.0f;
+        };
+        float wnext = fetch(warp);
         for (int p = warp; p < n2; p += nwarps) {
-            const float f = fbf[p];
-            const float2* srow = s + p * wt;
-            float2 v0 = make_float2(0.0f, 0.0f), v1 = make_float2(0.0f, 0.0f);
-            const int c0 = lane, c1 = lane + 32;
-            if (c0 < a.xt && x0 + c0 < a.nk) v0 = rcmc_mf_sample(a, cp0, x0 + c0, f, srow, a.hl + c0, err_flag);
-            if (c1 < a.xt && x0 + c1 < a.nk) v1 = rcmc_mf_sample(a, cp1, x0 + c1, f, srow, a.hl + c1, err_flag);
+            const RowRec rec = t.rows[p];
+            float2* srow = s + p * wt;
+            float2 va = make_float2(0.0f, 0.0f), vb = va;
+            if (lane < kRcmcBufFloats) wbuf[lane] = wnext;
+            __syncwarp();
+            wnext = fetch(p + nwarps);
+            if (rec.code >= 0) {
+                rcmc_mf_pair(a, rec, wbuf, edge, ca, cb, x, srow, c, &va, &vb);
+            } else if (rec.code == kRowSlow) {
+                if (x < a.nk) va = rcmc_mf_sample(a, az_col_params(a, x), x, rec.bf, srow, a.hl + c, err_flag);
+                if (x + 1 < a.nk)
+                    vb = rcmc_mf_sample(a, az_col_params(a, x + 1), x + 1, rec.bf, srow, a.hl + c + 1, err_flag);
+            }
             if (a.absolute_phase) {
-                const float2* phs = az_rd_phase_table(const_cast<ColParams*>(cps), a);
-                if (c0 < a.xt) v0 = cmul(v0, phs[c0]);
-                if (c1 < a.xt) v1 = cmul(v1, phs[c1]);
+                va = cmul(va, t.phs[c]);
+                vb = cmul(vb, t.phs[c + 1]);
             }
             __syncwarp();
-            if (c0 < a.xt) s[p * wt + a.hl + c0] = v0;
-            if (c1 < a.xt) s[p * wt + a.hl + c1] = v1;
+            if (2 * lane < a.xt) *reinterpret_cast<float4*>(srow + a.hl + c) = make_float4(va.x, va.y, vb.x, vb.y);
             __syncwarp();
         }
     }
@@ -1196,24 +1500,32 @@ ASARF_HD ASARF_INLINE void az_rd_body(const AzRdArgs& a, int tile, int k1, int t
     {
         float2 rowbuf[64];
         for (int p = 0; p < n2; ++p) {
-            const float f = fbf[p];
+            const RowRec rec = t.rows[p];
+            float2* srow = s + p * wt;
             for (int c = 0; c < a.xt; ++c) {
-                rowbuf[c] = (x0 + c < a.nk) ? rcmc_mf_sample(a, cps[c], x0 + c, f, s + p * wt, a.hl + c, err_flag)
-                                            : make_float2(0.0f, 0.0f);
-                if (a.absolute_phase) rowbuf[c] = cmul(rowbuf[c], az_rd_phase_table(const_cast<ColParams*>(cps), a)[c]);
+                if (rec.code >= 0) {
+                    if (!(c & 1))  // with the column after it
+                        rcmc_mf_pair(a, rec, rcmc_weights(a, rec.code), edge, t.cols[c], t.cols[c + 1], x0 + c, srow,
+                                     c, &rowbuf[c], &rowbuf[c + 1]);
+                } else if (rec.code == kRowSlow && x0 + c < a.nk) {
+                    rowbuf[c] = rcmc_mf_sample(a, az_col_params(a, x0 + c), x0 + c, rec.bf, srow, a.hl + c, err_flag);
+                } else {
+                    rowbuf[c] = make_float2(0.0f, 0.0f);
+                }
             }
-            for (int c = 0; c < a.xt; ++c) s[p * wt + a.hl + c] = rowbuf[c];
+            for (int c = 0; c < a.xt; ++c)
+                srow[a.hl + c] = a.absolute_phase ? cmul(rowbuf[c], t.phs[c]) : rowbuf[c];
         }
     }
 #endif
     // the inverse transform's last stage stores the block's rows k1 * n2 + r directly
     if constexpr (R0 > 0)
-        fft_inverse_pairs_cs3<R0, R1, R2, AzRdOut, (R0 <= 5 && R1 <= 5 && R2 <= 5)>(s + a.hl, a.xt, wt, a.plan2.tw,
-                                                                                   tid, nthr, AzRdOut{&a, x0, k1});
+        fft_inverse_pairs_cs3<R0, R1, R2, AzRdOut, (R0 <= 5 && R1 <= 5 && R2 <= 5)>(s + a.hl, a.xt, wt, a.plan2.tw, tid,
+                                                                                   nthr, AzRdOut(a, x0, k1));
     else if (az_rd_packed_twiddles(a.plan2))
-        fft_inverse_pairs<AzRdOut, true>(a.plan2, s + a.hl, a.xt, wt, tid, nthr, AzRdOut{&a, x0, k1});
+        fft_inverse_pairs<AzRdOut, true>(a.plan2, s + a.hl, a.xt, wt, tid, nthr, AzRdOut(a, x0, k1));
     else
-        fft_inverse_pairs<AzRdOut, false>(a.plan2, s + a.hl, a.xt, wt, tid, nthr, AzRdOut{&a, x0, k1});
+        fft_inverse_pairs<AzRdOut, false>(a.plan2, s + a.hl, a.xt, wt, tid, nthr, AzRdOut(a, x0, k1));
 }
 
 // ----------------------------------------------------------------------------- level-0 packets

@@ -99,7 +99,8 @@ int backend_az_strided(const AzStridedArgs& a, const void*, int tiles, int nbloc
         if (plan_is(a.plan1, 9, 5, 5)) emu_az_strided<9, 5, 5, 32>(a, tiles, nblocks, sh);
         else emu_az_strided<9, 4, 5, 32>(a, tiles, nblocks, sh);
     } else {
-        emu_az_strided<0, 0, 0, 0>(a, tiles, nblocks, sh);
+        if (a.xt == 32) emu_az_strided<0, 0, 0, 32>(a, tiles, nblocks, sh);
+        else emu_az_strided<0, 0, 0, 16>(a, tiles, nblocks, sh);
     }
     return ASARF_OK;
 }
@@ -108,13 +109,17 @@ template <int R0, int R1, int R2>
 static void emu_az_rd(const AzRdArgs& a, int tiles, int nblocks, LaunchShape sh, unsigned int* err) {
     TileBuf buf(sh.smem + 128);
     float2* s = buf.data();
-    ColParams* cps = reinterpret_cast<ColParams*>(s + static_cast<size_t>(a.n2) * a.wt);
-    float* fbf = az_rd_freq_table(cps, a);
+    const AzRdTables tab(a, s);
     for (int b = 0; b < nblocks; ++b)
         for (int t = 0; t < tiles; ++t) {
-            az_rd_tables(a, t, b, 0, 1, cps, fbf);
-            az_rd_body<true, R0, R1, R2>(a, t, b, 0, 1, s, cps, fbf, err, false);
+            az_rd_tables(a, t, b, 0, 1, tab);
+            az_rd_body<true, R0, R1, R2>(a, t, b, 0, 1, s, tab, err, false);
         }
+}
+
+int backend_rcmc_table(float* table, void*) {
+    for (int n = 0; n <= kRcmcNodes; ++n) rcmc_weight_row(n, table + static_cast<size_t>(n) * kRcmcRowFloats);
+    return ASARF_OK;
 }
 
 // The same instantiation choice as the device backend (block_schedule_compiled).

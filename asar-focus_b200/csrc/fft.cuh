@@ -92,6 +92,15 @@ ASARF_HD ASARF_INLINE float2 pfma(float2 a, float c, float2 b) {
 #endif
 }
 
+// a * c + b, lane by lane
+ASARF_HD ASARF_INLINE float2 pfma2(float2 a, float2 c, float2 b) {
+#if defined(__CUDA_ARCH__)
+    return __ffma2_rn(a, c, b);
+#else
+    return make_float2(__builtin_fmaf(a.x, c.x, b.x), __builtin_fmaf(a.y, c.y, b.y));
+#endif
+}
+
 // r + mul_mi(p) and r - mul_mi(p): the swap of p's parts folded into two scalar adds
 template <bool INV>
 ASARF_HD ASARF_INLINE float2 add_mi(float2 r, float2 p) {
@@ -481,19 +490,19 @@ ASARF_HD ASARF_INLINE void pair_item(float2* s, int b, int j, int cp, int M, int
     }
 }
 
-template <int R, bool INV, bool TW_FIRST, bool PRE = false, class Epi = NoEpi, bool PTW = false>
-ASARF_HD ASARF_INLINE void fft_stage_pair(float2* s, int n, int S, const FastDiv& sdiv, int npair, const FastDiv& pdiv,
-                                          int ldc, const float2* __restrict__ tw, int tid, int nthr,
-                                          const float2* pre = nullptr, const Epi& epi = Epi()) {
+// Run-time length n and span S over NPAIR column pairs of row stride LDC.
+template <int R, bool INV, bool TW_FIRST, int NPAIR, int LDC, bool PRE, bool PTW>
+ASARF_HD ASARF_INLINE void fft_stage_pair(float2* s, int n, int S, const FastDiv& sdiv, const float2* __restrict__ tw,
+                                          int tid, int nthr, const float2* pre = nullptr) {
     const int M = S * R;
-    const int items = (n / R) * npair;
+    const int items = (n / R) * NPAIR;
     const int tw_step = n / M;
     for (int t = tid; t < items; t += nthr) {
-        const int bj = static_cast<int>(fdiv_u(t, pdiv));
-        const int cp = t - bj * npair;
-        const int b = static_cast<int>(fdiv_u(bj, sdiv));
+        const int bj = t / NPAIR;
+        const int cp = t - bj * NPAIR;
+        const int b = static_cast<int>(fdiv_u(static_cast<unsigned int>(bj), sdiv));
         const int j = bj - b * S;
-        pair_item<R, INV, TW_FIRST, PRE, Epi, PTW>(s, b, j, cp, M, S, ldc, tw_step, tw, pre, epi);
+        pair_item<R, INV, TW_FIRST, PRE, NoEpi, PTW>(s, b, j, cp, M, S, LDC, tw_step, tw, pre, NoEpi());
     }
 }
 
@@ -515,45 +524,55 @@ ASARF_HD ASARF_INLINE void fft_stage_pair_ct(float2* s, const float2* __restrict
     }
 }
 
-// The same stage with the length N and span S compile-time constants and the column count
-// run-time (npair pairs, divider pdiv, row stride ldc): the range-Doppler block, whose tile
-// width follows the scene's range walk.  PTW: packed twiddle products.
-template <int R, bool INV, bool TW_FIRST, int N, int S, class Epi = NoEpi, bool PTW = false>
-ASARF_HD ASARF_INLINE void fft_stage_pair_cs(float2* s, int npair, const FastDiv& pdiv, int ldc,
-                                             const float2* __restrict__ tw, int tid, int nthr,
-                                             const Epi& epi = Epi()) {
-    constexpr int M = S * R;
-    const int items = (N / R) * npair;
-    for (int t = tid; t < items; t += nthr) {
-        const int bj = static_cast<int>(fdiv_u(t, pdiv));
-        const int cp = t - bj * npair;
-        const int b = bj / S;
-        const int j = bj - b * S;
-        pair_item<R, INV, TW_FIRST, false, Epi, PTW>(s, b, j, cp, M, S, ldc, N / M, tw, nullptr, epi);
+// Column pairs of the range-Doppler block's stages, dealt to warps: a task is one butterfly row
+// (bj) over the first 32 column pairs, a pair per lane, so that block, offset and twiddle are the
+// warp's and a row's accesses are 512 contiguous bytes; the pairs past the 32nd are packed
+// into further tasks of 32 (pair, row) items.  ERS: 25 rows of 40 pairs are 25 + 7 tasks, two
+// rounds of the block's 16 warps.
+struct PairTasks {
+    int npair, full, rem;  // pairs, pairs of a main task, pairs past the 32nd
+    unsigned int rem_m;    // ceil(2^32 / rem)
+    ASARF_HD ASARF_INLINE explicit PairTasks(int n) : npair(n), full(n < 32 ? n : 32), rem(n - full), rem_m(0) {
+        if (rem > 1) rem_m = 0xffffffffu / static_cast<unsigned int>(rem) + 1u;
     }
+};
+
+// One stage over the tasks: fixed length NN and span SS when positive, else n, S and divider sdiv.
+template <int R, bool INV, bool TW_FIRST, int NN, int SS, class Epi, bool PTW>
+ASARF_HD ASARF_INLINE void fft_stage_pair_w(float2* s, int n_, int S_, const FastDiv& sdiv, const PairTasks& pt, int ldc,
+                                            const float2* __restrict__ tw, int tid, int nthr, const Epi& epi = Epi()) {
+    const int n = NN > 0 ? NN : n_, S = SS > 0 ? SS : S_;
+    const int M = S * R, nbj = n / R, tw_step = n / M;
+    auto item = [&](int bj, int cp) {
+        const int b = SS > 0 ? bj / (SS > 0 ? SS : 1) : static_cast<int>(fdiv_u(static_cast<unsigned int>(bj), sdiv));
+        pair_item<R, INV, TW_FIRST, false, Epi, PTW>(s, b, bj - b * S, cp, M, S, ldc, tw_step, tw, nullptr, epi);
+    };
+#if defined(__CUDA_ARCH__)
+    const int lane = tid & 31, nrem = (nbj * pt.rem + 31) >> 5;
+    for (int task = tid >> 5; task < nbj + nrem; task += nthr >> 5) {
+        int bj = task, cp = lane;
+        bool ok = lane < pt.full;
+        if (task >= nbj) {
+            const int t = (task - nbj) * 32 + lane;
+            bj = pt.rem > 1 ? static_cast<int>(__umulhi(static_cast<unsigned int>(t), pt.rem_m)) : t;
+            cp = 32 + t - bj * pt.rem;
+            ok = bj < nbj;
+        }
+        if (ok) item(bj, cp);
+    }
+#else
+    (void)tid;
+    (void)nthr;
+    for (int bj = 0; bj < nbj; ++bj)
+        for (int cp = 0; cp < pt.npair; ++cp) item(bj, cp);
+#endif
 }
 
-// Column-pair stages take the prime-power radices: a larger composite radix holds twice its
-// length in registers per column pair, which lifts the azimuth kernels from 64 to 128
-// registers per thread and halves their resident CTAs (measured slower despite fewer passes).
-// NINE adds radix 9 (two radix-3 DFTs in registers, 36 values per column pair: 71 registers
-// in the strided kernel, whose occupancy shared memory limits anyway) for plans that merge
-// factors 3 * 3; it is compiled only where such plans run, since every extra case costs the
-// other kernels registers.  PTW selects the packed twiddle products: the strided kernel uses them,
-// the range-Doppler block for radix <= 5 schedules only (az_rd_packed_twiddles).
-template <bool INV, bool TW_FIRST, bool NINE = false, bool PRE = false, class Epi = NoEpi, bool PTW = false>
-ASARF_HD ASARF_INLINE void fft_stage_pair_dispatch(int R, float2* s, int n, int S, const FastDiv& sdiv, int npair,
-                                                   const FastDiv& pdiv, int ldc, const float2* __restrict__ tw,
-                                                   int tid, int nthr, const float2* pre = nullptr,
-                                                   const Epi& epi = Epi()) {
-#define ASARF_PAIR(RR) \
-    fft_stage_pair<RR, INV, TW_FIRST, PRE, Epi, PTW>(s, n, S, sdiv, npair, pdiv, ldc, tw, tid, nthr, pre, epi)
-    if constexpr (NINE) {
-        if (R == 9) {
-            ASARF_PAIR(9);
-            return;
-        }
-    }
+template <bool INV, bool TW_FIRST, class Epi, bool PTW>
+ASARF_HD ASARF_INLINE void fft_stage_pair_w_dispatch(int R, float2* s, int n, int S, const FastDiv& sdiv,
+                                                     const PairTasks& pt, int ldc, const float2* __restrict__ tw,
+                                                     int tid, int nthr, const Epi& epi = Epi()) {
+#define ASARF_PAIR(RR) fft_stage_pair_w<RR, INV, TW_FIRST, 0, 0, Epi, PTW>(s, n, S, sdiv, pt, ldc, tw, tid, nthr, epi)
     switch (R) {
         case 2: ASARF_PAIR(2); break;
         case 3: ASARF_PAIR(3); break;
@@ -565,48 +584,71 @@ ASARF_HD ASARF_INLINE void fft_stage_pair_dispatch(int R, float2* s, int n, int 
 #undef ASARF_PAIR
 }
 
-// Column-pair forms of fft_forward / fft_inverse / fft_inverse_dif (ncol and ldc even).
-template <bool NINE = false, bool PTW = false>
+// Column-pair stages take the prime-power radices: a larger composite radix holds twice its
+// length in registers per column pair, which lifts the azimuth kernels from 64 to 128
+// registers per thread and halves their resident CTAs (measured slower despite fewer passes).
+// NINE adds radix 9 (two radix-3 DFTs in registers, 36 values per column pair: 71 registers
+// in the strided kernel, whose occupancy shared memory limits anyway) for plans that merge
+// factors 3 * 3; it is compiled only where such plans run, since every extra case costs the
+// other kernels registers.  PTW selects the packed twiddle products: the strided kernel uses them,
+// the range-Doppler block for radix <= 5 schedules only (az_rd_packed_twiddles).
+template <bool INV, bool TW_FIRST, int NPAIR, int LDC, bool PRE>
+ASARF_HD ASARF_INLINE void fft_stage_pair_dispatch(int R, float2* s, int n, int S, const FastDiv& sdiv,
+                                                   const float2* __restrict__ tw, int tid, int nthr,
+                                                   const float2* pre = nullptr) {
+#define ASARF_PAIR(RR) fft_stage_pair<RR, INV, TW_FIRST, NPAIR, LDC, PRE, true>(s, n, S, sdiv, tw, tid, nthr, pre)
+    switch (R) {
+        case 2: ASARF_PAIR(2); break;
+        case 3: ASARF_PAIR(3); break;
+        case 4: ASARF_PAIR(4); break;
+        case 5: ASARF_PAIR(5); break;
+        case 7: ASARF_PAIR(7); break;
+        case 9: ASARF_PAIR(9); break;
+        default: ASARF_PAIR(8); break;
+    }
+#undef ASARF_PAIR
+}
+
+// Column-pair forms of fft_forward / fft_inverse (ncol and ldc even) of the range-Doppler block.
+template <bool PTW>
 ASARF_HD ASARF_INLINE void fft_forward_pairs(const FftPlan& p, float2* s, int ncol, int ldc, int tid, int nthr) {
-    const int npair = ncol >> 1;
-    const FastDiv pdiv = make_fastdiv(static_cast<unsigned int>(npair));
+    const PairTasks pt(ncol >> 1);
     for (int i = 0; i < p.nst; ++i) {
-        fft_stage_pair_dispatch<false, false, NINE, false, NoEpi, PTW>(p.radix[i], s, p.n, p.span[i], p.sdiv[i], npair,
-                                                                      pdiv, ldc, p.tw, tid, nthr);
+        fft_stage_pair_w_dispatch<false, false, NoEpi, PTW>(p.radix[i], s, p.n, p.span[i], p.sdiv[i], pt, ldc, p.tw, tid,
+                                                            nthr);
         ASARF_SYNC();
     }
 }
 
-// With an active epilogue the last stage writes through it and the tile is left unfinished.
-template <class Epi = NoEpi, bool PTW = false>
+// The last stage writes through its epilogue and the tile is left unfinished.
+template <class Epi, bool PTW>
 ASARF_HD ASARF_INLINE void fft_inverse_pairs(const FftPlan& p, float2* s, int ncol, int ldc, int tid, int nthr,
-                                             const Epi& epi = Epi()) {
-    const int npair = ncol >> 1;
-    const FastDiv pdiv = make_fastdiv(static_cast<unsigned int>(npair));
-    for (int i = p.nst - 1; i >= 0; --i) {
-        if (Epi::kActive && i == 0)
-            fft_stage_pair_dispatch<true, true, false, false, Epi, PTW>(p.radix[i], s, p.n, p.span[i], p.sdiv[i],
-                                                                        npair, pdiv, ldc, p.tw, tid, nthr, nullptr, epi);
-        else
-            fft_stage_pair_dispatch<true, true, false, false, NoEpi, PTW>(p.radix[i], s, p.n, p.span[i], p.sdiv[i],
-                                                                          npair, pdiv, ldc, p.tw, tid, nthr);
+                                             const Epi& epi) {
+    const PairTasks pt(ncol >> 1);
+    for (int i = p.nst - 1; i > 0; --i) {
+        fft_stage_pair_w_dispatch<true, true, NoEpi, PTW>(p.radix[i], s, p.n, p.span[i], p.sdiv[i], pt, ldc, p.tw, tid,
+                                                          nthr);
+        ASARF_SYNC();
+    }
+    fft_stage_pair_w_dispatch<true, true, Epi, PTW>(p.radix[0], s, p.n, p.span[0], p.sdiv[0], pt, ldc, p.tw, tid, nthr,
+                                                    epi);
+}
+
+// Forward DIF, and inverse in DIF form whose input row l is first multiplied by conj(pre[l]) (folded
+// into stage 0), of the strided azimuth pass: NPAIR column pairs of row stride LDC.
+template <int NPAIR, int LDC>
+ASARF_HD ASARF_INLINE void fft_forward_pairs_xt(const FftPlan& p, float2* s, int tid, int nthr) {
+    for (int i = 0; i < p.nst; ++i) {
+        fft_stage_pair_dispatch<false, false, NPAIR, LDC, false>(p.radix[i], s, p.n, p.span[i], p.sdiv[i], p.tw, tid, nthr);
         ASARF_SYNC();
     }
 }
-
-// pre (optional): per-row table whose conjugate multiplies the input (folded into stage 0).
-template <bool NINE = false, bool PTW = false>
-ASARF_HD ASARF_INLINE void fft_inverse_dif_pairs(const FftPlan& p, float2* s, int ncol, int ldc, int tid, int nthr,
-                                                 const float2* pre = nullptr) {
-    const int npair = ncol >> 1;
-    const FastDiv pdiv = make_fastdiv(static_cast<unsigned int>(npair));
-    for (int i = 0; i < p.nst; ++i) {
-        if (i == 0 && pre)
-            fft_stage_pair_dispatch<true, false, NINE, true, NoEpi, PTW>(p.radix[i], s, p.n, p.span[i], p.sdiv[i],
-                                                                        npair, pdiv, ldc, p.tw, tid, nthr, pre);
-        else
-            fft_stage_pair_dispatch<true, false, NINE, false, NoEpi, PTW>(p.radix[i], s, p.n, p.span[i], p.sdiv[i],
-                                                                         npair, pdiv, ldc, p.tw, tid, nthr);
+template <int NPAIR, int LDC>
+ASARF_HD ASARF_INLINE void fft_inverse_dif_pairs_xt(const FftPlan& p, float2* s, int tid, int nthr, const float2* pre) {
+    fft_stage_pair_dispatch<true, false, NPAIR, LDC, true>(p.radix[0], s, p.n, p.span[0], p.sdiv[0], p.tw, tid, nthr, pre);
+    ASARF_SYNC();
+    for (int i = 1; i < p.nst; ++i) {
+        fft_stage_pair_dispatch<true, false, NPAIR, LDC, false>(p.radix[i], s, p.n, p.span[i], p.sdiv[i], p.tw, tid, nthr);
         ASARF_SYNC();
     }
 }
@@ -614,7 +656,7 @@ ASARF_HD ASARF_INLINE void fft_inverse_dif_pairs(const FftPlan& p, float2* s, in
 // Compile-time three-stage column-pair transforms (radices R0, R1, R2 first stage first, NPAIR
 // column pairs of row stride LDC): the forward DIF and the inverse in DIF form of the strided
 // azimuth pass, with the same stage sequence, twiddle tables and rounding as the run-time
-// versions above (fft_forward_pairs / fft_inverse_dif_pairs), so the results are identical.
+// versions above (fft_forward_pairs_xt / fft_inverse_dif_pairs_xt), so the results are identical.
 template <int R0, int R1, int R2, int NPAIR, int LDC, bool PTW>
 ASARF_HD ASARF_INLINE void fft_forward_pairs_ct3(float2* s, const float2* __restrict__ tw, int tid, int nthr) {
     constexpr int N = R0 * R1 * R2;
@@ -641,32 +683,31 @@ ASARF_HD ASARF_INLINE void fft_inverse_dif_pairs_ct3(float2* s, const float2* __
 // Three-stage forward DIF (fft_forward_pairs) and inverse DIT with epilogue (fft_inverse_pairs)
 // of a compile-time radix schedule R0, R1, R2 over a run-time number of columns: the same
 // stages, twiddles and rounding as the run-time versions.
-template <int R0, int R1, int R2, bool PTW = false>
+template <int R0, int R1, int R2, bool PTW>
 ASARF_HD ASARF_INLINE void fft_forward_pairs_cs3(float2* s, int ncol, int ldc, const float2* __restrict__ tw, int tid,
                                                  int nthr) {
     constexpr int N = R0 * R1 * R2;
-    const int npair = ncol >> 1;
-    const FastDiv pdiv = make_fastdiv(static_cast<unsigned int>(npair));
-    fft_stage_pair_cs<R0, false, false, N, N / R0, NoEpi, PTW>(s, npair, pdiv, ldc, tw, tid, nthr);
+    const PairTasks pt(ncol >> 1);
+    const FastDiv none{1u, 0u, 0u};
+    fft_stage_pair_w<R0, false, false, N, N / R0, NoEpi, PTW>(s, N, 0, none, pt, ldc, tw, tid, nthr);
     ASARF_SYNC();
-    fft_stage_pair_cs<R1, false, false, N, R2, NoEpi, PTW>(s, npair, pdiv, ldc, tw, tid, nthr);
+    fft_stage_pair_w<R1, false, false, N, R2, NoEpi, PTW>(s, N, 0, none, pt, ldc, tw, tid, nthr);
     ASARF_SYNC();
-    fft_stage_pair_cs<R2, false, false, N, 1, NoEpi, PTW>(s, npair, pdiv, ldc, tw, tid, nthr);
+    fft_stage_pair_w<R2, false, false, N, 1, NoEpi, PTW>(s, N, 0, none, pt, ldc, tw, tid, nthr);
     ASARF_SYNC();
 }
 
-template <int R0, int R1, int R2, class Epi = NoEpi, bool PTW = false>
+template <int R0, int R1, int R2, class Epi, bool PTW>
 ASARF_HD ASARF_INLINE void fft_inverse_pairs_cs3(float2* s, int ncol, int ldc, const float2* __restrict__ tw, int tid,
-                                                 int nthr, const Epi& epi = Epi()) {
+                                                 int nthr, const Epi& epi) {
     constexpr int N = R0 * R1 * R2;
-    const int npair = ncol >> 1;
-    const FastDiv pdiv = make_fastdiv(static_cast<unsigned int>(npair));
-    fft_stage_pair_cs<R2, true, true, N, 1, NoEpi, PTW>(s, npair, pdiv, ldc, tw, tid, nthr);
+    const PairTasks pt(ncol >> 1);
+    const FastDiv none{1u, 0u, 0u};
+    fft_stage_pair_w<R2, true, true, N, 1, NoEpi, PTW>(s, N, 0, none, pt, ldc, tw, tid, nthr);
     ASARF_SYNC();
-    fft_stage_pair_cs<R1, true, true, N, R2, NoEpi, PTW>(s, npair, pdiv, ldc, tw, tid, nthr);
+    fft_stage_pair_w<R1, true, true, N, R2, NoEpi, PTW>(s, N, 0, none, pt, ldc, tw, tid, nthr);
     ASARF_SYNC();
-    fft_stage_pair_cs<R0, true, true, N, N / R0, Epi, PTW>(s, npair, pdiv, ldc, tw, tid, nthr, epi);
-    ASARF_SYNC();
+    fft_stage_pair_w<R0, true, true, N, N / R0, Epi, PTW>(s, N, 0, none, pt, ldc, tw, tid, nthr, epi);
 }
 
 template <bool INV>

@@ -657,7 +657,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
         delete p;
         return set_error(ASARF_ERR_INVALID, "strided_tile_width must be 16 or 32");
     }
-    p->xt2 = az_rd_tile_width(p->n2, p->hl, p->hr);
+    p->xt2 = az_rd_tile_width(p->n2, p->hl, p->hr, opt.absolute_phase != 0);
     if (opt.az_tile_width != 0) {
         if (opt.az_tile_width < 16 || opt.az_tile_width > 64 || (opt.az_tile_width & 1)) {
             delete p;
@@ -668,7 +668,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     if (opt.precision == ASARF_PRECISION_SPLIT && opt.az_tile_width == 0) {
         // the split block holds the DFT matrix (16 KB) besides the tile: the widest tile that
         // still leaves two blocks resident per SM
-        while (p->xt2 > 16 && az_rd_smem(p->n2, p->xt2 + p->hl + p->hr, p->xt2) + 2 * kSplitMatrixBytes >
+        while (p->xt2 > 16 && az_rd_smem(p->n2, p->xt2 + p->hl + p->hr, p->xt2, opt.absolute_phase != 0) + 2 * kSplitMatrixBytes >
                                   kAzRdTwoBlockSmem)
             p->xt2 -= 2;
     }
@@ -768,7 +768,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     float2* tw2 = p->alloc<float2>(p->n2);
     int* drev2 = p->alloc<int>(p->n2);
     float2* twN = p->alloc<float2>(p->az_pad);
-    float* win = p->alloc<float>(16);
+    float* rcmc = p->alloc<float>(static_cast<size_t>(kRcmcNodes + 1) * kRcmcRowFloats);
     float* rsl_dev = p->alloc<float>(p->nx);
     // FBAQ4 records: reconstruction tables permuted to [block id][raw code], and the
     // statistics partials of every 32-column x kFbaqStatsLines tile
@@ -788,16 +788,13 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     constexpr int kPstatBlocks = 4 * 148;
     double* pstat_dev = opt.sq_stats ? p->alloc<double>(5 * kPstatBlocks + 4) : nullptr;
     if (!p->bufA || !p->bufB || !p->acc || !p->state || !p->raw_dev || !p->swst_dev || !p->out_dev || !rc_tw ||
-        !p->rc_mf || !tw1 || !drev1 || !tw2 || !drev2 || !twN || !win || !rsl_dev || (fbaq && (!lut_dev || !part_dev || !facc_dev)) ||
+        !p->rc_mf || !tw1 || !drev1 || !tw2 || !drev2 || !twN || !rcmc || !rsl_dev || (fbaq && (!lut_dev || !part_dev || !facc_dev)) ||
         (opt.sq_stats && !pstat_dev)) {
         const size_t need = p->bytes;
         delete p;
         return set_error(ASARF_ERR_NOMEM, "device allocation failed (plan needs about %zu MB)",
                          (need + 2 * img * sizeof(float2)) >> 20);
     }
-    float w16[16];
-    for (int n = 0; n < 16; ++n)  // numpy.blackman(16) (sar/range_doppler_algorithm.cu:49-52)
-        w16[n] = static_cast<float>(0.42 - 0.5 * std::cos(2 * kPi * n / 15) + 0.08 * std::cos(4 * kPi * n / 15));
     rc = 0;
     rc |= mem_h2d(rc_tw, p->rc.tw.data(), sizeof(float2) * p->rc_len, nullptr);
     rc |= mem_h2d(p->rc_mf, mf.data(), sizeof(float2) * p->rc_len, nullptr);
@@ -807,7 +804,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     rc |= mem_h2d(tw2, p->f2.tw.data(), sizeof(float2) * p->n2, nullptr);
     rc |= mem_h2d(drev2, p->f2.drev.data(), sizeof(int) * p->n2, nullptr);
     rc |= mem_h2d(twN, p->fN.tw.data(), sizeof(float2) * p->az_pad, nullptr);
-    rc |= mem_h2d(win, w16, sizeof(w16), nullptr);
+    rc |= backend_rcmc_table(rcmc, nullptr);
     rc |= mem_h2d(rsl_dev, rsl.data(), sizeof(float) * p->nx, nullptr);
     if (fbaq) {
         std::vector<float> lut(2 * 4096);
@@ -960,12 +957,12 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     d.range_spacing = s.range_spacing;
     for (int k = 0; k < 3; ++k) d.vr_poly[k] = static_cast<float>(p->vr_poly[k]);
     d.state = p->state;
-    d.win = win;
+    d.rcmc = rcmc;
     d.absolute_phase = opt.absolute_phase ? 1 : 0;
     d.compiled = p->a_fwd.compiled = p->a_inv.compiled = opt.compiled_schedules ? 1 : 0;
     d.lambda_d = s.wavelength;
     p->tiles2 = (p->nk + p->xt2 - 1) / p->xt2;
-    p->sh_rd = {512, az_rd_smem(p->n2, d.wt, d.xt)};
+    p->sh_rd = {512, az_rd_smem(p->n2, d.wt, d.xt, opt.absolute_phase != 0)};
 
     // detected products without a kept SLC: the inverse azimuth pass writes |z|^2 rows into
     // bufA (free once the range-Doppler block has read it) and the tail reads those

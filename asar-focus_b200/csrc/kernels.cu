@@ -164,7 +164,7 @@ __device__ __forceinline__ const uint8_t* stage_record(uint8_t* buf, const uint8
 // into shared memory (the sub-16-byte tail with plain loads) while the others wait.
 template <int FMT>
 __global__ void __launch_bounds__(512) k_range_compress(RangeCompressArgs a) {
-    extern __shared__ __align__(1024) unsigned char smem_rc_raw[];
+    extern __shared__ __align__(128) unsigned char smem_rc_raw[];
     float2* s = reinterpret_cast<float2*>(smem_rc_raw);
     __shared__ uint64_t bar;
     const uint8_t* line = nullptr;
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(512) k_range_compress(RangeCompressArgs a) {
 // Compile-time-scheduled variant (L in kCtLengths).
 template <int L, int FMT>
 __global__ void __launch_bounds__(CtSchedule<L>::nthr, 2) k_range_compress_ct(RangeCompressArgs a) {
-    extern __shared__ __align__(1024) unsigned char smem_rcc_raw[];
+    extern __shared__ __align__(128) unsigned char smem_rcc_raw[];
     float2* s = reinterpret_cast<float2*>(smem_rcc_raw);
     __shared__ uint64_t bar;
     const uint8_t* line = nullptr;
@@ -216,10 +216,10 @@ __global__ void __launch_bounds__(CtSchedule<L>::nthr, 2) k_range_compress_ct(Ra
 }
 
 // Strided azimuth pass: the [n1][xt] tile (rows r*n2 + b) arrives by 3-D TMA boxes.
-// R0..XT > 0: compile-time transform schedule and tile width (az_strided_body).
-template <int R0 = 0, int R1 = 0, int R2 = 0, int XT = 0>
+// R0..R2 > 0: compile-time transform schedule; XT: tile width (az_strided_body).
+template <int R0, int R1, int R2, int XT>
 __global__ void __launch_bounds__(512) k_az_strided(AzStridedArgs a, const __grid_constant__ CUtensorMap map) {
-    extern __shared__ __align__(1024) unsigned char smem_as_raw[];
+    extern __shared__ __align__(128) unsigned char smem_as_raw[];
     float2* s = reinterpret_cast<float2*>(smem_as_raw);
     float2* tw = s + static_cast<size_t>(a.n1) * a.xt;
     int* row = reinterpret_cast<int*>(tw + a.n1);
@@ -241,12 +241,13 @@ __global__ void __launch_bounds__(512) k_az_strided(AzStridedArgs a, const __gri
 // boxes; columns left of 0 and right of nk are filled with zeros by the TMA unit.
 // R0..R2 > 0: compile-time radix schedule of the n2 transforms (az_rd_body).
 template <int R0 = 0, int R1 = 0, int R2 = 0>
-__global__ void __launch_bounds__(512) k_az_rd(AzRdArgs a, unsigned int* err, const __grid_constant__ CUtensorMap map) {
-    extern __shared__ __align__(1024) unsigned char smem_rd_raw[];
+__global__ void __launch_bounds__(512, 2) k_az_rd(AzRdArgs a, unsigned int* err, const __grid_constant__ CUtensorMap map) {
+    // (128-byte alignment: a larger one pads the static barrier below to as much, and two blocks
+    // of kAzRdTwoBlockSmem bytes would no longer fit)
+    extern __shared__ __align__(128) unsigned char smem_rd_raw[];
     const int wt = a.wt;
     float2* s = reinterpret_cast<float2*>(smem_rd_raw);
-    ColParams* cps = reinterpret_cast<ColParams*>(s + static_cast<size_t>(a.n2) * wt);
-    float* fbf = az_rd_freq_table(cps, a);
+    const AzRdTables t(a, s);
     __shared__ uint64_t bar;
     if (a.use_tma && threadIdx.x == 0) {
         mbar_init(&bar, 1);
@@ -256,11 +257,10 @@ __global__ void __launch_bounds__(512) k_az_rd(AzRdArgs a, unsigned int* err, co
             tma_load_2d(s + static_cast<size_t>(r0) * wt, &map, &bar, x, blockIdx.y * a.n2 + r0);
     }
     // column constants and row frequencies are computed while the tile is in flight
-    az_rd_tables(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, cps, fbf);
+    az_rd_tables(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, t);
     __syncthreads();
     if (a.use_tma) mbar_wait(&bar, 0, err);
-    az_rd_body<true, R0, R1, R2>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, s, cps, fbf, err,
-                                 a.use_tma != 0);
+    az_rd_body<true, R0, R1, R2>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, s, t, err, a.use_tma != 0);
 }
 
 // ----------------------------------------------------------------------------- split precision
@@ -355,22 +355,20 @@ __device__ bool split_forward(const AzRdArgs& a, const AzRdSplit& sp, float2* s,
     }
     // radix-R DFT over r of every (slot, column pair): rows R * slot + r, no twiddles
     const int npair = wt >> 1;
-    fft_stage_pair_dispatch<false, false>(R, s, a.n2, 1, make_fastdiv(1u), npair,
-                                          make_fastdiv(static_cast<unsigned int>(npair)), wt, a.plan2.tw, tid,
-                                          blockDim.x);
+    fft_stage_pair_w_dispatch<false, false, NoEpi, false>(R, s, a.n2, 1, make_fastdiv(1u), PairTasks(npair), wt,
+                                                          a.plan2.tw, tid, blockDim.x);
     __syncthreads();
     return true;
 }
 
 __global__ void __launch_bounds__(512, 2) k_az_rd_split(AzRdArgs a, AzRdSplit sp, unsigned int* err,
                                                         const __grid_constant__ CUtensorMap map) {
-    extern __shared__ __align__(1024) unsigned char smem_rds_raw[];
+    extern __shared__ __align__(128) unsigned char smem_rds_raw[];
     unsigned char* b_hi = smem_rds_raw;
     unsigned char* b_lo = b_hi + kSplitMatrixBytes;
     float2* s = reinterpret_cast<float2*>(b_lo + kSplitMatrixBytes);
     const int wt = a.wt;
-    ColParams* cps = reinterpret_cast<ColParams*>(s + static_cast<size_t>(a.n2) * wt);
-    float* fbf = az_rd_freq_table(cps, a);
+    const AzRdTables t(a, s);
     __shared__ uint64_t bar, mbar;
     __shared__ uint32_t tmem_base;
     if (threadIdx.x < 32) tmem_alloc(&tmem_base, kSplitTmemCols);
@@ -386,7 +384,7 @@ __global__ void __launch_bounds__(512, 2) k_az_rd_split(AzRdArgs a, AzRdSplit sp
     const uint4* bsrc = reinterpret_cast<const uint4*>(sp.bmat);
     for (int i = threadIdx.x; i < 2 * kSplitMatrixBytes / 16; i += blockDim.x)
         reinterpret_cast<uint4*>(b_hi)[i] = __ldg(bsrc + i);
-    az_rd_tables(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, cps, fbf);
+    az_rd_tables(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, t);
     fence_async_smem();  // B is read by the tensor cores
     tc_fence_before_sync();
     __syncthreads();
@@ -394,11 +392,16 @@ __global__ void __launch_bounds__(512, 2) k_az_rd_split(AzRdArgs a, AzRdSplit sp
     const uint32_t tmem = tmem_base;
     mbar_wait(&bar, 0, err);
     if (split_forward(a, sp, s, b_hi, b_lo, tmem, &mbar, err))
-        az_rd_body<false>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, s, cps, fbf, err, true);
+        az_rd_body<false>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, s, t, err, true);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     if (threadIdx.x < 32) tmem_dealloc(tmem, kSplitTmemCols);
+}
+
+__global__ void __launch_bounds__(128) k_rcmc_table(float* table) {
+    const int n = blockIdx.x * 128 + threadIdx.x;
+    if (n <= kRcmcNodes) rcmc_weight_row(n, table + static_cast<size_t>(n) * kRcmcRowFloats);
 }
 
 __global__ void __launch_bounds__(512, 2) k_tail(TailArgs a, unsigned int* err) {
@@ -563,7 +566,8 @@ int backend_az_strided(const AzStridedArgs& a, const void* tmap, int tiles, int 
         if (plan_is(a.plan1, 9, 5, 5)) return launch_az_strided<9, 5, 5, 32>(a, tmap, tiles, nblocks, sh, stream);
         return launch_az_strided<9, 4, 5, 32>(a, tmap, tiles, nblocks, sh, stream);
     }
-    return launch_az_strided<0, 0, 0, 0>(a, tmap, tiles, nblocks, sh, stream);
+    if (a.xt == 32) return launch_az_strided<0, 0, 0, 32>(a, tmap, tiles, nblocks, sh, stream);
+    return launch_az_strided<0, 0, 0, 16>(a, tmap, tiles, nblocks, sh, stream);
 }
 
 template <int R0, int R1, int R2>
@@ -592,6 +596,11 @@ int backend_az_rd_split(const AzRdArgs& a, const AzRdSplit& sp, const void* tmap
     if (rc) return rc;
     k_az_rd_split<<<dim3(tiles, nblocks), sh.threads, sh.smem, S(stream)>>>(a, sp, err, tmap_or_zero(tmap));
     return check_launch("az_rd_split");
+}
+
+int backend_rcmc_table(float* table, void* stream) {
+    k_rcmc_table<<<kRcmcNodes / 128 + 1, 128, 0, S(stream)>>>(table);
+    return check_launch("rcmc_table");
 }
 
 int backend_make_tmap(void* out, int rank, void* base, const unsigned long long* dims,

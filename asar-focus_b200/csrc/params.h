@@ -185,7 +185,7 @@ struct AzRdArgs {
     double slant, range_spacing;
     float vr_poly[3];
     const FocusState* state;
-    const float* win;     // 16 RCMC window taps
+    const float* rcmc;    // interpolation weights by walk fraction (rcmc_weight_row)
     int use_tma;
     int n2_box;           // rows per TMA box
     int absolute_phase;   // 1: multiply column x by exp(j (4 pi R0 / lambda + pi dc_off^2 / Ka)) (FP64)

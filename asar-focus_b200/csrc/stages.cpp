@@ -291,8 +291,9 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
         return set_error(ASARF_ERR_INVALID, "range_doppler: azimuth size %d is not 2^a3^b5^c7^d", N);
     // tables + a finalised state carrying the Doppler polynomial
     DevBuf tw1(sizeof(float2) * n1), dr1(sizeof(int) * n1), tw2(sizeof(float2) * n2), dr2(sizeof(int) * n2),
-        twN(sizeof(float2) * N), st(sizeof(FocusState));
-    if (!tw1.p || !dr1.p || !tw2.p || !dr2.p || !twN.p || !st.p) return nomem();
+        twN(sizeof(float2) * N), st(sizeof(FocusState)),
+        rcmc(sizeof(float) * static_cast<size_t>(kRcmcNodes + 1) * kRcmcRowFloats);
+    if (!tw1.p || !dr1.p || !tw2.p || !dr2.p || !twN.p || !st.p || !rcmc.p) return nomem();
     FocusState hs{};
     for (int k = 0; k < 3; ++k) {
         hs.dc_poly[k] = prm->dc_poly[k];
@@ -306,6 +307,7 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     if (!rc) rc = mem_h2d(dr2.p, f2.drev.data(), sizeof(int) * n2, stream);
     if (!rc) rc = mem_h2d(twN.p, fN.tw.data(), sizeof(float2) * N, stream);
     if (!rc) rc = mem_h2d(st.p, &hs, sizeof(hs), stream);
+    if (!rc) rc = backend_rcmc_table(rcmc.as<float>(), stream);
     if (!rc) rc = mem_zero(d_out, sizeof(float2) * static_cast<size_t>(x_stride) * y_stride, stream);
     if (rc) return rc;
     f1.plan.tw = tw1.as<float2>();
@@ -356,7 +358,7 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     d.hl = kRcmcTaps / 2;
     d.hr = rcmc_right_halo(walk);
     if ((d.hl + d.hr) & 1) ++d.hr;  // column-pair transforms need an even tile width
-    d.xt = az_rd_tile_width(n2, d.hl, d.hr);
+    d.xt = az_rd_tile_width(n2, d.hl, d.hr, false);
     d.wt = d.xt + d.hl + d.hr;
     d.prf = static_cast<float>(prm->prf);
     d.bin_step = d.prf / static_cast<float>(N);
@@ -367,8 +369,9 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     d.range_spacing = prm->range_spacing;
     for (int k = 0; k < 3; ++k) d.vr_poly[k] = static_cast<float>(prm->vr_poly[k]);
     d.state = dstate;
+    d.rcmc = rcmc.as<float>();
     const LaunchShape sh_st{256, az_strided_smem(n1, xt1)};
-    const LaunchShape sh_rd{512, az_rd_smem(n2, d.wt, d.xt)};
+    const LaunchShape sh_rd{512, az_rd_smem(n2, d.wt, d.xt, false)};
     if (sh_st.smem > smem_optin_limit() || sh_rd.smem > smem_optin_limit())
         return set_error(ASARF_ERR_INVALID, "range_doppler: tiles exceed shared memory (n1 %d, n2 %d)", n1, n2);
     const int tiles1 = (x_size + xt1 - 1) / xt1, tiles2 = (x_size + d.xt - 1) / d.xt;
