@@ -13,6 +13,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -55,7 +56,7 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
     objdir = PKG / "_build"
     objdir.mkdir(exist_ok=True)
     common = ["-std=c++17", "-O3", "-lineinfo", f"-I{INC}", f"-I{CSRC}", "-Xcompiler", "-fPIC"]
-    objs = []
+    objs, cmds = [], []
     for src in ("kernels.cu", "noalloc.cu", "host.cpp", "stages.cpp", "batch.cpp", "strip.cpp", "l0.cpp"):
         obj = objdir / (src + ".o")
         cmd = [NVCC, *GENCODE, *common, "-c", str(CSRC / src), "-o", str(obj)]
@@ -63,8 +64,10 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
             cmd += ["-Xptxas", "-v"]
         if src.endswith(".cpp"):
             cmd = [NVCC, *common, "-x", "cu", *GENCODE, "-c", str(CSRC / src), "-o", str(obj)]
-        _run(cmd)
+        cmds.append(cmd)
         objs.append(str(obj))
+    with ThreadPoolExecutor() as pool:
+        list(pool.map(_run, cmds))
     _run([NVCC, *GENCODE, "-shared", "-o", str(LIB), *objs, "-lcudart"])
     return LIB
 

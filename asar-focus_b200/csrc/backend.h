@@ -21,7 +21,7 @@ int backend_finalize(const FinalizeArgs& a, void* stream);
 int backend_raw_stats_fbaq(const RawStatsArgs& a, int gx, int gy, void* stream);
 int backend_stats_fold(const RawStatsArgs& a, int tiles_y, void* stream);
 int backend_range_compress(const RangeCompressArgs& a, int lines, LaunchShape sh, void* stream);
-int backend_az_strided(const AzStridedArgs& a, const void* tmap, int tiles, int nblocks, LaunchShape sh, void* stream);
+int backend_az_strided(const AzStridedArgs& a, const void* tmap, int tiles, LaunchShape sh, void* stream);
 int backend_az_rd(const AzRdArgs& a, const void* tmap, int tiles, int nblocks, LaunchShape sh, unsigned int* err,
                   void* stream);
 // interpolation weights of AzRdArgs::rcmc: (kRcmcNodes + 1) rows of kRcmcRowFloats

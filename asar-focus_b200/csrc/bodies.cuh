@@ -853,83 +853,121 @@ ASARF_HD ASARF_INLINE void range_compress_ct_body(const RangeCompressArgs& a, in
 // write the digit-reversed transform output straight to its destination rows.
 // Together with the contiguous pass this is the transpose-free equivalent of the reference's
 // transpose + batched row FFT + transpose (sar/range_doppler_algorithm.cu:314-326, 381-391).
-// Per-block tables of the strided pass, staged in shared memory while the tile is in flight:
-// tw[p] = W_N^{b * k1} and row[p] = destination row, for transform position p (forward:
+// A block takes NB adjacent b: their tiles lie side by side as one [n1][NB * XT] tile (one TMA
+// box), so that short lengths n1 still give a block's threads and its loads enough to do.
+// Per-block tables, staged in shared memory while the tile is in flight: tw[k * n1 + p] =
+// W_N^{(b + k) k1} and row[p] = destination row of b, for transform position p (forward:
 // k1 = drev1(p), digit-reversed output; inverse: tw indexed by the natural input row k1 = p,
 // row by the digit-reversed output position).  b * k1 < N, so no reduction is needed.
 ASARF_HD ASARF_INLINE void az_strided_tables(const AzStridedArgs& a, int b, int tid, int nthr, float2* tw, int* row) {
     for (int p = tid; p < a.n1; p += nthr) {
         const int kd = ASARF_LDG(a.drev1 + p);
-        tw[p] = ASARF_LDG(a.twn + b * (a.inverse ? p : kd));
+        for (int k = 0; k < a.nb; ++k)
+            if (b + k < a.n2) tw[k * a.n1 + p] = ASARF_LDG(a.twn + (b + k) * (a.inverse ? p : kd));
         row[p] = kd * a.n2 + b;
     }
 }
 
-// XT: the tile width (16 or 32).  R0, R1, R2 > 0: the transform's radix schedule as compile-time
-// constants (it must be the plan's: the planner picks this instantiation only when it is).
-template <int R0, int R1, int R2, int XT>
+// Tiles of a block: as many as keep n1 * nb at 256 rows of 32 columns (64 KB, three blocks per SM)
+// while the grid still has three blocks per SM (5000 lines of 4913 columns, n1 = 40: 147 us forward
+// with one, 85 with four; n1 = 225 takes one).
+inline int az_strided_tiles_per_block(int n1, int n2, int tiles) {
+    int nb = 1;
+    while (nb < 8 && 2 * nb * n1 <= 256 && static_cast<long long>(tiles) * (n2 / (2 * nb)) >= 3 * 148) nb *= 2;
+    return nb;
+}
+
+// XT: the tile width (16 or 32), NB tiles.  R0, R1, R2 > 0: the transform's radix schedule as
+// compile-time constants (it must be the plan's: the planner picks this instantiation only when it
+// is).  b: the first tile's.
+template <int R0, int R1, int R2, int XT, int NB>
 ASARF_HD ASARF_INLINE void az_strided_body(const AzStridedArgs& a, int tile, int b, int tid, int nthr, float2* s,
                                            const float2* tw, const int* rowmap, bool preloaded) {
+    constexpr int LDC = XT * NB, PAIRS = XT / 2, NPAIR = LDC / 2;
     const int n1 = R0 > 0 ? R0 * R1 * R2 : a.n1;
-    constexpr int xt = XT;
-    const int x0 = tile * xt;
-    auto row_of = [](int t) { return t / XT; };
-    // tile [r][c] = row r*n2 + b, column x0 + c (natural order; columns >= nk read as 0)
+    const int x0 = tile * XT;
+    // tile [r][k][c] = row r*n2 + b + k, column x0 + c (natural order; columns >= nk read as 0)
     if (!preloaded) {
-        for (int t = tid; t < n1 * xt; t += nthr) {
-            const int r = row_of(t), c = t - r * xt;
-            const int row = r * a.n2 + b;
-            const int x = x0 + c;
+        for (int t = tid; t < n1 * LDC; t += nthr) {
+            const int r = t / LDC, k = t % LDC / XT;
+            const int row = r * a.n2 + b + k;
+            const int x = x0 + t % XT;
             float2 v = make_float2(0.0f, 0.0f);
-            if (row < a.valid_rows && x < a.nk) v = a.in[static_cast<long long>(row) * a.pitch + x];
+            if (b + k < a.n2 && row < a.valid_rows && x < a.nk) v = a.in[static_cast<long long>(row) * a.pitch + x];
             s[t] = v;
         }
+        ASARF_SYNC();
     } else if (a.valid_rows < n1 * a.n2) {
         // rows past the data hold stale values in memory: they are zero by definition
-        const int r0 = (a.valid_rows - b + a.n2 - 1) / a.n2;
-        for (int t = r0 * xt + tid; t < n1 * xt; t += nthr) s[t] = make_float2(0.0f, 0.0f);
+        const int r0 = a.valid_rows > b + NB - 1 ? (a.valid_rows - (b + NB - 1) + a.n2 - 1) / a.n2 : 0;
+        for (int t = r0 * LDC + tid; t < n1 * LDC; t += nthr)
+            if (t / LDC * a.n2 + b + t % LDC / XT >= a.valid_rows) s[t] = make_float2(0.0f, 0.0f);
+        ASARF_SYNC();
     }
-    ASARF_SYNC();
     if (!a.inverse) {
         // (writing the last stage straight to HBM, as the range-Doppler block does, measured
         // slower here: its rows scatter through the digit-reversed row map)
         if constexpr (R0 > 0)
-            fft_forward_pairs_ct3<R0, R1, R2, XT / 2, XT, true>(s, a.plan1.tw, tid, nthr);
+            fft_forward_pairs_ct3<R0, R1, R2, NPAIR, LDC, true>(s, a.plan1.tw, tid, nthr);
         else
-            fft_forward_pairs_xt<XT / 2, XT>(a.plan1, s, tid, nthr);
-        for (int t = tid; t < n1 * xt; t += nthr) {
-            const int p = row_of(t), c = t - p * xt;
-            const int x = x0 + c;
-            if (x < a.nk) a.out[static_cast<long long>(rowmap[p]) * a.pitch + x] = cmul(s[t], tw[p]);
+            fft_forward_pairs_xt<NPAIR, LDC>(a.plan1, s, tid, nthr);
+        const bool aligned = (a.pitch & 1) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
+        for (int t = tid; t < n1 * NPAIR; t += nthr) {
+            const int p = t / NPAIR, k = t % NPAIR / PAIRS;
+            const int x = x0 + 2 * (t % PAIRS);
+            if (b + k >= a.n2 || x >= a.nk) continue;
+            const float4 v = *reinterpret_cast<const float4*>(s + 2 * t);
+            const float2 w = tw[k * n1 + p];
+            const float2 u0 = cmul(make_float2(v.x, v.y), w), u1 = cmul(make_float2(v.z, v.w), w);
+            float2* dst = a.out + static_cast<long long>(rowmap[p] + k) * a.pitch + x;
+            if (aligned && x + 1 < a.nk) {
+                *reinterpret_cast<float4*>(dst) = make_float4(u0.x, u0.y, u1.x, u1.y);
+            } else {
+                dst[0] = u0;
+                if (x + 1 < a.nk) dst[1] = u1;
+            }
         }
     } else {
         // conj(twiddle) of row k1 applied as the first stage loads the row
         if constexpr (R0 > 0)
-            fft_inverse_dif_pairs_ct3<R0, R1, R2, XT / 2, XT, true>(s, a.plan1.tw, tid, nthr, tw);
+            fft_inverse_dif_pairs_ct3<R0, R1, R2, PAIRS, NPAIR, LDC, true>(s, a.plan1.tw, tid, nthr, tw);
         else
-            fft_inverse_dif_pairs_xt<XT / 2, XT>(a.plan1, s, tid, nthr, tw);
+            fft_inverse_dif_pairs_xt<PAIRS, NPAIR, LDC>(a.plan1, s, tid, nthr, tw);
         const int lo = a.state ? a.state->first_line : 0;
         const int hi = a.state ? lo + a.state->n_lines : n1 * a.n2;
-        for (int t = tid; t < n1 * xt; t += nthr) {
-            const int p = row_of(t), c = t - p * xt;
-            const int row = rowmap[p];
-            const int x = x0 + c;
-            if (x < a.nk && row >= lo && row < hi) {
-                const float2 v = s[t];
-                const float2 u = make_float2(fmul_rn(v.x, a.scale), fmul_rn(v.y, a.scale));
-                const long long o = static_cast<long long>(row - a.out_row0) * a.pitch + x;
-                if (a.out_intensity)
-                    a.out_intensity[o] = fma_rn(u.x, u.x, fmul_rn(u.y, u.y));  // the tail's |z|^2, same rounding
-                else
-                    a.out[o] = u;
+        const bool aligned = (a.pitch & 1) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 &&
+                             (reinterpret_cast<uintptr_t>(a.out_intensity) & 7) == 0;
+        for (int t = tid; t < n1 * NPAIR; t += nthr) {
+            const int p = t / NPAIR, k = t % NPAIR / PAIRS;
+            const int x = x0 + 2 * (t % PAIRS);
+            const int row = rowmap[p] + k;
+            if (b + k >= a.n2 || x >= a.nk || row < lo || row >= hi) continue;
+            const float4 v = *reinterpret_cast<const float4*>(s + 2 * t);
+            const float2 u0 = make_float2(fmul_rn(v.x, a.scale), fmul_rn(v.y, a.scale));
+            const float2 u1 = make_float2(fmul_rn(v.z, a.scale), fmul_rn(v.w, a.scale));
+            const long long o = static_cast<long long>(row - a.out_row0) * a.pitch + x;
+            if (a.out_intensity) {
+                // the tail's |z|^2, same rounding
+                const float i0 = fma_rn(u0.x, u0.x, fmul_rn(u0.y, u0.y)), i1 = fma_rn(u1.x, u1.x, fmul_rn(u1.y, u1.y));
+                if (aligned && x + 1 < a.nk) {
+                    *reinterpret_cast<float2*>(a.out_intensity + o) = make_float2(i0, i1);
+                } else {
+                    a.out_intensity[o] = i0;
+                    if (x + 1 < a.nk) a.out_intensity[o + 1] = i1;
+                }
+            } else if (aligned && x + 1 < a.nk) {
+                *reinterpret_cast<float4*>(a.out + o) = make_float4(u0.x, u0.y, u1.x, u1.y);
+            } else {
+                a.out[o] = u0;
+                if (x + 1 < a.nk) a.out[o + 1] = u1;
             }
         }
     }
 }
 
-// Shared-memory bytes of the strided pass: tile, twiddle table, row table.
-inline size_t az_strided_smem(int n1, int xt) {
-    return sizeof(float2) * static_cast<size_t>(n1) * xt + sizeof(float2) * n1 + sizeof(int) * n1;
+// Shared-memory bytes of the strided pass: tiles, twiddle tables, row table.
+inline size_t az_strided_smem(int n1, int xt, int nb) {
+    return (sizeof(float2) * static_cast<size_t>(n1) * xt + sizeof(float2) * n1) * nb + sizeof(int) * n1;
 }
 
 // ----------------------------------------------------------------------------- range-Doppler block
@@ -1391,6 +1429,11 @@ inline int az_rd_tile_width(int n2, int hl, int hr, bool absolute_phase) {
     while (xt > 16 && az_rd_smem(n2, xt + hl + hr, xt, absolute_phase) > kAzRdTwoBlockSmem) xt -= 2;
     return xt;
 }
+
+// Blocks the B200 holds at a time (two on each of 148 SMs), and the fewest that a split other than the
+// one at sqrt(N) may leave: below that a longer n2 would only idle SMs.
+constexpr int kAzRdRound = 2 * 148;
+constexpr int kAzRdMinBlocks = 3 * kAzRdRound / 2;
 
 // Epilogue of the range-Doppler block: row r of the inverse transform, column pair cp.
 struct AzRdOut {

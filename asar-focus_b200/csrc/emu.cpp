@@ -83,24 +83,33 @@ int backend_range_compress(const RangeCompressArgs& a, int lines, LaunchShape sh
 }
 
 // The same instantiation choice as the device backend (strided_schedule_compiled).
-template <int R0, int R1, int R2, int XT>
-static void emu_az_strided(const AzStridedArgs& a, int tiles, int nblocks, LaunchShape sh) {
+template <int R0, int R1, int R2, int XT, int NB>
+static void emu_az_strided(const AzStridedArgs& a, int tiles, LaunchShape sh) {
     TileBuf s(sh.smem);
-    float2* tw = s.data() + static_cast<size_t>(a.n1) * a.xt;
-    int* row = reinterpret_cast<int*>(tw + a.n1);
-    for (int b = 0; b < nblocks; ++b) {
+    float2* tw = s.data() + static_cast<size_t>(a.n1) * XT * NB;
+    int* row = reinterpret_cast<int*>(tw + a.n1 * NB);
+    for (int b = 0; b < a.n2; b += NB) {
         az_strided_tables(a, b, 0, 1, tw, row);
-        for (int t = 0; t < tiles; ++t) az_strided_body<R0, R1, R2, XT>(a, t, b, 0, 1, s.data(), tw, row, false);
+        for (int t = 0; t < tiles; ++t) az_strided_body<R0, R1, R2, XT, NB>(a, t, b, 0, 1, s.data(), tw, row, false);
     }
 }
 
-int backend_az_strided(const AzStridedArgs& a, const void*, int tiles, int nblocks, LaunchShape sh, void*) {
-    if (a.compiled && strided_schedule_compiled(a.plan1, a.xt)) {
-        if (plan_is(a.plan1, 9, 5, 5)) emu_az_strided<9, 5, 5, 32>(a, tiles, nblocks, sh);
-        else emu_az_strided<9, 4, 5, 32>(a, tiles, nblocks, sh);
+int backend_az_strided(const AzStridedArgs& a, const void*, int tiles, LaunchShape sh, void*) {
+    if (a.compiled && a.nb == 1 && strided_schedule_compiled(a.plan1, a.xt)) {
+#define ASARF_CASE(R0, R1, R2) \
+    if (plan_is(a.plan1, R0, R1, R2)) emu_az_strided<R0, R1, R2, 32, 1>(a, tiles, sh);
+        ASARF_STRIDED_SCHEDULES(ASARF_CASE)
+#undef ASARF_CASE
+    } else if (a.xt == 16) {
+        emu_az_strided<0, 0, 0, 16, 1>(a, tiles, sh);
+    } else if (a.nb == 2) {
+        emu_az_strided<0, 0, 0, 32, 2>(a, tiles, sh);
+    } else if (a.nb == 4) {
+        emu_az_strided<0, 0, 0, 32, 4>(a, tiles, sh);
+    } else if (a.nb == 8) {
+        emu_az_strided<0, 0, 0, 32, 8>(a, tiles, sh);
     } else {
-        if (a.xt == 32) emu_az_strided<0, 0, 0, 32>(a, tiles, nblocks, sh);
-        else emu_az_strided<0, 0, 0, 16>(a, tiles, nblocks, sh);
+        emu_az_strided<0, 0, 0, 32, 1>(a, tiles, sh);
     }
     return ASARF_OK;
 }
@@ -125,8 +134,10 @@ int backend_rcmc_table(float* table, void*) {
 // The same instantiation choice as the device backend (block_schedule_compiled).
 int backend_az_rd(const AzRdArgs& a, const void*, int tiles, int nblocks, LaunchShape sh, unsigned int* err, void*) {
     if (a.compiled && block_schedule_compiled(a.plan2)) {
-        if (plan_is(a.plan2, 5, 5, 5)) emu_az_rd<5, 5, 5>(a, tiles, nblocks, sh, err);
-        else emu_az_rd<8, 7, 3>(a, tiles, nblocks, sh, err);
+#define ASARF_CASE(R0, R1, R2) \
+    if (plan_is(a.plan2, R0, R1, R2)) emu_az_rd<R0, R1, R2>(a, tiles, nblocks, sh, err);
+        ASARF_BLOCK_SCHEDULES(ASARF_CASE)
+#undef ASARF_CASE
     } else {
         emu_az_rd<0, 0, 0>(a, tiles, nblocks, sh, err);
     }

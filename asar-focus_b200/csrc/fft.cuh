@@ -320,7 +320,8 @@ ASARF_HD ASARF_INLINE void dft_composite(float2* v) {
 // Any radix the schedules use: the direct small DFTs, or a composite of two of them.
 template <int R, bool INV>
 ASARF_HD ASARF_INLINE void dft_any(float2* v) {
-    if constexpr (R == 9) dft_composite<3, 3, INV>(v);
+    if constexpr (R == 6) dft_composite<3, 2, INV>(v);
+    else if constexpr (R == 9) dft_composite<3, 3, INV>(v);
     else if constexpr (R == 12) dft_composite<4, 3, INV>(v);
     else if constexpr (R == 16) dft_composite<4, 4, INV>(v);
     else if constexpr (R == 24) dft_composite<8, 3, INV>(v);
@@ -490,8 +491,9 @@ ASARF_HD ASARF_INLINE void pair_item(float2* s, int b, int j, int cp, int M, int
     }
 }
 
-// Run-time length n and span S over NPAIR column pairs of row stride LDC.
-template <int R, bool INV, bool TW_FIRST, int NPAIR, int LDC, bool PRE, bool PTW>
+// Run-time length n and span S over NPAIR column pairs of row stride LDC.  PRE > 0: a table pre of n
+// rows for every PRE column pairs.
+template <int R, bool INV, bool TW_FIRST, int NPAIR, int LDC, int PRE, bool PTW>
 ASARF_HD ASARF_INLINE void fft_stage_pair(float2* s, int n, int S, const FastDiv& sdiv, const float2* __restrict__ tw,
                                           int tid, int nthr, const float2* pre = nullptr) {
     const int M = S * R;
@@ -502,16 +504,16 @@ ASARF_HD ASARF_INLINE void fft_stage_pair(float2* s, int n, int S, const FastDiv
         const int cp = t - bj * NPAIR;
         const int b = static_cast<int>(fdiv_u(static_cast<unsigned int>(bj), sdiv));
         const int j = bj - b * S;
-        pair_item<R, INV, TW_FIRST, PRE, NoEpi, PTW>(s, b, j, cp, M, S, LDC, tw_step, tw, pre, NoEpi());
+        pair_item<R, INV, TW_FIRST, (PRE > 0), NoEpi, PTW>(s, b, j, cp, M, S, LDC, tw_step, tw,
+                                                           PRE > 0 ? pre + cp / (PRE > 0 ? PRE : 1) * n : nullptr, NoEpi());
     }
 }
 
 // The same stage with every size a compile-time constant (length N, span S, NPAIR column pairs
 // of row stride LDC): the index arithmetic folds into constant multiplies and shifts.
-template <int R, bool INV, bool TW_FIRST, int N, int S, int NPAIR, int LDC, bool PRE = false, class Epi = NoEpi,
-          bool PTW = false>
+template <int R, bool INV, bool TW_FIRST, int N, int S, int NPAIR, int LDC, int PRE, bool PTW>
 ASARF_HD ASARF_INLINE void fft_stage_pair_ct(float2* s, const float2* __restrict__ tw, int tid, int nthr,
-                                             const float2* pre = nullptr, const Epi& epi = Epi()) {
+                                             const float2* pre = nullptr) {
     constexpr int M = S * R;
     constexpr int ITEMS = (N / R) * NPAIR;
     constexpr int TW_STEP = N / M;
@@ -520,7 +522,8 @@ ASARF_HD ASARF_INLINE void fft_stage_pair_ct(float2* s, const float2* __restrict
         const int cp = t - bj * NPAIR;
         const int b = bj / S;
         const int j = bj - b * S;
-        pair_item<R, INV, TW_FIRST, PRE, Epi, PTW>(s, b, j, cp, M, S, LDC, TW_STEP, tw, pre, epi);
+        pair_item<R, INV, TW_FIRST, (PRE > 0), NoEpi, PTW>(s, b, j, cp, M, S, LDC, TW_STEP, tw,
+                                                           PRE > 0 ? pre + cp / (PRE > 0 ? PRE : 1) * N : nullptr, NoEpi());
     }
 }
 
@@ -578,6 +581,7 @@ ASARF_HD ASARF_INLINE void fft_stage_pair_w_dispatch(int R, float2* s, int n, in
         case 3: ASARF_PAIR(3); break;
         case 4: ASARF_PAIR(4); break;
         case 5: ASARF_PAIR(5); break;
+        case 6: ASARF_PAIR(6); break;
         case 7: ASARF_PAIR(7); break;
         default: ASARF_PAIR(8); break;
     }
@@ -592,7 +596,7 @@ ASARF_HD ASARF_INLINE void fft_stage_pair_w_dispatch(int R, float2* s, int n, in
 // factors 3 * 3; it is compiled only where such plans run, since every extra case costs the
 // other kernels registers.  PTW selects the packed twiddle products: the strided kernel uses them,
 // the range-Doppler block for radix <= 5 schedules only (az_rd_packed_twiddles).
-template <bool INV, bool TW_FIRST, int NPAIR, int LDC, bool PRE>
+template <bool INV, bool TW_FIRST, int NPAIR, int LDC, int PRE>
 ASARF_HD ASARF_INLINE void fft_stage_pair_dispatch(int R, float2* s, int n, int S, const FastDiv& sdiv,
                                                    const float2* __restrict__ tw, int tid, int nthr,
                                                    const float2* pre = nullptr) {
@@ -602,6 +606,7 @@ ASARF_HD ASARF_INLINE void fft_stage_pair_dispatch(int R, float2* s, int n, int 
         case 3: ASARF_PAIR(3); break;
         case 4: ASARF_PAIR(4); break;
         case 5: ASARF_PAIR(5); break;
+        case 6: ASARF_PAIR(6); break;
         case 7: ASARF_PAIR(7); break;
         case 9: ASARF_PAIR(9); break;
         default: ASARF_PAIR(8); break;
@@ -635,20 +640,21 @@ ASARF_HD ASARF_INLINE void fft_inverse_pairs(const FftPlan& p, float2* s, int nc
 }
 
 // Forward DIF, and inverse in DIF form whose input row l is first multiplied by conj(pre[l]) (folded
-// into stage 0), of the strided azimuth pass: NPAIR column pairs of row stride LDC.
+// into stage 0; a table for every PRE column pairs), of the strided azimuth pass: NPAIR column
+// pairs of row stride LDC.
 template <int NPAIR, int LDC>
 ASARF_HD ASARF_INLINE void fft_forward_pairs_xt(const FftPlan& p, float2* s, int tid, int nthr) {
     for (int i = 0; i < p.nst; ++i) {
-        fft_stage_pair_dispatch<false, false, NPAIR, LDC, false>(p.radix[i], s, p.n, p.span[i], p.sdiv[i], p.tw, tid, nthr);
+        fft_stage_pair_dispatch<false, false, NPAIR, LDC, 0>(p.radix[i], s, p.n, p.span[i], p.sdiv[i], p.tw, tid, nthr);
         ASARF_SYNC();
     }
 }
-template <int NPAIR, int LDC>
+template <int PRE, int NPAIR, int LDC>
 ASARF_HD ASARF_INLINE void fft_inverse_dif_pairs_xt(const FftPlan& p, float2* s, int tid, int nthr, const float2* pre) {
-    fft_stage_pair_dispatch<true, false, NPAIR, LDC, true>(p.radix[0], s, p.n, p.span[0], p.sdiv[0], p.tw, tid, nthr, pre);
+    fft_stage_pair_dispatch<true, false, NPAIR, LDC, PRE>(p.radix[0], s, p.n, p.span[0], p.sdiv[0], p.tw, tid, nthr, pre);
     ASARF_SYNC();
     for (int i = 1; i < p.nst; ++i) {
-        fft_stage_pair_dispatch<true, false, NPAIR, LDC, false>(p.radix[i], s, p.n, p.span[i], p.sdiv[i], p.tw, tid, nthr);
+        fft_stage_pair_dispatch<true, false, NPAIR, LDC, 0>(p.radix[i], s, p.n, p.span[i], p.sdiv[i], p.tw, tid, nthr);
         ASARF_SYNC();
     }
 }
@@ -660,23 +666,23 @@ ASARF_HD ASARF_INLINE void fft_inverse_dif_pairs_xt(const FftPlan& p, float2* s,
 template <int R0, int R1, int R2, int NPAIR, int LDC, bool PTW>
 ASARF_HD ASARF_INLINE void fft_forward_pairs_ct3(float2* s, const float2* __restrict__ tw, int tid, int nthr) {
     constexpr int N = R0 * R1 * R2;
-    fft_stage_pair_ct<R0, false, false, N, N / R0, NPAIR, LDC, false, NoEpi, PTW>(s, tw, tid, nthr);
+    fft_stage_pair_ct<R0, false, false, N, N / R0, NPAIR, LDC, 0, PTW>(s, tw, tid, nthr);
     ASARF_SYNC();
-    fft_stage_pair_ct<R1, false, false, N, N / (R0 * R1), NPAIR, LDC, false, NoEpi, PTW>(s, tw, tid, nthr);
+    fft_stage_pair_ct<R1, false, false, N, N / (R0 * R1), NPAIR, LDC, 0, PTW>(s, tw, tid, nthr);
     ASARF_SYNC();
-    fft_stage_pair_ct<R2, false, false, N, 1, NPAIR, LDC, false, NoEpi, PTW>(s, tw, tid, nthr);
+    fft_stage_pair_ct<R2, false, false, N, 1, NPAIR, LDC, 0, PTW>(s, tw, tid, nthr);
     ASARF_SYNC();
 }
 
-template <int R0, int R1, int R2, int NPAIR, int LDC, bool PTW>
+template <int R0, int R1, int R2, int PRE, int NPAIR, int LDC, bool PTW>
 ASARF_HD ASARF_INLINE void fft_inverse_dif_pairs_ct3(float2* s, const float2* __restrict__ tw, int tid, int nthr,
                                                      const float2* pre) {
     constexpr int N = R0 * R1 * R2;
-    fft_stage_pair_ct<R0, true, false, N, N / R0, NPAIR, LDC, true, NoEpi, PTW>(s, tw, tid, nthr, pre);
+    fft_stage_pair_ct<R0, true, false, N, N / R0, NPAIR, LDC, PRE, PTW>(s, tw, tid, nthr, pre);
     ASARF_SYNC();
-    fft_stage_pair_ct<R1, true, false, N, N / (R0 * R1), NPAIR, LDC, false, NoEpi, PTW>(s, tw, tid, nthr);
+    fft_stage_pair_ct<R1, true, false, N, N / (R0 * R1), NPAIR, LDC, 0, PTW>(s, tw, tid, nthr);
     ASARF_SYNC();
-    fft_stage_pair_ct<R2, true, false, N, 1, NPAIR, LDC, false, NoEpi, PTW>(s, tw, tid, nthr);
+    fft_stage_pair_ct<R2, true, false, N, 1, NPAIR, LDC, 0, PTW>(s, tw, tid, nthr);
     ASARF_SYNC();
 }
 

@@ -363,8 +363,27 @@ int32_t fft_size_above(int32_t v) {
 
 bool build_fft(int n, HostFft& h) { return build_fft_radices(n, factorize(n), h); }
 
+// The two or three factors of at most `most`, largest first, with the fewest factors, then the smallest
+// sum; empty when n has none.
+static std::vector<int> few_radices(int n, int most) {
+    for (int a = 2; a <= most; ++a)  // smallest sum first: the factors nearest to each other
+        if (n % a == 0 && n / a <= a && n / a >= 2) return {a, n / a};
+    std::vector<int> best;
+    int best_sum = 1 << 30;
+    for (int a = 2; a <= most; ++a)
+        for (int b = 2; b <= a; ++b) {
+            if (n % (a * b) != 0) continue;
+            const int c = n / (a * b);
+            if (c <= b && c >= 2 && a + b + c < best_sum) best_sum = a + b + c, best = {a, b, c};
+        }
+    return best;
+}
+
 std::vector<int> strided_radices(int n) {
-    // the default factors with each pair of 3s merged into a 9 (first, so that the short
+    if (n == 180) return {9, 4, 5};  // the compiled schedule
+    std::vector<int> best = few_radices(n, 9);
+    if (!best.empty()) return best;
+    // longer: the default factors with each pair of 3s merged into a 9 (first, so that the short
     // radices run on the shortest spans)
     std::vector<int> rest, out;
     int threes = 0;
@@ -378,6 +397,47 @@ std::vector<int> strided_radices(int n) {
     out.insert(out.end(), rest.begin(), rest.end());
     if (threes & 1) out.push_back(3);
     return out;
+}
+
+std::vector<int> block_radices(int n) {
+    if (n == 168) return {8, 7, 3};
+    const std::vector<int> best = few_radices(n, 8);
+    return best.empty() ? factorize(n) : best;
+}
+
+static int largest_divisor_to_root(int N) {
+    int best = 1;
+    for (int d = 1; static_cast<long long>(d) * d <= N; ++d)
+        if (N % d == 0) best = d;
+    return best;
+}
+
+// The strided pass costs about the same whatever n1 (az_strided_tiles_per_block), so n2 is the divisor
+// with the least time in range-Doppler blocks: a block's time, in us as fitted to blocks of 49 to
+// 175 rows (6.5 + 0.142 n2; radices up to 5 run 7 % faster, run-time schedules 10 % slower, a fourth
+// stage costs 6), times the rounds of the 296 resident blocks.  Longer blocks win until their tile
+// loses columns (n2 > 168).  5616 x 4999: n2 = 50, the divisor at sqrt(N), 400 us in the block, n2 =
+// 125 248 us.
+int choose_az_n2(int N, int nk, int hl, int hr, bool absolute_phase) {
+    const int root = largest_divisor_to_root(N);
+    int best = root;
+    double best_cost = 1e300;
+    for (int d = 48; d <= 256 && d < N; ++d) {
+        if (N % d != 0 || N / d > 640) continue;
+        const int xt = az_rd_tile_width(d, hl, hr, absolute_phase);
+        const double blocks = static_cast<double>((nk + xt - 1) / xt) * (N / d);
+        if (blocks < kAzRdMinBlocks) continue;
+        const std::vector<int> radices = block_radices(d);
+        HostFft f;
+        if (!build_fft_radices(d, radices, f)) continue;
+        double t = 6.5 + 0.142 * d + 6.0 * std::max(0, f.plan.nst - 3);
+        if (*std::max_element(radices.begin(), radices.end()) <= 5) t *= 0.93;
+        if (!block_schedule_compiled(f.plan)) t *= 1.1;
+        const double rounds = blocks / kAzRdRound;
+        const double cost = t * (rounds < 4.0 ? std::ceil(rounds) : rounds + 0.5);
+        if (cost < best_cost) best_cost = cost, best = d;
+    }
+    return best;
 }
 
 bool build_fft_radices(int n, const std::vector<int>& f, HostFft& h) {
@@ -589,44 +649,11 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
         delete p;
         return set_error(ASARF_ERR_INVALID, "range FFT length %d must be >= range_size and 2^a3^b5^c7^d", p->rc_len);
     }
-    // azimuth split N = n1 * n2, n2 = largest divisor <= sqrt(N) unless the caller names one
-    {
-        const int N = p->az_pad;
-        int best = 1;
-        for (int d = 1; static_cast<long long>(d) * d <= N; ++d)
-            if (N % d == 0) best = d;
-        if (opt.az_n2 > 0) {
-            if (N % opt.az_n2 != 0 || opt.az_n2 < 16 || opt.az_n2 > 256) {
-                delete p;
-                return set_error(ASARF_ERR_INVALID, "az_n2 %d must divide the azimuth FFT size %d and lie in [16, 256]",
-                                 opt.az_n2, N);
-            }
-            best = opt.az_n2;
-        }
-        p->n2 = best;
-        p->n1 = N / best;
-        if (p->n2 < 2) {
-            delete p;
-            return set_error(ASARF_ERR_INVALID, "azimuth FFT size %d cannot be split", N);
-        }
-    }
     // compile-time lengths use their own three-pass radix sequence (and so its output order)
     int ctr[3];
     const int n_ctr = ct_radices(p->rc_len, ctr);
     const bool rc_ok = n_ctr ? build_fft_radices(p->rc_len, std::vector<int>(ctr, ctr + n_ctr), p->rc)
                              : build_fft(p->rc_len, p->rc);
-    // the split-precision form takes the contiguous transform's last radix as its FP32 pass, so
-    // that pass gets the largest radix (smallest tensor-core DFT)
-    std::vector<int> f2_radices = factorize(p->n2);
-    if (opt.precision == ASARF_PRECISION_SPLIT && !f2_radices.empty()) {
-        auto big = std::max_element(f2_radices.begin(), f2_radices.end());
-        std::rotate(big, big + 1, f2_radices.end());
-    }
-    if (!rc_ok || !build_fft_radices(p->n1, strided_radices(p->n1), p->f1) ||
-        !build_fft_radices(p->n2, f2_radices, p->f2) || !build_fft(p->az_pad, p->fN)) {
-        delete p;
-        return set_error(ASARF_ERR_INVALID, "FFT schedule failed");
-    }
     // Vr polynomial
     if (s.vr_poly_given) {
         for (int k = 0; k < 3; ++k) p->vr_poly[k] = s.vr_poly[k];
@@ -649,6 +676,40 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
         p->hl = kRcmcTaps / 2;
         p->hr = rcmc_right_halo(walk);
         if ((p->hl + p->hr) & 1) ++p->hr;  // even tile width: TMA rows are whole 16-byte units
+    }
+    // azimuth split N = n1 * n2: choose_az_n2 unless the caller names one (the split-precision form,
+    // whose tensor-core part bounds n2, takes the largest divisor <= sqrt(N))
+    {
+        const int N = p->az_pad;
+        int best = opt.precision == ASARF_PRECISION_SPLIT
+                       ? largest_divisor_to_root(N)
+                       : choose_az_n2(N, p->nk, p->hl, p->hr, opt.absolute_phase != 0);
+        if (opt.az_n2 > 0) {
+            if (N % opt.az_n2 != 0 || opt.az_n2 < 16 || opt.az_n2 > 256) {
+                delete p;
+                return set_error(ASARF_ERR_INVALID, "az_n2 %d must divide the azimuth FFT size %d and lie in [16, 256]",
+                                 opt.az_n2, N);
+            }
+            best = opt.az_n2;
+        }
+        p->n2 = best;
+        p->n1 = N / best;
+        if (p->n2 < 2) {
+            delete p;
+            return set_error(ASARF_ERR_INVALID, "azimuth FFT size %d cannot be split", N);
+        }
+    }
+    // the split-precision form takes the contiguous transform's last radix as its FP32 pass, so
+    // that pass gets the largest radix (smallest tensor-core DFT)
+    std::vector<int> f2_radices = opt.precision == ASARF_PRECISION_SPLIT ? factorize(p->n2) : block_radices(p->n2);
+    if (opt.precision == ASARF_PRECISION_SPLIT && !f2_radices.empty()) {
+        auto big = std::max_element(f2_radices.begin(), f2_radices.end());
+        std::rotate(big, big + 1, f2_radices.end());
+    }
+    if (!rc_ok || !build_fft_radices(p->n1, strided_radices(p->n1), p->f1) ||
+        !build_fft_radices(p->n2, f2_radices, p->f2) || !build_fft(p->az_pad, p->fN)) {
+        delete p;
+        return set_error(ASARF_ERR_INVALID, "FFT schedule failed");
     }
     p->pitch = (p->nk + 31) / 32 * 32;
     p->xt1 = (p->n1 * 32 * 8 <= 160 * 1024) ? 32 : 16;
@@ -931,7 +992,8 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     p->a_inv.scale = 1.0f / static_cast<float>(p->az_pad);
     p->a_inv.inverse = 1;
     p->tiles1 = (p->nk + p->xt1 - 1) / p->xt1;
-    p->sh_st = {256, az_strided_smem(p->n1, p->xt1)};
+    p->a_fwd.nb = p->a_inv.nb = p->xt1 == 32 ? az_strided_tiles_per_block(p->n1, p->n2, p->tiles1) : 1;
+    p->sh_st = {256, az_strided_smem(p->n1, p->xt1, p->a_fwd.nb)};
 
     AzRdArgs& d = p->a_rd;
     d.in = p->bufA;
@@ -1021,7 +1083,8 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
         const unsigned long long d3[3] = {2ull * p->nk, static_cast<unsigned long long>(p->n2),
                                           static_cast<unsigned long long>(p->n1)};
         const unsigned long long s3[2] = {row_bytes, row_bytes * p->n2};
-        const unsigned int b3[3] = {static_cast<unsigned int>(2 * p->xt1), 1u, static_cast<unsigned int>(n1_box)};
+        const unsigned int b3[3] = {static_cast<unsigned int>(2 * p->xt1), static_cast<unsigned int>(p->a_fwd.nb),
+                                    static_cast<unsigned int>(n1_box)};
         const unsigned long long d2[2] = {2ull * p->nk, static_cast<unsigned long long>(p->az_pad)};
         const unsigned long long s2[1] = {row_bytes};
         const unsigned int b2[2] = {static_cast<unsigned int>(2 * d.wt), static_cast<unsigned int>(n2_box)};
@@ -1097,7 +1160,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     dm.split_m = p->split ? p->a_split.m : 0;
     dm.az_tile_width = p->xt2;
     dm.strided_tile_width = p->xt1;
-    dm.compiled_schedules = (p->a_fwd.compiled && strided_schedule_compiled(p->a_fwd.plan1, p->a_fwd.xt) ? 1 : 0) |
+    dm.compiled_schedules = (p->a_fwd.compiled && p->a_fwd.nb == 1 && strided_schedule_compiled(p->a_fwd.plan1, p->a_fwd.xt) ? 1 : 0) |
                             (p->a_rd.compiled && block_schedule_compiled(p->a_rd.plan2) ? 2 : 0);
     *out = p;
     return ASARF_OK;
@@ -1163,7 +1226,7 @@ int asarf_focus(asarf_plan* p, const uint8_t* d_raw, const uint16_t* d_swst, int
     rc = backend_range_compress(r, p->na, p->sh_rc, stream);
     if (rc) return rc;
     mark();
-    rc = backend_az_strided(p->a_fwd, p->use_tma ? p->tmapA3 : nullptr, p->tiles1, p->n2, p->sh_st, stream);
+    rc = backend_az_strided(p->a_fwd, p->use_tma ? p->tmapA3 : nullptr, p->tiles1, p->sh_st, stream);
     if (rc) return rc;
     mark();
     rc = p->split ? backend_az_rd_split(p->a_rd, p->a_split, p->tmapA2, p->tiles2, p->n1, p->sh_rd_split,
@@ -1172,7 +1235,7 @@ int asarf_focus(asarf_plan* p, const uint8_t* d_raw, const uint16_t* d_swst, int
                                   &p->state->errors, stream);
     if (rc) return rc;
     mark();
-    rc = backend_az_strided(p->a_inv, p->use_tma ? p->tmapB3 : nullptr, p->tiles1, p->n2, p->sh_st, stream);
+    rc = backend_az_strided(p->a_inv, p->use_tma ? p->tmapB3 : nullptr, p->tiles1, p->sh_st, stream);
     if (rc) return rc;
     mark();
     if (!p->skip_tail && p->opt.product == ASARF_PRODUCT_IMS_MDS) {

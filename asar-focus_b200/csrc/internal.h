@@ -28,6 +28,11 @@ bool build_fft(int n, HostFft& h);
 bool build_fft_radices(int n, const std::vector<int>& radices, HostFft& h);
 // radices of the strided azimuth pass: pairs of 3s merged into radix 9
 std::vector<int> strided_radices(int n);
+// radices of the contiguous azimuth pass: three of at most 8 when n allows, largest first
+std::vector<int> block_radices(int n);
+// Contiguous length n2 of the azimuth split N = n1 * n2 for nk columns (halo hl, hr of the
+// range-Doppler tile).
+int choose_az_n2(int N, int nk, int hl, int hr, bool absolute_phase);
 int choose_rc_len(int nr);
 int32_t fft_size_above(int32_t v);
 void matched_filter_table(const std::complex<float>* chirp, int nc, const HostFft& fft, std::vector<float2>& mf);

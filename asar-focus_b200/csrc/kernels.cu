@@ -215,26 +215,27 @@ __global__ void __launch_bounds__(CtSchedule<L>::nthr, 2) k_range_compress_ct(Ra
     range_compress_ct_body<L, FMT>(a, blockIdx.x, threadIdx.x, s, line);
 }
 
-// Strided azimuth pass: the [n1][xt] tile (rows r*n2 + b) arrives by 3-D TMA boxes.
-// R0..R2 > 0: compile-time transform schedule; XT: tile width (az_strided_body).
-template <int R0, int R1, int R2, int XT>
-__global__ void __launch_bounds__(512) k_az_strided(AzStridedArgs a, const __grid_constant__ CUtensorMap map) {
+// Strided azimuth pass: the [n1][NB][XT] tiles (rows r*n2 + b + k) arrive by 3-D TMA boxes.
+// R0..R2 > 0: compile-time transform schedule (az_strided_body).
+template <int R0, int R1, int R2, int XT, int NB>
+__global__ void __launch_bounds__(256, 3) k_az_strided(AzStridedArgs a, const __grid_constant__ CUtensorMap map) {
     extern __shared__ __align__(128) unsigned char smem_as_raw[];
     float2* s = reinterpret_cast<float2*>(smem_as_raw);
-    float2* tw = s + static_cast<size_t>(a.n1) * a.xt;
-    int* row = reinterpret_cast<int*>(tw + a.n1);
+    float2* tw = s + static_cast<size_t>(a.n1) * XT * NB;
+    int* row = reinterpret_cast<int*>(tw + a.n1 * NB);
     __shared__ uint64_t bar;
+    const int b = blockIdx.y * NB;
     if (a.use_tma && threadIdx.x == 0) {
         mbar_init(&bar, 1);
-        mbar_expect_tx(&bar, static_cast<uint32_t>(sizeof(float2) * a.n1 * a.xt));
+        mbar_expect_tx(&bar, static_cast<uint32_t>(sizeof(float2) * a.n1 * XT * NB));
         for (int r0 = 0; r0 < a.n1; r0 += a.n1_box)
-            tma_load_3d(s + static_cast<size_t>(r0) * a.xt, &map, &bar, 2 * blockIdx.x * a.xt, blockIdx.y, r0);
+            tma_load_3d(s + static_cast<size_t>(r0) * XT * NB, &map, &bar, 2 * blockIdx.x * XT, b, r0);
     }
     // twiddle and row tables are gathered while the tile is in flight
-    az_strided_tables(a, blockIdx.y, threadIdx.x, blockDim.x, tw, row);
+    az_strided_tables(a, b, threadIdx.x, blockDim.x, tw, row);
     __syncthreads();
     if (a.use_tma) mbar_wait(&bar, 0, a.state ? &const_cast<FocusState*>(a.state)->errors : nullptr);
-    az_strided_body<R0, R1, R2, XT>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, s, tw, row, a.use_tma != 0);
+    az_strided_body<R0, R1, R2, XT, NB>(a, blockIdx.x, b, threadIdx.x, blockDim.x, s, tw, row, a.use_tma != 0);
 }
 
 // Range-Doppler block: the [n2][wt] tile (contiguous rows, range halo) arrives by 2-D TMA
@@ -551,23 +552,28 @@ static CUtensorMap tmap_or_zero(const void* tmap) {
     return m;
 }
 
-template <int R0, int R1, int R2, int XT>
-static int launch_az_strided(const AzStridedArgs& a, const void* tmap, int tiles, int nblocks, LaunchShape sh,
-                             void* stream) {
-    int rc = ensure_smem(k_az_strided<R0, R1, R2, XT>, sh.smem, "az_strided");
+template <int R0, int R1, int R2, int XT, int NB>
+static int launch_az_strided(const AzStridedArgs& a, const void* tmap, int tiles, LaunchShape sh, void* stream) {
+    int rc = ensure_smem(k_az_strided<R0, R1, R2, XT, NB>, sh.smem, "az_strided");
     if (rc) return rc;
-    k_az_strided<R0, R1, R2, XT><<<dim3(tiles, nblocks), sh.threads, sh.smem, S(stream)>>>(a, tmap_or_zero(tmap));
+    k_az_strided<R0, R1, R2, XT, NB><<<dim3(tiles, (a.n2 + NB - 1) / NB), sh.threads, sh.smem, S(stream)>>>(
+        a, tmap_or_zero(tmap));
     return check_launch("az_strided");
 }
 
 // The compiled schedules (strided_schedule_compiled) when the plan allows them.
-int backend_az_strided(const AzStridedArgs& a, const void* tmap, int tiles, int nblocks, LaunchShape sh, void* stream) {
-    if (a.compiled && strided_schedule_compiled(a.plan1, a.xt)) {
-        if (plan_is(a.plan1, 9, 5, 5)) return launch_az_strided<9, 5, 5, 32>(a, tmap, tiles, nblocks, sh, stream);
-        return launch_az_strided<9, 4, 5, 32>(a, tmap, tiles, nblocks, sh, stream);
+int backend_az_strided(const AzStridedArgs& a, const void* tmap, int tiles, LaunchShape sh, void* stream) {
+    if (a.compiled && a.nb == 1 && strided_schedule_compiled(a.plan1, a.xt)) {
+#define ASARF_CASE(R0, R1, R2) \
+    if (plan_is(a.plan1, R0, R1, R2)) return launch_az_strided<R0, R1, R2, 32, 1>(a, tmap, tiles, sh, stream);
+        ASARF_STRIDED_SCHEDULES(ASARF_CASE)
+#undef ASARF_CASE
     }
-    if (a.xt == 32) return launch_az_strided<0, 0, 0, 32>(a, tmap, tiles, nblocks, sh, stream);
-    return launch_az_strided<0, 0, 0, 16>(a, tmap, tiles, nblocks, sh, stream);
+    if (a.xt == 16) return launch_az_strided<0, 0, 0, 16, 1>(a, tmap, tiles, sh, stream);
+    if (a.nb == 2) return launch_az_strided<0, 0, 0, 32, 2>(a, tmap, tiles, sh, stream);
+    if (a.nb == 4) return launch_az_strided<0, 0, 0, 32, 4>(a, tmap, tiles, sh, stream);
+    if (a.nb == 8) return launch_az_strided<0, 0, 0, 32, 8>(a, tmap, tiles, sh, stream);
+    return launch_az_strided<0, 0, 0, 32, 1>(a, tmap, tiles, sh, stream);
 }
 
 template <int R0, int R1, int R2>
@@ -583,8 +589,10 @@ static int launch_az_rd(const AzRdArgs& a, const void* tmap, int tiles, int nblo
 int backend_az_rd(const AzRdArgs& a, const void* tmap, int tiles, int nblocks, LaunchShape sh, unsigned int* err,
                   void* stream) {
     if (a.compiled && block_schedule_compiled(a.plan2)) {
-        if (plan_is(a.plan2, 5, 5, 5)) return launch_az_rd<5, 5, 5>(a, tmap, tiles, nblocks, sh, err, stream);
-        return launch_az_rd<8, 7, 3>(a, tmap, tiles, nblocks, sh, err, stream);
+#define ASARF_CASE(R0, R1, R2) \
+    if (plan_is(a.plan2, R0, R1, R2)) return launch_az_rd<R0, R1, R2>(a, tmap, tiles, nblocks, sh, err, stream);
+        ASARF_BLOCK_SCHEDULES(ASARF_CASE)
+#undef ASARF_CASE
     }
     return launch_az_rd<0, 0, 0>(a, tmap, tiles, nblocks, sh, err, stream);
 }

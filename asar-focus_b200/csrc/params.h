@@ -127,17 +127,27 @@ struct RangeCompressArgs {
     const float* lut_q;
 };
 
-// Transform schedules with compile-time instantiations of the azimuth kernels (the strided
-// lengths 225 = 9 x 5 x 5 and 180 = 9 x 4 x 5 at the 32-column tile, the block lengths
-// 125 = 5 x 5 x 5 and 168 = 8 x 7 x 3 of the ERS-like and ASAR IM-like scenes); every other
-// schedule runs the run-time loops, with the same arithmetic.
+// Transform schedules with compile-time instantiations of the azimuth kernels; every other
+// schedule runs the run-time loops, with the same arithmetic (block lengths take 10 % longer there,
+// strided ones 9 to 25 %).  ASARF_BLOCK_SCHEDULES: block lengths n2 of choose_az_n2, between them a
+// divisor of nearly every azimuth length above 1500; ASARF_STRIDED_SCHEDULES: strided lengths n1
+// at the 32-column tile.
+#define ASARF_BLOCK_SCHEDULES(X)                                                                      \
+    X(5, 5, 5) X(8, 7, 3) X(7, 7, 2) X(5, 5, 4) X(7, 5, 3) X(6, 6, 3) X(7, 4, 4) X(6, 5, 4) X(7, 6, 3) \
+    X(8, 4, 4) X(7, 5, 4) X(6, 6, 4) X(7, 7, 3) X(6, 5, 5) X(8, 5, 4) X(7, 5, 5)
+#define ASARF_STRIDED_SCHEDULES(X) X(9, 5, 5) X(9, 4, 5)
+
 ASARF_HD inline bool plan_is(const FftPlan& p, int r0, int r1, int r2) {
     return p.nst == 3 && p.radix[0] == r0 && p.radix[1] == r1 && p.radix[2] == r2;
 }
 ASARF_HD inline bool strided_schedule_compiled(const FftPlan& p, int xt) {
-    return xt == 32 && (plan_is(p, 9, 5, 5) || plan_is(p, 9, 4, 5));
+#define ASARF_IS(R0, R1, R2) || plan_is(p, R0, R1, R2)
+    return xt == 32 && (false ASARF_STRIDED_SCHEDULES(ASARF_IS));
 }
-ASARF_HD inline bool block_schedule_compiled(const FftPlan& p) { return plan_is(p, 5, 5, 5) || plan_is(p, 8, 7, 3); }
+ASARF_HD inline bool block_schedule_compiled(const FftPlan& p) {
+    return false ASARF_BLOCK_SCHEDULES(ASARF_IS);
+#undef ASARF_IS
+}
 
 struct AzStridedArgs {
     const float2* in;
@@ -148,7 +158,8 @@ struct AzStridedArgs {
     const int* drev1;
     const float2* twn;    // exp(-2 pi i m / N), N = n1 * n2
     int nk;
-    int xt;               // columns per block
+    int xt;               // columns per tile
+    int nb;               // adjacent b (tiles side by side) per block: 1, 2, 4 or 8
     int valid_rows;       // forward: rows at or beyond this are zero
     const FocusState* state;  // inverse: rows outside the results window are not stored
     float scale;          // inverse: 1 / N as the reference multiplies

@@ -282,12 +282,23 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     if (!prm || !d_src || !d_out || x_size < 17 || y_size <= 1 || x_stride < x_size || y_stride < y_size)
         return set_error(ASARF_ERR_INVALID, "range_doppler: bad arguments");
     const int N = y_stride;
-    int n2 = 1;
-    for (int d = 1; static_cast<long long>(d) * d <= N; ++d)
-        if (N % d == 0) n2 = d;
+    // RCMC halo from the largest walk at |f| <= PRF
+    double vr_min = 1e30;
+    for (int x = 0; x < x_size; x += std::max(1, x_size / 64)) {
+        const double v = (prm->vr_poly[0] * x + prm->vr_poly[1]) * x + prm->vr_poly[2];
+        vr_min = std::min(vr_min, std::fabs(v));
+    }
+    const double rmax = prm->slant_range_first + x_size * prm->range_spacing;
+    const double walk =
+        prm->wavelength * prm->wavelength * prm->prf * prm->prf * rmax / (8 * vr_min * vr_min) / prm->range_spacing;
+    const int hl = kRcmcTaps / 2;
+    int hr = rcmc_right_halo(walk);
+    if ((hl + hr) & 1) ++hr;  // column-pair transforms need an even tile width
+    const int n2 = choose_az_n2(N, x_size, hl, hr, false);
     const int n1 = N / n2;
     HostFft f1, f2, fN;
-    if (n2 < 2 || !build_fft_radices(n1, strided_radices(n1), f1) || !build_fft(n2, f2) || !build_fft(N, fN))
+    if (n2 < 2 || !build_fft_radices(n1, strided_radices(n1), f1) || !build_fft_radices(n2, block_radices(n2), f2) ||
+        !build_fft(N, fN))
         return set_error(ASARF_ERR_INVALID, "range_doppler: azimuth size %d is not 2^a3^b5^c7^d", N);
     // tables + a finalised state carrying the Doppler polynomial
     DevBuf tw1(sizeof(float2) * n1), dr1(sizeof(int) * n1), tw2(sizeof(float2) * n2), dr2(sizeof(int) * n2),
@@ -336,15 +347,6 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     inv.valid_rows = N;
     inv.scale = 1.0f / static_cast<float>(N);
     inv.inverse = 1;
-    // RCMC halo from the largest walk at |f| <= PRF
-    double vr_min = 1e30;
-    for (int x = 0; x < x_size; x += std::max(1, x_size / 64)) {
-        const double v = (prm->vr_poly[0] * x + prm->vr_poly[1]) * x + prm->vr_poly[2];
-        vr_min = std::min(vr_min, std::fabs(v));
-    }
-    const double rmax = prm->slant_range_first + x_size * prm->range_spacing;
-    const double walk =
-        prm->wavelength * prm->wavelength * prm->prf * prm->prf * rmax / (8 * vr_min * vr_min) / prm->range_spacing;
     AzRdArgs d{};
     d.in = src;
     d.out = out;
@@ -355,9 +357,8 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     d.plan2 = f2.plan;
     d.drev2 = dr2.as<int>();
     d.nk = x_size;
-    d.hl = kRcmcTaps / 2;
-    d.hr = rcmc_right_halo(walk);
-    if ((d.hl + d.hr) & 1) ++d.hr;  // column-pair transforms need an even tile width
+    d.hl = hl;
+    d.hr = hr;
     d.xt = az_rd_tile_width(n2, d.hl, d.hr, false);
     d.wt = d.xt + d.hl + d.hr;
     d.prf = static_cast<float>(prm->prf);
@@ -370,14 +371,15 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     for (int k = 0; k < 3; ++k) d.vr_poly[k] = static_cast<float>(prm->vr_poly[k]);
     d.state = dstate;
     d.rcmc = rcmc.as<float>();
-    const LaunchShape sh_st{256, az_strided_smem(n1, xt1)};
+    const int tiles1 = (x_size + xt1 - 1) / xt1, tiles2 = (x_size + d.xt - 1) / d.xt;
+    fwd.nb = inv.nb = xt1 == 32 ? az_strided_tiles_per_block(n1, n2, tiles1) : 1;
+    const LaunchShape sh_st{256, az_strided_smem(n1, xt1, fwd.nb)};
     const LaunchShape sh_rd{512, az_rd_smem(n2, d.wt, d.xt, false)};
     if (sh_st.smem > smem_optin_limit() || sh_rd.smem > smem_optin_limit())
         return set_error(ASARF_ERR_INVALID, "range_doppler: tiles exceed shared memory (n1 %d, n2 %d)", n1, n2);
-    const int tiles1 = (x_size + xt1 - 1) / xt1, tiles2 = (x_size + d.xt - 1) / d.xt;
-    rc = backend_az_strided(fwd, nullptr, tiles1, n2, sh_st, stream);
+    rc = backend_az_strided(fwd, nullptr, tiles1, sh_st, stream);
     if (!rc) rc = backend_az_rd(d, nullptr, tiles2, n1, sh_rd, &dstate->errors, stream);
-    if (!rc) rc = backend_az_strided(inv, nullptr, tiles1, n2, sh_st, stream);
+    if (!rc) rc = backend_az_strided(inv, nullptr, tiles1, sh_st, stream);
     // rows past the data block still hold the spectrum stage's values: clear them
     if (!rc && y_size < N)
         rc = mem_zero(out + static_cast<size_t>(y_size) * x_stride,
