@@ -337,8 +337,11 @@ void split_dft_tables(int n, int R, const std::vector<int>& drev, std::vector<un
 }
 
 void matched_filter_table(const std::complex<float>* chirp, int nc, const HostFft& fft, std::vector<float2>& mf) {
-    // conj(DFT_L(replica)) / L in FP64, stored in the forward transform's digit-reversed order
+    // conj(DFT_L(replica)) / L in FP64, stored in the forward transform's digit-reversed order, with
+    // the gain error of the forward and the inverse transform taken back
     const int L = fft.plan.n;
+    int ct[3];
+    const double scale = 1.0 / (L * (1.0 + 2.0 * transform_gain(fft, ct_radices(L, ct) == fft.plan.nst)));
     mf.assign(L, make_float2(0.0f, 0.0f));
     std::vector<std::complex<double>> w(L);
     for (int m = 0; m < L; ++m) w[m] = std::polar(1.0, -2.0 * kPi * m / L);
@@ -349,7 +352,7 @@ void matched_filter_table(const std::complex<float>* chirp, int nc, const HostFf
             const long long idx = (static_cast<long long>(n) * k) % L;
             acc += std::complex<double>(chirp[n].real(), chirp[n].imag()) * w[idx];
         }
-        const std::complex<double> h = std::conj(acc) / static_cast<double>(L);
+        const std::complex<double> h = std::conj(acc) * scale;
         mf[pos] = make_float2(static_cast<float>(h.real()), static_cast<float>(h.imag()));
     }
 }
@@ -359,6 +362,61 @@ int32_t fft_size_above(int32_t v) {
     for (int n = v + 1; n <= 131072; ++n)
         if (smooth(n)) return n;
     return -1;
+}
+
+// Mean gain error of the R-point DFT as the kernels form it: its response to unit impulses, where only
+// the rounding of its constants shows.
+template <int R>
+static double dft_gain_of() {
+    double sum = 0.0;
+    for (int m = 0; m < R; ++m) {
+        float2 v[R];
+        for (int k = 0; k < R; ++k) v[k] = make_float2(k == m ? 1.0f : 0.0f, 0.0f);
+        dft_any<R, false>(v);
+        for (int k = 0; k < R; ++k) {
+            const double a = -2.0 * kPi * (m * k % R) / R;
+            sum += v[k].x * std::cos(a) + v[k].y * std::sin(a) - 1.0;
+        }
+    }
+    return sum / (R * R);
+}
+
+static double dft_gain(int R) {
+    switch (R) {
+        case 3: return dft_gain_of<3>();
+        case 5: return dft_gain_of<5>();
+        case 6: return dft_gain_of<6>();
+        case 7: return dft_gain_of<7>();
+        case 8: return dft_gain_of<8>();
+        case 9: return dft_gain_of<9>();
+        case 12: return dft_gain_of<12>();
+        case 16: return dft_gain_of<16>();
+        case 24: return dft_gain_of<24>();
+        case 32: return dft_gain_of<32>();
+        default: return 0.0;  // 2 and 4 have no constants
+    }
+}
+
+double transform_gain(const HostFft& h, bool table_powers) {
+    double total = 0.0;
+    for (int i = 0; i < h.plan.nst; ++i) {
+        const int R = h.plan.radix[i], S = h.plan.span[i], step = h.plan.n / (S * R);
+        // a stage's outputs average w~^q conj(w^q) over its offsets j and powers q, w~^q from the table
+        // or by the recurrence of pair_twiddle
+        double sum = 0.0;
+        for (int j = 1; j < S; ++j) {
+            const float2 w1 = h.tw[static_cast<size_t>(j) * step];
+            float2 w = w1;
+            for (int q = 1; q < R; ++q) {
+                if (table_powers) w = h.tw[static_cast<size_t>(j) * q * step];
+                const double a = -2.0 * kPi * static_cast<double>(static_cast<long long>(j) * q % (S * R)) / (S * R);
+                sum += w.x * std::cos(a) + w.y * std::sin(a) - 1.0;
+                w = make_float2(std::fma(-w1.y, w.y, w1.x * w.x), std::fma(w1.x, w.y, w1.y * w.x));
+            }
+        }
+        total += sum / (static_cast<double>(S) * R) + dft_gain(R);
+    }
+    return total;
 }
 
 bool build_fft(int n, HostFft& h) { return build_fft_radices(n, factorize(n), h); }
@@ -989,7 +1047,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     p->a_inv.out = p->bufB;
     p->a_inv.valid_rows = p->az_pad;
     p->a_inv.state = p->state;
-    p->a_inv.scale = 1.0f / static_cast<float>(p->az_pad);
+    p->a_inv.scale = azimuth_scale(p->az_pad, p->f1, p->f2);
     p->a_inv.inverse = 1;
     p->tiles1 = (p->nk + p->xt1 - 1) / p->xt1;
     p->a_fwd.nb = p->a_inv.nb = p->xt1 == 32 ? az_strided_tiles_per_block(p->n1, p->n2, p->tiles1) : 1;

@@ -33,6 +33,15 @@ std::vector<int> block_radices(int n);
 // Contiguous length n2 of the azimuth split N = n1 * n2 for nk columns (halo hl, hr of the
 // range-Doppler tile).
 int choose_az_n2(int N, int nk, int hl, int hr, bool absolute_phase);
+// Mean gain error of a transform with this schedule: its float twiddles (from the table at every power,
+// or by recurrence) and radix constants are rounded, which scales all outputs alike by some 1e-8 to
+// 1e-7; its inverse has the same.
+double transform_gain(const HostFft& h, bool table_powers);
+// 1 / N of the azimuth transforms with that gain taken back: over the two forward and two inverse
+// passes it is the one error of theirs that all samples share.
+inline float azimuth_scale(int N, const HostFft& f1, const HostFft& f2) {
+    return static_cast<float>(1.0 / (N * (1.0 + 2.0 * (transform_gain(f1, false) + transform_gain(f2, false)))));
+}
 int choose_rc_len(int nr);
 int32_t fft_size_above(int32_t v);
 void matched_filter_table(const std::complex<float>* chirp, int nc, const HostFft& fft, std::vector<float2>& mf);

@@ -345,7 +345,7 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     inv.in = out;
     inv.out = out;
     inv.valid_rows = N;
-    inv.scale = 1.0f / static_cast<float>(N);
+    inv.scale = azimuth_scale(N, f1, f2);
     inv.inverse = 1;
     AzRdArgs d{};
     d.in = src;
