@@ -34,18 +34,22 @@ int backend_condition(const ConditionArgs& a, int rows, void* stream);
 int backend_product_stats(const ProductStatsArgs& a, void* stream);  // partials then fold
 
 // per-stage kernels
-int backend_decode(const DecodeArgs& a, long long n, void* stream);
-int backend_decode_fbaq(const DecodeFbaqArgs& a, long long n, void* stream);
+int backend_decode(const DecodeArgs& a, void* stream);
+int backend_decode_fbaq(const DecodeFbaqArgs& a, void* stream);
 int backend_img_moments(const ImgMomentsArgs& a, int blocks, void* stream);
 int backend_iq_apply(const IqApplyArgs& a, long long n, void* stream);
 int backend_zero_nans(float2* img, long long n, void* stream);
-int backend_accc(const AcccArgs& a, int blocks, void* stream);
+int backend_accc(const AcccArgs& a, int grid_x, int grid_y, void* stream);
 int backend_rc_rows(const RcRowsArgs& a, int rows, LaunchShape sh, void* stream);
 int backend_multilook(const MultilookArgs& a, void* stream);
 int backend_ers_unpack(const ErsUnpackArgs& a, void* stream);
 int backend_asar_unpack(const AsarUnpackArgs& a, void* stream);
-int backend_rsl(const RslArgs& a, long long n, void* stream);
-int backend_srgr(const SrgrArgs& a, long long n, void* stream);
+int backend_rsl(const RslArgs& a, void* stream);
+int backend_srgr(const SrgrArgs& a, void* stream);
+
+// tables
+int backend_matched_filter(const MatchedFilterArgs& a, void* stream);
+int backend_twiddles(const TwiddleArgs& a, void* stream);
 
 void* mem_alloc(size_t bytes);
 void mem_free(void* p);
@@ -54,6 +58,7 @@ int mem_d2h(void* dst, const void* src, size_t n, void* stream);
 int mem_d2d(void* dst, const void* src, size_t n, void* stream);
 int mem_d2d_2d(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t rows, void* stream);
 int mem_zero(void* dst, size_t n, void* stream);
+int mem_zero_2d(void* dst, size_t pitch, size_t width, size_t rows, void* stream);
 int stream_sync(void* stream);
 void* event_create();
 void event_destroy(void* e);

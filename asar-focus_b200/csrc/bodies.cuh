@@ -2088,89 +2088,105 @@ ASARF_HD ASARF_INLINE void product_stats_fold(const ProductStatsArgs& a, int tid
 // ============================================================================= per-stage bodies
 
 // ConvertErsImSamplesToComplexKernel (envisat_format/src/envisat_format_kernels.cu:116-134)
-// after the NaN pre-fill of ConvertRawSampleSetsToComplex (main_flow.cc:537-540): one item
-// per (line, range sample).
-ASARF_HD ASARF_INLINE void decode_item(const DecodeArgs& a, long long idx) {
-    const int y = static_cast<int>(idx / a.nr);
-    const int x = static_cast<int>(idx - static_cast<long long>(y) * a.nr);
+// after the NaN pre-fill of ConvertRawSampleSetsToComplex (main_flow.cc:537-540): line y.
+ASARF_HD ASARF_INLINE void decode_row(const DecodeArgs& a, int y, int tid, int nthr) {
     const int off = a.swst ? 4 * (static_cast<int>(a.swst[y]) - a.min_swst) : 0;
-    const int i = x - off;
-    float2 v = make_float2(qnan_f(), qnan_f());
-    if (i >= 0 && i < a.spl) {
-        const uint8_t* p = a.raw + static_cast<long long>(y) * a.line_bytes + 2ll * i;
-        v = make_float2(static_cast<float>(p[0]), static_cast<float>(p[1]));
+    const uint8_t* rec = a.raw + static_cast<long long>(y) * a.line_bytes;
+    float2* row = a.img + static_cast<long long>(y) * a.stride;
+    const bool even = (reinterpret_cast<uintptr_t>(rec) & 1) == 0;
+#pragma unroll 4
+    for (int x = tid; x < a.nr; x += nthr) {
+        const int i = x - off;
+        float2 v = make_float2(qnan_f(), qnan_f());
+        if (i >= 0 && i < a.spl) {
+            const unsigned int w = even ? ASARF_LDG(reinterpret_cast<const uint16_t*>(rec) + i)
+                                        : static_cast<unsigned int>(rec[2 * i] | (rec[2 * i + 1] << 8));
+            v = make_float2(static_cast<float>(w & 0xffu), static_cast<float>(w >> 8));
+        }
+        row[x] = v;
     }
-    a.img[static_cast<long long>(y) * a.stride + x] = v;
 }
 
 // ConvertAsarImBlocksToComplexKernel (envisat_format/src/envisat_format_kernels.cu:160-209) as
-// a gather over output pixels: sample r = x - (swst[y] - min_swst) of record y through the
+// a gather over the pixels of line y: sample r = x - (swst[y] - min_swst) of record y through the
 // instrument-file tables, NaN where the record holds no sample.
-ASARF_HD ASARF_INLINE void decode_fbaq_item(const DecodeFbaqArgs& a, long long idx) {
-    const int y = static_cast<int>(idx / a.nr);
-    const int x = static_cast<int>(idx - static_cast<long long>(y) * a.nr);
-    const int r = x - (a.swst ? static_cast<int>(a.swst[y]) - a.min_swst : 0);
-    float2 v = make_float2(qnan_f(), qnan_f());
-    if (r >= 0) {
-        const uint8_t* rec = a.raw + static_cast<long long>(y) * a.line_bytes;
-        const int len = fbaq_len(rec, a.line_bytes);
-        const int b = r / 63;
-        const int j = r + b + 1;
-        if (j < len) {
-            const int id = rec[2 + 64 * b];
-            const int cw = rec[2 + j];
-            v = make_float2(ASARF_LDG(a.lut_i + fbaq4_index(id, cw >> 4)), ASARF_LDG(a.lut_q + fbaq4_index(id, cw & 15)));
+ASARF_HD ASARF_INLINE void decode_fbaq_row(const DecodeFbaqArgs& a, int y, int tid, int nthr) {
+    const int off = a.swst ? static_cast<int>(a.swst[y]) - a.min_swst : 0;
+    const uint8_t* rec = a.raw + static_cast<long long>(y) * a.line_bytes;
+    const int len = fbaq_len(rec, a.line_bytes);
+    float2* row = a.img + static_cast<long long>(y) * a.stride;
+    for (int x = tid; x < a.nr; x += nthr) {
+        const int r = x - off;
+        float2 v = make_float2(qnan_f(), qnan_f());
+        if (r >= 0) {
+            const int b = r / 63;
+            const int j = r + b + 1;
+            if (j < len) {
+                const int id = rec[2 + 64 * b];
+                const int cw = rec[2 + j];
+                v = make_float2(ASARF_LDG(a.lut_i + fbaq4_index(id, cw >> 4)),
+                                ASARF_LDG(a.lut_q + fbaq4_index(id, cw & 15)));
+            }
         }
+        row[x] = v;
     }
-    a.img[static_cast<long long>(y) * a.stride + x] = v;
 }
 
 ASARF_HD ASARF_INLINE bool is_nan_f(float v) { return v != v; }
 
+// DevicePaddedImage::ZeroNaNs (cuda_util/device_padded_image.cu:322-329): only pixels that hold a NaN
+// are written, so an image without any costs one read.
+ASARF_HD ASARF_INLINE void zero_nan_item(float2* img, long long i) {
+    float2 v = img[i];
+    if (is_nan_f(v.x) || is_nan_f(v.y)) {
+        if (is_nan_f(v.x)) v.x = 0.0f;
+        if (is_nan_f(v.y)) v.y = 0.0f;
+        img[i] = v;
+    }
+}
+
 // Moment partials for RawDataCorrection / CalcMean / CalcStdDev
 // (sar/iq_correction.cu:40-138, cuda_util/device_padded_image.cu:156-257): block `blk` sums
 // rows [blk*rpb, ...) in double, NaN samples skipped; deterministic in-block tree.
+ASARF_HD ASARF_INLINE void img_moments_add(double acc[6], float2 v) {
+    if (is_nan_f(v.x) || is_nan_f(v.y)) return;
+    const double i = v.x, q = v.y;
+    acc[0] += 1.0;
+    acc[1] += i;
+    acc[2] += q;
+    acc[3] += i * i;
+    acc[4] += q * q;
+    acc[5] += i * q;
+}
 ASARF_HD ASARF_INLINE void img_moments_body(const ImgMomentsArgs& a, int blk, int tid, int nthr, double* red) {
-    double acc[12];
-    for (int k = 0; k < 12; ++k) acc[k] = 0.0;
+    double data[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, pad[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     const int y0 = blk * a.rows_per_block;
     const int y1 = (y0 + a.rows_per_block < a.y_size) ? y0 + a.rows_per_block : a.y_size;
     for (int y = y0; y < y1; ++y) {
         const float2* row = a.img + static_cast<long long>(y) * a.x_stride;
-        for (int x = tid; x < a.x_stride; x += nthr) {
-            const float2 v = row[x];
-            if (is_nan_f(v.x) || is_nan_f(v.y)) continue;
-            const int o = x < a.x_size ? 0 : 6;
-            if (a.centered) {
-                if (o) continue;
-                const float di = fsub_rn(v.x, a.mean_i), dq = fsub_rn(v.y, a.mean_q);
-                acc[3] += static_cast<double>(fmul_rn(di, di));
-                acc[4] += static_cast<double>(fmul_rn(dq, dq));
-                acc[0] += 1.0;
-                continue;
-            }
-            const double i = v.x, q = v.y;
-            acc[o + 0] += 1.0;
-            acc[o + 1] += i;
-            acc[o + 2] += q;
-            acc[o + 3] += i * i;
-            acc[o + 4] += q * q;
-            acc[o + 5] += i * q;
+        int x = tid;
+        for (; x + 3 * nthr < a.x_size; x += 4 * nthr) {  // four loads in flight
+            const float2 v0 = row[x], v1 = row[x + nthr], v2 = row[x + 2 * nthr], v3 = row[x + 3 * nthr];
+            img_moments_add(data, v0);
+            img_moments_add(data, v1);
+            img_moments_add(data, v2);
+            img_moments_add(data, v3);
         }
+        for (; x < a.x_size; x += nthr) img_moments_add(data, row[x]);
+        for (; x < a.x_stride; x += nthr) img_moments_add(pad, row[x]);
     }
-    for (int k = 0; k < 12; ++k) red[k * nthr + tid] = acc[k];
+    for (int k = 0; k < 6; ++k) red[k * nthr + tid] = data[k], red[(6 + k) * nthr + tid] = pad[k];
     ASARF_SYNC();
 #if defined(__CUDA_ARCH__)
     for (int w = nthr / 2; w > 0; w >>= 1) {
-        if (tid < w)
-            for (int k = 0; k < 12; ++k) red[k * nthr + tid] += red[k * nthr + tid + w];
+        for (int t = tid; t < 12 * w; t += nthr) {
+            const int k = t / w, i = t - k * w;
+            red[k * nthr + i] += red[k * nthr + i + w];
+        }
         ASARF_SYNC();
     }
-    if (tid == 0)
-        for (int k = 0; k < 12; ++k) a.partial[blk * 12 + k] = red[k * nthr];
-#else
-    for (int k = 0; k < 12; ++k) a.partial[blk * 12 + k] = red[k * nthr];
 #endif
+    for (int k = tid; k < 12; k += nthr) a.partial[blk * 12 + k] = red[k * nthr];
 }
 
 // CorrectDCBias + ApplyGainCorrection + ApplyPhaseCorrection (sar/iq_correction.cu:140-178)
@@ -2185,23 +2201,46 @@ ASARF_HD ASARF_INLINE void iq_apply_item(const IqApplyArgs& a, long long idx) {
 }
 
 // PhaseDifference partials of CalculateDopplerCentroid (sar/fractional_doppler_centroid.cu:33-69):
-// per block of rows and per column x (columns up to nblk*step, which may reach into the
-// padding as the reference's last block does), the FP64 sum over pairs (y-1, y), y >= 1,
-// of conj(z[y-1]) z[y]; the host adds columns into range blocks in a fixed order.
-ASARF_HD ASARF_INLINE void accc_body(const AcccArgs& a, int blk, int tid, int nthr) {
-    const int y0 = blk * a.rows_per_block;
+// block (bx, by) takes kAcccCols columns (up to nblk*step, which may reach into the padding as the
+// reference's last block does) of rows_per_block rows; a thread sums its column's pairs (y-1, y),
+// y >= 1, of conj(z[y-1]) z[y] in FP64, reading each row once, and the columns of each Doppler
+// block are added in order.  (One block per 256 rows, all columns in turn, left 28 blocks for a
+// 7000-line image, 1346 us.)
+ASARF_HD ASARF_INLINE void accc_body(const AcccArgs& a, int bx, int by, int grid_x, int tid, int nthr, double* cols) {
+    const int y0 = by * a.rows_per_block;
     const int y1 = (y0 + a.rows_per_block < a.y_size) ? y0 + a.rows_per_block : a.y_size;
-    const int xend = a.nblk * a.step < a.x_stride ? a.nblk * a.step : a.x_stride;
-    for (int x = tid; x < xend; x += nthr) {
+    const int x0 = bx * kAcccCols;
+    constexpr int kBatch = 8;
+    for (int t = tid; t < kAcccCols; t += nthr) {
         double re = 0.0, im = 0.0;
-        for (int y = (y0 > 1 ? y0 : 1); y < y1; ++y) {
-            const float2 p = a.img[static_cast<long long>(y - 1) * a.x_stride + x];
-            const float2 c = a.img[static_cast<long long>(y) * a.x_stride + x];
-            re += static_cast<double>(p.x) * c.x + static_cast<double>(p.y) * c.y;
-            im += static_cast<double>(p.x) * c.y - static_cast<double>(p.y) * c.x;
+        if (x0 + t < a.xend) {
+            const float2* col = a.img + x0 + t;
+            float2 p = col[static_cast<long long>(y0 > 0 ? y0 - 1 : 0) * a.x_stride];
+            for (int y = y0 > 0 ? y0 : 1; y < y1; y += kBatch) {
+                float2 c[kBatch];
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u)
+                    c[u] = y + u < y1 ? col[static_cast<long long>(y + u) * a.x_stride] : make_float2(0.0f, 0.0f);
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u) {
+                    if (y + u >= y1) break;
+                    re += static_cast<double>(p.x) * c[u].x + static_cast<double>(p.y) * c[u].y;
+                    im += static_cast<double>(p.x) * c[u].y - static_cast<double>(p.y) * c[u].x;
+                    p = c[u];
+                }
+            }
         }
-        a.partial[(static_cast<long long>(blk) * xend + x) * 2] = re;
-        a.partial[(static_cast<long long>(blk) * xend + x) * 2 + 1] = im;
+        cols[2 * t] = re;
+        cols[2 * t + 1] = im;
+    }
+    ASARF_SYNC();
+    const int b0 = x0 / a.step;
+    double* out = a.partial + (static_cast<long long>(by) * grid_x + bx) * a.span * 2;
+    for (int t = tid; t < 2 * a.span; t += nthr) {
+        const int lo = (b0 + t / 2) * a.step - x0, hi = lo + a.step;
+        double acc = 0.0;
+        for (int c = lo > 0 ? lo : 0; c < hi && c < kAcccCols; ++c) acc += cols[2 * c + (t & 1)];
+        out[t] = acc;
     }
 }
 
@@ -2219,8 +2258,102 @@ ASARF_HD ASARF_INLINE void rc_rows_body(const RcRowsArgs& a, int y, int tid, int
     for (int l = tid; l < a.x_zero_end; l += nthr) row[l] = l < a.nk ? s[l] : make_float2(0.0f, 0.0f);
 }
 
-// TimeDomainAzimuthLook (sar/az_multilook.cu:25-80): one output line per block.
+// The same with a compile-time schedule (lengths in kCtLengths), as the planned path's range
+// compression: 7000 lines of 5616 samples 522 -> RCUS us.
+template <int L>
+ASARF_HD ASARF_INLINE void rc_rows_ct_body(const RcRowsArgs& a, int y, int tid, float2* s) {
+    constexpr int NTHR = CtSchedule<L>::nthr;
+    constexpr int PER = (L + NTHR - 1) / NTHR;
+    float2* row = a.img + static_cast<long long>(y) * a.stride;
+    ct_phase<NTHR>(
+        [&](int t) {
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                const int l = t + k * NTHR;
+                if (L % NTHR != 0 && l >= L) break;
+                s[ct_pad<L>(l)] = l < a.nr ? row[l] : make_float2(0.0f, 0.0f);
+            }
+        },
+        tid);
+    ct_fft_mf_ifft<L>(s, a.ctw, a.mf, tid, RcOut{row, a.nk});
+    ct_phase<NTHR, false>([&](int t) {
+        for (int x = a.nk + t; x < a.x_zero_end; x += NTHR) row[x] = make_float2(0.0f, 0.0f);
+    }, tid);
+}
+
+// exp(2 pi i m / n) in FP64
+ASARF_HD ASARF_INLINE void unit_root(long long m, int n, double* c, double* s) {
+#if defined(__CUDA_ARCH__)
+    sincospi(2.0 * static_cast<double>(m) / n, s, c);
+#else
+    const double a = 2.0 * 3.14159265358979323846 * static_cast<double>(m) / n;
+    *c = cos(a);
+    *s = sin(a);
+#endif
+}
+
+// Part `part` of `parts` of the sum behind matched-filter position pos: the replica's samples of that
+// stretch against exp(-2 pi i n k / L), stepped by a rotation in FP64 (L * nc terms: on one host
+// thread 17 ms of every per-stage range compression and of every plan, here about 20 us).
+ASARF_HD ASARF_INLINE void matched_filter_sum(const MatchedFilterArgs& a, int pos, int part, int parts, double* re,
+                                              double* im) {
+    const int L = a.plan.n;
+    int rem = pos, k = 0, mult = 1;
+    for (int i = 0; i < a.plan.nst; ++i) {
+        const int q = rem / a.plan.span[i];
+        rem -= q * a.plan.span[i];
+        k += q * mult;
+        mult *= a.plan.radix[i];
+    }
+    const int len = (a.nc + parts - 1) / parts, n0 = part * len, n1 = n0 + len < a.nc ? n0 + len : a.nc;
+    double c, s, wc, ws, sr = 0.0, si = 0.0;
+    unit_root(-(static_cast<long long>(n0) * k % L), L, &c, &s);
+    unit_root(-static_cast<long long>(k), L, &wc, &ws);
+    for (int n = n0; n < n1; ++n) {
+        const float2 v = ASARF_LDG(a.chirp + n);
+        sr += v.x * c - v.y * s;
+        si += v.x * s + v.y * c;
+        const double t = c * wc - s * ws;
+        s = c * ws + s * wc;
+        c = t;
+    }
+    *re = sr;
+    *im = si;
+}
+ASARF_HD ASARF_INLINE void matched_filter_store(const MatchedFilterArgs& a, int pos, double re, double im) {
+    const int R = a.last_radix;
+    const int at = R > 0 ? (pos % R) * (a.plan.n / R) + pos / R : pos;
+    a.mf[at] = make_float2(static_cast<float>(re * a.scale), static_cast<float>(-im * a.scale));
+}
+
+// Entry i of a twiddle table.
+ASARF_HD ASARF_INLINE void twiddle_item(const TwiddleArgs& a, int i) {
+    long long m = i;
+    int n = a.n;
+    if (a.r[0] > 0) {
+        int at = i;
+        for (int k = 0; k < 2; ++k) {  // pass k: (r_k - 1) * S entries exp(-2 pi i j q / M), q outer
+            const int S = n / a.r[k];
+            if (at < (a.r[k] - 1) * S) {
+                m = static_cast<long long>(at / S + 1) * (at % S) % n;
+                break;
+            }
+            at -= (a.r[k] - 1) * S;
+            n = S;
+        }
+    }
+    double c, s;
+    unit_root(-m, n, &c, &s);
+    a.out[i] = make_float2(static_cast<float>(c), static_cast<float>(s));
+}
+inline int twiddle_count(const TwiddleArgs& a) {
+    return a.r[0] > 0 ? (a.r[0] - 1) * (a.n / a.r[0]) + (a.r[1] - 1) * (a.n / a.r[0] / a.r[1]) : a.n;
+}
+
+// TimeDomainAzimuthLook (sar/az_multilook.cu:25-80): one output line per block.  A column's window
+// rows (at most 6) are loaded before any is summed.
 ASARF_HD ASARF_INLINE void multilook_row_body(const MultilookArgs& a, int y, int tid, int nthr) {
+    constexpr int kRows = 6;
     const float in_idx = fmul_rn(static_cast<float>(y), a.ratio);
     const float mu = fsub_rn(in_idx, static_cast<float>(static_cast<int>(in_idx)));
     int s0 = static_cast<int>(fsub_rn(in_idx, 2.0f)), e0 = static_cast<int>(fadd_rn(in_idx, 2.0f));
@@ -2233,14 +2366,23 @@ ASARF_HD ASARF_INLINE void multilook_row_body(const MultilookArgs& a, int y, int
     const int c1 = e1 > s1 ? e1 - s1 : 0;
     const int r_lo = s0 < s1 ? s0 : s1;
     const int r_hi = e0 > e1 ? e0 : e1;
+    const int nr = r_hi - r_lo;
+    const float2* first = a.slc + static_cast<long long>(r_lo) * a.x_size;
     for (int c = tid; c < a.x_size; c += nthr) {
+        float2 z[kRows];
+#pragma unroll
+        for (int k = 0; k < kRows; ++k)
+            z[k] = k < nr ? first[static_cast<long long>(k) * a.x_size + c] : make_float2(0.0f, 0.0f);
         float sum0 = 0.0f, sum1 = 0.0f;
-        for (int r = r_lo; r < r_hi; ++r) {
-            const float2 v = a.slc[static_cast<long long>(r) * a.x_size + c];
+        auto add = [&](int r, float2 v) {
             const float p2 = fma_rn(v.x, v.x, fmul_rn(v.y, v.y));
             if (r >= s0 && r < e0) sum0 = fadd_rn(sum0, p2);
             if (r >= s1 && r < e1) sum1 = fadd_rn(sum1, p2);
-        }
+        };
+#pragma unroll
+        for (int k = 0; k < kRows; ++k)
+            if (k < nr) add(r_lo + k, z[k]);
+        for (int r = r_lo + kRows; r < r_hi; ++r) add(r, a.slc[static_cast<long long>(r) * a.x_size + c]);
         if (c0) sum0 = fdiv_rn(sum0, static_cast<float>(c0));
         if (c1) sum1 = fdiv_rn(sum1, static_cast<float>(c1));
         float val = 0.0f;
@@ -2249,25 +2391,30 @@ ASARF_HD ASARF_INLINE void multilook_row_body(const MultilookArgs& a, int y, int
     }
 }
 
-// CorrectionKernel of RangeSpreadingLossCorrection (sar/range_spreading_loss.cu:29-52).
-ASARF_HD ASARF_INLINE void rsl_item(const RslArgs& a, long long idx) {
-    const int x = static_cast<int>(idx % a.range_size);
+// Rows a column's gain or resampling index serves in the two kernels below, which each form it once
+// (an FP64 power, a polynomial and a division a pixel bound them before).
+constexpr int kColumnRows = 32;
+
+// CorrectionKernel of RangeSpreadingLossCorrection (sar/range_spreading_loss.cu:29-52): column x of rows
+// [y0, y1).
+ASARF_HD ASARF_INLINE void rsl_column(const RslArgs& a, int x, int y0, int y1) {
     const double r = a.slant_first + x * a.range_spacing;
     const double ratio = a.ref_range / r;
     const float g = static_cast<float>(1.0 / sqrt(pow(ratio, 3.0)));
-    a.img[idx] = fmul_rn(a.img[idx], g);
+    float* p = a.img + static_cast<long long>(y0) * a.range_size + x;
+#pragma unroll 8
+    for (int y = y0; y < y1; ++y, p += a.range_size) *p = fmul_rn(*p, g);
 }
 
-// SrGrInterpolation (sar/srgr.cu:49-71) with the float Horner / IEEE divide / truncation index.
-ASARF_HD ASARF_INLINE void srgr_item(const SrgrArgs& a, long long idx) {
-    const int y = static_cast<int>(idx / a.out_x);
-    const int xg = static_cast<int>(idx - static_cast<long long>(y) * a.out_x);
+// SrGrInterpolation (sar/srgr.cu:49-71) with the float Horner / IEEE divide / truncation index: ground
+// column xg of rows [y0, y1).
+ASARF_HD ASARF_INLINE void srgr_column(const SrgrArgs& a, int xg, int y0, int y1) {
     const float gd = fmul_rn(static_cast<float>(xg), a.ground_spacing);
     const float rd = polyval_f32(a.grsr, gd);
     const float ridx = fdiv_rn(rd, a.range_spacing);
     int i0 = static_cast<int>(ridx);
     const float dx = fsub_rn(ridx, static_cast<float>(i0));
-    if (a.start && y == 0) {
+    if (a.start && y0 == 0) {
         a.start[xg] = i0;
         a.frac[xg] = dx;
     }
@@ -2276,9 +2423,13 @@ ASARF_HD ASARF_INLINE void srgr_item(const SrgrArgs& a, long long idx) {
         if (a.err) atomic_or_u32(a.err, kErrSrgrIndex);
         i0 = i0 < 0 ? 0 : a.in_x - 2;
     }
-    const float* row = a.in + static_cast<long long>(y) * a.in_x;
-    const float v0 = row[i0], v1 = row[i0 + 1];
-    a.out[idx] = fma_rn(dx, fsub_rn(v1, v0), v0);
+    const float* in = a.in + static_cast<long long>(y0) * a.in_x + i0;
+    float* out = a.out + static_cast<long long>(y0) * a.out_x + xg;
+#pragma unroll 8
+    for (int y = y0; y < y1; ++y, in += a.in_x, out += a.out_x) {
+        const float v0 = in[0], v1 = in[1];
+        *out = fma_rn(dx, fsub_rn(v1, v0), v0);
+    }
 }
 
 }  // namespace asarf

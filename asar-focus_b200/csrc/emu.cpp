@@ -160,8 +160,8 @@ int backend_asar_unpack(const AsarUnpackArgs& a, void*) {
     return ASARF_OK;
 }
 
-int backend_decode(const DecodeArgs& a, long long n, void*) {
-    for (long long i = 0; i < n; ++i) decode_item(a, i);
+int backend_decode(const DecodeArgs& a, void*) {
+    for (int y = 0; y < a.lines; ++y) decode_row(a, y, 0, 1);
     return ASARF_OK;
 }
 int backend_product_stats(const ProductStatsArgs& a, void*) {
@@ -176,8 +176,8 @@ int backend_condition(const ConditionArgs& a, int rows, void*) {
     return ASARF_OK;
 }
 
-int backend_decode_fbaq(const DecodeFbaqArgs& a, long long n, void*) {
-    for (long long i = 0; i < n; ++i) decode_fbaq_item(a, i);
+int backend_decode_fbaq(const DecodeFbaqArgs& a, void*) {
+    for (int y = 0; y < a.lines; ++y) decode_fbaq_row(a, y, 0, 1);
     return ASARF_OK;
 }
 
@@ -191,31 +191,57 @@ int backend_iq_apply(const IqApplyArgs& a, long long n, void*) {
     return ASARF_OK;
 }
 int backend_zero_nans(float2* img, long long n, void*) {
-    for (long long i = 0; i < n; ++i) {
-        if (is_nan_f(img[i].x)) img[i].x = 0.0f;
-        if (is_nan_f(img[i].y)) img[i].y = 0.0f;
-    }
+    for (long long i = 0; i < n; ++i) zero_nan_item(img, i);
     return ASARF_OK;
 }
-int backend_accc(const AcccArgs& a, int blocks, void*) {
-    for (int b = 0; b < blocks; ++b) accc_body(a, b, 0, 1);
+int backend_accc(const AcccArgs& a, int grid_x, int grid_y, void*) {
+    std::vector<double> cols(2 * kAcccCols);
+    for (int by = 0; by < grid_y; ++by)
+        for (int bx = 0; bx < grid_x; ++bx) accc_body(a, bx, by, grid_x, 0, 1, cols.data());
     return ASARF_OK;
+}
+template <int L>
+static void emu_rc_rows_ct(const RcRowsArgs& a, int rows, float2* s) {
+    for (int y = 0; y < rows; ++y) rc_rows_ct_body<L>(a, y, 0, s);
 }
 int backend_rc_rows(const RcRowsArgs& a, int rows, LaunchShape sh, void*) {
     std::vector<float2> s(sh.smem / sizeof(float2) + 1);
+    switch (a.ctw ? a.plan.n : 0) {
+        case 768: emu_rc_rows_ct<768>(a, rows, s.data()); return ASARF_OK;
+        case 1024: emu_rc_rows_ct<1024>(a, rows, s.data()); return ASARF_OK;
+        case 1536: emu_rc_rows_ct<1536>(a, rows, s.data()); return ASARF_OK;
+        case 2048: emu_rc_rows_ct<2048>(a, rows, s.data()); return ASARF_OK;
+        case 3072: emu_rc_rows_ct<3072>(a, rows, s.data()); return ASARF_OK;
+        case 4096: emu_rc_rows_ct<4096>(a, rows, s.data()); return ASARF_OK;
+        case 6144: emu_rc_rows_ct<6144>(a, rows, s.data()); return ASARF_OK;
+        case 8192: emu_rc_rows_ct<8192>(a, rows, s.data()); return ASARF_OK;
+        default: break;
+    }
     for (int y = 0; y < rows; ++y) rc_rows_body(a, y, 0, 1, s.data());
+    return ASARF_OK;
+}
+int backend_matched_filter(const MatchedFilterArgs& a, void*) {
+    for (int pos = 0; pos < a.plan.n; ++pos) {
+        double re, im;
+        matched_filter_sum(a, pos, 0, 1, &re, &im);
+        matched_filter_store(a, pos, re, im);
+    }
+    return ASARF_OK;
+}
+int backend_twiddles(const TwiddleArgs& a, void*) {
+    for (int i = 0, n = twiddle_count(a); i < n; ++i) twiddle_item(a, i);
     return ASARF_OK;
 }
 int backend_multilook(const MultilookArgs& a, void*) {
     for (int y = 0; y < a.out_y; ++y) multilook_row_body(a, y, 0, 1);
     return ASARF_OK;
 }
-int backend_rsl(const RslArgs& a, long long n, void*) {
-    for (long long i = 0; i < n; ++i) rsl_item(a, i);
+int backend_rsl(const RslArgs& a, void*) {
+    for (int x = 0; x < a.range_size; ++x) rsl_column(a, x, 0, a.az_size);
     return ASARF_OK;
 }
-int backend_srgr(const SrgrArgs& a, long long n, void*) {
-    for (long long i = 0; i < n; ++i) srgr_item(a, i);
+int backend_srgr(const SrgrArgs& a, void*) {
+    for (int x = 0; x < a.out_x; ++x) srgr_column(a, x, 0, a.y_size);
     return ASARF_OK;
 }
 
@@ -240,6 +266,10 @@ int mem_d2d_2d(void* dst, size_t dpitch, const void* src, size_t spitch, size_t 
 }
 int mem_zero(void* dst, size_t n, void*) {
     std::memset(dst, 0, n);
+    return ASARF_OK;
+}
+int mem_zero_2d(void* dst, size_t pitch, size_t width, size_t rows, void*) {
+    for (size_t r = 0; r < rows; ++r) std::memset(static_cast<char*>(dst) + r * pitch, 0, width);
     return ASARF_OK;
 }
 int stream_sync(void*) { return ASARF_OK; }

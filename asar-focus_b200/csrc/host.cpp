@@ -336,25 +336,26 @@ void split_dft_tables(int n, int R, const std::vector<int>& drev, std::vector<un
         }
 }
 
-void matched_filter_table(const std::complex<float>* chirp, int nc, const HostFft& fft, std::vector<float2>& mf) {
-    // conj(DFT_L(replica)) / L in FP64, stored in the forward transform's digit-reversed order, with
-    // the gain error of the forward and the inverse transform taken back
-    const int L = fft.plan.n;
+MatchedFilterArgs matched_filter_args(const float2* d_chirp, int nc, const HostFft& fft, float2* d_mf) {
+    MatchedFilterArgs a{};
     int ct[3];
-    const double scale = 1.0 / (L * (1.0 + 2.0 * transform_gain(fft, ct_radices(L, ct) == fft.plan.nst)));
-    mf.assign(L, make_float2(0.0f, 0.0f));
-    std::vector<std::complex<double>> w(L);
-    for (int m = 0; m < L; ++m) w[m] = std::polar(1.0, -2.0 * kPi * m / L);
-    for (int pos = 0; pos < L; ++pos) {
-        const int k = fft.drev[pos];
-        std::complex<double> acc(0.0, 0.0);
-        for (int n = 0; n < nc; ++n) {
-            const long long idx = (static_cast<long long>(n) * k) % L;
-            acc += std::complex<double>(chirp[n].real(), chirp[n].imag()) * w[idx];
-        }
-        const std::complex<double> h = std::conj(acc) * scale;
-        mf[pos] = make_float2(static_cast<float>(h.real()), static_cast<float>(h.imag()));
-    }
+    const bool compiled = ct_radices(fft.plan.n, ct) == fft.plan.nst;
+    a.chirp = d_chirp;
+    a.nc = nc;
+    a.plan = fft.plan;
+    // 1 / L, with the gain error of the forward and the inverse transform taken back
+    a.scale = 1.0 / (fft.plan.n * (1.0 + 2.0 * transform_gain(fft, compiled)));
+    a.last_radix = compiled ? ct[2] : 0;
+    a.mf = d_mf;
+    return a;
+}
+
+TwiddleArgs ct_twiddle_args(int L, float2* d_out) {
+    TwiddleArgs a{};
+    a.n = L;
+    a.out = d_out;
+    ct_radices(L, a.r);
+    return a;
 }
 
 int32_t fft_size_above(int32_t v) {
@@ -530,6 +531,27 @@ bool build_fft_radices(int n, const std::vector<int>& f, HostFft& h) {
         h.tw[m] = make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a)));
     }
     return true;
+}
+
+int largest_divisor_le(int n, int cap) {
+    for (int d = std::min(n, cap); d >= 1; --d)
+        if (n % d == 0) return d;
+    return 1;
+}
+
+bool make_azimuth_maps(float2* a, float2* b, int nk, long long pitch, int n1, int n2, int xt, int nb, int n1_box, int wt,
+                       int n2_box, void* map_a3, void* map_b3, void* map_a2) {
+    if (wt % 2 != 0) return false;
+    const unsigned long long row_bytes = static_cast<unsigned long long>(pitch) * sizeof(float2);
+    const unsigned long long d3[3] = {2ull * nk, static_cast<unsigned long long>(n2), static_cast<unsigned long long>(n1)};
+    const unsigned long long s3[2] = {row_bytes, row_bytes * n2};
+    const unsigned int b3[3] = {static_cast<unsigned int>(2 * xt), static_cast<unsigned int>(nb),
+                                static_cast<unsigned int>(n1_box)};
+    const unsigned long long d2[2] = {2ull * nk, static_cast<unsigned long long>(n1) * n2};
+    const unsigned long long s2[1] = {row_bytes};
+    const unsigned int b2[2] = {static_cast<unsigned int>(2 * wt), static_cast<unsigned int>(n2_box)};
+    return backend_make_tmap(map_a3, 3, a, d3, s3, b3) == ASARF_OK && backend_make_tmap(map_b3, 3, b, d3, s3, b3) == ASARF_OK &&
+           backend_make_tmap(map_a2, 2, a, d2, s2, b2) == ASARF_OK;
 }
 
 int choose_rc_len(int nr) {
@@ -765,7 +787,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
         std::rotate(big, big + 1, f2_radices.end());
     }
     if (!rc_ok || !build_fft_radices(p->n1, strided_radices(p->n1), p->f1) ||
-        !build_fft_radices(p->n2, f2_radices, p->f2) || !build_fft(p->az_pad, p->fN)) {
+        !build_fft_radices(p->n2, f2_radices, p->f2)) {
         delete p;
         return set_error(ASARF_ERR_INVALID, "FFT schedule failed");
     }
@@ -792,30 +814,9 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
             p->xt2 -= 2;
     }
 
-    // chirp matched filter in the forward transform's output order, scaled by 1/L
+    // the replica behind the matched filter
     std::vector<std::complex<float>> chirp;
-    generate_chirp(s.chirp_kr, s.range_sampling_rate, p->nc, s.apply_window != 0, p->rc_len, chirp);
-    std::vector<float2> mf;
-    matched_filter_table(chirp.data(), p->nc, p->rc, mf);
-    std::vector<float2> ctw;
-    if (n_ctr) {
-        // transposed filter (position b*R + q at q*(L/R) + b) and the per-pass twiddle tables
-        const int L = p->rc_len, R = ctr[n_ctr - 1], nb = L / R;
-        std::vector<float2> t(mf.size());
-        for (int b = 0; b < nb; ++b)
-            for (int q = 0; q < R; ++q) t[static_cast<size_t>(q) * nb + b] = mf[static_cast<size_t>(b) * R + q];
-        mf.swap(t);
-        int m = L;
-        for (int k = 0; k + 1 < n_ctr; ++k) {
-            const int S = m / ctr[k], M = m;
-            for (int q = 1; q < ctr[k]; ++q)
-                for (int j = 0; j < S; ++j) {
-                    const double a = -2.0 * kPi * static_cast<double>(static_cast<long long>(j) * q % M) / M;
-                    ctw.push_back(make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a))));
-                }
-            m = S;
-        }
-    }
+    generate_chirp(s.chirp_kr, s.range_sampling_rate, p->nc, s.apply_window != 0, p->nc, chirp);
 
     // results-window variants (CalcResultsWindow, main_flow.cc:155-201) and their tails
     const int max_ap = max_aperture_pixels(s);
@@ -881,7 +882,9 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     p->out_dev = p->alloc<float>(static_cast<size_t>(p->out_bytes + 3) / 4);
     float2* rc_tw = p->alloc<float2>(p->rc_len);
     p->rc_mf = p->alloc<float2>(p->rc_len);
-    float2* ct_tw = ctw.empty() ? nullptr : p->alloc<float2>(ctw.size());
+    TwiddleArgs ctw = ct_twiddle_args(p->rc_len, nullptr);
+    float2* ct_tw = ctw.out = n_ctr ? p->alloc<float2>(static_cast<size_t>(twiddle_count(ctw))) : nullptr;
+    float2* chirp_dev = p->alloc<float2>(static_cast<size_t>(p->nc));
     float2* tw1 = p->alloc<float2>(p->n1);
     int* drev1 = p->alloc<int>(p->n1);
     float2* tw2 = p->alloc<float2>(p->n2);
@@ -907,7 +910,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     constexpr int kPstatBlocks = 4 * 148;
     double* pstat_dev = opt.sq_stats ? p->alloc<double>(5 * kPstatBlocks + 4) : nullptr;
     if (!p->bufA || !p->bufB || !p->acc || !p->state || !p->raw_dev || !p->swst_dev || !p->out_dev || !rc_tw ||
-        !p->rc_mf || !tw1 || !drev1 || !tw2 || !drev2 || !twN || !rcmc || !rsl_dev || (fbaq && (!lut_dev || !part_dev || !facc_dev)) ||
+        !p->rc_mf || !chirp_dev || (n_ctr && !ct_tw) || !tw1 || !drev1 || !tw2 || !drev2 || !twN || !rcmc || !rsl_dev || (fbaq && (!lut_dev || !part_dev || !facc_dev)) ||
         (opt.sq_stats && !pstat_dev)) {
         const size_t need = p->bytes;
         delete p;
@@ -916,13 +919,14 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     }
     rc = 0;
     rc |= mem_h2d(rc_tw, p->rc.tw.data(), sizeof(float2) * p->rc_len, nullptr);
-    rc |= mem_h2d(p->rc_mf, mf.data(), sizeof(float2) * p->rc_len, nullptr);
-    if (ct_tw) rc |= mem_h2d(ct_tw, ctw.data(), sizeof(float2) * ctw.size(), nullptr);
+    rc |= mem_h2d(chirp_dev, chirp.data(), sizeof(float2) * p->nc, nullptr);
+    rc |= backend_matched_filter(matched_filter_args(chirp_dev, p->nc, p->rc, p->rc_mf), nullptr);
+    if (ct_tw) rc |= backend_twiddles(ctw, nullptr);
     rc |= mem_h2d(tw1, p->f1.tw.data(), sizeof(float2) * p->n1, nullptr);
     rc |= mem_h2d(drev1, p->f1.drev.data(), sizeof(int) * p->n1, nullptr);
     rc |= mem_h2d(tw2, p->f2.tw.data(), sizeof(float2) * p->n2, nullptr);
     rc |= mem_h2d(drev2, p->f2.drev.data(), sizeof(int) * p->n2, nullptr);
-    rc |= mem_h2d(twN, p->fN.tw.data(), sizeof(float2) * p->az_pad, nullptr);
+    rc |= backend_twiddles(TwiddleArgs{twN, p->az_pad, {0, 0, 0}}, nullptr);
     rc |= backend_rcmc_table(rcmc, nullptr);
     rc |= mem_h2d(rsl_dev, rsl.data(), sizeof(float) * p->nx, nullptr);
     if (fbaq) {
@@ -1130,26 +1134,11 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
 
     // ---- TMA tensor maps (all tiles come from this GPU's own buffers; loads only)
     {
-        auto largest_divisor_le = [](int n, int cap) {
-            for (int d = std::min(n, cap); d >= 1; --d)
-                if (n % d == 0) return d;
-            return 1;
-        };
         const int n1_box = largest_divisor_le(p->n1, 256);
         const int n2_box = largest_divisor_le(p->n2, 256);
-        const unsigned long long row_bytes = static_cast<unsigned long long>(p->pitch) * sizeof(float2);
-        const unsigned long long d3[3] = {2ull * p->nk, static_cast<unsigned long long>(p->n2),
-                                          static_cast<unsigned long long>(p->n1)};
-        const unsigned long long s3[2] = {row_bytes, row_bytes * p->n2};
-        const unsigned int b3[3] = {static_cast<unsigned int>(2 * p->xt1), static_cast<unsigned int>(p->a_fwd.nb),
-                                    static_cast<unsigned int>(n1_box)};
-        const unsigned long long d2[2] = {2ull * p->nk, static_cast<unsigned long long>(p->az_pad)};
-        const unsigned long long s2[1] = {row_bytes};
-        const unsigned int b2[2] = {static_cast<unsigned int>(2 * d.wt), static_cast<unsigned int>(n2_box)};
-        const bool shapes_ok = (d.wt % 2 == 0) && 2 * d.wt <= 256 && 2 * p->xt1 <= 256;
-        p->use_tma = shapes_ok && backend_make_tmap(p->tmapA3, 3, p->bufA, d3, s3, b3) == ASARF_OK &&
-                     backend_make_tmap(p->tmapB3, 3, p->bufB, d3, s3, b3) == ASARF_OK &&
-                     backend_make_tmap(p->tmapA2, 2, p->bufA, d2, s2, b2) == ASARF_OK;
+        p->use_tma = 2 * d.wt <= 256 && make_azimuth_maps(p->bufA, p->bufB, p->nk, p->pitch, p->n1, p->n2, p->xt1,
+                                                          p->a_fwd.nb, n1_box, d.wt, n2_box, p->tmapA3, p->tmapB3,
+                                                          p->tmapA2);
         p->a_fwd.use_tma = p->a_inv.use_tma = d.use_tma = p->use_tma ? 1 : 0;
         p->a_fwd.n1_box = p->a_inv.n1_box = n1_box;
         d.n2_box = n2_box;

@@ -6,6 +6,7 @@
 
 #include "asarf.h"
 #include "fft.cuh"
+#include "params.h"
 
 namespace asarf {
 
@@ -42,8 +43,17 @@ double transform_gain(const HostFft& h, bool table_powers);
 inline float azimuth_scale(int N, const HostFft& f1, const HostFft& f2) {
     return static_cast<float>(1.0 / (N * (1.0 + 2.0 * (transform_gain(f1, false) + transform_gain(f2, false)))));
 }
+int largest_divisor_le(int n, int cap);
+// TMA maps (128-byte blobs) of the azimuth passes over an image pair a, b of n1 * n2 rows of `pitch`
+// complex values, nk of them data: strided views of a and b (nb tiles of xt columns, n1_box of the
+// n1 rows a box) and the contiguous view of a (wt columns, n2_box rows).
+bool make_azimuth_maps(float2* a, float2* b, int nk, long long pitch, int n1, int n2, int xt, int nb, int n1_box, int wt,
+                       int n2_box, void* map_a3, void* map_b3, void* map_a2);
 int choose_rc_len(int nr);
 int32_t fft_size_above(int32_t v);
-void matched_filter_table(const std::complex<float>* chirp, int nc, const HostFft& fft, std::vector<float2>& mf);
+// Device tables of a range transform: the matched filter (fft.plan.n entries) from a replica of nc
+// samples in device memory, and the twiddle tables of a compile-time length.
+MatchedFilterArgs matched_filter_args(const float2* d_chirp, int nc, const HostFft& fft, float2* d_mf);
+TwiddleArgs ct_twiddle_args(int L, float2* d_out);
 
 }  // namespace asarf

@@ -417,23 +417,65 @@ __global__ void __launch_bounds__(256) k_items(Args a, long long n) {
         Item(a, i);
 }
 
-ASARF_HD ASARF_INLINE void zero_nan_item(float2* const& img, long long i) {
-    float2 v = img[i];
-    if (is_nan_f(v.x)) v.x = 0.0f;
-    if (is_nan_f(v.y)) v.y = 0.0f;
-    img[i] = v;
+__global__ void __launch_bounds__(256) k_decode(DecodeArgs a) { decode_row(a, blockIdx.x, threadIdx.x, 256); }
+
+__global__ void __launch_bounds__(256) k_decode_fbaq(DecodeFbaqArgs a) {
+    decode_fbaq_row(a, blockIdx.x, threadIdx.x, 256);
+}
+
+__global__ void __launch_bounds__(256) k_zero_nans(float2* img, long long n) {
+    const long long step = static_cast<long long>(gridDim.x) * 256;
+#pragma unroll 4
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += step) zero_nan_item(img, i);
 }
 
 __global__ void __launch_bounds__(256) k_img_moments(ImgMomentsArgs a) {
     __shared__ double red[12 * 256];
-    img_moments_body(a, blockIdx.x, threadIdx.x, blockDim.x, red);
+    img_moments_body(a, blockIdx.x, threadIdx.x, 256, red);
 }
 
-__global__ void __launch_bounds__(256) k_accc(AcccArgs a) { accc_body(a, blockIdx.x, threadIdx.x, blockDim.x); }
+__global__ void __launch_bounds__(kAcccCols) k_accc(AcccArgs a) {
+    __shared__ double cols[2 * kAcccCols];
+    accc_body(a, blockIdx.x, blockIdx.y, gridDim.x, threadIdx.x, kAcccCols, cols);
+}
 
 __global__ void __launch_bounds__(512) k_rc_rows(RcRowsArgs a) {
     extern __shared__ float2 smem_rcr[];
     rc_rows_body(a, blockIdx.x, threadIdx.x, blockDim.x, smem_rcr);
+}
+
+template <int L>
+__global__ void __launch_bounds__(CtSchedule<L>::nthr, 2) k_rc_rows_ct(RcRowsArgs a) {
+    extern __shared__ float2 smem_rcrc[];
+    rc_rows_ct_body<L>(a, blockIdx.x, threadIdx.x, smem_rcrc);
+}
+
+// Matched filter: eight threads share a position's sum.
+__global__ void __launch_bounds__(256) k_matched_filter(MatchedFilterArgs a) {
+    const int pos = blockIdx.x * 32 + (threadIdx.x >> 3);
+    double re = 0.0, im = 0.0;
+    if (pos < a.plan.n) matched_filter_sum(a, pos, threadIdx.x & 7, 8, &re, &im);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        re += __shfl_xor_sync(0xffffffffu, re, o);
+        im += __shfl_xor_sync(0xffffffffu, im, o);
+    }
+    if (pos < a.plan.n && (threadIdx.x & 7) == 0) matched_filter_store(a, pos, re, im);
+}
+
+__global__ void __launch_bounds__(128) k_twiddles(TwiddleArgs a, int count) {
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    if (i < count) twiddle_item(a, i);
+}
+
+__global__ void __launch_bounds__(128) k_rsl(RslArgs a) {
+    const int x = blockIdx.x * 128 + threadIdx.x, y0 = blockIdx.y * kColumnRows;
+    if (x < a.range_size) rsl_column(a, x, y0, min(y0 + kColumnRows, a.az_size));
+}
+
+__global__ void __launch_bounds__(128) k_srgr(SrgrArgs a) {
+    const int x = blockIdx.x * 128 + threadIdx.x, y0 = blockIdx.y * kColumnRows;
+    if (x < a.out_x) srgr_column(a, x, y0, min(y0 + kColumnRows, a.y_size));
 }
 
 // Level-0 gathers: one warp per line, eight lines per block.  A line's own loads form a chain
@@ -646,8 +688,8 @@ int backend_tail(const TailArgs& a, int rows, LaunchShape sh, unsigned int* err,
     return check_launch("tail");
 }
 
-int backend_decode(const DecodeArgs& a, long long n, void* stream) {
-    k_items<DecodeArgs, decode_item><<<grid_for(n), 256, 0, S(stream)>>>(a, n);
+int backend_decode(const DecodeArgs& a, void* stream) {
+    k_decode<<<a.lines, 256, 0, S(stream)>>>(a);
     return check_launch("decode");
 }
 int backend_product_stats(const ProductStatsArgs& a, void* stream) {
@@ -662,8 +704,8 @@ int backend_condition(const ConditionArgs& a, int rows, void* stream) {
     k_condition<<<rows, 256, 0, S(stream)>>>(a);
     return check_launch("condition");
 }
-int backend_decode_fbaq(const DecodeFbaqArgs& a, long long n, void* stream) {
-    k_items<DecodeFbaqArgs, decode_fbaq_item><<<grid_for(n), 256, 0, S(stream)>>>(a, n);
+int backend_decode_fbaq(const DecodeFbaqArgs& a, void* stream) {
+    k_decode_fbaq<<<a.lines, 256, 0, S(stream)>>>(a);
     return check_launch("decode_fbaq");
 }
 int backend_img_moments(const ImgMomentsArgs& a, int blocks, void* stream) {
@@ -675,18 +717,49 @@ int backend_iq_apply(const IqApplyArgs& a, long long n, void* stream) {
     return check_launch("iq_apply");
 }
 int backend_zero_nans(float2* img, long long n, void* stream) {
-    k_items<float2*, zero_nan_item><<<grid_for(n), 256, 0, S(stream)>>>(img, n);
+    k_zero_nans<<<grid_for(n), 256, 0, S(stream)>>>(img, n);
     return check_launch("zero_nans");
 }
-int backend_accc(const AcccArgs& a, int blocks, void* stream) {
-    k_accc<<<blocks, 256, 0, S(stream)>>>(a);
+int backend_accc(const AcccArgs& a, int grid_x, int grid_y, void* stream) {
+    k_accc<<<dim3(grid_x, grid_y), kAcccCols, 0, S(stream)>>>(a);
     return check_launch("accc");
 }
+
+template <int L>
+static int launch_rc_rows_ct(const RcRowsArgs& a, int rows, size_t smem, void* stream) {
+    int rc = ensure_smem(k_rc_rows_ct<L>, smem, "rc_rows");
+    if (rc) return rc;
+    k_rc_rows_ct<L><<<rows, CtSchedule<L>::nthr, smem, S(stream)>>>(a);
+    return check_launch("rc_rows");
+}
+
 int backend_rc_rows(const RcRowsArgs& a, int rows, LaunchShape sh, void* stream) {
+    switch (a.ctw ? a.plan.n : 0) {
+        case 768: return launch_rc_rows_ct<768>(a, rows, sh.smem, stream);
+        case 1024: return launch_rc_rows_ct<1024>(a, rows, sh.smem, stream);
+        case 1536: return launch_rc_rows_ct<1536>(a, rows, sh.smem, stream);
+        case 2048: return launch_rc_rows_ct<2048>(a, rows, sh.smem, stream);
+        case 3072: return launch_rc_rows_ct<3072>(a, rows, sh.smem, stream);
+        case 4096: return launch_rc_rows_ct<4096>(a, rows, sh.smem, stream);
+        case 6144: return launch_rc_rows_ct<6144>(a, rows, sh.smem, stream);
+        case 8192: return launch_rc_rows_ct<8192>(a, rows, sh.smem, stream);
+        default: break;
+    }
     int rc = ensure_smem(k_rc_rows, sh.smem, "rc_rows");
     if (rc) return rc;
     k_rc_rows<<<rows, sh.threads, sh.smem, S(stream)>>>(a);
     return check_launch("rc_rows");
+}
+
+int backend_matched_filter(const MatchedFilterArgs& a, void* stream) {
+    k_matched_filter<<<(a.plan.n + 31) / 32, 256, 0, S(stream)>>>(a);
+    return check_launch("matched_filter");
+}
+
+int backend_twiddles(const TwiddleArgs& a, void* stream) {
+    const int count = twiddle_count(a);
+    k_twiddles<<<(count + 127) / 128, 128, 0, S(stream)>>>(a, count);
+    return check_launch("twiddles");
 }
 int backend_ers_unpack(const ErsUnpackArgs& a, void* stream) {
     if (a.lines <= 0) return ASARF_OK;
@@ -703,12 +776,12 @@ int backend_multilook(const MultilookArgs& a, void* stream) {
     k_multilook<<<a.out_y, 256, 0, S(stream)>>>(a);
     return check_launch("multilook");
 }
-int backend_rsl(const RslArgs& a, long long n, void* stream) {
-    k_items<RslArgs, rsl_item><<<grid_for(n), 256, 0, S(stream)>>>(a, n);
+int backend_rsl(const RslArgs& a, void* stream) {
+    k_rsl<<<dim3((a.range_size + 127) / 128, (a.az_size + kColumnRows - 1) / kColumnRows), 128, 0, S(stream)>>>(a);
     return check_launch("rsl");
 }
-int backend_srgr(const SrgrArgs& a, long long n, void* stream) {
-    k_items<SrgrArgs, srgr_item><<<grid_for(n), 256, 0, S(stream)>>>(a, n);
+int backend_srgr(const SrgrArgs& a, void* stream) {
+    k_srgr<<<dim3((a.out_x + 127) / 128, (a.y_size + kColumnRows - 1) / kColumnRows), 128, 0, S(stream)>>>(a);
     return check_launch("srgr");
 }
 
@@ -745,6 +818,10 @@ int mem_d2d_2d(void* dst, size_t dpitch, const void* src, size_t spitch, size_t 
 }
 int mem_zero(void* dst, size_t n, void* stream) {
     return cuda_rc(cudaMemsetAsync(dst, 0, n, S(stream)), "memset");
+}
+int mem_zero_2d(void* dst, size_t pitch, size_t width, size_t rows, void* stream) {
+    if (width == 0 || rows == 0) return ASARF_OK;
+    return cuda_rc(cudaMemset2DAsync(dst, pitch, 0, width, rows, S(stream)), "2D memset");
 }
 int stream_sync(void* stream) { return cuda_rc(cudaStreamSynchronize(S(stream)), "stream sync"); }
 

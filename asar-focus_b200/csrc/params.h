@@ -356,8 +356,6 @@ struct ImgMomentsArgs {
     int x_size, y_size, x_stride;
     int rows_per_block;
     double* partial;    // [blocks][12]
-    float mean_i, mean_q;   // second pass: sums of (I - mean)^2, (Q - mean)^2 over the data region
-    int centered;
 };
 
 struct IqApplyArgs {
@@ -366,11 +364,14 @@ struct IqApplyArgs {
     float dc_i, dc_q, gain, sin_c, cos_c;
 };
 
+constexpr int kAcccCols = 256;  // columns of one block
 struct AcccArgs {
     const float2* img;
     int x_size, y_size, x_stride;
     int step, nblk, rows_per_block;
-    double* partial;    // [blocks][nblk][2]
+    int xend;           // columns that enter: nblk * step, at most x_stride
+    int span;           // Doppler blocks kAcccCols columns can touch
+    double* partial;    // [row blocks][column blocks][span][2]
 };
 
 struct RcRowsArgs {
@@ -378,7 +379,27 @@ struct RcRowsArgs {
     long long stride;
     int nr, nk, x_zero_end;  // inputs x < nr; keep x < nk; zero [nk, x_zero_end)
     FftPlan plan;
-    const float2* mf;
+    const float2* mf;     // compile-time lengths: transposed, with ctw (fft_ct.cuh)
+    const float2* ctw;
+};
+
+// Matched filter mf = conj(DFT_L(chirp)) * scale in the order of plan's forward transform, L =
+// plan.n; last_radix > 0: transposed for the compile-time lengths (position b * R + q at q * (L / R) + b).
+struct MatchedFilterArgs {
+    const float2* chirp;
+    int nc;
+    FftPlan plan;
+    double scale;
+    int last_radix;
+    float2* mf;
+};
+
+// Twiddle tables: out[m] = exp(-2 pi i m / n), m < n; or, with r[0] > 0, the per-pass tables of the
+// compile-time length n with radices r (fft_ct.cuh).
+struct TwiddleArgs {
+    float2* out;
+    int n;
+    int r[3];
 };
 
 struct MultilookArgs {

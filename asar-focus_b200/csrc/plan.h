@@ -48,7 +48,7 @@ struct asarf_plan {
     uint8_t* raw_dev = nullptr;
     uint16_t* swst_dev = nullptr;
     float* out_dev = nullptr;
-    HostFft rc, f1, f2, fN;
+    HostFft rc, f1, f2;
     float2* rc_mf = nullptr;
     // launch argument blocks
     RawStatsArgs a_stats{};

@@ -32,11 +32,31 @@ struct DevBuf {
 
 int nomem() { return set_error(ASARF_ERR_NOMEM, "device allocation failed"); }
 
+// Several arrays in one device allocation (a call's scratch: one cudaMalloc and one cudaFree).
+struct Scratch {
+    std::vector<size_t> at;
+    size_t bytes = 0;
+    void* p = nullptr;
+    int add(size_t n) {
+        at.push_back(bytes);
+        bytes += (n + 255) / 256 * 256;
+        return static_cast<int>(at.size()) - 1;
+    }
+    bool alloc() { return (p = mem_alloc(bytes)) != nullptr; }
+    template <class T>
+    T* as(int k) const {
+        return reinterpret_cast<T*>(static_cast<unsigned char*>(p) + at[static_cast<size_t>(k)]);
+    }
+    Scratch() = default;
+    ~Scratch() { mem_free(p); }
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+};
+
 // NaN-aware moments of the data block and of the padding columns, summed on the host in a
 // fixed order.
-int image_moments(const float2* img, int x_size, int y_size, int x_stride, float mean_i, float mean_q, int centered,
-                  double out[12], void* stream) {
-    const int rpb = 16;
+int image_moments(const float2* img, int x_size, int y_size, int x_stride, double out[12], void* stream) {
+    const int rpb = 8;
     const int blocks = (y_size + rpb - 1) / rpb;
     DevBuf part(sizeof(double) * 12 * static_cast<size_t>(blocks));
     if (!part.p) return nomem();
@@ -47,9 +67,6 @@ int image_moments(const float2* img, int x_size, int y_size, int x_stride, float
     a.x_stride = x_stride;
     a.rows_per_block = rpb;
     a.partial = part.as<double>();
-    a.mean_i = mean_i;
-    a.mean_q = mean_q;
-    a.centered = centered;
     int rc = backend_img_moments(a, blocks, stream);
     if (rc) return rc;
     std::vector<double> h(12 * static_cast<size_t>(blocks));
@@ -83,7 +100,7 @@ int asarf_convert_ers_samples(const uint8_t* d_raw, int32_t raw_line_bytes, int3
     a.min_swst = min_swst;
     a.img = static_cast<float2*>(d_img);
     a.stride = img_stride;
-    int rc = backend_decode(a, static_cast<long long>(lines) * range_size, stream);
+    int rc = backend_decode(a, stream);
     if (rc) return rc;
     return stream_sync(stream);
 }
@@ -105,7 +122,7 @@ int asarf_convert_asar_blocks(const uint8_t* d_raw, int32_t record_bytes, int32_
     a.lut_q = d_lut_q;
     a.img = static_cast<float2*>(d_img);
     a.stride = img_stride;
-    int rc = backend_decode_fbaq(a, static_cast<long long>(records) * range_size, stream);
+    int rc = backend_decode_fbaq(a, stream);
     if (rc) return rc;
     return stream_sync(stream);
 }
@@ -154,21 +171,18 @@ int asarf_raw_data_correction(void* d_img, int32_t x_size, int32_t y_size, int32
         return set_error(ASARF_ERR_INVALID, "raw_data_correction: bad arguments");
     float2* img = static_cast<float2*>(d_img);
     double m[12];
-    int rc = image_moments(img, x_size, y_size, x_stride, 0.0f, 0.0f, 0, m, stream);
+    int rc = image_moments(img, x_size, y_size, x_stride, m, stream);
     if (rc) return rc;
     const double total = n_total_samples > 0 ? static_cast<double>(n_total_samples) : static_cast<double>(x_size) * y_size;
     const float totf = static_cast<float>(total);
     // CalcMean: float(double sum) / float(total)
     const float dc_i = static_cast<float>(m[1]) / totf;
     const float dc_q = static_cast<float>(m[2]) / totf;
-    double c[12];
-    rc = image_moments(img, x_size, y_size, x_stride, dc_i, dc_q, 1, c, stream);
-    if (rc) return rc;
-    const float std_i = std::sqrt(static_cast<float>(c[3]) / totf);
-    const float std_q = std::sqrt(static_cast<float>(c[4]) / totf);
-    // gain / phase sums over x < XStride after the DC step, both regions (closed forms)
+    // sums over x < XStride after the DC step, both regions (closed forms of the FP64 moments)
     const double di = dc_i, dq = dc_q;
     auto sq = [&](int o, int s1, int s2, double d) { return m[o + s2] - 2.0 * d * m[o + s1] + m[o] * d * d; };
+    const float std_i = std::sqrt(static_cast<float>(sq(0, 1, 3, di)) / totf);
+    const float std_q = std::sqrt(static_cast<float>(sq(0, 2, 4, dq)) / totf);
     const double i1sq = sq(0, 1, 3, di) + sq(6, 1, 3, di);
     const double q1sq = sq(0, 2, 4, dq) + sq(6, 2, 4, dq);
     auto cross = [&](int o) { return m[o + 5] - dq * m[o + 1] - di * m[o + 2] + m[o] * di * dq; };
@@ -215,24 +229,30 @@ int asarf_doppler_centroid(const void* d_img, int32_t x_size, int32_t y_size, in
     a.step = x_size / 32;
     a.nblk = (x_size + a.step - 1) / a.step;
     a.rows_per_block = 256;
-    const int blocks = (y_size + a.rows_per_block - 1) / a.rows_per_block;
-    const int xend = std::min(a.nblk * a.step, x_stride);
-    DevBuf part(sizeof(double) * 2 * static_cast<size_t>(xend) * blocks);
+    a.xend = std::min(a.nblk * a.step, x_stride);
+    a.span = (kAcccCols - 1) / a.step + 2;
+    const int gx = (a.xend + kAcccCols - 1) / kAcccCols, gy = (y_size + a.rows_per_block - 1) / a.rows_per_block;
+    const size_t count = 2 * static_cast<size_t>(a.span) * gx * gy;
+    DevBuf part(sizeof(double) * count);
     if (!part.p) return nomem();
     a.partial = part.as<double>();
-    int rc = backend_accc(a, blocks, stream);
+    int rc = backend_accc(a, gx, gy, stream);
     if (rc) return rc;
-    std::vector<double> h(2 * static_cast<size_t>(xend) * blocks);
-    rc = mem_d2h(h.data(), part.p, sizeof(double) * h.size(), stream);
+    std::vector<double> h(count);
+    rc = mem_d2h(h.data(), part.p, sizeof(double) * count, stream);
     if (rc) return rc;
     rc = stream_sync(stream);
     if (rc) return rc;
     std::vector<double> re(a.nblk, 0.0), im(a.nblk, 0.0), xs(a.nblk), ys(a.nblk);
-    for (int b = 0; b < blocks; ++b)
-        for (int x = 0; x < xend; ++x) {
-            re[x / a.step] += h[(static_cast<size_t>(b) * xend + x) * 2];
-            im[x / a.step] += h[(static_cast<size_t>(b) * xend + x) * 2 + 1];
-        }
+    for (int by = 0; by < gy; ++by)
+        for (int bx = 0; bx < gx; ++bx)
+            for (int k = 0; k < a.span; ++k) {
+                const int b = bx * kAcccCols / a.step + k;
+                if (b >= a.nblk) break;
+                const double* v = &h[2 * (static_cast<size_t>(a.span) * (static_cast<size_t>(by) * gx + bx) + k)];
+                re[b] += v[0];
+                im[b] += v[1];
+            }
     for (int k = 0; k < a.nblk; ++k) {
         ys[k] = prf * (std::atan2(im[k], re[k]) / (2.0 * 3.14159265358979323846));
         xs[k] = static_cast<double>((k * a.step + (k + 1) * a.step) / 2);
@@ -249,15 +269,23 @@ int asarf_range_compression(void* d_img, int32_t x_size, int32_t y_size, int32_t
     if (chirp_len != x_stride) return set_error(ASARF_ERR_INVALID, "Range padding and chirp size mismatch");
     HostFft fft;
     const int L = choose_rc_len(x_size);
-    if (L < x_size || !build_fft(L, fft)) return set_error(ASARF_ERR_INVALID, "range_compression: no FFT length");
-    std::vector<std::complex<float>> chirp(chirp_samples);
-    for (int i = 0; i < chirp_samples; ++i) chirp[i] = {chirp_padded[2 * i], chirp_padded[2 * i + 1]};
-    std::vector<float2> mf;
-    matched_filter_table(chirp.data(), chirp_samples, fft, mf);
-    DevBuf tw(sizeof(float2) * L), mfd(sizeof(float2) * L);
-    if (!tw.p || !mfd.p) return nomem();
-    int rc = mem_h2d(tw.p, fft.tw.data(), sizeof(float2) * L, stream);
-    if (!rc) rc = mem_h2d(mfd.p, mf.data(), sizeof(float2) * L, stream);
+    int ct[3];
+    const int n_ct = L >= x_size ? ct_radices(L, ct) : 0;
+    if (L < x_size || !(n_ct ? build_fft_radices(L, std::vector<int>(ct, ct + n_ct), fft) : build_fft(L, fft)))
+        return set_error(ASARF_ERR_INVALID, "range_compression: no FFT length");
+    const LaunchShape sh{512, sizeof(float2) * static_cast<size_t>(n_ct ? ct_smem_elems_of(L) : L)};
+    if (sh.smem > smem_optin_limit())
+        return set_error(ASARF_ERR_INVALID, "range_compression: range FFT of %d samples exceeds shared memory", L);
+    TwiddleArgs tw = n_ct ? ct_twiddle_args(L, nullptr) : TwiddleArgs{nullptr, L, {0, 0, 0}};
+    Scratch m;
+    const int k_chirp = m.add(sizeof(float2) * chirp_samples), k_mf = m.add(sizeof(float2) * L),
+              k_tw = m.add(sizeof(float2) * twiddle_count(tw));
+    if (!m.alloc()) return nomem();
+    tw.out = m.as<float2>(k_tw);
+    int rc = mem_h2d(m.as<float2>(k_chirp), chirp_padded, sizeof(float2) * chirp_samples, stream);
+    if (!rc) rc = backend_matched_filter(matched_filter_args(m.as<float2>(k_chirp), chirp_samples, fft, m.as<float2>(k_mf)),
+                                         stream);
+    if (!rc) rc = backend_twiddles(tw, stream);
     if (rc) return rc;
     RcRowsArgs a{};
     a.img = static_cast<float2*>(d_img);
@@ -266,11 +294,9 @@ int asarf_range_compression(void* d_img, int32_t x_size, int32_t y_size, int32_t
     a.nk = x_size - chirp_samples;
     a.x_zero_end = x_stride;
     a.plan = fft.plan;
-    a.plan.tw = tw.as<float2>();
-    a.mf = mfd.as<float2>();
-    const LaunchShape sh{512, sizeof(float2) * static_cast<size_t>(L)};
-    if (sh.smem > smem_optin_limit())
-        return set_error(ASARF_ERR_INVALID, "range_compression: range FFT of %d samples exceeds shared memory", L);
+    a.plan.tw = n_ct ? nullptr : tw.out;
+    a.ctw = n_ct ? tw.out : nullptr;
+    a.mf = m.as<float2>(k_mf);
     rc = backend_rc_rows(a, y_size, sh, stream);
     if (rc) return rc;
     if (new_x_size) *new_x_size = a.nk;
@@ -296,15 +322,21 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     if ((hl + hr) & 1) ++hr;  // column-pair transforms need an even tile width
     const int n2 = choose_az_n2(N, x_size, hl, hr, false);
     const int n1 = N / n2;
-    HostFft f1, f2, fN;
-    if (n2 < 2 || !build_fft_radices(n1, strided_radices(n1), f1) || !build_fft_radices(n2, block_radices(n2), f2) ||
-        !build_fft(N, fN))
+    HostFft f1, f2;
+    if (n2 < 2 || !build_fft_radices(n1, strided_radices(n1), f1) || !build_fft_radices(n2, block_radices(n2), f2))
         return set_error(ASARF_ERR_INVALID, "range_doppler: azimuth size %d is not 2^a3^b5^c7^d", N);
     // tables + a finalised state carrying the Doppler polynomial
-    DevBuf tw1(sizeof(float2) * n1), dr1(sizeof(int) * n1), tw2(sizeof(float2) * n2), dr2(sizeof(int) * n2),
-        twN(sizeof(float2) * N), st(sizeof(FocusState)),
-        rcmc(sizeof(float) * static_cast<size_t>(kRcmcNodes + 1) * kRcmcRowFloats);
-    if (!tw1.p || !dr1.p || !tw2.p || !dr2.p || !twN.p || !st.p || !rcmc.p) return nomem();
+    Scratch m;
+    const int k_tw1 = m.add(sizeof(float2) * n1), k_dr1 = m.add(sizeof(int) * n1), k_tw2 = m.add(sizeof(float2) * n2),
+              k_dr2 = m.add(sizeof(int) * n2), k_twn = m.add(sizeof(float2) * N), k_st = m.add(sizeof(FocusState)),
+              k_rcmc = m.add(sizeof(float) * static_cast<size_t>(kRcmcNodes + 1) * kRcmcRowFloats);
+    if (!m.alloc()) return nomem();
+    float2* tw1 = m.as<float2>(k_tw1);
+    int* dr1 = m.as<int>(k_dr1);
+    float2* tw2 = m.as<float2>(k_tw2);
+    int* dr2 = m.as<int>(k_dr2);
+    float2* twN = m.as<float2>(k_twn);
+    float* rcmc = m.as<float>(k_rcmc);
     FocusState hs{};
     for (int k = 0; k < 3; ++k) {
         hs.dc_poly[k] = prm->dc_poly[k];
@@ -312,18 +344,17 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     }
     hs.first_line = 0;
     hs.n_lines = y_size;  // inverse pass stores the data rows only
-    int rc = mem_h2d(tw1.p, f1.tw.data(), sizeof(float2) * n1, stream);
-    if (!rc) rc = mem_h2d(dr1.p, f1.drev.data(), sizeof(int) * n1, stream);
-    if (!rc) rc = mem_h2d(tw2.p, f2.tw.data(), sizeof(float2) * n2, stream);
-    if (!rc) rc = mem_h2d(dr2.p, f2.drev.data(), sizeof(int) * n2, stream);
-    if (!rc) rc = mem_h2d(twN.p, fN.tw.data(), sizeof(float2) * N, stream);
-    if (!rc) rc = mem_h2d(st.p, &hs, sizeof(hs), stream);
-    if (!rc) rc = backend_rcmc_table(rcmc.as<float>(), stream);
-    if (!rc) rc = mem_zero(d_out, sizeof(float2) * static_cast<size_t>(x_stride) * y_stride, stream);
+    FocusState* dstate = m.as<FocusState>(k_st);
+    int rc = mem_h2d(tw1, f1.tw.data(), sizeof(float2) * n1, stream);
+    if (!rc) rc = mem_h2d(dr1, f1.drev.data(), sizeof(int) * n1, stream);
+    if (!rc) rc = mem_h2d(tw2, f2.tw.data(), sizeof(float2) * n2, stream);
+    if (!rc) rc = mem_h2d(dr2, f2.drev.data(), sizeof(int) * n2, stream);
+    if (!rc) rc = mem_h2d(dstate, &hs, sizeof(hs), stream);
+    if (!rc) rc = backend_twiddles(TwiddleArgs{twN, N, {0, 0, 0}}, stream);
+    if (!rc) rc = backend_rcmc_table(rcmc, stream);
     if (rc) return rc;
-    f1.plan.tw = tw1.as<float2>();
-    f2.plan.tw = tw2.as<float2>();
-    FocusState* dstate = st.as<FocusState>();
+    f1.plan.tw = tw1;
+    f2.plan.tw = tw2;
     float2* src = static_cast<float2*>(d_src);
     float2* out = static_cast<float2*>(d_out);
     const int xt1 = (n1 * 32 * 8 <= 160 * 1024) ? 32 : 16;
@@ -334,8 +365,8 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     fwd.n1 = n1;
     fwd.n2 = n2;
     fwd.plan1 = f1.plan;
-    fwd.drev1 = dr1.as<int>();
-    fwd.twn = twN.as<float2>();
+    fwd.drev1 = dr1;
+    fwd.twn = twN;
     fwd.nk = x_size;
     fwd.xt = xt1;
     fwd.valid_rows = N;  // the reference transforms every row of the padded image
@@ -355,7 +386,7 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     d.n2 = n2;
     d.az_pad = N;
     d.plan2 = f2.plan;
-    d.drev2 = dr2.as<int>();
+    d.drev2 = dr2;
     d.nk = x_size;
     d.hl = hl;
     d.hr = hr;
@@ -370,17 +401,31 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     d.range_spacing = prm->range_spacing;
     for (int k = 0; k < 3; ++k) d.vr_poly[k] = static_cast<float>(prm->vr_poly[k]);
     d.state = dstate;
-    d.rcmc = rcmc.as<float>();
+    d.rcmc = rcmc;
     const int tiles1 = (x_size + xt1 - 1) / xt1, tiles2 = (x_size + d.xt - 1) / d.xt;
     fwd.nb = inv.nb = xt1 == 32 ? az_strided_tiles_per_block(n1, n2, tiles1) : 1;
     const LaunchShape sh_st{256, az_strided_smem(n1, xt1, fwd.nb)};
     const LaunchShape sh_rd{512, az_rd_smem(n2, d.wt, d.xt, false)};
     if (sh_st.smem > smem_optin_limit() || sh_rd.smem > smem_optin_limit())
         return set_error(ASARF_ERR_INVALID, "range_doppler: tiles exceed shared memory (n1 %d, n2 %d)", n1, n2);
-    rc = backend_az_strided(fwd, nullptr, tiles1, sh_st, stream);
-    if (!rc) rc = backend_az_rd(d, nullptr, tiles2, n1, sh_rd, &dstate->errors, stream);
-    if (!rc) rc = backend_az_strided(inv, nullptr, tiles1, sh_st, stream);
-    // rows past the data block still hold the spectrum stage's values: clear them
+    // tiles by TMA where the caller's rows are 16-byte aligned, as the planned path's always are
+    alignas(64) unsigned char map_src3[128], map_out3[128], map_src2[128];
+    bool tma = x_stride % 2 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 &&
+               (reinterpret_cast<uintptr_t>(out) & 15) == 0 && 2 * d.wt <= 256;
+    if (tma) {
+        fwd.n1_box = inv.n1_box = largest_divisor_le(n1, 256);
+        d.n2_box = largest_divisor_le(n2, 256);
+        tma = make_azimuth_maps(src, out, x_size, x_stride, n1, n2, xt1, fwd.nb, fwd.n1_box, d.wt, d.n2_box, map_src3,
+                                map_out3, map_src2);
+    }
+    fwd.use_tma = inv.use_tma = d.use_tma = tma ? 1 : 0;
+    fwd.compiled = inv.compiled = d.compiled = 1;
+    rc = backend_az_strided(fwd, tma ? map_src3 : nullptr, tiles1, sh_st, stream);
+    if (!rc) rc = backend_az_rd(d, tma ? map_src2 : nullptr, tiles2, n1, sh_rd, &dstate->errors, stream);
+    if (!rc) rc = backend_az_strided(inv, tma ? map_out3 : nullptr, tiles1, sh_st, stream);
+    // everything outside the data block is zero: columns past it, and the rows past it, which still
+    // hold the spectrum stage's values
+    if (!rc) rc = mem_zero_2d(out + x_size, sizeof(float2) * x_stride, sizeof(float2) * (x_stride - x_size), y_size, stream);
     if (!rc && y_size < N)
         rc = mem_zero(out + static_cast<size_t>(y_size) * x_stride,
                       sizeof(float2) * static_cast<size_t>(N - y_size) * x_stride, stream);
@@ -422,7 +467,7 @@ int asarf_range_spreading_loss(float* d_img, int32_t range_size, int32_t azimuth
     a.slant_first = slant_range_first;
     a.range_spacing = range_spacing;
     a.ref_range = reference_range;
-    int rc = backend_rsl(a, static_cast<long long>(range_size) * azimuth_size, stream);
+    int rc = backend_rsl(a, stream);
     if (rc) return rc;
     return stream_sync(stream);
 }
@@ -440,7 +485,7 @@ static int srgr_common(const float* d_in, int32_t in_x, int32_t y_size, const do
     a.out = d_out;
     a.start = d_start;
     a.frac = d_frac;
-    int rc = backend_srgr(a, static_cast<long long>(out_x) * y_size, stream);
+    int rc = backend_srgr(a, stream);
     if (rc) return rc;
     return stream_sync(stream);
 }
