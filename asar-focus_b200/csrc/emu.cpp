@@ -247,6 +247,11 @@ int backend_srgr(const SrgrArgs& a, void*) {
 
 void* mem_alloc(size_t bytes) { return std::calloc(1, bytes ? bytes : 1); }
 void mem_free(void* p) { std::free(p); }
+void* scratch_alloc(size_t bytes, void*, bool* pooled) {
+    *pooled = false;
+    return mem_alloc(bytes);
+}
+void scratch_free(void* p, void*, bool) { mem_free(p); }
 int mem_h2d(void* dst, const void* src, size_t n, void*) {
     std::memcpy(dst, src, n);
     return ASARF_OK;

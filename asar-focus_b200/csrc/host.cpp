@@ -402,14 +402,13 @@ double transform_gain(const HostFft& h, bool table_powers) {
     double total = 0.0;
     for (int i = 0; i < h.plan.nst; ++i) {
         const int R = h.plan.radix[i], S = h.plan.span[i], step = h.plan.n / (S * R);
-        // a stage's outputs average w~^q conj(w^q) over its offsets j and powers q, w~^q from the table
-        // or by the recurrence of pair_twiddle
+        // a stage's outputs average w~^q conj(w^q) over its offsets j and powers q, w~^q by the
+        // recurrence of pair_twiddle (table entries are rounded each for itself and average out)
         double sum = 0.0;
-        for (int j = 1; j < S; ++j) {
+        for (int j = 1; j < S && !table_powers; ++j) {
             const float2 w1 = h.tw[static_cast<size_t>(j) * step];
             float2 w = w1;
             for (int q = 1; q < R; ++q) {
-                if (table_powers) w = h.tw[static_cast<size_t>(j) * q * step];
                 const double a = -2.0 * kPi * static_cast<double>(static_cast<long long>(j) * q % (S * R)) / (S * R);
                 sum += w.x * std::cos(a) + w.y * std::sin(a) - 1.0;
                 w = make_float2(std::fma(-w1.y, w.y, w1.x * w.x), std::fma(w1.x, w.y, w1.y * w.x));
@@ -488,7 +487,7 @@ int choose_az_n2(int N, int nk, int hl, int hr, bool absolute_phase) {
         if (blocks < kAzRdMinBlocks) continue;
         const std::vector<int> radices = block_radices(d);
         HostFft f;
-        if (!build_fft_radices(d, radices, f)) continue;
+        if (!build_fft_radices(d, radices, f, false)) continue;
         double t = 6.5 + 0.142 * d + 6.0 * std::max(0, f.plan.nst - 3);
         if (*std::max_element(radices.begin(), radices.end()) <= 5) t *= 0.93;
         if (!block_schedule_compiled(f.plan)) t *= 1.1;
@@ -499,7 +498,7 @@ int choose_az_n2(int N, int nk, int hl, int hr, bool absolute_phase) {
     return best;
 }
 
-bool build_fft_radices(int n, const std::vector<int>& f, HostFft& h) {
+bool build_fft_radices(int n, const std::vector<int>& f, HostFft& h, bool with_twiddles) {
     long long prod = 1;
     for (int r : f) prod *= r;
     if (f.empty() || prod != n || static_cast<int>(f.size()) > kMaxStages) return false;
@@ -525,8 +524,8 @@ bool build_fft_radices(int n, const std::vector<int>& f, HostFft& h) {
         }
         h.drev[p] = k;
     }
-    h.tw.resize(n);
-    for (int m = 0; m < n; ++m) {
+    h.tw.resize(with_twiddles ? n : 0);
+    for (int m = 0; m < n && with_twiddles; ++m) {
         const double a = -2.0 * kPi * static_cast<double>(m) / n;
         h.tw[m] = make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a)));
     }
@@ -732,7 +731,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     // compile-time lengths use their own three-pass radix sequence (and so its output order)
     int ctr[3];
     const int n_ctr = ct_radices(p->rc_len, ctr);
-    const bool rc_ok = n_ctr ? build_fft_radices(p->rc_len, std::vector<int>(ctr, ctr + n_ctr), p->rc)
+    const bool rc_ok = n_ctr ? build_fft_radices(p->rc_len, std::vector<int>(ctr, ctr + n_ctr), p->rc, false)
                              : build_fft(p->rc_len, p->rc);
     // Vr polynomial
     if (s.vr_poly_given) {
@@ -880,7 +879,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     p->raw_dev = p->alloc<uint8_t>(static_cast<size_t>(p->na) * s.raw_line_bytes);
     p->swst_dev = p->alloc<uint16_t>(p->na);
     p->out_dev = p->alloc<float>(static_cast<size_t>(p->out_bytes + 3) / 4);
-    float2* rc_tw = p->alloc<float2>(p->rc_len);
+    float2* rc_tw = n_ctr ? nullptr : p->alloc<float2>(p->rc_len);
     p->rc_mf = p->alloc<float2>(p->rc_len);
     TwiddleArgs ctw = ct_twiddle_args(p->rc_len, nullptr);
     float2* ct_tw = ctw.out = n_ctr ? p->alloc<float2>(static_cast<size_t>(twiddle_count(ctw))) : nullptr;
@@ -909,7 +908,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     FloatStatAccum* facc_dev = fbaq ? p->alloc<FloatStatAccum>(1) : nullptr;
     constexpr int kPstatBlocks = 4 * 148;
     double* pstat_dev = opt.sq_stats ? p->alloc<double>(5 * kPstatBlocks + 4) : nullptr;
-    if (!p->bufA || !p->bufB || !p->acc || !p->state || !p->raw_dev || !p->swst_dev || !p->out_dev || !rc_tw ||
+    if (!p->bufA || !p->bufB || !p->acc || !p->state || !p->raw_dev || !p->swst_dev || !p->out_dev || (!n_ctr && !rc_tw) ||
         !p->rc_mf || !chirp_dev || (n_ctr && !ct_tw) || !tw1 || !drev1 || !tw2 || !drev2 || !twN || !rcmc || !rsl_dev || (fbaq && (!lut_dev || !part_dev || !facc_dev)) ||
         (opt.sq_stats && !pstat_dev)) {
         const size_t need = p->bytes;
@@ -918,7 +917,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
                          (need + 2 * img * sizeof(float2)) >> 20);
     }
     rc = 0;
-    rc |= mem_h2d(rc_tw, p->rc.tw.data(), sizeof(float2) * p->rc_len, nullptr);
+    if (rc_tw) rc |= mem_h2d(rc_tw, p->rc.tw.data(), sizeof(float2) * p->rc_len, nullptr);
     rc |= mem_h2d(chirp_dev, chirp.data(), sizeof(float2) * p->nc, nullptr);
     rc |= backend_matched_filter(matched_filter_args(chirp_dev, p->nc, p->rc, p->rc_mf), nullptr);
     if (ct_tw) rc |= backend_twiddles(ctw, nullptr);

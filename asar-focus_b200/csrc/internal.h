@@ -25,8 +25,9 @@ int max_aperture_pixels(const asarf_scene& s);
 int srgr_poly(const asarf_scene& s, double slant_first, int range_size, int azimuth_size, double lti, double poly[5],
               int* ng);
 bool build_fft(int n, HostFft& h);
-// Same with an explicit radix sequence (product n), e.g. a compile-time schedule's.
-bool build_fft_radices(int n, const std::vector<int>& radices, HostFft& h);
+// Same with an explicit radix sequence (product n), e.g. a compile-time schedule's; without the
+// twiddle table where only the schedule and order are wanted.
+bool build_fft_radices(int n, const std::vector<int>& radices, HostFft& h, bool with_twiddles = true);
 // radices of the strided azimuth pass: pairs of 3s merged into radix 9
 std::vector<int> strided_radices(int n);
 // radices of the contiguous azimuth pass: three of at most 8 when n allows, largest first

@@ -13,6 +13,7 @@
 #include "asarf.h"
 #include "backend.h"
 #include "bodies.cuh"
+#include "context_cache.h"
 #include "tc.cuh"
 #include "tma.cuh"
 
@@ -796,6 +797,51 @@ void* mem_alloc(size_t bytes) {
 
 void mem_free(void* p) {
     if (p) cudaFree(p);
+}
+
+// The library's scratch pool of the current context (keyed by the context's id, as a pool made before a
+// device reset must not be used after it), or null.
+static cudaMemPool_t scratch_pool() {
+    static ContextAddressCache<64> pools;
+    unsigned long long id = 0;
+    if (current_context_id(&id) != ASARF_OK || id == 0) return nullptr;
+    void* pool = nullptr;
+    pools.get(id, [](void** out) {
+        int dev = 0, supported = 0;
+        cudaGetDevice(&dev);
+        cudaMemPool_t made = nullptr;
+        if (cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, dev) == cudaSuccess && supported) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            unsigned long long keep = kScratchKept;
+            if (cudaMemPoolCreate(&made, &props) != cudaSuccess) made = nullptr;
+            if (made && cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+                cudaMemPoolDestroy(made);
+                made = nullptr;
+            }
+        }
+        cudaGetLastError();
+        *out = made;
+        return 0;
+    }, &pool);
+    return static_cast<cudaMemPool_t>(pool);
+}
+
+void* scratch_alloc(size_t bytes, void* stream, bool* pooled) {
+    void* p = nullptr;
+    cudaMemPool_t pool = scratch_pool();
+    *pooled = pool && cudaMallocFromPoolAsync(&p, bytes, pool, S(stream)) == cudaSuccess;
+    if (*pooled) return p;
+    cudaGetLastError();
+    return mem_alloc(bytes);
+}
+
+void scratch_free(void* p, void* stream, bool pooled) {
+    if (!p) return;
+    if (pooled) cudaFreeAsync(p, S(stream));
+    else cudaFree(p);
 }
 
 static int cuda_rc(cudaError_t e, const char* what) {

@@ -27,19 +27,6 @@
 #include "context_cache.h"
 
 namespace asarf {
-namespace {
-
-// Accumulators + finalisation state: 5.8 KB + ~1 KB, inside a fixed 8 KiB array.
-struct NoallocScratch {
-    StatAccum acc;
-    FocusState state;
-};
-constexpr size_t kNoallocScratchBytes = 8192;
-static_assert(sizeof(NoallocScratch) <= kNoallocScratchBytes, "scratch layout exceeds the static array");
-
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocScratchBytes];
-
-ContextAddressCache<64> g_scratch_cache;
 
 // Unique id of the calling thread's current CUDA context (0 when none is current yet),
 // through the driver entry points the runtime exposes.
@@ -60,15 +47,29 @@ int current_context_id(unsigned long long* id) {
         cudaGetLastError();
     });
     if (!get_current || !get_id)
-        return set_error(ASARF_ERR_CUDA, "raw_statistics_noalloc: cuCtxGetCurrent / cuCtxGetId unavailable");
+        return set_error(ASARF_ERR_CUDA, "cuCtxGetCurrent / cuCtxGetId unavailable");
     CUcontext ctx = nullptr;
     if (get_current(&ctx) != CUDA_SUCCESS)
-        return set_error(ASARF_ERR_CUDA, "raw_statistics_noalloc: cuCtxGetCurrent failed");
+        return set_error(ASARF_ERR_CUDA, "cuCtxGetCurrent failed");
     *id = 0;
     if (ctx && get_id(ctx, id) != CUDA_SUCCESS)
-        return set_error(ASARF_ERR_CUDA, "raw_statistics_noalloc: cuCtxGetId failed");
+        return set_error(ASARF_ERR_CUDA, "cuCtxGetId failed");
     return ASARF_OK;
 }
+
+namespace {
+
+// Accumulators + finalisation state: 5.8 KB + ~1 KB, inside a fixed 8 KiB array.
+struct NoallocScratch {
+    StatAccum acc;
+    FocusState state;
+};
+constexpr size_t kNoallocScratchBytes = 8192;
+static_assert(sizeof(NoallocScratch) <= kNoallocScratchBytes, "scratch layout exceeds the static array");
+
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocScratchBytes];
+
+ContextAddressCache<64> g_scratch_cache;
 
 int resolve_scratch(void** p) {
     *p = nullptr;

@@ -18,55 +18,46 @@ using namespace asarf;
 
 namespace {
 
-struct DevBuf {
-    void* p = nullptr;
-    explicit DevBuf(size_t n) : p(mem_alloc(n)) {}
-    ~DevBuf() { mem_free(p); }
-    DevBuf(const DevBuf&) = delete;
-    DevBuf& operator=(const DevBuf&) = delete;
-    template <class T>
-    T* as() const {
-        return static_cast<T*>(p);
-    }
-};
-
-int nomem() { return set_error(ASARF_ERR_NOMEM, "device allocation failed"); }
-
-// Several arrays in one device allocation (a call's scratch: one cudaMalloc and one cudaFree).
+// A call's device arrays in one allocation (scratch_alloc) on its stream.
 struct Scratch {
+    void* stream;
     std::vector<size_t> at;
     size_t bytes = 0;
     void* p = nullptr;
+    bool pooled = false;
+    explicit Scratch(void* s) : stream(s) {}
+    ~Scratch() { scratch_free(p, stream, pooled); }
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
     int add(size_t n) {
         at.push_back(bytes);
         bytes += (n + 255) / 256 * 256;
         return static_cast<int>(at.size()) - 1;
     }
-    bool alloc() { return (p = mem_alloc(bytes)) != nullptr; }
+    bool alloc() { return (p = scratch_alloc(bytes, stream, &pooled)) != nullptr; }
     template <class T>
     T* as(int k) const {
         return reinterpret_cast<T*>(static_cast<unsigned char*>(p) + at[static_cast<size_t>(k)]);
     }
-    Scratch() = default;
-    ~Scratch() { mem_free(p); }
-    Scratch(const Scratch&) = delete;
-    Scratch& operator=(const Scratch&) = delete;
 };
+
+int nomem() { return set_error(ASARF_ERR_NOMEM, "device allocation failed"); }
 
 // NaN-aware moments of the data block and of the padding columns, summed on the host in a
 // fixed order.
 int image_moments(const float2* img, int x_size, int y_size, int x_stride, double out[12], void* stream) {
     const int rpb = 8;
     const int blocks = (y_size + rpb - 1) / rpb;
-    DevBuf part(sizeof(double) * 12 * static_cast<size_t>(blocks));
-    if (!part.p) return nomem();
+    Scratch part(stream);
+    part.add(sizeof(double) * 12 * static_cast<size_t>(blocks));
+    if (!part.alloc()) return nomem();
     ImgMomentsArgs a{};
     a.img = img;
     a.x_size = x_size;
     a.y_size = y_size;
     a.x_stride = x_stride;
     a.rows_per_block = rpb;
-    a.partial = part.as<double>();
+    a.partial = part.as<double>(0);
     int rc = backend_img_moments(a, blocks, stream);
     if (rc) return rc;
     std::vector<double> h(12 * static_cast<size_t>(blocks));
@@ -233,9 +224,10 @@ int asarf_doppler_centroid(const void* d_img, int32_t x_size, int32_t y_size, in
     a.span = (kAcccCols - 1) / a.step + 2;
     const int gx = (a.xend + kAcccCols - 1) / kAcccCols, gy = (y_size + a.rows_per_block - 1) / a.rows_per_block;
     const size_t count = 2 * static_cast<size_t>(a.span) * gx * gy;
-    DevBuf part(sizeof(double) * count);
-    if (!part.p) return nomem();
-    a.partial = part.as<double>();
+    Scratch part(stream);
+    part.add(sizeof(double) * count);
+    if (!part.alloc()) return nomem();
+    a.partial = part.as<double>(0);
     int rc = backend_accc(a, gx, gy, stream);
     if (rc) return rc;
     std::vector<double> h(count);
@@ -271,13 +263,13 @@ int asarf_range_compression(void* d_img, int32_t x_size, int32_t y_size, int32_t
     const int L = choose_rc_len(x_size);
     int ct[3];
     const int n_ct = L >= x_size ? ct_radices(L, ct) : 0;
-    if (L < x_size || !(n_ct ? build_fft_radices(L, std::vector<int>(ct, ct + n_ct), fft) : build_fft(L, fft)))
+    if (L < x_size || !(n_ct ? build_fft_radices(L, std::vector<int>(ct, ct + n_ct), fft, false) : build_fft(L, fft)))
         return set_error(ASARF_ERR_INVALID, "range_compression: no FFT length");
     const LaunchShape sh{512, sizeof(float2) * static_cast<size_t>(n_ct ? ct_smem_elems_of(L) : L)};
     if (sh.smem > smem_optin_limit())
         return set_error(ASARF_ERR_INVALID, "range_compression: range FFT of %d samples exceeds shared memory", L);
     TwiddleArgs tw = n_ct ? ct_twiddle_args(L, nullptr) : TwiddleArgs{nullptr, L, {0, 0, 0}};
-    Scratch m;
+    Scratch m(stream);
     const int k_chirp = m.add(sizeof(float2) * chirp_samples), k_mf = m.add(sizeof(float2) * L),
               k_tw = m.add(sizeof(float2) * twiddle_count(tw));
     if (!m.alloc()) return nomem();
@@ -326,7 +318,7 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     if (n2 < 2 || !build_fft_radices(n1, strided_radices(n1), f1) || !build_fft_radices(n2, block_radices(n2), f2))
         return set_error(ASARF_ERR_INVALID, "range_doppler: azimuth size %d is not 2^a3^b5^c7^d", N);
     // tables + a finalised state carrying the Doppler polynomial
-    Scratch m;
+    Scratch m(stream);
     const int k_tw1 = m.add(sizeof(float2) * n1), k_dr1 = m.add(sizeof(int) * n1), k_tw2 = m.add(sizeof(float2) * n2),
               k_dr2 = m.add(sizeof(int) * n2), k_twn = m.add(sizeof(float2) * N), k_st = m.add(sizeof(FocusState)),
               k_rcmc = m.add(sizeof(float) * static_cast<size_t>(kRcmcNodes + 1) * kRcmcRowFloats);
