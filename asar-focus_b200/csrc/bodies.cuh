@@ -439,12 +439,18 @@ ASARF_HD ASARF_INLINE bool fbaq_sample(const uint8_t* rec, int len, int r, const
     return true;
 }
 
-// Statistics of FBAQ4 records: the sums of k_raw_stats over the decoded float samples, in
+// Statistics of FBAQ4 records: the sums of k_raw_stats over the decoded samples, in
 // FP64.  Tile (bx, by) = 32 columns x kFbaqStatsLines lines; warp w of the block takes lines
 // [y0 + w * sub, y0 + (w + 1) * sub) of the tile, lane = column.  Per-lane sums are combined
 // over the warps, then over the lanes (moments: fixed pairwise tree; lag sums: per Doppler
 // block in lane order), and the tile's partials are written, not accumulated: the fold sums
 // them in a fixed order, so the statistics do not depend on scheduling.
+// Where all records of a tile have the same SWST shift and length (nearly all tiles), a lane's
+// sample has one place in every record: no index arithmetic per line, no masks, and the sums over
+// single samples of the pairs follow from the moments and the range's end samples, so a line costs
+// nine FP64 operations instead of fifteen.  The tables hold doubles (the float entries, exactly):
+// four conversions a sample went at a sixteenth of the FP32 rate.  The next lines' bytes are
+// loaded while these are summed.  176 x 15 tiles of a 5616 x 30000 scene: 632 -> 325 us.
 constexpr int kFbaqSums = 15;  // 6 moments + 9 lag sums
 constexpr int kFoldTree = 256; // leaves of the moment tree of the fold (column tiles wrap onto them)
 struct FbaqStatsSmem {
@@ -453,80 +459,171 @@ struct FbaqStatsSmem {
     double red[kFbaqStatsWarps][kFbaqSums][32];
 };
 
+// One column over lines [wy0, wy1) of records that hold its sample at code byte j of the block data,
+// block id at 64 b: the moments and lag sums, the pair (wy0 - 1, wy0) included when wy0 > 0.
+ASARF_HD ASARF_INLINE void fbaq_column(const RawStatsArgs& a, int b, int j, int wy0, int wy1, double v[kFbaqSums]) {
+    const uint8_t* base = a.raw + 2;
+    auto bytes = [&](int y, int& id, int& cw) {
+        const uint8_t* rec = base + static_cast<long long>(y) * a.line_bytes;
+        id = ASARF_LDG(rec + 64 * b);
+        cw = ASARF_LDG(rec + j);
+    };
+    auto value = [&](int id, int cw, double& i, double& q) {
+        i = ASARF_LDG(a.lut_i + 16 * id + (cw >> 4));
+        q = ASARF_LDG(a.lut_q + 16 * id + (cw & 15));
+    };
+    double pi = 0.0, pq = 0.0, fi = 0.0, fq = 0.0;  // previous sample; the first one, when it ends no pair
+    double si = 0.0, sq = 0.0, sii = 0.0, sqq = 0.0, siq = 0.0, lac = 0.0, lbd = 0.0, lad = 0.0, lbc = 0.0;
+    auto add = [&](double ci, double cq) {
+        si += ci;
+        sq += cq;
+        sii += ci * ci;
+        sqq += cq * cq;
+        siq += ci * cq;
+        lac += pi * ci;
+        lbd += pq * cq;
+        lad += pi * cq;
+        lbc += pq * ci;
+        pi = ci;
+        pq = cq;
+    };
+    int id[kStatsBatch], cw[kStatsBatch], y = wy0;
+    if (wy0 > 0) {
+        bytes(wy0 - 1, id[0], cw[0]);
+        value(id[0], cw[0], pi, pq);
+    } else {  // line 0: no pair (its products with the zero predecessor vanish)
+        bytes(0, id[0], cw[0]);
+        value(id[0], cw[0], fi, fq);
+        add(fi, fq);
+        y = 1;
+    }
+    const double ai = wy0 > 0 ? pi : fi, aq = wy0 > 0 ? pq : fq;  // first sample of the first pair
+    const double bi = wy0 > 0 ? 0.0 : fi, bq = wy0 > 0 ? 0.0 : fq;
+    if (y + kStatsBatch <= wy1) {
+#pragma unroll
+        for (int u = 0; u < kStatsBatch; ++u) bytes(y + u, id[u], cw[u]);
+    }
+    for (; y + kStatsBatch <= wy1; y += kStatsBatch) {
+        constexpr int kHalf = kStatsBatch / 2;
+        double ci[kHalf], cq[kHalf];
+#pragma unroll
+        for (int u = 0; u < kHalf; ++u) value(id[u], cw[u], ci[u], cq[u]);
+#pragma unroll
+        for (int u = 0; u < kHalf; ++u) add(ci[u], cq[u]);
+#pragma unroll
+        for (int u = 0; u < kHalf; ++u) value(id[kHalf + u], cw[kHalf + u], ci[u], cq[u]);
+        if (y + 2 * kStatsBatch <= wy1) {
+#pragma unroll
+            for (int u = 0; u < kStatsBatch; ++u) bytes(y + kStatsBatch + u, id[u], cw[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kHalf; ++u) add(ci[u], cq[u]);
+    }
+    for (; y < wy1; ++y) {
+        double ci, cq;
+        bytes(y, id[0], cw[0]);
+        value(id[0], cw[0], ci, cq);
+        add(ci, cq);
+    }
+    const int n = wy1 - wy0, np = wy0 > 0 ? n : n - 1;
+    v[0] = n, v[1] = si, v[2] = sq, v[3] = sii, v[4] = sqq, v[5] = siq;
+    // over the pairs: second samples are all but an unpaired first one, first samples those less the
+    // last plus the one before the range
+    const double c = si - bi, d = sq - bq;
+    v[6] = np, v[7] = np ? c - pi + ai : 0.0, v[8] = np ? d - pq + aq : 0.0, v[9] = np ? c : 0.0, v[10] = np ? d : 0.0;
+    v[11] = lac, v[12] = lbd, v[13] = lad, v[14] = lbc;
+}
+
+// The same for records of any shift and length: lane sums of column x straight to red[k][lane].
+#if defined(__CUDA_ARCH__)
+static __device__ __noinline__
+#else
+static inline
+#endif
+void fbaq_column_masked(const RawStatsArgs& a, const FbaqStatsSmem* sm, int x, int ys, int wy0, int wy1,
+                        double (*red)[32], int lane) {
+    const FastDiv d63 = make_fastdiv(63u);
+    double v[kFbaqSums];
+    for (int k = 0; k < kFbaqSums; ++k) v[k] = 0.0;
+    double pi = 0.0, pq = 0.0;
+    bool pf = false;
+    for (int y = wy0 > 0 ? wy0 - 1 : 0; y < wy1; ++y) {
+        const int r = x - sm->off[y - ys];
+        const int b = r > 0 ? static_cast<int>(fdiv_u(static_cast<unsigned int>(r), d63)) : 0;
+        const int j = r + b + 1;
+        const bool f = r >= 0 && j < sm->len[y - ys];
+        double ci = 0.0, cq = 0.0;
+        if (f) {
+            const uint8_t* rec = a.raw + static_cast<long long>(y) * a.line_bytes + 2;
+            const int id = rec[64 * b], cw = rec[j];
+            ci = ASARF_LDG(a.lut_i + 16 * id + (cw >> 4));
+            cq = ASARF_LDG(a.lut_q + 16 * id + (cw & 15));
+        }
+        if (y >= wy0 && f) {
+            v[0] += 1.0;
+            v[1] += ci;
+            v[2] += cq;
+            v[3] += ci * ci;
+            v[4] += cq * cq;
+            v[5] += ci * cq;
+            if (y > 0 && pf) {
+                v[6] += 1.0;
+                v[7] += pi;
+                v[8] += pq;
+                v[9] += ci;
+                v[10] += cq;
+                v[11] += pi * ci;
+                v[12] += pq * cq;
+                v[13] += pi * cq;
+                v[14] += pq * ci;
+            }
+        }
+        pi = ci;
+        pq = cq;
+        pf = f;
+    }
+    for (int k = 0; k < kFbaqSums; ++k) red[k][lane] = v[k];
+}
+
+// Lines of tile row by with one shift and length: those of its first line in (*off, *len).
+ASARF_HD ASARF_INLINE bool fbaq_line_like(const RawStatsArgs& a, int y, int off, int len) {
+    return (a.swst ? static_cast<int>(a.swst[y]) - a.min_swst : 0) == off &&
+           fbaq_len(a.raw + static_cast<long long>(y) * a.line_bytes, a.line_bytes) == len;
+}
+ASARF_HD ASARF_INLINE int fbaq_tile_start(int by) { return by > 0 ? by * kFbaqStatsLines - 1 : 0; }
+
 ASARF_HD ASARF_INLINE void raw_stats_fbaq_body(const RawStatsArgs& a, int bx, int by, int tid, int nthr,
                                                FbaqStatsSmem* sm) {
     const int y0 = by * kFbaqStatsLines;
     const int y1 = (y0 + kFbaqStatsLines < a.na) ? y0 + kFbaqStatsLines : a.na;
-    const int ys = y0 > 0 ? y0 - 1 : 0;
-    for (int y = ys + tid; y < y1; y += nthr) {
-        sm->off[y - ys] = a.swst ? static_cast<int>(a.swst[y]) - a.min_swst : 0;
-        sm->len[y - ys] = fbaq_len(a.raw + static_cast<long long>(y) * a.line_bytes, a.line_bytes);
+    const int ys = fbaq_tile_start(by);
+    const bool same = a.uniform[by] != 0;
+    const int off0 = a.swst ? static_cast<int>(a.swst[ys]) - a.min_swst : 0;
+    const int len0 = fbaq_len(a.raw + static_cast<long long>(ys) * a.line_bytes, a.line_bytes);
+    if (!same) {
+        for (int y = ys + tid; y < y1; y += nthr) {
+            sm->off[y - ys] = a.swst ? static_cast<int>(a.swst[y]) - a.min_swst : 0;
+            sm->len[y - ys] = fbaq_len(a.raw + static_cast<long long>(y) * a.line_bytes, a.line_bytes);
+        }
+        ASARF_SYNC();
     }
-    ASARF_SYNC();
-    const FastDiv d63 = make_fastdiv(63u);
     constexpr int sub = kFbaqStatsLines / kFbaqStatsWarps;
     for (int t = tid; t < 32 * kFbaqStatsWarps; t += nthr) {
         const int lane = t & 31, w = t >> 5;
         const int x = bx * 32 + lane;
         const int wy0 = y0 + w * sub;
         const int wy1 = (wy0 + sub < y1) ? wy0 + sub : y1;
+        const bool any = x < a.nr && wy0 < wy1;
+        if (any && !same) {
+            fbaq_column_masked(a, sm, x, ys, wy0, wy1, sm->red[w], lane);
+            continue;
+        }
         double v[kFbaqSums];
 #pragma unroll
         for (int k = 0; k < kFbaqSums; ++k) v[k] = 0.0;
-        float pi = 0.0f, pq = 0.0f;
-        bool pf = false;
-        const int start = wy0 > 0 ? wy0 - 1 : 0;
-        if (x < a.nr && wy0 < wy1) {
-            for (int yb = start; yb < wy1; yb += kStatsBatch) {
-                float iv[kStatsBatch], qv[kStatsBatch];
-                bool f[kStatsBatch];
-                // branch-free batch: an absent sample reads byte 0 of its record's block data
-                // (inside the record: every record holds at least one block byte) and is masked
-#pragma unroll
-                for (int u = 0; u < kStatsBatch; ++u) {
-                    const int y = yb + u < wy1 ? yb + u : wy1 - 1;
-                    const int r = x - sm->off[y - ys];
-                    const int rr = r > 0 ? r : 0;
-                    const int b = static_cast<int>(fdiv_u(static_cast<unsigned int>(rr), d63));
-                    const int j = rr + b + 1;
-                    f[u] = (yb + u < wy1) && r >= 0 && j < sm->len[y - ys];
-                    const uint8_t* rec = a.raw + static_cast<long long>(y) * a.line_bytes + 2;
-                    const int id = rec[f[u] ? 64 * b : 0];
-                    const int cw = rec[f[u] ? j : 0];
-                    iv[u] = ASARF_LDG(a.lut_i + 16 * id + (cw >> 4));
-                    qv[u] = ASARF_LDG(a.lut_q + 16 * id + (cw & 15));
-                }
-#pragma unroll
-                for (int u = 0; u < kStatsBatch; ++u) {
-                    const int y = yb + u;
-                    if (y >= wy1) break;
-                    const double ci = f[u] ? iv[u] : 0.0, cq = f[u] ? qv[u] : 0.0;
-                    if (y >= wy0 && f[u]) {
-                        v[0] += 1.0;
-                        v[1] += ci;
-                        v[2] += cq;
-                        v[3] += ci * ci;
-                        v[4] += cq * cq;
-                        v[5] += ci * cq;
-                        if (y > 0 && pf) {
-                            const double ai = pi, aq = pq;
-                            v[6] += 1.0;
-                            v[7] += ai;
-                            v[8] += aq;
-                            v[9] += ci;
-                            v[10] += cq;
-                            v[11] += ai * ci;
-                            v[12] += aq * cq;
-                            v[13] += ai * cq;
-                            v[14] += aq * ci;
-                        }
-                    }
-                    pi = f[u] ? iv[u] : 0.0f;
-                    pq = f[u] ? qv[u] : 0.0f;
-                    pf = f[u];
-                }
-            }
-        }
+        const int r = x - off0;
+        const int b = r >= 0 ? r / 63 : 0;
+        if (any && r >= 0 && r + b + 1 < len0) fbaq_column(a, b, r + b + 1, wy0, wy1, v);
 #pragma unroll
         for (int k = 0; k < kFbaqSums; ++k) sm->red[w][k][lane] = v[k];
     }
@@ -2259,7 +2356,7 @@ ASARF_HD ASARF_INLINE void rc_rows_body(const RcRowsArgs& a, int y, int tid, int
 }
 
 // The same with a compile-time schedule (lengths in kCtLengths), as the planned path's range
-// compression: 7000 lines of 5616 samples 522 -> RCUS us.
+// compression: 7000 lines of 5616 samples 522 -> 242 us.
 template <int L>
 ASARF_HD ASARF_INLINE void rc_rows_ct_body(const RcRowsArgs& a, int y, int tid, float2* s) {
     constexpr int NTHR = CtSchedule<L>::nthr;

@@ -35,6 +35,14 @@ int backend_raw_stats(const RawStatsArgs& a, int gx, int gy, void*) {
 
 int backend_raw_stats_fbaq(const RawStatsArgs& a, int gx, int gy, void*) {
     std::vector<FbaqStatsSmem> sm(1);
+    for (int by = 0; by < gy; ++by) {
+        const int ys = fbaq_tile_start(by);
+        const int off = a.swst ? static_cast<int>(a.swst[ys]) - a.min_swst : 0;
+        const int len = fbaq_len(a.raw + static_cast<long long>(ys) * a.line_bytes, a.line_bytes);
+        a.uniform[by] = 1;
+        for (int y = ys; y < (by + 1) * kFbaqStatsLines && y < a.na; ++y)
+            if (!fbaq_line_like(a, y, off, len)) a.uniform[by] = 0;
+    }
     for (int by = 0; by < gy; ++by)
         for (int bx = 0; bx < gx; ++bx) raw_stats_fbaq_body(a, bx, by, 0, 1, sm.data());
     return ASARF_OK;

@@ -904,12 +904,14 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     }
     const int fb_slots = 6 + 9 * fb_span;
     float* lut_dev = fbaq ? p->alloc<float>(2 * 4096) : nullptr;
+    int* uniform_dev = fbaq ? p->alloc<int>(static_cast<size_t>(fb_tiles_y)) : nullptr;
+    double* dlut_dev = fbaq ? p->alloc<double>(2 * 4096) : nullptr;
     double* part_dev = fbaq ? p->alloc<double>(static_cast<size_t>(fb_tiles_y) * fb_tiles_x * fb_slots) : nullptr;
     FloatStatAccum* facc_dev = fbaq ? p->alloc<FloatStatAccum>(1) : nullptr;
     constexpr int kPstatBlocks = 4 * 148;
     double* pstat_dev = opt.sq_stats ? p->alloc<double>(5 * kPstatBlocks + 4) : nullptr;
     if (!p->bufA || !p->bufB || !p->acc || !p->state || !p->raw_dev || !p->swst_dev || !p->out_dev || (!n_ctr && !rc_tw) ||
-        !p->rc_mf || !chirp_dev || (n_ctr && !ct_tw) || !tw1 || !drev1 || !tw2 || !drev2 || !twN || !rcmc || !rsl_dev || (fbaq && (!lut_dev || !part_dev || !facc_dev)) ||
+        !p->rc_mf || !chirp_dev || (n_ctr && !ct_tw) || !tw1 || !drev1 || !tw2 || !drev2 || !twN || !rcmc || !rsl_dev || (fbaq && (!lut_dev || !dlut_dev || !uniform_dev || !part_dev || !facc_dev)) ||
         (opt.sq_stats && !pstat_dev)) {
         const size_t need = p->bytes;
         delete p;
@@ -936,6 +938,8 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
                 lut[4096 + 16 * id + code] = s.fbaq_q_lut[fbaq4_index(id, code)];
             }
         rc |= mem_h2d(lut_dev, lut.data(), sizeof(float) * lut.size(), nullptr);
+        const std::vector<double> dlut(lut.begin(), lut.end());
+        rc |= mem_h2d(dlut_dev, dlut.data(), sizeof(double) * dlut.size(), nullptr);
     }
     rc |= mem_zero(p->state, sizeof(FocusState), nullptr);
     rc |= mem_zero(p->acc, sizeof(StatAccum), nullptr);  // each run's finalisation leaves it zero again
@@ -973,8 +977,9 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     }
     p->stats_gy = (p->na + st.lines_per_cta - 1) / st.lines_per_cta;
     if (fbaq) {
-        st.lut_i = lut_dev;
-        st.lut_q = lut_dev + 4096;
+        st.lut_i = dlut_dev;
+        st.lut_q = dlut_dev + 4096;
+        st.uniform = uniform_dev;
         st.part = part_dev;
         st.facc = facc_dev;
         st.tiles_x = fb_tiles_x;
@@ -1026,8 +1031,8 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     }
     const int rc_elems = n_ctr ? ct_smem_elems_of(p->rc_len) : p->rc_len;  // compile-time lengths: padded tile
     p->raw_smem_offset = static_cast<int>((sizeof(float2) * static_cast<size_t>(rc_elems) + 127) / 128 * 128);
-    const size_t raw_area = fbaq ? static_cast<size_t>(s.raw_line_bytes) + 16
-                                 : (2 * static_cast<size_t>(s.samples_per_line) + 15) / 16 * 16;
+    // the record, where it starts in a 16-byte word
+    const size_t raw_area = (fbaq ? static_cast<size_t>(s.raw_line_bytes) : 2 * static_cast<size_t>(s.samples_per_line)) + 16;
     p->sh_rc = {512, static_cast<size_t>(p->raw_smem_offset) + raw_area};
 
     AzStridedArgs& f = p->a_fwd;
@@ -1265,8 +1270,6 @@ int asarf_focus(asarf_plan* p, const uint8_t* d_raw, const uint16_t* d_swst, int
     r.raw = d_raw;
     r.swst = d_swst;
     r.min_swst = min_swst;
-    const bool aligned = (reinterpret_cast<uintptr_t>(d_raw) % 16 == 0) && (p->scene.raw_line_bytes % 16 == 0);
-    r.bulk_bytes = (p->use_tma && aligned && !fbaq) ? (2 * p->scene.samples_per_line) / 16 * 16 : 0;
     r.raw_smem_offset = p->raw_smem_offset;
     mark();
     rc = backend_range_compress(r, p->na, p->sh_rc, stream);

@@ -33,7 +33,20 @@ __global__ void __launch_bounds__(kStatsCols, kStatsBlocksPerSm) k_raw_stats(Raw
     raw_stats_body<ALIGNED>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, &sm);
 }
 
-__global__ void __launch_bounds__(32 * kFbaqStatsWarps, 3) k_raw_stats_fbaq(RawStatsArgs a) {
+// Which tile rows of the statistics have records of one shift and length (every column tile would
+// otherwise read all its records' length fields, a 32-byte sector each).
+__global__ void __launch_bounds__(1024) k_fbaq_uniform(RawStatsArgs a) {
+    const int ys = fbaq_tile_start(blockIdx.x);
+    const int y1 = min((static_cast<int>(blockIdx.x) + 1) * kFbaqStatsLines, a.na);
+    const int off = a.swst ? static_cast<int>(a.swst[ys]) - a.min_swst : 0;
+    const int len = fbaq_len(a.raw + static_cast<long long>(ys) * a.line_bytes, a.line_bytes);
+    bool same = true;
+    for (int y = ys + threadIdx.x; y < y1; y += 1024) same = same && fbaq_line_like(a, y, off, len);
+    same = __syncthreads_and(same) != 0;
+    if (threadIdx.x == 0) a.uniform[blockIdx.x] = same ? 1 : 0;
+}
+
+__global__ void __launch_bounds__(32 * kFbaqStatsWarps, 4) k_raw_stats_fbaq(RawStatsArgs a) {
     __shared__ FbaqStatsSmem sm;
     raw_stats_fbaq_body(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, &sm);
 }
@@ -143,77 +156,53 @@ __global__ void __launch_bounds__(kFinalizeThreads) k_finalize(FinalizeArgs a) {
     }
 }
 
-// FBAQ4 record into shared memory: its 16-byte-aligned interior with vector loads, the
-// unaligned head and tail bytewise, so nothing outside the record is read (records are not
-// 16-byte multiples).  The copy starts at buf + (address mod 16), which keeps the interior
-// aligned in shared memory as well; buf itself is 16-byte aligned.
-__device__ __forceinline__ const uint8_t* stage_record(uint8_t* buf, const uint8_t* rec, int n) {
+// Raw record of n bytes into shared memory: its 16-byte aligned interior by one bulk copy of thread 0,
+// the bytes before and after it (records start and end anywhere) by plain loads, so nothing outside
+// the record is read.  The copy starts at buf + (address mod 16), buf 16-byte aligned, which keeps
+// the interior aligned in shared memory as well.  (Lines off 16-byte alignment decoded from global
+// memory sample by sample, FBAQ4 records moved by vector loads: 17011 lines of 10386 bytes 803 ->
+// 626 us, 30000 FBAQ4 records 1287 -> 1238 us.)
+__device__ __forceinline__ const uint8_t* stage_record(uint8_t* buf, const uint8_t* rec, int n, uint64_t* bar,
+                                                       unsigned int* err) {
     const int lead = static_cast<int>(reinterpret_cast<uintptr_t>(rec) & 15);
     const int head = min(n, (16 - lead) & 15);
-    const int nv = (n - head) >> 4;
+    const int body = (n - head) & ~15;
     uint8_t* dst = buf + lead;
+    if (threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        mbar_expect_tx(bar, static_cast<uint32_t>(body));
+        if (body) bulk_load(dst + head, rec + head, static_cast<uint32_t>(body), bar);
+    }
     for (int i = threadIdx.x; i < head; i += blockDim.x) dst[i] = rec[i];
-    const uint4* src4 = reinterpret_cast<const uint4*>(rec + head);
-    uint4* dst4 = reinterpret_cast<uint4*>(dst + head);
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) dst4[i] = __ldg(src4 + i);
-    for (int i = head + 16 * nv + threadIdx.x; i < n; i += blockDim.x) dst[i] = rec[i];
+    for (int i = head + body + threadIdx.x; i < n; i += blockDim.x) dst[i] = rec[i];
     __syncthreads();
+    mbar_wait(bar, 0, err);
     return dst;
 }
 
-// One raw line per block; with bulk_bytes > 0 thread 0 fetches the line with one bulk copy
-// into shared memory (the sub-16-byte tail with plain loads) while the others wait.
+// One raw line per block.
+template <int FMT>
+__device__ __forceinline__ const uint8_t* stage_line(const RangeCompressArgs& a, unsigned char* smem, uint64_t* bar) {
+    const int n = FMT == kRawAsarFbaq4 ? static_cast<int>(a.line_bytes) : 2 * a.spl;
+    return stage_record(smem + a.raw_smem_offset, a.raw + static_cast<long long>(blockIdx.x) * a.line_bytes, n, bar,
+                        &const_cast<FocusState*>(a.state)->errors);
+}
+
 template <int FMT>
 __global__ void __launch_bounds__(512) k_range_compress(RangeCompressArgs a) {
     extern __shared__ __align__(128) unsigned char smem_rc_raw[];
-    float2* s = reinterpret_cast<float2*>(smem_rc_raw);
     __shared__ uint64_t bar;
-    const uint8_t* line = nullptr;
-    if constexpr (FMT == kRawAsarFbaq4) {
-        line = stage_record(smem_rc_raw + a.raw_smem_offset, a.raw + static_cast<long long>(blockIdx.x) * a.line_bytes,
-                            static_cast<int>(a.line_bytes));
-    } else if (a.bulk_bytes > 0) {
-        uint8_t* buf = smem_rc_raw + a.raw_smem_offset;
-        const uint8_t* src = a.raw + static_cast<long long>(blockIdx.x) * a.line_bytes;
-        const int total = 2 * a.spl;
-        if (threadIdx.x == 0) {
-            mbar_init(&bar, 1);
-            mbar_expect_tx(&bar, static_cast<uint32_t>(a.bulk_bytes));
-            bulk_load(buf, src, static_cast<uint32_t>(a.bulk_bytes), &bar);
-        }
-        for (int i = a.bulk_bytes + threadIdx.x; i < total; i += blockDim.x) buf[i] = src[i];
-        __syncthreads();
-        mbar_wait(&bar, 0, &const_cast<FocusState*>(a.state)->errors);
-        line = buf;
-    }
-    range_compress_body<FMT>(a, blockIdx.x, threadIdx.x, blockDim.x, s, line);
+    const uint8_t* line = stage_line<FMT>(a, smem_rc_raw, &bar);
+    range_compress_body<FMT>(a, blockIdx.x, threadIdx.x, blockDim.x, reinterpret_cast<float2*>(smem_rc_raw), line);
 }
 
 // Compile-time-scheduled variant (L in kCtLengths).
 template <int L, int FMT>
 __global__ void __launch_bounds__(CtSchedule<L>::nthr, 2) k_range_compress_ct(RangeCompressArgs a) {
     extern __shared__ __align__(128) unsigned char smem_rcc_raw[];
-    float2* s = reinterpret_cast<float2*>(smem_rcc_raw);
     __shared__ uint64_t bar;
-    const uint8_t* line = nullptr;
-    if constexpr (FMT == kRawAsarFbaq4) {
-        line = stage_record(smem_rcc_raw + a.raw_smem_offset, a.raw + static_cast<long long>(blockIdx.x) * a.line_bytes,
-                            static_cast<int>(a.line_bytes));
-    } else if (a.bulk_bytes > 0) {
-        uint8_t* buf = smem_rcc_raw + a.raw_smem_offset;
-        const uint8_t* src = a.raw + static_cast<long long>(blockIdx.x) * a.line_bytes;
-        const int total = 2 * a.spl;
-        if (threadIdx.x == 0) {
-            mbar_init(&bar, 1);
-            mbar_expect_tx(&bar, static_cast<uint32_t>(a.bulk_bytes));
-            bulk_load(buf, src, static_cast<uint32_t>(a.bulk_bytes), &bar);
-        }
-        for (int i = a.bulk_bytes + threadIdx.x; i < total; i += blockDim.x) buf[i] = src[i];
-        __syncthreads();
-        mbar_wait(&bar, 0, &const_cast<FocusState*>(a.state)->errors);
-        line = buf;
-    }
-    range_compress_ct_body<L, FMT>(a, blockIdx.x, threadIdx.x, s, line);
+    const uint8_t* line = stage_line<FMT>(a, smem_rcc_raw, &bar);
+    range_compress_ct_body<L, FMT>(a, blockIdx.x, threadIdx.x, reinterpret_cast<float2*>(smem_rcc_raw), line);
 }
 
 // Strided azimuth pass: the [n1][NB][XT] tiles (rows r*n2 + b + k) arrive by 3-D TMA boxes.
@@ -545,6 +534,9 @@ int backend_finalize(const FinalizeArgs& a, void* stream) {
 }
 
 int backend_raw_stats_fbaq(const RawStatsArgs& a, int gx, int gy, void* stream) {
+    k_fbaq_uniform<<<gy, 1024, 0, S(stream)>>>(a);
+    int rc = check_launch("fbaq_uniform");
+    if (rc) return rc;
     k_raw_stats_fbaq<<<dim3(gx, gy), 32 * kFbaqStatsWarps, 0, S(stream)>>>(a);
     return check_launch("raw_stats_fbaq");
 }

@@ -96,8 +96,9 @@ struct RawStatsArgs {
     int gpb;              // 4-column groups per Doppler block: ceil(dc_step / 4)
     StatAccum* acc;
     // ASAR FBAQ4 records (k_raw_stats_fbaq): FP64 partial sums of each 32-column tile
-    const float* lut_i;   // [256 block ids][16 raw codes]
-    const float* lut_q;
+    const double* lut_i;  // [256 block ids][16 raw codes], the float tables' values
+    const double* lut_q;
+    int* uniform;         // [tiles_y]: 1 when all records of the tile row have one SWST shift and length
     double* part;         // [tiles_y][tiles_x][part_slots]
     FloatStatAccum* facc; // folded sums
     int tiles_x;          // ceil(nr / 32)
@@ -120,7 +121,6 @@ struct RangeCompressArgs {
     int nk;
     float2* out;
     long long out_pitch;
-    int bulk_bytes;       // raw bytes per line fetched by one bulk copy (multiple of 16; 0 = plain loads)
     int raw_smem_offset;  // byte offset of the raw-line buffer in shared memory
     int format;           // RawFormat of the records
     const float* lut_i;   // ASAR FBAQ4 records: [256 block ids][16 raw codes]
