@@ -918,27 +918,26 @@ struct RcOut {
     }
 };
 
+// Corrected samples of a raw line.
+template <int FMT>
+struct RcSource {
+    static constexpr bool kActive = true;
+    const RangeCompressArgs& a;
+    const IqCorr st;
+    const LineDecoder<FMT> dec;
+    ASARF_HD ASARF_INLINE RcSource(const RangeCompressArgs& args, const FocusState& fs, int y, const uint8_t* raw_line)
+        : a(args), st(fs), dec(args, y, raw_line) {}
+    ASARF_HD ASARF_INLINE float2 operator()(int l) const { return dec(a, st, l); }
+};
+
 // Same transform with a compile-time schedule (lengths in kCtLengths): all loops unrolled,
 // all index arithmetic constant.
 template <int L, int FMT = kRawErsBytes>
 ASARF_HD ASARF_INLINE void range_compress_ct_body(const RangeCompressArgs& a, int y, int tid, float2* s,
                                                   const uint8_t* raw_line) {
-    constexpr int NTHR = CtSchedule<L>::nthr;
-    constexpr int PER = (L + NTHR - 1) / NTHR;
-    const IqCorr st(*a.state);
-    const LineDecoder<FMT> dec(a, y, raw_line);
-    ct_phase<NTHR>(
-        [&](int t) {
-#pragma unroll
-            for (int k = 0; k < PER; ++k) {
-                const int l = t + k * NTHR;
-                if (L % NTHR != 0 && l >= L) break;
-                s[ct_pad<L>(l)] = dec(a, st, l);
-            }
-        },
-        tid);
-    // the last inverse pass stores the kept samples x < Nk of the line directly
-    ct_fft_mf_ifft<L>(s, a.ctw, a.mf, tid, RcOut{a.out + static_cast<long long>(y) * a.out_pitch, a.nk});
+    // the first pass decodes the samples it transforms, the last inverse pass stores the kept ones
+    ct_fft_mf_ifft<L>(s, a.ctw, a.mf, tid, RcSource<FMT>{a, *a.state, y, raw_line},
+                      RcOut{a.out + static_cast<long long>(y) * a.out_pitch, a.nk});
 }
 
 // ----------------------------------------------------------------------------- azimuth strided pass
@@ -2355,24 +2354,20 @@ ASARF_HD ASARF_INLINE void rc_rows_body(const RcRowsArgs& a, int y, int tid, int
     for (int l = tid; l < a.x_zero_end; l += nthr) row[l] = l < a.nk ? s[l] : make_float2(0.0f, 0.0f);
 }
 
+struct RowSource {
+    static constexpr bool kActive = true;
+    const float2* row;
+    int nr;
+    ASARF_HD ASARF_INLINE float2 operator()(int l) const { return l < nr ? row[l] : make_float2(0.0f, 0.0f); }
+};
+
 // The same with a compile-time schedule (lengths in kCtLengths), as the planned path's range
 // compression: 7000 lines of 5616 samples 522 -> 242 us.
 template <int L>
 ASARF_HD ASARF_INLINE void rc_rows_ct_body(const RcRowsArgs& a, int y, int tid, float2* s) {
     constexpr int NTHR = CtSchedule<L>::nthr;
-    constexpr int PER = (L + NTHR - 1) / NTHR;
     float2* row = a.img + static_cast<long long>(y) * a.stride;
-    ct_phase<NTHR>(
-        [&](int t) {
-#pragma unroll
-            for (int k = 0; k < PER; ++k) {
-                const int l = t + k * NTHR;
-                if (L % NTHR != 0 && l >= L) break;
-                s[ct_pad<L>(l)] = l < a.nr ? row[l] : make_float2(0.0f, 0.0f);
-            }
-        },
-        tid);
-    ct_fft_mf_ifft<L>(s, a.ctw, a.mf, tid, RcOut{row, a.nk});
+    ct_fft_mf_ifft<L>(s, a.ctw, a.mf, tid, RowSource{row, a.nr}, RcOut{row, a.nk});
     ct_phase<NTHR, false>([&](int t) {
         for (int x = a.nk + t; x < a.x_zero_end; x += NTHR) row[x] = make_float2(0.0f, 0.0f);
     }, tid);

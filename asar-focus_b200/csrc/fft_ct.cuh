@@ -4,7 +4,7 @@
 // samples), so the planner picks it from the lengths below and the whole transform is
 // instantiated with constant radices, spans and per-thread item counts.
 //
-// Each length is three passes of composite radices (8, 12, 16, 24 or 32), each pass one
+// Each length is three passes of composite radices (6, 8, 12, 16, 24 or 32), each pass one
 // register-resident DFT per item: three shared-memory round trips per transform instead
 // of one per radix-2..8 stage.  The last forward pass, the matched-filter multiply and the
 // first inverse pass touch the same R contiguous positions, so one thread does all three in
@@ -25,25 +25,41 @@
 namespace asarf {
 
 // ----------------------------------------------------------------------------- schedules
+// Threads of a block, resident blocks an SM must hold (the register cap), radices.  A pass is L / R
+// butterflies, so the thread counts are those that share every pass's butterflies evenly, or nearly,
+// and the blocks are the most that registers (80 a thread, 64 at least for a radix of 24) and shared
+// memory (the tile and the staged record) leave room for: what a barrier idles in one line's passes
+// the others fill.  A last radix of 16 reads and writes the tile with fewer passes over its banks
+// than 8 or 12 do.  Range compression of 12000 byte lines (FBAQ4 records), us, the schedules before
+// (two blocks per SM asked for) and these:
+//   768:  8 8 12 x 96 threads    53,       now  46      3072: 16 16 12 x 256  219 (265), now 169 (209)
+//   1024: 8 8 16 x 128           66,       now  56      4096: 16 16 16 x 256  270 (352), now 235 (295)
+//   1536: 24 8 8 x 192          158,       now  84      6144: 24 16 16 x 384  398 (508), now 379 (461)
+//   2048: 16 16 8 x 128         135 (172), now 105 (130)
+// Also timed: 1024 = 16 8 8 60, 4 16 16 58; 1536 = 24 8 8 x 64 91, 12 8 16 91; 2048 = 8 16 16 109
+// (134); 3072 = 12 16 16 176 (222), 96 threads 205; 4096 x 128 267 (311); 6144 = 24 16 16 x 256 392
+// (453), 16 16 24 397 (482), 24 16 16 x 128 424; 8192 = 32 16 16 545 (685), 16 32 16 602 (674),
+// 32 16 16 x 512 751, against the 561 (664) of the one kept: its tile leaves room for two blocks.
 template <int L>
 struct CtSchedule {
     static constexpr int count = 0;
 };
-#define ASARF_CT_SCHEDULE(LEN, NT, R0, R1, R2)   \
-    template <>                                  \
-    struct CtSchedule<LEN> {                     \
-        static constexpr int r[] = {R0, R1, R2}; \
-        static constexpr int count = 3;          \
-        static constexpr int nthr = NT;          \
+#define ASARF_CT_SCHEDULE(LEN, NT, BLK, R0, R1, R2) \
+    template <>                                      \
+    struct CtSchedule<LEN> {                         \
+        static constexpr int r[] = {R0, R1, R2};     \
+        static constexpr int count = 3;              \
+        static constexpr int nthr = NT;              \
+        static constexpr int blocks = BLK;           \
     }
-ASARF_CT_SCHEDULE(768, 96, 8, 8, 12);
-ASARF_CT_SCHEDULE(1024, 128, 8, 8, 16);
-ASARF_CT_SCHEDULE(1536, 192, 24, 8, 8);
-ASARF_CT_SCHEDULE(2048, 128, 16, 16, 8);
-ASARF_CT_SCHEDULE(3072, 256, 16, 16, 12);
-ASARF_CT_SCHEDULE(4096, 256, 16, 16, 16);
-ASARF_CT_SCHEDULE(6144, 384, 24, 16, 16);
-ASARF_CT_SCHEDULE(8192, 256, 16, 16, 32);
+ASARF_CT_SCHEDULE(768, 96, 6, 12, 8, 8);
+ASARF_CT_SCHEDULE(1024, 64, 10, 8, 8, 16);
+ASARF_CT_SCHEDULE(1536, 96, 8, 6, 16, 16);
+ASARF_CT_SCHEDULE(2048, 128, 6, 16, 8, 16);
+ASARF_CT_SCHEDULE(3072, 192, 4, 16, 12, 16);
+ASARF_CT_SCHEDULE(4096, 256, 3, 16, 16, 16);
+ASARF_CT_SCHEDULE(6144, 256, 3, 16, 24, 16);
+ASARF_CT_SCHEDULE(8192, 256, 2, 16, 16, 32);
 #undef ASARF_CT_SCHEDULE
 
 constexpr int kCtLengths[] = {768, 1024, 1536, 2048, 3072, 4096, 6144, 8192};
@@ -111,12 +127,19 @@ ASARF_HD ASARF_INLINE void ct_phase(F&& phase, int tid) {
 #endif
 }
 
+// Inputs come from the tile.
+struct NoSrc {
+    static constexpr bool kActive = false;
+};
+
 // One pass I < count-1 (span S > 1, a multiple of Q): forward DIF (DFT, then twiddle output q
 // by W_M^{jq}) or inverse DIT (conjugate twiddles on the inputs, then the inverse DFT).
 // An active Epi receives each output (natural position, value) instead of the tile: the last
-// inverse pass hands the line straight to its destination.
-template <int L, int I, bool INV, class Epi = NoEpi>
-ASARF_HD ASARF_INLINE void ct_pass(float2* s, const float2* __restrict__ ctw, int t, const Epi& epi = Epi{}) {
+// inverse pass hands the line straight to its destination.  An active Src gives each input (natural
+// position) instead of the tile: the first forward pass forms the line's samples as it reads them.
+template <int L, int I, bool INV, class Epi = NoEpi, class Src = NoSrc>
+ASARF_HD ASARF_INLINE void ct_pass(float2* s, const float2* __restrict__ ctw, int t, const Epi& epi = Epi{},
+                                   const Src& src = Src{}) {
     constexpr int NTHR = CtSchedule<L>::nthr;
     constexpr int R = CtSchedule<L>::r[I];
     constexpr int S = ct_span<L, I>();
@@ -136,7 +159,10 @@ ASARF_HD ASARF_INLINE void ct_pass(float2* s, const float2* __restrict__ ctw, in
         float2* p = s + ct_pad<L>(b * M + j);
         float2 v[R];
 #pragma unroll
-        for (int m = 0; m < R; ++m) v[m] = p[m * STRIDE];
+        for (int m = 0; m < R; ++m) {
+            if constexpr (Src::kActive) v[m] = src(b * M + j + m * S);
+            else v[m] = p[m * STRIDE];
+        }
         if (INV) {
             if (j != 0) {
 #pragma unroll
@@ -185,16 +211,20 @@ ASARF_HD ASARF_INLINE void ct_middle(float2* s, const float2* __restrict__ mf, i
     }
 }
 
-// Forward transform, matched filter, inverse transform of the padded tile s (natural order
-// in, unscaled); the last pass hands its outputs to epi (natural position, value) and ends
-// without a barrier, every other pass ends with one.
-template <int L, class Epi>
+// Forward transform, matched filter, inverse transform (unscaled) through the padded tile s: the
+// first pass takes its inputs from src (natural position), the last hands its outputs to epi
+// (natural position, value) and ends without a barrier, every other pass ends with one.
+// The samples are formed where they are first used: decoding the line into the tile and reading it
+// back took a fifth of the kernel's shared-memory passes and a barrier (5616 x 28000, L = 6144:
+// 1000 -> 926 us).
+template <int L, class Src, class Epi>
 ASARF_HD ASARF_INLINE void ct_fft_mf_ifft(float2* s, const float2* __restrict__ ctw, const float2* __restrict__ mf,
-                                          int tid, const Epi& epi) {
+                                          int tid, const Src& src, const Epi& epi) {
     constexpr int NTHR = CtSchedule<L>::nthr;
     static_assert(CtSchedule<L>::count == 3, "three-pass schedules");
     static_assert(Epi::kActive, "the last pass writes through its epilogue");
-    ct_phase<NTHR>([&](int t) { ct_pass<L, 0, false>(s, ctw, t); }, tid);
+    static_assert(Src::kActive, "the first pass reads through its source");
+    ct_phase<NTHR>([&](int t) { ct_pass<L, 0, false>(s, ctw, t, NoEpi{}, src); }, tid);
     ct_phase<NTHR>([&](int t) { ct_pass<L, 1, false>(s, ctw, t); }, tid);
     ct_phase<NTHR>([&](int t) { ct_middle<L>(s, mf, t); }, tid);
     ct_phase<NTHR>([&](int t) { ct_pass<L, 1, true>(s, ctw, t); }, tid);

@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(512) k_range_compress(RangeCompressArgs a) {
 
 // Compile-time-scheduled variant (L in kCtLengths).
 template <int L, int FMT>
-__global__ void __launch_bounds__(CtSchedule<L>::nthr, 2) k_range_compress_ct(RangeCompressArgs a) {
+__global__ void __launch_bounds__(CtSchedule<L>::nthr, CtSchedule<L>::blocks) k_range_compress_ct(RangeCompressArgs a) {
     extern __shared__ __align__(128) unsigned char smem_rcc_raw[];
     __shared__ uint64_t bar;
     const uint8_t* line = stage_line<FMT>(a, smem_rcc_raw, &bar);
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(512) k_rc_rows(RcRowsArgs a) {
 }
 
 template <int L>
-__global__ void __launch_bounds__(CtSchedule<L>::nthr, 2) k_rc_rows_ct(RcRowsArgs a) {
+__global__ void __launch_bounds__(CtSchedule<L>::nthr, CtSchedule<L>::blocks) k_rc_rows_ct(RcRowsArgs a) {
     extern __shared__ float2 smem_rcrc[];
     rc_rows_ct_body<L>(a, blockIdx.x, threadIdx.x, smem_rcrc);
 }
