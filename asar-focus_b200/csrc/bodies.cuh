@@ -103,9 +103,15 @@ ASARF_HD inline bool polyfit_qr(const double* x, const double* y, int m, int deg
 // of one Doppler block inside an aligned group of 4 (columns 4g .. 4g + 3, one 8-byte window per
 // line, byte-lane dot products for all sums; a group that straddles a Doppler block boundary is
 // two units, one per block, each masking the other's columns), so every sum a thread keeps
-// belongs to a single Doppler block, and kStatsBatch lines are loaded before any is consumed.
-// A window is one aligned 8-byte load when the raw base and line stride are 8-byte aligned,
+// belongs to a single Doppler block, and kStatsBatch lines are read before any is consumed.
+// A window is one aligned 8-byte word when the raw base and line stride are 8-byte aligned,
 // otherwise the three aligned 4-byte words around it, funnelled into place.
+//
+// Unaligned lines' bytes under a block's columns (2 KB a line) arrive in a ring of kStatsStages batches
+// in shared memory, a bulk copy per line, the batches ahead in flight while one is summed: 5193 x
+// 17011, 10386-byte lines, 212 -> 118 us; batches of 16 lines in two stages 172.  Both forms are bound
+// by instructions and the chain of batches (315 MB in 113 us are 2.8 TB/s), so a block whose lines
+// have one SWST shift checks its windows once: aligned lines of 5616 x 28000 140 -> 113 us.
 constexpr int kStatsCols = 256;
 constexpr int kStatsBatch = 8;
 constexpr int kStatsMaxLines = 256;
@@ -136,10 +142,46 @@ inline int stats_lines_per_block(int na, int gx, int slots) {
     return kStatsLinesPerBlock;
 }
 
+constexpr int kStatsStages = 4;
+// a line's bytes in the ring: at most kStatsCols groups of 4 columns, from a 16-byte boundary on
+constexpr int kStatsSlotBytes = 8 * kStatsCols + 32;
+constexpr size_t kStatsRingBytes = static_cast<size_t>(kStatsStages) * kStatsBatch * kStatsSlotBytes;
+
 struct RawStatsSmem {
     unsigned long long mom[6];
     unsigned long long lag[kMaxDcBlocks][9];
     int off[kStatsMaxLines + 1];  // SWST shift of the block's lines (and the line before)
+    int same;                     // 1: all those shifts are equal
+    int x_lo, x_hi;               // columns the block's units read
+    int sample0[kStatsStages * kStatsBatch];  // ring offset of the lines' sample 0 (may lie before the slot)
+    uint64_t full[kStatsStages];  // mbarriers: a batch's bytes have arrived
+};
+
+// Batch k of a statistics block's lines [ys, y1): the line before the block's first (its lag-sum
+// partner) is a batch of its own, so every following batch holds kStatsBatch counted lines.
+struct StatsBatches {
+    int ys, y0, y1, count;
+    ASARF_HD ASARF_INLINE StatsBatches(int y0_, int y1_) : ys(y0_ > 0 ? y0_ - 1 : 0), y0(y0_), y1(y1_) {
+        count = (ys < y0 ? 1 : 0) + (y1 - y0 + kStatsBatch - 1) / kStatsBatch;
+    }
+    ASARF_HD ASARF_INLINE void lines(int k, int* yg, int* ye) const {
+        const int pre = ys < y0 ? 1 : 0;
+        *yg = k < pre ? ys : y0 + (k - pre) * kStatsBatch;
+        *ye = k < pre ? y0 : (*yg + kStatsBatch < y1 ? *yg + kStatsBatch : y1);
+    }
+};
+
+// Lines read in place (the caller-scratch statistics and the host emulation).  kMargin: samples past a window that the words around it reach.
+template <bool ALIGNED>
+struct StatsRowsInPlace {
+    static constexpr bool kCollective = false;
+    static constexpr int kMargin = ALIGNED ? 0 : 1;
+    const RawStatsArgs& a;
+    ASARF_HD ASARF_INLINE void begin(int) const {}
+    ASARF_HD ASARF_INLINE void end(int) const {}
+    ASARF_HD ASARF_INLINE const uint8_t* row(int, int, int y) const {
+        return a.raw + static_cast<long long>(y) * a.line_bytes;
+    }
 };
 
 // Host side: work units and grid width of the statistics kernel for this raw buffer.
@@ -222,76 +264,82 @@ ASARF_HD ASARF_INLINE void raw_stats_reduce(RawStatsSmem* sm, bool valid, int bl
 
 // The columns of `colmask` (bit k: column x0 + k) of the aligned group at x0 (x0 % 4 == 0), all in
 // one Doppler block.  A line's four samples are the 8 bytes (I0 Q0 I1 Q1 | I2 Q2 I3 Q3) at
-// raw + y*line_bytes + 2*(x0 - off) (the SWST shift is a multiple of 4 samples, so with ALIGNED the
-// window stays 8-byte aligned on every line; without, it starts at any even address, and a window
-// at the very start or end of its record is read sample by sample, so that the words around a
-// window never leave the record: 5193 x 17011, 10386-byte lines, 206 us, against 296 one column and
-// one 2-byte load at a time).  Samples outside the record or the mask are zero bytes, which
-// drop out of every sum.
-template <bool ALIGNED>
-ASARF_HD ASARF_INLINE void raw_stats_quad(const RawStatsArgs& a, const RawStatsSmem* sm, int x0, unsigned int colmask,
-                                          int y0, int y1, int ys, unsigned long long mv[6], unsigned int lv[9]) {
+// row + 2*(x0 - off) (the SWST shift is a multiple of 4 samples, so with ALIGNED the window stays
+// 8-byte aligned on every line; without, it starts at any even address).  A window that leaves its
+// record is read sample by sample.  Samples outside the record or the mask are zero bytes, which
+// drop out of every sum.  Where the block's lines have one shift, a window that lies inside one
+// record lies inside all: its batches are read with nothing checked per line.  With kCollective rows
+// every thread of the block runs the batches, an idle one at another's columns with none its own.
+template <bool ALIGNED, class Rows>
+ASARF_HD ASARF_INLINE void raw_stats_quad(const RawStatsArgs& a, const RawStatsSmem* sm, const Rows& rows, int x0,
+                                          unsigned int colmask, const StatsBatches& bt, unsigned long long mv[6],
+                                          unsigned int lv[9]) {
+    const int y0 = bt.y0, ys = bt.ys;
+    const int i_same = x0 - sm->off[0];
+    const bool inside = sm->same && i_same >= Rows::kMargin && i_same + 4 + Rows::kMargin <= a.spl;
     constexpr unsigned int kLo = 0x00ff00ffu, kOnes = 0x01010101u;
     const unsigned int colbits = colmask;
     const int ncol = popc_u32(colmask);
     unsigned int cnt = 0, si = 0, sq = 0, sii = 0, sqq = 0, siq = 0;
     unsigned int l0 = 0, l1 = 0, l2 = 0, l3 = 0, l4 = 0, l5 = 0, l6 = 0, l7 = 0, l8 = 0;
     unsigned int pI0 = 0, pI1 = 0, pQ0 = 0, pQ1 = 0, pfb = 0;
-    const uint8_t* base = a.raw + 2ll * x0;
     // byte masks of the group's columns: in the packed I (or Q) word byte k is column k; in the
     // two raw words column k is the 16-bit lane k % 2 of word k / 2
     const unsigned int cm = ((colmask & 1u) ? 0x000000ffu : 0u) | ((colmask & 2u) ? 0x0000ff00u : 0u) |
                             ((colmask & 4u) ? 0x00ff0000u : 0u) | ((colmask & 8u) ? 0xff000000u : 0u);
-    // the line before the block's first (its lag-sum partner) is a batch of its own, so every
-    // following batch holds kStatsBatch counted lines
-    for (int yg = ys, ye = (ys < y0 ? y0 : (ys + kStatsBatch < y1 ? ys + kStatsBatch : y1)); yg < y1;
-         yg = ye, ye = (ye + kStatsBatch < y1 ? ye + kStatsBatch : y1)) {
-        // loads only in this loop (nothing consumes them), so all kStatsBatch lines are in flight
+    for (int k = 0; k < bt.count; ++k) {
+        int yg, ye;
+        bt.lines(k, &yg, &ye);
+        rows.begin(k);
         uint2 w[kStatsBatch];
-        unsigned int fbv[kStatsBatch];
-        bool vec[kStatsBatch];
+        unsigned int fbv[kStatsBatch], whole = 0;
+        // the whole 8-byte window at p is inside its record
+        auto window = [](const uint8_t* p) -> uint2 {
+            if constexpr (ALIGNED) {
+                return *reinterpret_cast<const uint2*>(p);
+            } else {
+                const unsigned int odd = static_cast<unsigned int>(reinterpret_cast<uintptr_t>(p) & 2);
+                const uint32_t* q = reinterpret_cast<const uint32_t*>(p - odd);
+                const uint32_t q0 = q[0], q1 = q[1], q2 = odd ? q[2] : 0u;
+                return make_uint2(funnel_r(q0, q1, 8 * odd), funnel_r(q1, q2, 8 * odd));
+            }
+        };
+        bool interior = ye - yg == kStatsBatch && pfb == colbits;
+        if (interior && inside) {
 #pragma unroll
-        for (int u = 0; u < kStatsBatch; ++u) {
-            const int y = yg + u;
-            w[u] = make_uint2(0u, 0u);
-            fbv[u] = 0u;
-            vec[u] = false;
-            if (y < ye) {
-                const int off = sm->off[y - ys];
-                const int i = x0 - off;
-                constexpr int kMargin = ALIGNED ? 0 : 1;  // samples the words around a window reach past it
-                if (i >= kMargin && i + 4 + kMargin <= a.spl) {
-                    // the whole 8-byte window is inside the record
-                    const uint8_t* p = base + static_cast<long long>(y) * a.line_bytes - 2ll * off;
-                    if constexpr (ALIGNED) {
-                        w[u] = *reinterpret_cast<const uint2*>(p);
+            for (int u = 0; u < kStatsBatch; ++u) w[u] = window(rows.row(k, u, yg + u) + 2ll * i_same);
+        } else {
+#pragma unroll
+            for (int u = 0; u < kStatsBatch; ++u) {
+                const int y = yg + u;
+                w[u] = make_uint2(0u, 0u);
+                fbv[u] = 0u;
+                if (y < ye && colbits) {
+                    const int i = x0 - sm->off[y - ys];
+                    const uint8_t* p = rows.row(k, u, y) + 2ll * i;
+                    if (i >= Rows::kMargin && i + 4 + Rows::kMargin <= a.spl) {
+                        w[u] = window(p);
+                        fbv[u] = colbits;
+                        whole |= 1u << u;
                     } else {
-                        const unsigned int odd = static_cast<unsigned int>(reinterpret_cast<uintptr_t>(p) & 2);
-                        const uint32_t* q = reinterpret_cast<const uint32_t*>(p - odd);
-                        const uint32_t q0 = q[0], q1 = q[1], q2 = odd ? q[2] : 0u;
-                        w[u] = make_uint2(funnel_r(q0, q1, 8 * odd), funnel_r(q1, q2, 8 * odd));
-                    }
-                    fbv[u] = colbits;
-                    vec[u] = true;
-                } else {
-                    // record edge: sample by sample
-                    const uint8_t* row = a.raw + static_cast<long long>(y) * a.line_bytes;
-                    for (int k = 0; k < 4; ++k) {
-                        if (!((colbits >> k) & 1u) || i + k < 0 || i + k >= a.spl) continue;
-                        const unsigned int v = *reinterpret_cast<const uint16_t*>(row + 2ll * (i + k));
-                        if (k < 2) w[u].x |= v << (16 * k);
-                        else w[u].y |= v << (16 * (k - 2));
-                        fbv[u] |= 1u << k;
+                        // record edge: sample by sample
+                        for (int c = 0; c < 4; ++c) {
+                            if (!((colbits >> c) & 1u) || i + c < 0 || i + c >= a.spl) continue;
+                            const unsigned int v = *reinterpret_cast<const uint16_t*>(p + 2 * c);
+                            if (c < 2) w[u].x |= v << (16 * c);
+                            else w[u].y |= v << (16 * (c - 2));
+                            fbv[u] |= 1u << c;
+                        }
                     }
                 }
             }
+            interior = interior && (whole == (1u << kStatsBatch) - 1u || colbits == 0u);
         }
+        rows.end(k);
         // Interior batch: every line and the one before it counted, filled and read through a
         // whole window.  The group's I and Q bytes are packed into one word each, so every sum
-        // is one byte-lane dot product and nothing is masked per line.
-        bool interior = ye - yg == kStatsBatch && pfb == colbits;
-#pragma unroll
-        for (int u = 0; u < kStatsBatch; ++u) interior = interior && vec[u];
+        // is one byte-lane dot product and nothing is masked per line (an idle thread takes this path
+        // with its warp and sums zeros).
         if (interior) {
             unsigned int pI = byte_perm(pI0, pI1, 0x6420u), pQ = byte_perm(pQ0, pQ1, 0x6420u);
             unsigned int psI = dp4(pI, kOnes, 0u), psQ = dp4(pQ, kOnes, 0u);
@@ -370,34 +418,53 @@ ASARF_HD ASARF_INLINE void raw_stats_quad(const RawStatsArgs& a, const RawStatsS
     lv[0] = l0, lv[1] = l1, lv[2] = l2, lv[3] = l3, lv[4] = l4, lv[5] = l5, lv[6] = l6, lv[7] = l7, lv[8] = l8;
 }
 
-template <bool ALIGNED>
-ASARF_HD ASARF_INLINE void raw_stats_body(const RawStatsArgs& a, int bx, int by, int tid, int nthr,
-                                          RawStatsSmem* sm) {
-    unsigned long long* flat = &sm->mom[0];
-    const int nflat = 6 + a.nblk * 9;
-    for (int i = tid; i < 6 + kMaxDcBlocks * 9; i += nthr) flat[i] = 0ull;
-    const int y0 = by * a.lines_per_cta;
-    const int y1 = (y0 + a.lines_per_cta < a.na) ? y0 + a.lines_per_cta : a.na;
-    const int ys = y0 > 0 ? y0 - 1 : 0;
-    for (int y = ys + tid; y < y1; y += nthr) sm->off[y - ys] = a.swst ? 4 * (static_cast<int>(a.swst[y]) - a.min_swst) : 0;
-    ASARF_SYNC();
-    const FastDiv dgpb = make_fastdiv(static_cast<unsigned int>(a.gpb));
-    for (int c = tid; c < kStatsCols; c += nthr) {
-        const int unit = bx * kStatsCols + c;
-        unsigned long long mv[6] = {0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
-        unsigned int lv[9] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-        // group k of Doppler block blk: the aligned group at (block start & ~3) + 4k, the
-        // block's columns [xs, xe) in it
-        const int blk = static_cast<int>(fdiv_u(static_cast<unsigned int>(unit), dgpb));
+// Unit -> first column of its aligned group, its columns and its Doppler block: group k of block blk
+// is the aligned group at (block start & ~3) + 4k, the block's columns [xs, xe) in it.
+struct StatsUnit {
+    int blk, x0;
+    unsigned int colmask;
+    ASARF_HD ASARF_INLINE StatsUnit(const RawStatsArgs& a, const FastDiv& dgpb, int unit) {
+        blk = static_cast<int>(fdiv_u(static_cast<unsigned int>(unit), dgpb));
         const int xs = blk * a.dc_step;
         const int xe = (blk + 1) * a.dc_step < a.nr ? (blk + 1) * a.dc_step : a.nr;
-        const int x0 = (xs & ~3) + 4 * (unit - blk * a.gpb);
+        x0 = (xs & ~3) + 4 * (unit - blk * a.gpb);
         const int c_lo = xs > x0 ? xs - x0 : 0;
         const int c_hi = xe - x0 < 4 ? xe - x0 : 4;
-        const bool valid = blk < a.nblk && c_hi > c_lo;
-        const unsigned int colmask = valid ? ((1u << c_hi) - 1u) & ~((1u << c_lo) - 1u) : 0u;
-        if (valid) raw_stats_quad<ALIGNED>(a, sm, x0, colmask, y0, y1, ys, mv, lv);
-        raw_stats_reduce(sm, valid, blk, mv, lv);
+        colmask = blk < a.nblk && c_hi > c_lo ? ((1u << c_hi) - 1u) & ~((1u << c_lo) - 1u) : 0u;
+    }
+};
+
+// Lines of the block by, their SWST shifts and the block's accumulators in sm (the caller barriers).
+ASARF_HD ASARF_INLINE StatsBatches raw_stats_begin(const RawStatsArgs& a, int by, int tid, int nthr, RawStatsSmem* sm) {
+    unsigned long long* flat = &sm->mom[0];
+    for (int i = tid; i < 6 + kMaxDcBlocks * 9; i += nthr) flat[i] = 0ull;
+    const int y0 = by * a.lines_per_cta;
+    const StatsBatches bt(y0, y0 + a.lines_per_cta < a.na ? y0 + a.lines_per_cta : a.na);
+    bool same = true;
+    for (int y = bt.ys + tid; y < bt.y1; y += nthr) {
+        sm->off[y - bt.ys] = a.swst ? 4 * (static_cast<int>(a.swst[y]) - a.min_swst) : 0;
+        same = same && (!a.swst || a.swst[y] == a.swst[bt.ys]);
+    }
+#if defined(__CUDA_ARCH__)
+    same = __syncthreads_and(same) != 0;
+#endif
+    if (tid == 0) sm->same = same ? 1 : 0;
+    return bt;
+}
+
+template <bool ALIGNED, class Rows>
+ASARF_HD ASARF_INLINE void raw_stats_body(const RawStatsArgs& a, const Rows& rows, const StatsBatches& bt, int bx, int tid,
+                                          int nthr, RawStatsSmem* sm) {
+    const unsigned long long* flat = &sm->mom[0];
+    const int nflat = 6 + a.nblk * 9;
+    const FastDiv dgpb = make_fastdiv(static_cast<unsigned int>(a.gpb));
+    for (int c = tid; c < kStatsCols; c += nthr) {
+        const StatsUnit un(a, dgpb, bx * kStatsCols + c);
+        unsigned long long mv[6] = {0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
+        unsigned int lv[9] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+        if (un.colmask || Rows::kCollective)
+            raw_stats_quad<ALIGNED>(a, sm, rows, un.colmask ? un.x0 : sm->x_lo, un.colmask, bt, mv, lv);
+        raw_stats_reduce(sm, un.colmask != 0, un.blk, mv, lv);
     }
     ASARF_SYNC();
     unsigned long long* gflat = &a.acc->mom[0];
@@ -726,6 +793,7 @@ ASARF_HD inline FinalizeMap finalize_stats(const FinalizeArgs& a, FocusState* st
     FinalizeMap m;
     m.err = 0;
     if (n == 0.0) m.err |= kErrStatsEmpty;
+    if (!a.facc) m.err |= a.acc->errors;
     const float total = static_cast<float>(a.n_total);
     // mean: float(sum) / float(total)
     const float dc_i = static_cast<float>(SI) / total;

@@ -27,8 +27,9 @@ int backend_raw_stats(const RawStatsArgs& a, int gx, int gy, void*) {
     RawStatsSmem sm;
     for (int by = 0; by < gy; ++by)
         for (int bx = 0; bx < gx; ++bx) {
-            if (a.aligned) raw_stats_body<true>(a, bx, by, 0, 1, &sm);
-            else raw_stats_body<false>(a, bx, by, 0, 1, &sm);
+            const StatsBatches bt = raw_stats_begin(a, by, 0, 1, &sm);
+            if (a.aligned) raw_stats_body<true>(a, StatsRowsInPlace<true>{a}, bt, bx, 0, 1, &sm);
+            else raw_stats_body<false>(a, StatsRowsInPlace<false>{a}, bt, bx, 0, 1, &sm);
         }
     return ASARF_OK;
 }

@@ -968,9 +968,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     st.nblk = nblk;
     st.acc = p->acc;
     {
-        // block height for the grid of aligned raw buffers (the 4-column path, any address
-        // that is a multiple of 8: a null pointer stands for one); an unaligned buffer runs
-        // the one-column path over the same lines
+        // block height for the grid (the same for lines read in place and through the ring)
         RawStatsArgs shape = st;
         const int gx = raw_stats_grid_x(shape, nullptr);
         st.lines_per_cta = stats_lines_per_block(p->na, gx, backend_sm_count() * kStatsBlocksPerSm);

@@ -24,13 +24,103 @@ namespace {
 constexpr int kFinalizeThreads = 96;
 static_assert(kFinalizeThreads >= kMaxDcBlocks, "one Doppler block per thread");
 
-// Three blocks per SM (80 registers, no spills).  Four blocks at 64 registers spilled 176
-// bytes per thread in the batched loads and measured slower on the ERS-like scene:
-// 0.156 against 0.143 ms.
-template <bool ALIGNED>
+// Statistics lines through the ring of batches.  The warps take turns to issue one: lane u copies the bytes of
+// line u under the block's columns, from the 16-byte boundary before its first to the one after its
+// last; at the two ends of the raw buffer, where that would leave it, the odd bytes are moved by plain
+// loads.  A batch is issued into its slots once every thread has read the one they held.
+struct StatsRowsStaged {
+    static constexpr bool kCollective = true;
+    static constexpr int kMargin = 0;  // the words around a window stay inside its slot
+    const RawStatsArgs& a;
+    RawStatsSmem* sm;
+    const StatsBatches& bt;
+    unsigned char* ring;
+    __device__ __forceinline__ void issue(int k) const {
+        if (k >= bt.count) return;
+        const int lane = threadIdx.x & 31, stage = k % kStatsStages, slot = stage * kStatsBatch + lane;
+        int yg, ye;
+        bt.lines(k, &yg, &ye);
+        const int y = yg + lane;
+        uint32_t bytes = 0;
+        const uint8_t* src = nullptr;
+        unsigned char* dst = nullptr;
+        if (lane < kStatsBatch && y < ye) {
+            const int off = sm->off[y - bt.ys];
+            const int i0 = max(sm->x_lo - off, 0), i1 = min(sm->x_hi - off, a.spl);
+            if (i0 < i1) {
+                const uint8_t* row = a.raw + static_cast<long long>(y) * a.line_bytes;
+                const uint8_t *b0 = row + 2ll * i0, *b1 = row + 2ll * i1;
+                const int lead = static_cast<int>(reinterpret_cast<uintptr_t>(b0) & 15);
+                const int tail = static_cast<int>(-reinterpret_cast<uintptr_t>(b1) & 15);
+                const uint8_t *c0 = b0 - lead, *c1 = b1 + tail;
+                unsigned char* base = ring + slot * kStatsSlotBytes;
+                if (c0 < a.raw) {
+                    c0 += 16;
+                    for (const uint8_t* p = b0; p < c0 && p < b1; ++p) base[lead + (p - b0)] = *p;
+                }
+                if (c1 > a.raw + static_cast<long long>(a.na - 1) * a.line_bytes + 2ll * a.spl) {
+                    c1 -= 16;
+                    for (const uint8_t* p = c1 > b0 ? c1 : b0; p < b1; ++p) base[lead + (p - b0)] = *p;
+                }
+                if (c0 < c1) {
+                    bytes = static_cast<uint32_t>(c1 - c0);
+                    src = c0;
+                    dst = base + lead + (c0 - b0);
+                }
+                sm->sample0[slot] = slot * kStatsSlotBytes + lead - 2 * i0;
+            }
+        }
+        const uint32_t total = __reduce_add_sync(0xffffffffu, bytes);
+        if (lane == 0) mbar_expect_tx(&sm->full[stage], total);
+        __syncwarp();
+        fence_async_smem();
+        if (bytes) bulk_load(dst, src, bytes, &sm->full[stage]);
+    }
+    __device__ __forceinline__ void begin(int k) const {
+        mbar_wait(&sm->full[k % kStatsStages], (k / kStatsStages) & 1, &a.acc->errors);
+    }
+    __device__ __forceinline__ void end(int k) const {
+        __syncthreads();
+        if (static_cast<int>(threadIdx.x >> 5) == k % (kStatsCols / 32)) issue(k + kStatsStages);
+    }
+    __device__ __forceinline__ const uint8_t* row(int k, int u, int) const {
+        return ring + sm->sample0[k % kStatsStages * kStatsBatch + u];
+    }
+};
+
+// Lines on 8-byte boundaries: every window is one 8-byte load, read in place.  Three blocks per SM (80
+// registers): four blocks at 64 registers spilled 176 bytes per thread in the batched loads and
+// measured slower, 0.156 against 0.143 ms.
 __global__ void __launch_bounds__(kStatsCols, kStatsBlocksPerSm) k_raw_stats(RawStatsArgs a) {
     __shared__ RawStatsSmem sm;
-    raw_stats_body<ALIGNED>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, &sm);
+    const StatsBatches bt = raw_stats_begin(a, blockIdx.y, threadIdx.x, kStatsCols, &sm);
+    __syncthreads();
+    raw_stats_body<true>(a, StatsRowsInPlace<true>{a}, bt, blockIdx.x, threadIdx.x, kStatsCols, &sm);
+}
+
+// Any other lines, through the ring (three blocks per SM by their rings, too).
+__global__ void __launch_bounds__(kStatsCols, kStatsBlocksPerSm) k_raw_stats_ring(RawStatsArgs a) {
+    extern __shared__ __align__(128) unsigned char smem_rs_raw[];
+    __shared__ RawStatsSmem sm;
+    const int tid = threadIdx.x;
+    const StatsBatches bt = raw_stats_begin(a, blockIdx.y, tid, kStatsCols, &sm);
+    if (tid == 0) {
+        for (int i = 0; i < kStatsStages; ++i) mbar_init(&sm.full[i], 1);
+        sm.x_lo = 0x3fffffff;  // no unit: past every record
+        sm.x_hi = 0;
+    }
+    __syncthreads();
+    const StatsUnit un(a, make_fastdiv(static_cast<unsigned int>(a.gpb)), blockIdx.x * kStatsCols + tid);
+    if (un.colmask) {
+        atomicMin(&sm.x_lo, un.x0);
+        atomicMax(&sm.x_hi, un.x0 + 4);
+    }
+    __syncthreads();
+    const StatsRowsStaged rows{a, &sm, bt, smem_rs_raw};
+    if (tid < 32)
+        for (int k = 0; k < kStatsStages; ++k) rows.issue(k);
+    __syncthreads();
+    raw_stats_body<false>(a, rows, bt, blockIdx.x, tid, kStatsCols, &sm);
 }
 
 // Which tile rows of the statistics have records of one shift and length (every column tile would
@@ -148,6 +238,7 @@ __global__ void __launch_bounds__(kFinalizeThreads) k_finalize(FinalizeArgs a) {
     if (!a.facc) {
         unsigned long long* acc = &a.acc->mom[0];
         for (int i = tid; i < 6 + 9 * nblk; i += kFinalizeThreads) acc[i] = 0ull;
+        if (tid == 0) a.acc->errors = 0u;
     }
     if (tid < 32) {
         double poly[3] = {0.0, 0.0, 0.0};
@@ -523,8 +614,15 @@ cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
 }  // namespace
 
 int backend_raw_stats(const RawStatsArgs& a, int gx, int gy, void* stream) {
-    if (a.aligned) k_raw_stats<true><<<dim3(gx, gy), kStatsCols, 0, S(stream)>>>(a);
-    else k_raw_stats<false><<<dim3(gx, gy), kStatsCols, 0, S(stream)>>>(a);
+    // lines of 11232 bytes (28000): in place 113 us, through the ring 124; of 10386 (17011): 212 (three
+    // loads a window instead of one, and the line's checks) and 118
+    if (a.aligned) {
+        k_raw_stats<<<dim3(gx, gy), kStatsCols, 0, S(stream)>>>(a);
+    } else {
+        int rc = ensure_smem(k_raw_stats_ring, kStatsRingBytes, "raw_stats");
+        if (rc) return rc;
+        k_raw_stats_ring<<<dim3(gx, gy), kStatsCols, kStatsRingBytes, S(stream)>>>(a);
+    }
     return check_launch("raw_stats");
 }
 

@@ -107,7 +107,9 @@ int scratch_address(NoallocScratch** out) {
 template <bool ALIGNED>
 __global__ void __launch_bounds__(kStatsCols) k_noalloc_raw_stats(RawStatsArgs a) {
     __shared__ RawStatsSmem sm;
-    raw_stats_body<ALIGNED>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, &sm);
+    const StatsBatches bt = raw_stats_begin(a, blockIdx.y, threadIdx.x, blockDim.x, &sm);
+    __syncthreads();
+    raw_stats_body<ALIGNED>(a, StatsRowsInPlace<ALIGNED>{a}, bt, blockIdx.x, threadIdx.x, blockDim.x, &sm);
 }
 
 __global__ void k_noalloc_finalize(FinalizeArgs a, asarf_raw_stats* out) {

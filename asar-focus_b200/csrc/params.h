@@ -19,6 +19,7 @@ constexpr int kNumTailVariants = 2;
 struct StatAccum {
     unsigned long long mom[6];
     unsigned long long lag[kMaxDcBlocks][9];
+    unsigned int errors;  // kErrTmaTimeout of the statistics kernel
 };
 
 // ASAR FBAQ4 records: the same sums over the decoded float samples, in FP64, written (not
