@@ -1034,7 +1034,7 @@ ASARF_HD ASARF_INLINE void az_strided_tables(const AzStridedArgs& a, int b, int 
 
 // Tiles of a block: as many as keep n1 * nb at 256 rows of 32 columns (64 KB, three blocks per SM)
 // while the grid still has three blocks per SM (5000 lines of 4913 columns, n1 = 40: 147 us forward
-// with one, 85 with four; n1 = 225 takes one).
+// with one, 81 with four; n1 = 225 takes one).
 inline int az_strided_tiles_per_block(int n1, int n2, int tiles) {
     int nb = 1;
     while (nb < 8 && 2 * nb * n1 <= 256 && static_cast<long long>(tiles) * (n2 / (2 * nb)) >= 3 * 148) nb *= 2;

@@ -117,7 +117,7 @@ typedef struct asarf_options {
                                   (half the bytes written, and read again by the multilook) */
     int32_t compiled_schedules; /* 1 (default): azimuth transforms whose radix schedule has a compile-time
                                   instantiation (strided 225 = 9*5*5 and 180 = 9*4*5 at 32 columns,
-                                  blocks 125 = 5*5*5 and 168 = 8*7*3) run it; 0: run-time schedules only.
+                                  blocks 125 = 5*5*5, 168 = 8*7*3 and 14 more) run it; 0: run-time schedules only.
                                   Both give identical results */
 } asarf_options;
 
