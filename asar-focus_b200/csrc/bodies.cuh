@@ -799,8 +799,13 @@ ASARF_HD inline FinalizeMap finalize_stats(const FinalizeArgs& a, FocusState* st
     const float dc_i = static_cast<float>(SI) / total;
     const float dc_q = static_cast<float>(SQ) / total;
     const double di = dc_i, dq = dc_q;
-    const double cii = SII - 2.0 * di * SI + n * di * di;  // sum over filled of (I - dc_i)^2
-    const double cqq = SQQ - 2.0 * dq * SQ + n * dq * dq;
+    // sums over filled of (I - dc_i)^2, (Q - dc_q)^2: a dead channel's may round to just below zero
+    auto centred = [&](double s2, double s1, double d) {
+        const double c = s2 - 2.0 * d * s1 + n * d * d;
+        return c < 0.0 ? 0.0 : c;
+    };
+    const double cii = centred(SII, SI, di);
+    const double cqq = centred(SQQ, SQ, dq);
     const double ciq = SIQ - dq * SI - di * SQ + n * di * dq;
     // padding samples hold 0 - dc after the DC step and enter the gain / phase sums
     const double npad = static_cast<double>(a.n_pad);
