@@ -1592,10 +1592,12 @@ inline int rcmc_right_halo(double max_walk) { return kRcmcTaps / 2 - 1 + static_
 // room for two resident blocks per SM (2 x 512 threads at 64 registers fill the register file;
 // 228 KB of shared memory per SM, 1 KB reserved per block).  With one block per SM the
 // block-wide barriers of the FFT stages leave the SM idle (measured 2.63 -> 1.92 ms at n2 = 168).
+// Where the halo leaves no such width of at least 16, 16; less than that only to fit a block at all.
 constexpr size_t kAzRdTwoBlockSmem = 228 * 1024 / 2 - 1024 - 128;
-inline int az_rd_tile_width(int n2, int hl, int hr, bool absolute_phase) {
+inline int az_rd_tile_width(int n2, int hl, int hr, bool absolute_phase, size_t limit) {
     int xt = 64;
     while (xt > 16 && az_rd_smem(n2, xt + hl + hr, xt, absolute_phase) > kAzRdTwoBlockSmem) xt -= 2;
+    while (xt > 8 && az_rd_smem(n2, xt + hl + hr, xt, absolute_phase) > limit) xt -= 2;
     return xt;
 }
 

@@ -475,14 +475,18 @@ static int largest_divisor_to_root(int N) {
 // 175 rows (6.5 + 0.142 n2; radices up to 5 run 7 % faster, run-time schedules 10 % slower, a fourth
 // stage costs 6), times the rounds of the 296 resident blocks.  Longer blocks win until their tile
 // loses columns (n2 > 168).  5616 x 4999: n2 = 50, the divisor at sqrt(N), 400 us in the block, n2 =
-// 125 248 us.
+// 125 248 us.  A long range walk takes the tile its columns too: a length whose tile does not fit is
+// left out, one that leaves a single block per SM costs 37 % more (az_rd_tile_width).
 int choose_az_n2(int N, int nk, int hl, int hr, bool absolute_phase) {
     const int root = largest_divisor_to_root(N);
     int best = root;
     double best_cost = 1e300;
+    const size_t limit = smem_optin_limit();
     for (int d = 48; d <= 256 && d < N; ++d) {
         if (N % d != 0 || N / d > 640) continue;
-        const int xt = az_rd_tile_width(d, hl, hr, absolute_phase);
+        const int xt = az_rd_tile_width(d, hl, hr, absolute_phase, limit);
+        const size_t smem = az_rd_smem(d, xt + hl + hr, xt, absolute_phase);
+        if (smem > limit) continue;
         const double blocks = static_cast<double>((nk + xt - 1) / xt) * (N / d);
         if (blocks < kAzRdMinBlocks) continue;
         const std::vector<int> radices = block_radices(d);
@@ -491,6 +495,7 @@ int choose_az_n2(int N, int nk, int hl, int hr, bool absolute_phase) {
         double t = 6.5 + 0.142 * d + 6.0 * std::max(0, f.plan.nst - 3);
         if (*std::max_element(radices.begin(), radices.end()) <= 5) t *= 0.93;
         if (!block_schedule_compiled(f.plan)) t *= 1.1;
+        if (smem > kAzRdTwoBlockSmem) t *= 1.37;
         const double rounds = blocks / kAzRdRound;
         const double cost = t * (rounds < 4.0 ? std::ceil(rounds) : rounds + 0.5);
         if (cost < best_cost) best_cost = cost, best = d;
@@ -797,7 +802,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
         delete p;
         return set_error(ASARF_ERR_INVALID, "strided_tile_width must be 16 or 32");
     }
-    p->xt2 = az_rd_tile_width(p->n2, p->hl, p->hr, opt.absolute_phase != 0);
+    p->xt2 = az_rd_tile_width(p->n2, p->hl, p->hr, opt.absolute_phase != 0, smem_optin_limit());
     if (opt.az_tile_width != 0) {
         if (opt.az_tile_width < 16 || opt.az_tile_width > 64 || (opt.az_tile_width & 1)) {
             delete p;

@@ -406,7 +406,7 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     d.nk = x_size;
     d.hl = hl;
     d.hr = hr;
-    d.xt = az_rd_tile_width(n2, d.hl, d.hr, false);
+    d.xt = az_rd_tile_width(n2, d.hl, d.hr, false, smem_optin_limit());
     d.wt = d.xt + d.hl + d.hr;
     d.prf = static_cast<float>(prm->prf);
     d.bin_step = d.prf / static_cast<float>(N);
