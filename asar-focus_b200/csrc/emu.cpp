@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "context_cache.h"
+#include "internal.h"
 #include "asarf.h"
 #include "backend.h"
 #include "bodies.cuh"
@@ -383,6 +384,15 @@ extern "C" int asarf_emu_context_cache_probe(const unsigned long long* ids, int 
         addrs[i] = reinterpret_cast<unsigned long long>(p);
     }
     return resolutions;
+}
+
+// Test hook of the host emulation only: the range-Doppler tile (length n2, width wt) that the planner takes
+// for N = n1 * n2 rows of nk columns, and the rows of its TMA boxes.
+extern "C" void asarf_emu_rd_tile(int N, int nk, int hl, int hr, int* n2, int* wt, int* box_rows) {
+    using namespace asarf;
+    *n2 = choose_az_n2(N, nk, hl, hr, false);
+    *wt = az_rd_tile_width(*n2, hl, hr, false, smem_optin_limit()) + hl + hr;
+    *box_rows = rd_box_rows(*n2, *wt);
 }
 
 namespace asarf {

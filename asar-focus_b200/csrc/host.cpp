@@ -543,6 +543,12 @@ int largest_divisor_le(int n, int cap) {
     return 1;
 }
 
+int rd_box_rows(int n2, int wt) {
+    for (int d = std::min(n2, 256); d >= 1; --d)
+        if (n2 % d == 0 && (d == n2 || d * wt * sizeof(float2) % 128 == 0)) return d;
+    return 0;
+}
+
 bool make_azimuth_maps(float2* a, float2* b, int nk, long long pitch, int n1, int n2, int xt, int nb, int n1_box, int wt,
                        int n2_box, void* map_a3, void* map_b3, void* map_a2) {
     if (wt % 2 != 0) return false;
@@ -1142,8 +1148,8 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     // ---- TMA tensor maps (all tiles come from this GPU's own buffers; loads only)
     {
         const int n1_box = largest_divisor_le(p->n1, 256);
-        const int n2_box = largest_divisor_le(p->n2, 256);
-        p->use_tma = 2 * d.wt <= 256 && make_azimuth_maps(p->bufA, p->bufB, p->nk, p->pitch, p->n1, p->n2, p->xt1,
+        const int n2_box = rd_box_rows(p->n2, d.wt);
+        p->use_tma = 2 * d.wt <= 256 && n2_box > 0 && make_azimuth_maps(p->bufA, p->bufB, p->nk, p->pitch, p->n1, p->n2, p->xt1,
                                                           p->a_fwd.nb, n1_box, d.wt, n2_box, p->tmapA3, p->tmapB3,
                                                           p->tmapA2);
         p->a_fwd.use_tma = p->a_inv.use_tma = d.use_tma = p->use_tma ? 1 : 0;

@@ -45,6 +45,11 @@ inline float azimuth_scale(int N, const HostFft& f1, const HostFft& f2) {
     return static_cast<float>(1.0 / (N * (1.0 + 2.0 * (transform_gain(f1, false) + transform_gain(f2, false)))));
 }
 int largest_divisor_le(int n, int cap);
+// Rows of a TMA box of the range-Doppler tile (n2 rows of wt complex values): all n2 up to 256, else their
+// largest divisor whose boxes each start on a 128-byte boundary of shared memory, as a tensor copy must;
+// 0 where none does (n2 = 343, odd rows: the tile then arrives by plain loads).  The strided pass's
+// rows are whole multiples of 128 bytes.
+int rd_box_rows(int n2, int wt);
 // TMA maps (128-byte blobs) of the azimuth passes over an image pair a, b of n1 * n2 rows of `pitch`
 // complex values, nk of them data: strided views of a and b (nb tiles of xt columns, n1_box of the
 // n1 rows a box) and the contiguous view of a (wt columns, n2_box rows).

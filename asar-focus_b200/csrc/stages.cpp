@@ -428,9 +428,10 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     alignas(64) unsigned char map_src3[128], map_out3[128], map_src2[128];
     bool tma = x_stride % 2 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 &&
                (reinterpret_cast<uintptr_t>(out) & 15) == 0 && 2 * d.wt <= 256;
+    d.n2_box = rd_box_rows(n2, d.wt);
+    tma = tma && d.n2_box > 0;
     if (tma) {
         fwd.n1_box = inv.n1_box = largest_divisor_le(n1, 256);
-        d.n2_box = largest_divisor_le(n2, 256);
         tma = make_azimuth_maps(src, out, x_size, x_stride, n1, n2, xt1, fwd.nb, fwd.n1_box, d.wt, d.n2_box, map_src3,
                                 map_out3, map_src2);
     }
