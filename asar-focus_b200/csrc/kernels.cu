@@ -1,6 +1,7 @@
 // CUDA kernels of the focusing path (sm_100a) and their launchers.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -550,13 +551,17 @@ __global__ void __launch_bounds__(128) k_twiddles(TwiddleArgs a, int count) {
 }
 
 __global__ void __launch_bounds__(128) k_rsl(RslArgs a) {
-    const int x = blockIdx.x * 128 + threadIdx.x, y0 = blockIdx.y * kColumnRows;
-    if (x < a.range_size) rsl_column(a, x, y0, min(y0 + kColumnRows, a.az_size));
+    const int x = blockIdx.x * 128 + threadIdx.x;
+    if (x >= a.range_size) return;
+    for (long long y0 = blockIdx.y * kColumnRows; y0 < a.az_size; y0 += gridDim.y * kColumnRows)
+        rsl_column(a, x, static_cast<int>(y0), static_cast<int>(min(y0 + kColumnRows, static_cast<long long>(a.az_size))));
 }
 
 __global__ void __launch_bounds__(128) k_srgr(SrgrArgs a) {
-    const int x = blockIdx.x * 128 + threadIdx.x, y0 = blockIdx.y * kColumnRows;
-    if (x < a.out_x) srgr_column(a, x, y0, min(y0 + kColumnRows, a.y_size));
+    const int x = blockIdx.x * 128 + threadIdx.x;
+    if (x >= a.out_x) return;
+    for (long long y0 = blockIdx.y * kColumnRows; y0 < a.y_size; y0 += gridDim.y * kColumnRows)
+        srgr_column(a, x, static_cast<int>(y0), static_cast<int>(min(y0 + kColumnRows, static_cast<long long>(a.y_size))));
 }
 
 // Level-0 gathers: one warp per line, eight lines per block.  A line's own loads form a chain
@@ -583,6 +588,9 @@ int grid_for(long long n) {
     long long g = (n + 255) / 256;
     return static_cast<int>(g < 148 * 32 ? (g > 0 ? g : 1) : 148 * 32);
 }
+
+// Grid height of the column kernels, whose blocks stride over the rows past it.
+int column_blocks(int rows) { return static_cast<int>(std::min((rows + kColumnRows - 1ll) / kColumnRows, 1ll * kMaxGridY)); }
 
 int check_launch(const char* what) {
     cudaError_t e = cudaGetLastError();
@@ -868,11 +876,11 @@ int backend_multilook(const MultilookArgs& a, void* stream) {
     return check_launch("multilook");
 }
 int backend_rsl(const RslArgs& a, void* stream) {
-    k_rsl<<<dim3((a.range_size + 127) / 128, (a.az_size + kColumnRows - 1) / kColumnRows), 128, 0, S(stream)>>>(a);
+    k_rsl<<<dim3((a.range_size + 127) / 128, column_blocks(a.az_size)), 128, 0, S(stream)>>>(a);
     return check_launch("rsl");
 }
 int backend_srgr(const SrgrArgs& a, void* stream) {
-    k_srgr<<<dim3((a.out_x + 127) / 128, (a.y_size + kColumnRows - 1) / kColumnRows), 128, 0, S(stream)>>>(a);
+    k_srgr<<<dim3((a.out_x + 127) / 128, column_blocks(a.y_size)), 128, 0, S(stream)>>>(a);
     return check_launch("srgr");
 }
 

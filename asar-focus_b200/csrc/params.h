@@ -367,6 +367,8 @@ struct IqApplyArgs {
     float dc_i, dc_q, gain, sin_c, cos_c;
 };
 
+constexpr int kMaxGridY = 65535;  // a launch grid's height
+
 constexpr int kAcccCols = 256;  // columns of one block
 struct AcccArgs {
     const float2* img;

@@ -243,7 +243,7 @@ int asarf_doppler_centroid(const void* d_img, int32_t x_size, int32_t y_size, in
     a.x_stride = x_stride;
     a.step = x_size / 32;
     a.nblk = (x_size + a.step - 1) / a.step;
-    a.rows_per_block = 256;
+    a.rows_per_block = std::max(256, (y_size + kMaxGridY - 1) / kMaxGridY);
     a.xend = std::min(a.nblk * a.step, x_stride);
     a.span = (kAcccCols - 1) / a.step + 2;
     const int gx = (a.xend + kAcccCols - 1) / kAcccCols, gy = (y_size + a.rows_per_block - 1) / a.rows_per_block;
