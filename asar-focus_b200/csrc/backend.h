@@ -70,6 +70,7 @@ int mem_d2d_2d(void* dst, size_t dpitch, const void* src, size_t spitch, size_t 
 int mem_zero(void* dst, size_t n, void* stream);
 int mem_zero_2d(void* dst, size_t pitch, size_t width, size_t rows, void* stream);
 int stream_sync(void* stream);
+bool stream_capturing(void* stream);  // work on it is recorded, not run
 void* event_create();
 void event_destroy(void* e);
 int event_record(void* e, void* stream);

@@ -12,6 +12,7 @@
 #include "asarf.h"
 #include "backend.h"
 #include "bodies.cuh"
+#include "plan.h"
 
 namespace asarf {
 
@@ -22,9 +23,15 @@ struct TileBuf {
     explicit TileBuf(size_t bytes) : v(bytes / sizeof(float4) + 2) {}
     float2* data() { return reinterpret_cast<float2*>(v.data()); }
 };
+
+// Test hooks: a finalisation that fails to launch, and a stream under capture, on which the statistics,
+// their finalisation and the clearing of their accumulators are recorded and not run.
+bool g_fail_finalize = false;
+bool g_capturing = false;
 }  // namespace
 
 int backend_raw_stats(const RawStatsArgs& a, int gx, int gy, void*) {
+    if (g_capturing) return ASARF_OK;
     RawStatsSmem sm;
     for (int by = 0; by < gy; ++by)
         for (int bx = 0; bx < gx; ++bx) {
@@ -57,6 +64,11 @@ int backend_stats_fold(const RawStatsArgs& a, int tiles_y, void*) {
 }
 
 int backend_finalize(const FinalizeArgs& a, void*) {
+    if (g_fail_finalize) {
+        g_fail_finalize = false;
+        return set_error(ASARF_ERR_CUDA, "finalize launch: made to fail");
+    }
+    if (g_capturing) return ASARF_OK;
     finalize_body(a);
     if (!a.facc) *a.acc = StatAccum{};  // as the device finalisation leaves it
     return ASARF_OK;
@@ -279,7 +291,9 @@ int mem_d2d_2d(void* dst, size_t dpitch, const void* src, size_t spitch, size_t 
         std::memcpy(static_cast<char*>(dst) + r * dpitch, static_cast<const char*>(src) + r * spitch, width);
     return ASARF_OK;
 }
+bool stream_capturing(void*) { return g_capturing; }
 int mem_zero(void* dst, size_t n, void*) {
+    if (g_capturing) return ASARF_OK;
     std::memset(dst, 0, n);
     return ASARF_OK;
 }
@@ -384,6 +398,17 @@ extern "C" int asarf_emu_context_cache_probe(const unsigned long long* ids, int 
         addrs[i] = reinterpret_cast<unsigned long long>(p);
     }
     return resolutions;
+}
+
+// Test hooks of the host emulation only: the next finalisation fails; the stream is under capture; a
+// plan's statistics accumulators are all zero.
+extern "C" void asarf_emu_fail_finalize() { asarf::g_fail_finalize = true; }
+extern "C" void asarf_emu_capture(int on) { asarf::g_capturing = on != 0; }
+extern "C" int asarf_emu_accumulators_clear(const asarf_plan* p) {
+    const unsigned char* b = reinterpret_cast<const unsigned char*>(p->acc);
+    for (size_t i = 0; i < sizeof(asarf::StatAccum); ++i)
+        if (b[i]) return 0;
+    return 1;
 }
 
 // Test hook of the host emulation only: the range-Doppler tile (length n2, width wt) that the planner takes

@@ -1238,6 +1238,18 @@ static constexpr int kKernelsPerRun = 7;
 static const char* const kKernelNames[kKernelsPerRun] = {"raw_stats", "finalize", "range_compress", "az_strided_fwd",
                                                           "az_rd", "az_strided_inv", "tail"};
 
+// The accumulators are zero between runs: the finalisation leaves them so, and a run that ends between
+// its statistics and its finalisation clears them in the same order, at once, so that neither the next
+// run nor a graph captured before adds to its sums.
+struct AccumulatorGuard {
+    asarf_plan* plan;
+    void* stream;
+    bool finalised = false;
+    ~AccumulatorGuard() {
+        if (!finalised && mem_zero(plan->acc, sizeof(StatAccum), stream) != ASARF_OK) plan->acc_dirty = true;
+    }
+};
+
 int asarf_focus(asarf_plan* p, const uint8_t* d_raw, const uint16_t* d_swst, int32_t min_swst, float* d_out,
                 void* stream) {
     if (!p || !d_raw || (!d_out && !p->skip_tail)) return set_error(ASARF_ERR_INVALID, "focus: null argument");
@@ -1254,10 +1266,13 @@ int asarf_focus(asarf_plan* p, const uint8_t* d_raw, const uint16_t* d_swst, int
         if (ev) event_record(ev[k], stream);
         ++k;
     };
-    // the accumulators are zero unless a run ended between its statistics and its finalisation
-    int rc = p->acc_dirty ? mem_zero(p->acc, sizeof(StatAccum), stream) : ASARF_OK;
-    if (rc) return rc;
-    p->acc_dirty = true;
+    int rc = ASARF_OK;
+    if (p->acc_dirty) {
+        rc = mem_zero(p->acc, sizeof(StatAccum), stream);
+        if (rc) return rc;
+        if (!stream_capturing(stream)) p->acc_dirty = false;  // (a captured clear has not run)
+    }
+    AccumulatorGuard sums{p, stream};
     RawStatsArgs st = p->a_stats;
     st.raw = d_raw;
     st.swst = d_swst;
@@ -1274,7 +1289,7 @@ int asarf_focus(asarf_plan* p, const uint8_t* d_raw, const uint16_t* d_swst, int
     mark();
     rc = backend_finalize(p->a_fin, stream);
     if (rc) return rc;
-    p->acc_dirty = false;
+    sums.finalised = true;
     RangeCompressArgs r = p->a_rc;
     r.raw = d_raw;
     r.swst = d_swst;

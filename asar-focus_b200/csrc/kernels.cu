@@ -967,6 +967,14 @@ int mem_zero_2d(void* dst, size_t pitch, size_t width, size_t rows, void* stream
     if (width == 0 || rows == 0) return ASARF_OK;
     return cuda_rc(cudaMemset2DAsync(dst, pitch, 0, width, rows, S(stream)), "2D memset");
 }
+bool stream_capturing(void* stream) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(S(stream), &st) != cudaSuccess) {
+        cudaGetLastError();  // the legacy stream beside another's capture: not capturing itself
+        return false;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
 int stream_sync(void* stream) { return cuda_rc(cudaStreamSynchronize(S(stream)), "stream sync"); }
 
 void* event_create() {

@@ -43,7 +43,7 @@ struct asarf_plan {
     float2* bufA = nullptr;
     float2* bufB = nullptr;
     StatAccum* acc = nullptr;
-    bool acc_dirty = false;       // a run's statistics were enqueued without its finalisation
+    bool acc_dirty = false;       // an interrupted run's sums could not be cleared
     FocusState* state = nullptr;
     uint8_t* raw_dev = nullptr;
     uint16_t* swst_dev = nullptr;
