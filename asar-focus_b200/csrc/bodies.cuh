@@ -1179,76 +1179,6 @@ ASARF_HD ASARF_INLINE float bin_frequency(int f, int az_pad, float step) {
     return fmul_rn(static_cast<float>(k), step);
 }
 
-// bf: the row's Doppler bin frequency (bin_frequency of its bin, from the block's row table).
-ASARF_HD ASARF_INLINE float2 rcmc_mf_sample(const AzRdArgs& a, const ColParams& cp, int x, float bf, const float2* srow,
-                                            int cs, unsigned int* err_flag) {
-    const float prf = a.prf;
-    const float half = a.half_prf;
-    // --- aliased frequency (the same test decides the matched-filter band and the RCMC walk)
-    float fn = bf;
-    if (cp.dc < 0.0f) {
-        if (bf > fadd_rn(half, cp.dc)) fn = fsub_rn(fn, prf);
-    } else if (cp.dc > 0.0f) {
-        if (fn < fadd_rn(-half, cp.dc)) fn = fadd_rn(fn, prf);
-    }
-    // outside the processed band the reference writes zero whatever RCMC gave
-    if (fn < cp.cut_lo || fn > cp.cut_hi) return make_float2(0.0f, 0.0f);
-    // --- RCMC: walk = lambda^2 fn^2 / (8 Vr^2) [float, IEEE divide] * R0 [double] / range spacing
-    const float num = fmul_rn(fmul_rn(fmul_rn(a.lambda, a.lambda), fn), fn);
-    const float shift = static_cast<float>(static_cast<double>(div_by_recip_rn(num, cp.den, cp.rden)) * cp.r0_dr);
-    const int walk = static_cast<int>(roundf(shift));
-    const int calc_x = x + walk;
-    float2 out = make_float2(0.0f, 0.0f);
-    if (!(calc_x - kRcmcTaps / 2 < 0 || calc_x + kRcmcTaps / 2 >= a.nk)) {
-        const int first = cs + walk - kRcmcTaps / 2;  // smem column of tap 0
-        if (first + 1 < 0 || first + kRcmcTaps - 1 > a.wt) {
-            atomic_or_u32(err_flag, kErrRcmcHalo);
-        } else {
-            // Windowed sinc at off - i, off = shift - walk + 8 in [7.5, 8.5]:
-            // sin(pi (off - i)) = (-1)^i sin(pi off), and the common factor sin(pi off) / pi
-            // cancels in the normalised sum, leaving weights (-1)^i W_i / (off - i).  The two end
-            // taps are skipped: their window values W_0 = W_15 = -1.4e-17 (a numpy.blackman
-            // rounding residue of an exact zero) give terms below half an ulp of every sum.
-            // With dl = off - 8 (exact) a weight is 1 / fma(dl, c_i, (8 - i) c_i), c_i = (-1)^i / W_i
-            // (constants): one FMA and one reciprocal per tap, within 2 ulp of the quotient since
-            // |8 - i| >= 1 wherever the constant term is not zero.  The normaliser sums in pairs.
-            const float off = fadd_rn(fsub_rn(shift, static_cast<float>(walk)), static_cast<float>(kRcmcTaps / 2));
-            const float dl = fsub_rn(off, static_cast<float>(kRcmcTaps / 2));
-            if (dl == 0.0f) {
-                out = srow[first + kRcmcTaps / 2];  // integer shift: sinc is a unit impulse
-            } else {
-                constexpr float kWin[kRcmcTaps] = ASARF_BLACKMAN16;
-                float2 acc = make_float2(0.0f, 0.0f);
-                float2 nrm2 = make_float2(0.0f, 0.0f);
-#pragma unroll
-                for (int i = 1; i < kRcmcTaps - 1; i += 2) {
-                    const float ca = -1.0f / kWin[i];  // i odd
-                    const float cb = 1.0f / kWin[i + 1];
-                    const float wa = rcp_approx(fma_rn(dl, ca, static_cast<float>(kRcmcTaps / 2 - i) * ca));
-                    const float wb = rcp_approx(fma_rn(dl, cb, static_cast<float>(kRcmcTaps / 2 - i - 1) * cb));
-                    acc = pfma(srow[first + i], wa, acc);
-                    acc = pfma(srow[first + i + 1], wb, acc);
-                    nrm2 = padd(nrm2, make_float2(wa, wb));
-                }
-                const float nrm = fadd_rn(nrm2.x, nrm2.y);
-                if (nrm != 0.0f) {
-                    const float inv = rcp_approx(nrm);
-                    out = make_float2(fmul_rn(acc.x, inv), fmul_rn(acc.y, inv));
-                }
-            }
-        }
-    }
-    // --- matched filter exp(-j pi fc^2 / Ka) * exp(-j 2 pi (dc_off / Ka) f), both phases
-    // rounded as the reference rounds them, combined into one reduced exponential
-    float fc = fsub_rn(bf, cp.dc_off);
-    if (fc > half) fc = fsub_rn(fc, prf);
-    else if (fc < -half) fc = fadd_rn(fc, prf);
-    const float pi = 3.14159265358979323846f;
-    const float mf_phase = div_by_recip_rn(fmul_rn(fmul_rn(pi, fc), fc), cp.ka, cp.rka);
-    const float sh_phase = fmul_rn(fmul_rn(fmul_rn(2.0f, pi), cp.dc_off_ka), bf);
-    return cmul(out, expj_neg_sum(mf_phase, sh_phase));
-}
-
 // Absolute-phase factor of column x: exp(j phi), phi = 4 pi R0 / lambda + pi dc_off^2 / Ka, in
 // FP64 (4 pi R0 / lambda is about 1.9e8 rad at 850 km; it is reduced modulo 2 pi before the
 // cast).  With it the matched filter is exp(-j pi f^2 / Ka) in the unaliased Doppler
@@ -1308,7 +1238,7 @@ ASARF_HD inline void rcmc_weight_row(int n, float* row) {
     }
 }
 
-// What a uniform row's samples need of their column.
+// What a sample needs of its column.
 struct ColUse {
     float den, rden;      // 8 Vr^2 and its rounded reciprocal
     float r0_hi, r0_lo;   // R0 / range spacing as a float pair
@@ -1372,6 +1302,165 @@ struct RowSpan {
 // lambda^2 fn^2 as rcmc_mf_sample rounds it.
 ASARF_HD ASARF_INLINE float rcmc_numerator(const AzRdArgs& a, float fn) {
     return fmul_rn(fmul_rn(fmul_rn(a.lambda, a.lambda), fn), fn);
+}
+
+// Range walk in samples, with the reference's roundings: the quotient num / den, times R0 / range spacing as
+// a float pair (the product's rounding differs from the FP64 one's only within 2^-45 of a tie).
+ASARF_HD ASARF_INLINE float rcmc_shift(const ColUse& c, float num) {
+    const float q = div_by_recip_rn(num, c.den, c.rden);
+    const float p = fmul_rn(q, c.r0_hi);
+    return fadd_rn(p, fma_rn(q, c.r0_lo, fma_rn(q, c.r0_hi, -p)));
+}
+
+// ---- rows that go sample by sample
+// What one sample decides for itself.  first: tile column of tap 0 (kNoTaps where the taps leave the line, or
+// the tile, which sets the error bit).
+struct SampleWalk {
+    static constexpr int kNoTaps = -2;
+    bool band;  // inside the processed band; outside it the reference writes zero whatever RCMC gave
+    int first;
+    float dl;   // walk past the integer walk
+};
+
+// bf: the row's Doppler bin frequency (bin_frequency of its bin, from the block's row table); cs: the
+// sample's tile column.
+ASARF_HD ASARF_INLINE SampleWalk rcmc_decide(const AzRdArgs& a, const ColUse& c, float dc, int x, float bf, int cs,
+                                             unsigned int* err_flag) {
+    const float prf = a.prf;
+    const float half = a.half_prf;
+    SampleWalk s{false, SampleWalk::kNoTaps, 0.0f};
+    // --- aliased frequency (the same test decides the matched-filter band and the RCMC walk)
+    float fn = bf;
+    if (dc < 0.0f) {
+        if (bf > fadd_rn(half, dc)) fn = fsub_rn(fn, prf);
+    } else if (dc > 0.0f) {
+        if (fn < fadd_rn(-half, dc)) fn = fadd_rn(fn, prf);
+    }
+    if (fn < fma_rn(-half, a.frac, c.dc_off) || fn > fma_rn(half, a.frac, c.dc_off)) return s;
+    s.band = true;
+    // --- RCMC: walk = lambda^2 fn^2 / (8 Vr^2) [float, IEEE divide] * R0 / range spacing
+    const float shift = rcmc_shift(c, rcmc_numerator(a, fn));
+    const int walk = static_cast<int>(roundf(shift));
+    const int calc_x = x + walk;
+    if (calc_x - kRcmcTaps / 2 < 0 || calc_x + kRcmcTaps / 2 >= a.nk) return s;
+    const int first = cs + walk - kRcmcTaps / 2;  // smem column of tap 0
+    if (first + 1 < 0 || first + kRcmcTaps - 1 > a.wt) {
+        atomic_or_u32(err_flag, kErrRcmcHalo);
+        return s;
+    }
+    // off = shift - walk + 8 in [7.5, 8.5] as the reference rounds it; off - 8 is exact
+    const float off = fadd_rn(fsub_rn(shift, static_cast<float>(walk)), static_cast<float>(kRcmcTaps / 2));
+    s.dl = fsub_rn(off, static_cast<float>(kRcmcTaps / 2));
+    s.first = first;
+    return s;
+}
+
+// Windowed sinc at off - i, off = shift - walk + 8 in [7.5, 8.5]:
+// sin(pi (off - i)) = (-1)^i sin(pi off), and the common factor sin(pi off) / pi
+// cancels in the normalised sum, leaving weights (-1)^i W_i / (off - i).  The two end
+// taps are skipped: their window values W_0 = W_15 = -1.4e-17 (a numpy.blackman
+// rounding residue of an exact zero) give terms below half an ulp of every sum.
+// With dl = off - 8 (exact) a weight is 1 / fma(dl, c_i, (8 - i) c_i), c_i = (-1)^i / W_i
+// (constants): one FMA and one reciprocal per tap, within 2 ulp of the quotient since
+// |8 - i| >= 1 wherever the constant term is not zero.  The normaliser sums in pairs.
+struct TapSum {
+    float2 acc, nrm2;
+    ASARF_HD ASARF_INLINE TapSum() : acc(make_float2(0.0f, 0.0f)), nrm2(acc) {}
+    // taps i (odd) and i + 1
+    ASARF_HD ASARF_INLINE void add(int i, float dl, float2 u, float2 v) {
+        constexpr float kWin[kRcmcTaps] = ASARF_BLACKMAN16;
+        const float ca = -1.0f / kWin[i], cb = 1.0f / kWin[i + 1];
+        const float wa = rcp_approx(fma_rn(dl, ca, static_cast<float>(kRcmcTaps / 2 - i) * ca));
+        const float wb = rcp_approx(fma_rn(dl, cb, static_cast<float>(kRcmcTaps / 2 - i - 1) * cb));
+        acc = pfma(u, wa, acc);
+        acc = pfma(v, wb, acc);
+        nrm2 = padd(nrm2, make_float2(wa, wb));
+    }
+    // centre: the sample at the integer walk, which a walk without fraction takes (a unit impulse)
+    ASARF_HD ASARF_INLINE float2 value(float dl, const float2* centre) const {
+        if (dl == 0.0f) return *centre;
+        const float nrm = fadd_rn(nrm2.x, nrm2.y);
+        if (nrm == 0.0f) return make_float2(0.0f, 0.0f);
+        const float inv = rcp_approx(nrm);
+        return make_float2(fmul_rn(acc.x, inv), fmul_rn(acc.y, inv));
+    }
+};
+
+ASARF_HD ASARF_INLINE float2 rcmc_taps(const float2* srow, const SampleWalk& w) {
+    if (w.first == SampleWalk::kNoTaps) return make_float2(0.0f, 0.0f);
+    const float2* s = srow + w.first;
+    TapSum t;
+#pragma unroll
+    for (int i = 1; i < kRcmcTaps - 1; i += 2) t.add(i, w.dl, s[i], s[i + 1]);
+    return t.value(w.dl, s + kRcmcTaps / 2);
+}
+
+// The taps of two adjacent samples with one integer walk: 15 columns, read as the 16-byte units from the even
+// one at or below the first (ODD: tap 1 is the unit's second sample).
+template <bool ODD>
+ASARF_HD ASARF_INLINE void rcmc_taps_pair(const float2* srow, const SampleWalk& wa, const SampleWalk& wb, float2* va,
+                                          float2* vb) {
+    const float4* q = reinterpret_cast<const float4*>(srow + (ODD ? wa.first : wa.first + 1));
+    TapSum ta, tb;
+    float4 d = q[0];
+    float2 lo = ODD ? make_float2(d.z, d.w) : make_float2(d.x, d.y);  // first sample's next tap
+#pragma unroll
+    for (int i = 1; i < kRcmcTaps - 1; i += 2) {
+        float2 mid, hi;
+        if (ODD) {
+            d = q[i / 2 + 1];
+            mid = make_float2(d.x, d.y), hi = make_float2(d.z, d.w);
+        } else {
+            mid = make_float2(d.z, d.w);
+            d = q[i / 2 + 1];
+            hi = make_float2(d.x, d.y);
+        }
+        ta.add(i, wa.dl, lo, mid);
+        tb.add(i, wb.dl, mid, hi);
+        lo = hi;
+    }
+    *va = ta.value(wa.dl, srow + wa.first + kRcmcTaps / 2);
+    *vb = tb.value(wb.dl, srow + wb.first + kRcmcTaps / 2);
+}
+
+// Matched filter exp(-j pi fc^2 / Ka) * exp(-j 2 pi (dc_off / Ka) f), both phases
+// rounded as the reference rounds them, combined into one reduced exponential.
+ASARF_HD ASARF_INLINE float2 mf_sample(const AzRdArgs& a, const ColUse& c, float bf, const SampleWalk& w, float2 v) {
+    if (!w.band) return make_float2(0.0f, 0.0f);
+    float fc = fsub_rn(bf, c.dc_off);
+    if (fc > a.half_prf) fc = fsub_rn(fc, a.prf);
+    else if (fc < -a.half_prf) fc = fadd_rn(fc, a.prf);
+    const float mf_phase = div_by_recip_rn(fmul_rn(fmul_rn(3.14159265358979323846f, fc), fc), c.ka, c.rka);
+    return cmul(v, expj_neg_sum(mf_phase, fmul_rn(c.sh, bf)));
+}
+
+// One sample, and two adjacent ones (columns x, x + 1, of which the first lies inside the line; cs even).
+// The columns' constants come from the lane's registers and the centroid table: formed anew for each
+// sample (two FP64 and three float divisions, two polynomials) they were most of a slow row.  Adjacent
+// samples nearly always share the integer walk, and then their loads: 16-byte units in place of 8-byte ones two
+// columns apart.  A third of the rows slow (centroid 1039 Hz, PRF 2080 Hz, 5616 x 9973, n2 = 100): 684 -> 604
+// us with the constants held, 593 with the loads shared (a lane per column and no table for any row: 607).
+ASARF_HD ASARF_INLINE float2 rcmc_mf_sample(const AzRdArgs& a, const ColUse& c, float dc, int x, float bf,
+                                            const float2* srow, int cs, unsigned int* err_flag) {
+    const SampleWalk w = rcmc_decide(a, c, dc, x, bf, cs, err_flag);
+    return mf_sample(a, c, bf, w, rcmc_taps(srow, w));
+}
+ASARF_HD ASARF_INLINE void rcmc_mf_samples(const AzRdArgs& a, const ColUse& ca, const ColUse& cb, float2 dc, int x,
+                                           float bf, const float2* srow, int cs, unsigned int* err_flag, float2* va,
+                                           float2* vb) {
+    const SampleWalk wa = rcmc_decide(a, ca, dc.x, x, bf, cs, err_flag);
+    SampleWalk wb{false, SampleWalk::kNoTaps, 0.0f};
+    if (x + 1 < a.nk) wb = rcmc_decide(a, cb, dc.y, x + 1, bf, cs + 1, err_flag);
+    float2 ua, ub;
+    if (wa.first != SampleWalk::kNoTaps && wb.first == wa.first + 1) {
+        if (wa.first & 1) rcmc_taps_pair<false>(srow, wa, wb, &ua, &ub);
+        else rcmc_taps_pair<true>(srow, wa, wb, &ua, &ub);
+    } else {
+        ua = rcmc_taps(srow, wa);
+        ub = rcmc_taps(srow, wb);
+    }
+    *va = mf_sample(a, ca, bf, wa, ua);
+    *vb = mf_sample(a, cb, bf, wb, ub);
 }
 
 struct RowRec {
@@ -1445,6 +1534,7 @@ struct AzRdTables {
     RowSpan* span;
     int* used;  // az_rd_used_columns
     float* weights;
+    float* dc;  // the columns' centroids
     float2* phs;
     RowRec* rows;
     ASARF_HD ASARF_INLINE AzRdTables(const AzRdArgs& a, float2* tile) {
@@ -1453,7 +1543,8 @@ struct AzRdTables {
         span = reinterpret_cast<RowSpan*>(cols + a.xt);
         used = reinterpret_cast<int*>(span + 2);
         weights = reinterpret_cast<float*>(cols);
-        phs = reinterpret_cast<float2*>(reinterpret_cast<unsigned char*>(cols) + az_rd_cols_bytes(a.xt));
+        dc = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(cols) + az_rd_cols_bytes(a.xt));
+        phs = reinterpret_cast<float2*>(dc + a.xt);
         rows = reinterpret_cast<RowRec*>(phs + (a.absolute_phase ? a.xt : 0));
     }
 };
@@ -1469,6 +1560,7 @@ ASARF_HD ASARF_INLINE void az_rd_tables(const AzRdArgs& a, int tile, int k1, int
         const ColParams cp = az_col_params(a, x0 + c);
         if (tid < a.xt) {
             t.cols[c].set(cp);
+            t.dc[c] = cp.dc;
             if (a.absolute_phase) t.phs[c] = az_abs_phase(a, cp, x0 + c);
         }
         RowSpan sp;
@@ -1480,6 +1572,7 @@ ASARF_HD ASARF_INLINE void az_rd_tables(const AzRdArgs& a, int tile, int k1, int
     for (int c = 0; c < a.xt; ++c) {
         const ColParams cp = az_col_params(a, x0 + c);
         t.cols[c].set(cp);
+        t.dc[c] = cp.dc;
         if (a.absolute_phase) t.phs[c] = az_abs_phase(a, cp, x0 + c);
         RowSpan o;
         o.set(cp);
@@ -1498,7 +1591,7 @@ ASARF_HD ASARF_INLINE void az_rd_tables(const AzRdArgs& a, int tile, int k1, int
 // Shared-memory bytes of the range-Doppler block.
 inline size_t az_rd_smem(int n2, int wt, int xt, bool absolute_phase) {
     return sizeof(float2) * static_cast<size_t>(n2) * wt + static_cast<size_t>(az_rd_cols_bytes(xt)) +
-           sizeof(RowRec) * static_cast<size_t>(n2) +
+           sizeof(float) * static_cast<size_t>(xt) + sizeof(RowRec) * static_cast<size_t>(n2) +
            (absolute_phase ? sizeof(float2) * static_cast<size_t>(xt) : 0);
 }
 
@@ -1539,14 +1632,9 @@ ASARF_HD ASARF_INLINE void rcmc_pair_taps(const float4* q, const float4* w, floa
     *vb = acc_b;
 }
 
-// Fraction of the range walk past the row's integer walk, with the reference's roundings
-// (rcmc_mf_sample): quotient num / den, times R0 / range spacing as a float pair (the product's
-// rounding differs from the FP64 one's only within 2^-45 of a tie), minus the walk, plus 8.
+// Fraction of the range walk past the row's integer walk, plus 8, with the reference's roundings.
 ASARF_HD ASARF_INLINE float rcmc_offset(const ColUse& c, float num, float walk) {
-    const float q = div_by_recip_rn(num, c.den, c.rden);
-    const float p = fmul_rn(q, c.r0_hi);
-    const float shift = fadd_rn(p, fma_rn(q, c.r0_lo, fma_rn(q, c.r0_hi, -p)));
-    return fadd_rn(fsub_rn(shift, walk), static_cast<float>(kRcmcTaps / 2));
+    return fadd_rn(fsub_rn(rcmc_shift(c, num), walk), static_cast<float>(kRcmcTaps / 2));
 }
 
 // Two adjacent columns x, x + 1 of a uniform row, interpolated and filtered: srow the tile row, c the
@@ -1696,9 +1784,7 @@ ASARF_HD ASARF_INLINE void az_rd_body(const AzRdArgs& a, int tile, int k1, int t
             if (rec.code >= 0) {
                 rcmc_mf_pair(a, rec, wbuf, edge, ca, cb, x, srow, c, &va, &vb);
             } else if (rec.code == kRowSlow) {
-                if (x < a.nk) va = rcmc_mf_sample(a, az_col_params(a, x), x, rec.bf, srow, a.hl + c, err_flag);
-                if (x + 1 < a.nk)
-                    vb = rcmc_mf_sample(a, az_col_params(a, x + 1), x + 1, rec.bf, srow, a.hl + c + 1, err_flag);
+                if (x < a.nk) rcmc_mf_samples(a, ca, cb, *reinterpret_cast<const float2*>(t.dc + c), x, rec.bf, srow, a.hl + c, err_flag, &va, &vb);
             }
             if (a.absolute_phase) {
                 va = cmul(va, t.phs[c]);
@@ -1722,7 +1808,7 @@ ASARF_HD ASARF_INLINE void az_rd_body(const AzRdArgs& a, int tile, int k1, int t
                         rcmc_mf_pair(a, rec, rcmc_weights(a, rec.code), edge, t.cols[c], t.cols[c + 1], x0 + c, srow,
                                      c, &rowbuf[c], &rowbuf[c + 1]);
                 } else if (rec.code == kRowSlow && x0 + c < a.nk) {
-                    rowbuf[c] = rcmc_mf_sample(a, az_col_params(a, x0 + c), x0 + c, rec.bf, srow, a.hl + c, err_flag);
+                    rowbuf[c] = rcmc_mf_sample(a, t.cols[c], t.dc[c], x0 + c, rec.bf, srow, a.hl + c, err_flag);
                 } else {
                     rowbuf[c] = make_float2(0.0f, 0.0f);
                 }
