@@ -1879,19 +1879,18 @@ ASARF_HD ASARF_INLINE void copy_units(const uint8_t* src, uint8_t* dst, int unit
 // line y, its SWST and PRI codes (big-endian, ISP bytes 38-39 and 40-41 after the 32 bytes of
 // sensing time and FEP annotation) to swst[y] / pri[y]; the FEP ISP length (11465) and the
 // auxiliary section's 0xAA marker are checked as ParseErsLevel0ImPackets checks them
-// (envisat_format/src/ers_im_parse.cc:423-453).  Block y.  Raw lines are multiples of 16 bytes,
-// so a 16-byte aligned raw buffer takes whole 16-byte units; any other one, and the end of a line
-// whose packet is not aligned, 2-byte words (packet offsets are even: whole MDSRs of 11498 bytes).
+// (envisat_format/src/ers_im_parse.cc:423-453).  A warp takes the line.  Its 16-byte aligned interior moves by
+// whole units, what lies before and after it (at most 15 and 31 bytes) by bytes: 28000 lines to a raw buffer
+// 2 bytes off 16-byte alignment 113 us, as aligned; all by 2-byte words 400.
 ASARF_HD ASARF_INLINE void ers_unpack_line(const ErsUnpackArgs& a, int y, int tid, int nthr) {
     const uint8_t* pk = a.mdsr + ASARF_LDG(a.offset + y);
     const uint8_t* src = pk + kErsMeasurementOffset;
     uint8_t* dst = a.raw + static_cast<long long>(y) * kErsMeasurementBytes;
-    const int units =
-        (reinterpret_cast<uintptr_t>(a.raw) & 15) == 0 ? copy_units_of(src, kErsMeasurementBytes) : 0;
-    copy_units<4>(src, dst, units, tid, nthr);
-    const uint16_t* src2 = reinterpret_cast<const uint16_t*>(src);
-    uint16_t* dst2 = reinterpret_cast<uint16_t*>(dst);
-    for (int i = 8 * units + tid; i < kErsMeasurementBytes / 2; i += nthr) dst2[i] = src2[i];
+    const int head = static_cast<int>((16 - (reinterpret_cast<uintptr_t>(dst) & 15)) & 15);
+    const int units = copy_units_of(src + head, kErsMeasurementBytes - head);
+    copy_units<4>(src + head, dst + head, units, tid, nthr);
+    for (int i = tid; i < head; i += nthr) dst[i] = src[i];
+    for (int i = head + 16 * units + tid; i < kErsMeasurementBytes; i += nthr) dst[i] = src[i];
     if (tid == 0) {
         const int isp_len = (pk[24] << 8) | pk[25];
         unsigned e = 0;
