@@ -11,6 +11,7 @@ Usage: python asar-focus_b200/build.py [--emu DIR]
 from __future__ import annotations
 
 import os
+import re
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -48,6 +49,30 @@ def _stale(target: Path, deps: list[Path]) -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def _cases(header: str, macro: str) -> list[str]:
+    """The argument lists of an X-macro: ``X(5, 5, 5) X(8, 7, 3)`` -> ["5, 5, 5", "8, 7, 3"]."""
+    text = (CSRC / header).read_text().replace("\\\n", " ")
+    m = re.search(rf"#define {macro}\(X\)(.*)", text)
+    return re.findall(r"X\(([^)]*)\)", m.group(1))
+
+
+def units() -> list[tuple[str, str, list[str]]]:
+    """(source, object name, macros) of every translation unit.  A unit is one module, loaded when the first of
+    its kernels is asked for, so each compiled schedule and length has its own."""
+    out = [(s, s, []) for s in ("kernels.cu", "az_rd_split.cu", "noalloc.cu", "host.cpp", "stages.cpp", "batch.cpp",
+                                "strip.cpp", "l0.cpp")]
+    tiles = [f"0, 0, 0, {xt}, {nb}" for xt, nb in ((16, 1), (32, 1), (32, 2), (32, 4), (32, 8))]
+    tiles += [f"{r}, 32, 1" for r in _cases("params.h", "ASARF_STRIDED_SCHEDULES")]
+    for src, macros, values in (
+            ("az_rd.cu", "R0 R1 R2", ["0, 0, 0"] + _cases("params.h", "ASARF_BLOCK_SCHEDULES")),
+            ("az_strided.cu", "R0 R1 R2 XT NB", tiles),
+            ("range_compress.cu", "LENGTH", ["0"] + _cases("fft_ct.cuh", "ASARF_CT_LENGTHS"))):
+        for v in values:
+            v = v.split(", ")
+            out.append((src, f"{src}.{'_'.join(v)}", [f"-DASARF_{m}={x}" for m, x in zip(macros.split(), v)]))
+    return out
+
+
 def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
     """Compile the product library (sm_100a)."""
     deps = _sources()
@@ -57,9 +82,9 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
     objdir.mkdir(exist_ok=True)
     common = ["-std=c++17", "-O3", "-lineinfo", f"-I{INC}", f"-I{CSRC}", "-Xcompiler", "-fPIC"]
     objs, cmds = [], []
-    for src in ("kernels.cu", "noalloc.cu", "host.cpp", "stages.cpp", "batch.cpp", "strip.cpp", "l0.cpp"):
-        obj = objdir / (src + ".o")
-        cmd = [NVCC, *GENCODE, *common, "-c", str(CSRC / src), "-o", str(obj)]
+    for src, name, macros in units():
+        obj = objdir / (name + ".o")
+        cmd = [NVCC, *GENCODE, *common, *macros, "-c", str(CSRC / src), "-o", str(obj)]
         if src.endswith(".cu") and verbose_ptxas:
             cmd += ["-Xptxas", "-v"]
         if src.endswith(".cpp"):
@@ -68,7 +93,7 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
         objs.append(str(obj))
     with ThreadPoolExecutor() as pool:
         list(pool.map(_run, cmds))
-    _run([NVCC, *GENCODE, "-shared", "-o", str(LIB), *objs, "-lcudart"])
+    _run([NVCC, *GENCODE, "-shared", "-Xlinker", "-z,defs", "-o", str(LIB), *objs, "-lcudart"])
     return LIB
 
 

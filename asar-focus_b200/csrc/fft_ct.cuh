@@ -62,7 +62,10 @@ ASARF_CT_SCHEDULE(6144, 256, 3, 16, 24, 16);
 ASARF_CT_SCHEDULE(8192, 256, 2, 16, 16, 32);
 #undef ASARF_CT_SCHEDULE
 
-constexpr int kCtLengths[] = {768, 1024, 1536, 2048, 3072, 4096, 6144, 8192};
+#define ASARF_CT_LENGTHS(X) X(768) X(1024) X(1536) X(2048) X(3072) X(4096) X(6144) X(8192)
+#define ASARF_LENGTH_ITEM(L) L,
+constexpr int kCtLengths[] = {ASARF_CT_LENGTHS(ASARF_LENGTH_ITEM)};
+#undef ASARF_LENGTH_ITEM
 
 // Radix sequence of a compile-time length (host: digit reversal, matched filter, tables).
 inline int ct_radices(int L, int* out) {

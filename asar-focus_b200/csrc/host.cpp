@@ -1197,6 +1197,17 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
                          a3);
     }
 
+    // load the kernels of this plan's schedules now, not in its first run (which may be a capture)
+    rc = backend_range_compress(p->a_rc, 0, p->sh_rc, nullptr);
+    if (!rc) rc = backend_az_strided(p->a_fwd, nullptr, 0, p->sh_st, nullptr);
+    if (!rc)
+        rc = p->split ? backend_az_rd_split(p->a_rd, p->a_split, p->tmapA2, 0, 0, p->sh_rd_split, nullptr, nullptr)
+                      : backend_az_rd(p->a_rd, nullptr, 0, 0, p->sh_rd, nullptr, nullptr);
+    if (rc) {
+        delete p;
+        return rc;
+    }
+
     asarf_dims& dm = p->dims;
     dm.nk = p->nk;
     dm.rg_pad_ref = p->rg_pad_ref;

@@ -1,12 +1,10 @@
-// CUDA kernels of the focusing path (sm_100a) and their launchers.
+// CUDA kernels of the focusing path (sm_100a) and their launchers: statistics, finalisation, tail, records and the
+// per-stage kernels.  The transform kernels are in range_compress.cu, az_strided.cu, az_rd.cu and az_rd_split.cu.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
-#include <map>
-#include <mutex>
-#include <utility>
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -15,7 +13,7 @@
 #include "backend.h"
 #include "bodies.cuh"
 #include "context_cache.h"
-#include "tc.cuh"
+#include "launch.cuh"
 #include "tma.cuh"
 
 namespace asarf {
@@ -248,240 +246,6 @@ __global__ void __launch_bounds__(kFinalizeThreads) k_finalize(FinalizeArgs a) {
     }
 }
 
-// Raw record of n bytes into shared memory: its 16-byte aligned interior by one bulk copy of thread 0,
-// the bytes before and after it (records start and end anywhere) by plain loads, so nothing outside
-// the record is read.  The copy starts at buf + (address mod 16), buf 16-byte aligned, which keeps
-// the interior aligned in shared memory as well.  (Lines off 16-byte alignment decoded from global
-// memory sample by sample, FBAQ4 records moved by vector loads: 17011 lines of 10386 bytes 803 ->
-// 626 us, 30000 FBAQ4 records 1287 -> 1238 us.)
-__device__ __forceinline__ const uint8_t* stage_record(uint8_t* buf, const uint8_t* rec, int n, uint64_t* bar,
-                                                       unsigned int* err) {
-    const int lead = static_cast<int>(reinterpret_cast<uintptr_t>(rec) & 15);
-    const int head = min(n, (16 - lead) & 15);
-    const int body = (n - head) & ~15;
-    uint8_t* dst = buf + lead;
-    if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        mbar_expect_tx(bar, static_cast<uint32_t>(body));
-        if (body) bulk_load(dst + head, rec + head, static_cast<uint32_t>(body), bar);
-    }
-    for (int i = threadIdx.x; i < head; i += blockDim.x) dst[i] = rec[i];
-    for (int i = head + body + threadIdx.x; i < n; i += blockDim.x) dst[i] = rec[i];
-    __syncthreads();
-    mbar_wait(bar, 0, err);
-    return dst;
-}
-
-// One raw line per block.
-template <int FMT>
-__device__ __forceinline__ const uint8_t* stage_line(const RangeCompressArgs& a, unsigned char* smem, uint64_t* bar) {
-    const int n = FMT == kRawAsarFbaq4 ? static_cast<int>(a.line_bytes) : 2 * a.spl;
-    return stage_record(smem + a.raw_smem_offset, a.raw + static_cast<long long>(blockIdx.x) * a.line_bytes, n, bar,
-                        &const_cast<FocusState*>(a.state)->errors);
-}
-
-template <int FMT>
-__global__ void __launch_bounds__(512) k_range_compress(RangeCompressArgs a) {
-    extern __shared__ __align__(128) unsigned char smem_rc_raw[];
-    __shared__ uint64_t bar;
-    const uint8_t* line = stage_line<FMT>(a, smem_rc_raw, &bar);
-    range_compress_body<FMT>(a, blockIdx.x, threadIdx.x, blockDim.x, reinterpret_cast<float2*>(smem_rc_raw), line);
-}
-
-// Compile-time-scheduled variant (L in kCtLengths).
-template <int L, int FMT>
-__global__ void __launch_bounds__(CtSchedule<L>::nthr, CtSchedule<L>::blocks) k_range_compress_ct(RangeCompressArgs a) {
-    extern __shared__ __align__(128) unsigned char smem_rcc_raw[];
-    __shared__ uint64_t bar;
-    const uint8_t* line = stage_line<FMT>(a, smem_rcc_raw, &bar);
-    range_compress_ct_body<L, FMT>(a, blockIdx.x, threadIdx.x, reinterpret_cast<float2*>(smem_rcc_raw), line);
-}
-
-// Strided azimuth pass: the [n1][NB][XT] tiles (rows r*n2 + b + k) arrive by 3-D TMA boxes.
-// R0..R2 > 0: compile-time transform schedule (az_strided_body).
-template <int R0, int R1, int R2, int XT, int NB>
-__global__ void __launch_bounds__(256, 3) k_az_strided(AzStridedArgs a, const __grid_constant__ CUtensorMap map) {
-    extern __shared__ __align__(128) unsigned char smem_as_raw[];
-    float2* s = reinterpret_cast<float2*>(smem_as_raw);
-    float2* tw = s + static_cast<size_t>(a.n1) * XT * NB;
-    int* row = reinterpret_cast<int*>(tw + a.n1 * NB);
-    __shared__ uint64_t bar;
-    const int b = blockIdx.y * NB;
-    if (a.use_tma && threadIdx.x == 0) {
-        mbar_init(&bar, 1);
-        mbar_expect_tx(&bar, static_cast<uint32_t>(sizeof(float2) * a.n1 * XT * NB));
-        for (int r0 = 0; r0 < a.n1; r0 += a.n1_box)
-            tma_load_3d(s + static_cast<size_t>(r0) * XT * NB, &map, &bar, 2 * blockIdx.x * XT, b, r0);
-    }
-    // twiddle and row tables are gathered while the tile is in flight
-    az_strided_tables(a, b, threadIdx.x, blockDim.x, tw, row);
-    __syncthreads();
-    if (a.use_tma) mbar_wait(&bar, 0, a.state ? &const_cast<FocusState*>(a.state)->errors : nullptr);
-    az_strided_body<R0, R1, R2, XT, NB>(a, blockIdx.x, b, threadIdx.x, blockDim.x, s, tw, row, a.use_tma != 0);
-}
-
-// Range-Doppler block: the [n2][wt] tile (contiguous rows, range halo) arrives by 2-D TMA
-// boxes; columns left of 0 and right of nk are filled with zeros by the TMA unit.
-// R0..R2 > 0: compile-time radix schedule of the n2 transforms (az_rd_body).
-template <int R0 = 0, int R1 = 0, int R2 = 0>
-__global__ void __launch_bounds__(512, 2) k_az_rd(AzRdArgs a, unsigned int* err, const __grid_constant__ CUtensorMap map) {
-    // (128-byte alignment: a larger one pads the static barrier below to as much, and two blocks
-    // of kAzRdTwoBlockSmem bytes would no longer fit)
-    extern __shared__ __align__(128) unsigned char smem_rd_raw[];
-    const int wt = a.wt;
-    float2* s = reinterpret_cast<float2*>(smem_rd_raw);
-    const AzRdTables t(a, s);
-    __shared__ uint64_t bar;
-    if (a.use_tma && threadIdx.x == 0) {
-        mbar_init(&bar, 1);
-        mbar_expect_tx(&bar, static_cast<uint32_t>(sizeof(float2) * a.n2 * wt));
-        const int x = 2 * (static_cast<int>(blockIdx.x) * a.xt - a.hl);
-        for (int r0 = 0; r0 < a.n2; r0 += a.n2_box)
-            tma_load_2d(s + static_cast<size_t>(r0) * wt, &map, &bar, x, blockIdx.y * a.n2 + r0);
-    }
-    // column constants and row frequencies are computed while the tile is in flight
-    az_rd_tables(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, t);
-    __syncthreads();
-    if (a.use_tma) mbar_wait(&bar, 0, err);
-    az_rd_body<true, R0, R1, R2>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, s, t, err, a.use_tma != 0);
-}
-
-// ----------------------------------------------------------------------------- split precision
-// Forward transform of the range-Doppler tile on the tensor cores.  Tile s[l][c], l < n2 =
-// R * m, c < wt.  Operand row rho = r * wt + c holds the sub-sequence x[r + R mm] (mm < m) of
-// column c as bf16 hi + lo parts (K = (mm, re / im)); it multiplies the m-point DFT matrix B
-// (hi + lo, output slot s = frequency k1(s)) as Ahi Bhi + Ahi Blo + Alo Bhi with FP32
-// accumulation, and the result times W_n2^(r k1(s)) goes back to row r + R s of column c (a
-// row of the same sub-sequence, already consumed).  The operands live in tensor memory
-// beside the accumulator (TMEM columns [0, 64) accumulator, [64, 96) A hi, [96, 128) A lo),
-// so shared memory holds only B and the tile and two blocks stay resident per SM, as in the
-// FP32 kernel.  Rounds of 128 operand rows: warp w writes TMEM lanes 32 (w % 4) .., K chunk
-// w / 4 (8 inputs), one thread issues the products, every thread reads back its lane.  A
-// radix-R FP32 pass over rows R s .. R s + R - 1 then leaves frequency k1(s) + m k2 at row
-// R s + k2: the digit-reversed order of the FP32 forward transform (k1(s) from that
-// transform's order table).  Returns false (error bit set, products drained) if a product did
-// not complete in time.
-constexpr uint32_t kSplitColAcc = 0, kSplitColAHi = 64, kSplitColALo = 96;
-
-__device__ bool split_forward(const AzRdArgs& a, const AzRdSplit& sp, float2* s, const unsigned char* b_hi,
-                              const unsigned char* b_lo, uint32_t tmem, uint64_t* mbar, unsigned int* err) {
-    const int tid = threadIdx.x, nthr = blockDim.x;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int wt = a.wt, R = sp.radix, m = sp.m;
-    const int rows = R * wt;
-    const int q = warp & 3, jb = warp >> 2;  // TMEM lane quarter, K chunk / accumulator column block
-    const uint32_t lane_base = static_cast<uint32_t>(32 * q) << 16;
-    const FastDiv dwt = make_fastdiv(static_cast<unsigned int>(wt));
-    constexpr uint32_t kIdesc = umma_idesc_bf16(kSplitRows, kSplitN);
-    constexpr uint32_t kSbo = kSplitK * 16;  // 8 rows x K bf16
-    (void)nthr;
-    uint32_t phase = 0;
-    for (int g0 = 0; g0 < rows; g0 += kSplitRows) {
-        const int rho = g0 + 32 * q + lane;
-        const bool live = rho < rows;
-        int r = 0, c = 0;
-        if (live) {
-            r = static_cast<int>(fdiv_u(static_cast<unsigned int>(rho), dwt));
-            c = rho - r * wt;
-        }
-        {
-            uint32_t hi[8], lo[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int mm = 8 * jb + i;
-                const float2 v = (live && mm < m) ? s[(r + R * mm) * wt + c] : make_float2(0.0f, 0.0f);
-                split_bf16x2(v.x, v.y, hi[i], lo[i]);
-            }
-            tmem_st8(tmem + lane_base + kSplitColAHi + 8u * jb, hi);
-            tmem_st8(tmem + lane_base + kSplitColALo + 8u * jb, lo);
-            tmem_wait_st();
-        }
-        tc_fence_before_sync();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after_sync();
-            const uint32_t bh = smem_u32(b_hi), bl = smem_u32(b_lo);
-#pragma unroll
-            for (int ks = 0; ks < kSplitK / 16; ++ks) {
-                const uint32_t o = 256u * ks;  // B: two 128-byte core-matrix columns per k-step
-                const uint64_t dbh = umma_smem_desc(bh + o, 128, kSbo), dbl = umma_smem_desc(bl + o, 128, kSbo);
-                const uint32_t ah = tmem + kSplitColAHi + 8u * ks, al = tmem + kSplitColALo + 8u * ks;
-                umma_bf16_ts(tmem + kSplitColAcc, ah, dbh, kIdesc, ks > 0);
-                umma_bf16_ts(tmem + kSplitColAcc, ah, dbl, kIdesc, true);
-                umma_bf16_ts(tmem + kSplitColAcc, al, dbh, kIdesc, true);
-            }
-            umma_commit(mbar);
-        }
-        const bool done = mbar_wait(mbar, phase, nullptr);
-        if (__syncthreads_or(!done)) {
-            if (tid == 0) atomicOr(err, kErrMmaTimeout);
-            mbar_wait(mbar, phase, nullptr);  // one more bounded wait for the products in flight
-            return false;
-        }
-        phase ^= 1u;
-        tc_fence_after_sync();
-        // accumulator: this warp's lanes, columns 16 jb .. (output slots 8 jb ..)
-        if (8 * jb < m) {  // warp-uniform
-            float v[16];
-            tmem_ld16(tmem + lane_base + kSplitColAcc + 16u * jb, v);
-            if (live) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int slot = 8 * jb + i;
-                    if (slot < m)
-                        s[(r + R * slot) * wt + c] = cmul(make_float2(v[2 * i], v[2 * i + 1]), __ldg(sp.tw + r * m + slot));
-                }
-            }
-        }
-        tc_fence_before_sync();
-        __syncthreads();
-    }
-    // radix-R DFT over r of every (slot, column pair): rows R * slot + r, no twiddles
-    const int npair = wt >> 1;
-    fft_stage_pair_w_dispatch<false, false, NoEpi, false>(R, s, a.n2, 1, make_fastdiv(1u), PairTasks(npair), wt,
-                                                          a.plan2.tw, tid, blockDim.x);
-    __syncthreads();
-    return true;
-}
-
-__global__ void __launch_bounds__(512, 2) k_az_rd_split(AzRdArgs a, AzRdSplit sp, unsigned int* err,
-                                                        const __grid_constant__ CUtensorMap map) {
-    extern __shared__ __align__(128) unsigned char smem_rds_raw[];
-    unsigned char* b_hi = smem_rds_raw;
-    unsigned char* b_lo = b_hi + kSplitMatrixBytes;
-    float2* s = reinterpret_cast<float2*>(b_lo + kSplitMatrixBytes);
-    const int wt = a.wt;
-    const AzRdTables t(a, s);
-    __shared__ uint64_t bar, mbar;
-    __shared__ uint32_t tmem_base;
-    if (threadIdx.x < 32) tmem_alloc(&tmem_base, kSplitTmemCols);
-    if (threadIdx.x == 0) {
-        mbar_init(&mbar, 1);
-        mbar_init(&bar, 1);
-        mbar_expect_tx(&bar, static_cast<uint32_t>(sizeof(float2) * a.n2 * wt));
-        const int x = 2 * (static_cast<int>(blockIdx.x) * a.xt - a.hl);
-        for (int r0 = 0; r0 < a.n2; r0 += a.n2_box)
-            tma_load_2d(s + static_cast<size_t>(r0) * wt, &map, &bar, x, blockIdx.y * a.n2 + r0);
-    }
-    // the DFT matrix images and the column / row tables while the tile is in flight
-    const uint4* bsrc = reinterpret_cast<const uint4*>(sp.bmat);
-    for (int i = threadIdx.x; i < 2 * kSplitMatrixBytes / 16; i += blockDim.x)
-        reinterpret_cast<uint4*>(b_hi)[i] = __ldg(bsrc + i);
-    az_rd_tables(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, t);
-    fence_async_smem();  // B is read by the tensor cores
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    const uint32_t tmem = tmem_base;
-    mbar_wait(&bar, 0, err);
-    if (split_forward(a, sp, s, b_hi, b_lo, tmem, &mbar, err))
-        az_rd_body<false>(a, blockIdx.x, blockIdx.y, threadIdx.x, blockDim.x, s, t, err, true);
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    if (threadIdx.x < 32) tmem_dealloc(tmem, kSplitTmemCols);
-}
-
 __global__ void __launch_bounds__(128) k_rcmc_table(float* table) {
     const int n = blockIdx.x * 128 + threadIdx.x;
     if (n <= kRcmcNodes) rcmc_weight_row(n, table + static_cast<size_t>(n) * kRcmcRowFloats);
@@ -519,17 +283,6 @@ __global__ void __launch_bounds__(256) k_img_moments(ImgMomentsArgs a) {
 __global__ void __launch_bounds__(kAcccCols) k_accc(AcccArgs a) {
     __shared__ double cols[2 * kAcccCols];
     accc_body(a, blockIdx.x, blockIdx.y, gridDim.x, threadIdx.x, kAcccCols, cols);
-}
-
-__global__ void __launch_bounds__(512) k_rc_rows(RcRowsArgs a) {
-    extern __shared__ float2 smem_rcr[];
-    rc_rows_body(a, blockIdx.x, threadIdx.x, blockDim.x, smem_rcr);
-}
-
-template <int L>
-__global__ void __launch_bounds__(CtSchedule<L>::nthr, CtSchedule<L>::blocks) k_rc_rows_ct(RcRowsArgs a) {
-    extern __shared__ float2 smem_rcrc[];
-    rc_rows_ct_body<L>(a, blockIdx.x, threadIdx.x, smem_rcrc);
 }
 
 // Matched filter: eight threads share a position's sum.
@@ -592,33 +345,6 @@ int grid_for(long long n) {
 // Grid height of the column kernels, whose blocks stride over the rows past it.
 int column_blocks(int rows) { return static_cast<int>(std::min((rows + kColumnRows - 1ll) / kColumnRows, 1ll * kMaxGridY)); }
 
-int check_launch(const char* what) {
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return set_error(ASARF_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
-    return ASARF_OK;
-}
-
-// Raise a kernel's dynamic shared-memory limit to `bytes` (once per kernel, device and size:
-// the default limit of 48 KiB counts the kernel's static shared memory too, so any dynamic
-// size is checked, not only those above 48 KiB).
-template <class K>
-int ensure_smem(K kernel, size_t bytes, const char* what) {
-    static std::mutex mu;
-    static std::map<std::pair<const void*, int>, size_t> done;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lock(mu);
-    const auto key = std::make_pair(reinterpret_cast<const void*>(kernel), dev);
-    auto it = done.find(key);
-    if (it != done.end() && it->second >= bytes) return ASARF_OK;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-    if (e != cudaSuccess) return set_error(ASARF_ERR_CUDA, "%s smem %zu: %s", what, bytes, cudaGetErrorString(e));
-    done[key] = bytes;
-    return ASARF_OK;
-}
-
-cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
-
 }  // namespace
 
 int backend_raw_stats(const RawStatsArgs& a, int gx, int gy, void* stream) {
@@ -652,54 +378,12 @@ int backend_stats_fold(const RawStatsArgs& a, int tiles_y, void* stream) {
     return check_launch("stats_fold");
 }
 
-template <int L, int FMT>
-static int launch_rc_ct(const RangeCompressArgs& a, int lines, size_t smem, void* stream) {
-    int rc = ensure_smem(k_range_compress_ct<L, FMT>, smem, "range_compress");
-    if (rc) return rc;
-    k_range_compress_ct<L, FMT><<<lines, CtSchedule<L>::nthr, smem, S(stream)>>>(a);
-    return check_launch("range_compress");
-}
-
-template <int FMT>
-static int launch_rc(const RangeCompressArgs& a, int lines, LaunchShape sh, void* stream) {
-    switch (a.plan.n) {
-        case 768: return launch_rc_ct<768, FMT>(a, lines, sh.smem, stream);
-        case 1024: return launch_rc_ct<1024, FMT>(a, lines, sh.smem, stream);
-        case 1536: return launch_rc_ct<1536, FMT>(a, lines, sh.smem, stream);
-        case 2048: return launch_rc_ct<2048, FMT>(a, lines, sh.smem, stream);
-        case 3072: return launch_rc_ct<3072, FMT>(a, lines, sh.smem, stream);
-        case 4096: return launch_rc_ct<4096, FMT>(a, lines, sh.smem, stream);
-        case 6144: return launch_rc_ct<6144, FMT>(a, lines, sh.smem, stream);
-        case 8192: return launch_rc_ct<8192, FMT>(a, lines, sh.smem, stream);
-        default: break;
-    }
-    int rc = ensure_smem(k_range_compress<FMT>, sh.smem, "range_compress");
-    if (rc) return rc;
-    k_range_compress<FMT><<<lines, sh.threads, sh.smem, S(stream)>>>(a);
-    return check_launch("range_compress");
-}
-
 int backend_range_compress(const RangeCompressArgs& a, int lines, LaunchShape sh, void* stream) {
-    if (a.format == kRawAsarFbaq4) return launch_rc<kRawAsarFbaq4>(a, lines, sh, stream);
-    return launch_rc<kRawErsBytes>(a, lines, sh, stream);
-}
-
-static CUtensorMap tmap_or_zero(const void* tmap) {
-    CUtensorMap m;
-    if (tmap)
-        std::memcpy(&m, tmap, sizeof(m));
-    else
-        std::memset(&m, 0, sizeof(m));
-    return m;
-}
-
-template <int R0, int R1, int R2, int XT, int NB>
-static int launch_az_strided(const AzStridedArgs& a, const void* tmap, int tiles, LaunchShape sh, void* stream) {
-    int rc = ensure_smem(k_az_strided<R0, R1, R2, XT, NB>, sh.smem, "az_strided");
-    if (rc) return rc;
-    k_az_strided<R0, R1, R2, XT, NB><<<dim3(tiles, (a.n2 + NB - 1) / NB), sh.threads, sh.smem, S(stream)>>>(
-        a, tmap_or_zero(tmap));
-    return check_launch("az_strided");
+#define ASARF_CASE(L) \
+    if (a.plan.n == L) return launch_range_compress<L>(a, lines, sh, stream);
+    ASARF_CT_LENGTHS(ASARF_CASE)
+#undef ASARF_CASE
+    return launch_range_compress<0>(a, lines, sh, stream);
 }
 
 // The compiled schedules (strided_schedule_compiled) when the plan allows them.
@@ -717,15 +401,6 @@ int backend_az_strided(const AzStridedArgs& a, const void* tmap, int tiles, Laun
     return launch_az_strided<0, 0, 0, 32, 1>(a, tmap, tiles, sh, stream);
 }
 
-template <int R0, int R1, int R2>
-static int launch_az_rd(const AzRdArgs& a, const void* tmap, int tiles, int nblocks, LaunchShape sh,
-                        unsigned int* err, void* stream) {
-    int rc = ensure_smem(k_az_rd<R0, R1, R2>, sh.smem, "az_rd");
-    if (rc) return rc;
-    k_az_rd<R0, R1, R2><<<dim3(tiles, nblocks), sh.threads, sh.smem, S(stream)>>>(a, err, tmap_or_zero(tmap));
-    return check_launch("az_rd");
-}
-
 // The compiled schedules (block_schedule_compiled) when the plan allows them.
 int backend_az_rd(const AzRdArgs& a, const void* tmap, int tiles, int nblocks, LaunchShape sh, unsigned int* err,
                   void* stream) {
@@ -736,15 +411,6 @@ int backend_az_rd(const AzRdArgs& a, const void* tmap, int tiles, int nblocks, L
 #undef ASARF_CASE
     }
     return launch_az_rd<0, 0, 0>(a, tmap, tiles, nblocks, sh, err, stream);
-}
-
-int backend_az_rd_split(const AzRdArgs& a, const AzRdSplit& sp, const void* tmap, int tiles, int nblocks,
-                        LaunchShape sh, unsigned int* err, void* stream) {
-    if (!tmap) return set_error(ASARF_ERR_INVALID, "az_rd_split: needs the TMA tile loads");
-    int rc = ensure_smem(k_az_rd_split, sh.smem, "az_rd_split");
-    if (rc) return rc;
-    k_az_rd_split<<<dim3(tiles, nblocks), sh.threads, sh.smem, S(stream)>>>(a, sp, err, tmap_or_zero(tmap));
-    return check_launch("az_rd_split");
 }
 
 int backend_rcmc_table(float* table, void* stream) {
@@ -824,30 +490,12 @@ int backend_accc(const AcccArgs& a, int grid_x, int grid_y, void* stream) {
     return check_launch("accc");
 }
 
-template <int L>
-static int launch_rc_rows_ct(const RcRowsArgs& a, int rows, size_t smem, void* stream) {
-    int rc = ensure_smem(k_rc_rows_ct<L>, smem, "rc_rows");
-    if (rc) return rc;
-    k_rc_rows_ct<L><<<rows, CtSchedule<L>::nthr, smem, S(stream)>>>(a);
-    return check_launch("rc_rows");
-}
-
 int backend_rc_rows(const RcRowsArgs& a, int rows, LaunchShape sh, void* stream) {
-    switch (a.ctw ? a.plan.n : 0) {
-        case 768: return launch_rc_rows_ct<768>(a, rows, sh.smem, stream);
-        case 1024: return launch_rc_rows_ct<1024>(a, rows, sh.smem, stream);
-        case 1536: return launch_rc_rows_ct<1536>(a, rows, sh.smem, stream);
-        case 2048: return launch_rc_rows_ct<2048>(a, rows, sh.smem, stream);
-        case 3072: return launch_rc_rows_ct<3072>(a, rows, sh.smem, stream);
-        case 4096: return launch_rc_rows_ct<4096>(a, rows, sh.smem, stream);
-        case 6144: return launch_rc_rows_ct<6144>(a, rows, sh.smem, stream);
-        case 8192: return launch_rc_rows_ct<8192>(a, rows, sh.smem, stream);
-        default: break;
-    }
-    int rc = ensure_smem(k_rc_rows, sh.smem, "rc_rows");
-    if (rc) return rc;
-    k_rc_rows<<<rows, sh.threads, sh.smem, S(stream)>>>(a);
-    return check_launch("rc_rows");
+#define ASARF_CASE(L) \
+    if (a.ctw && a.plan.n == L) return launch_rc_rows<L>(a, rows, sh, stream);
+    ASARF_CT_LENGTHS(ASARF_CASE)
+#undef ASARF_CASE
+    return launch_rc_rows<0>(a, rows, sh, stream);
 }
 
 int backend_matched_filter(const MatchedFilterArgs& a, void* stream) {

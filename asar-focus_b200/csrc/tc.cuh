@@ -64,9 +64,6 @@ __device__ __forceinline__ void tc_fence_before_sync() {
 }
 __device__ __forceinline__ void tc_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Generic-proxy shared-memory writes become visible to the tensor core (async proxy).
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
 // D[taddr] (+)= A * B with A in TMEM (lanes = rows, two 16-bit K elements per 32-bit column,
 // the lower K index in the low half) and B in shared memory, one elected thread.
 __device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,

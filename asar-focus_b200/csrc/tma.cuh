@@ -75,5 +75,7 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                  : "memory");
 }
 
+// Generic-proxy shared-memory accesses are ordered with the asynchronous ones after it (bulk copies, tensor cores).
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 }  // namespace asarf
