@@ -400,6 +400,13 @@ extern "C" int asarf_emu_context_cache_probe(const unsigned long long* ids, int 
     return resolutions;
 }
 
+// Test hook of the host emulation only: radices of a strided or contiguous azimuth length; returns their number.
+extern "C" int asarf_emu_radices(int n, int strided, int out[16]) {
+    const std::vector<int> r = strided ? asarf::strided_radices(n) : asarf::block_radices(n);
+    for (size_t i = 0; i < r.size() && i < 16; ++i) out[i] = r[i];
+    return static_cast<int>(r.size());
+}
+
 // Test hooks of the host emulation only: the next finalisation fails; the stream is under capture; a
 // plan's statistics accumulators are all zero.
 extern "C" void asarf_emu_fail_finalize() { asarf::g_fail_finalize = true; }

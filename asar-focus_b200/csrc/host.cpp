@@ -438,7 +438,9 @@ static std::vector<int> few_radices(int n, int most) {
 }
 
 std::vector<int> strided_radices(int n) {
-    if (n == 180) return {9, 4, 5};  // the compiled schedule
+#define ASARF_CASE(R0, R1, R2) \
+    if (n == R0 * R1 * R2) return {R0, R1, R2};
+    ASARF_STRIDED_SCHEDULES(ASARF_CASE)
     std::vector<int> best = few_radices(n, 9);
     if (!best.empty()) return best;
     // longer: the default factors with each pair of 3s merged into a 9 (first, so that the short
@@ -458,7 +460,8 @@ std::vector<int> strided_radices(int n) {
 }
 
 std::vector<int> block_radices(int n) {
-    if (n == 168) return {8, 7, 3};
+    ASARF_BLOCK_SCHEDULES(ASARF_CASE)
+#undef ASARF_CASE
     const std::vector<int> best = few_radices(n, 8);
     return best.empty() ? factorize(n) : best;
 }
