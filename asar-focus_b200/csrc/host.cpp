@@ -303,15 +303,18 @@ static float bf16_to_float(uint16_t h) {
 // as the B operand (rows = output (slot, re / im), K = input (mm, re / im)) in the canonical
 // no-swizzle K-major layout, bf16 hi image then lo image; and the twiddles W_n^(r k1(s)),
 // [r][s].  Output slot s holds frequency k1(s) = drev[R s] (the FP32 transform's order).
-// FP64 throughout, rounded once.
-void split_dft_tables(int n, int R, const std::vector<int>& drev, std::vector<unsigned char>& img,
+// FP64 throughout, rounded once.  Returns the matrix's mean gain error: bf16 hi + lo parts hold its entries to
+// 2^-18 or so, which over the few of a small m averages to some 1e-7 (m = 7: 2.7e-7).
+double split_dft_tables(int n, int R, const std::vector<int>& drev, std::vector<unsigned char>& img,
                       std::vector<float2>& tw) {
     const int m = n / R;
     img.assign(2 * static_cast<size_t>(kSplitMatrixBytes), 0);
+    double gain = 0.0;
     auto put = [&](int row, int k, double v) {
         const float f = static_cast<float>(v);
         const uint16_t hi = bf16_rn(f);
         const uint16_t lo = bf16_rn(f - bf16_to_float(hi));
+        gain += (static_cast<double>(bf16_to_float(hi)) + bf16_to_float(lo) - v) * v / (2.0 * m * m);  // each entry twice
         const uint32_t off = umma_offset(row, k, kSplitK);
         std::memcpy(&img[off], &hi, 2);
         std::memcpy(&img[kSplitMatrixBytes + off], &lo, 2);
@@ -334,6 +337,7 @@ void split_dft_tables(int n, int R, const std::vector<int>& drev, std::vector<un
             const double a = -2.0 * kPi * static_cast<double>((static_cast<long long>(r) * k1) % n) / n;
             tw[static_cast<size_t>(r) * m + sl] = make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a)));
         }
+    return gain;
 }
 
 MatchedFilterArgs matched_filter_args(const float2* d_chirp, int nc, const HostFft& fft, float2* d_mf) {
@@ -1067,7 +1071,7 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
     p->a_inv.out = p->bufB;
     p->a_inv.valid_rows = p->az_pad;
     p->a_inv.state = p->state;
-    p->a_inv.scale = azimuth_scale(p->az_pad, p->f1, p->f2);
+    p->a_inv.scale = azimuth_scale(p->az_pad, 2.0 * (transform_gain(p->f1, false) + transform_gain(p->f2, false)));
     p->a_inv.inverse = 1;
     p->tiles1 = (p->nk + p->xt1 - 1) / p->xt1;
     p->a_fwd.nb = p->a_inv.nb = p->xt1 == 32 ? az_strided_tiles_per_block(p->n1, p->n2, p->tiles1) : 1;
@@ -1170,7 +1174,10 @@ int asarf_plan_create(const asarf_scene* scene, const asarf_options* opt_in, asa
         if (p->use_tma && radix_ok && m >= 2 && 2 * m <= kSplitK && smem_split <= smem_optin_limit()) {
             std::vector<unsigned char> img;
             std::vector<float2> tws;
-            split_dft_tables(p->n2, R, p->f2.drev, img, tws);
+            // the matrix's own gain, the FP32 pass's, and that of the FP32 accumulation on the tensor cores:
+            // -0.6e-7 for each 16 of K, measured over 28 lengths of m = 2 .. 28 (-0.5 to 1.0e-7 about it)
+            const double gain = split_dft_tables(p->n2, R, p->f2.drev, img, tws) + dft_gain(R) - 0.6e-7 * ((2 * m + 15) / 16);
+            p->a_inv.scale = azimuth_scale(p->az_pad, 2.0 * transform_gain(p->f1, false) + transform_gain(p->f2, false) + gain);
             unsigned char* bmat = p->alloc<unsigned char>(img.size());
             float2* tw_dev = p->alloc<float2>(tws.size());
             if (!bmat || !tw_dev) {

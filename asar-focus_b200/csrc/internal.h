@@ -41,11 +41,9 @@ int choose_az_n2(int N, int nk, int hl, int hr, bool absolute_phase);
 // or by recurrence) and radix constants are rounded, which scales all outputs alike by some 1e-8 to
 // 1e-7; its inverse has the same.
 double transform_gain(const HostFft& h, bool table_powers);
-// 1 / N of the azimuth transforms with that gain taken back: over the two forward and two inverse
-// passes it is the one error of theirs that all samples share.
-inline float azimuth_scale(int N, const HostFft& f1, const HostFft& f2) {
-    return static_cast<float>(1.0 / (N * (1.0 + 2.0 * (transform_gain(f1, false) + transform_gain(f2, false)))));
-}
+// 1 / N of the azimuth transforms with `gain`, the sum of those of the two forward and two inverse passes, taken
+// back: it is the one error of theirs that all samples share.
+inline float azimuth_scale(int N, double gain) { return static_cast<float>(1.0 / (N * (1.0 + gain))); }
 int largest_divisor_le(int n, int cap);
 // Rows of a TMA box of the range-Doppler tile (n2 rows of wt complex values): all n2 up to 256, else their
 // largest divisor whose boxes each start on a 128-byte boundary of shared memory, as a tensor copy must;

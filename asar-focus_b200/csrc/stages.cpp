@@ -392,7 +392,7 @@ int asarf_range_doppler(const asarf_rda_params* prm, void* d_src, void* d_out, i
     inv.in = out;
     inv.out = out;
     inv.valid_rows = N;
-    inv.scale = azimuth_scale(N, f1, f2);
+    inv.scale = azimuth_scale(N, 2.0 * (transform_gain(f1, false) + transform_gain(f2, false)));
     inv.inverse = 1;
     AzRdArgs d{};
     d.in = src;
