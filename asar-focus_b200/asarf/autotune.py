@@ -10,8 +10,8 @@ shape costs a few dozen short runs.
 
 The cache is a JSON file (default ``~/.cache/asarf/autotune.json``, or ``cache=`` / the
 ASARF_AUTOTUNE_CACHE environment variable) mapping a shape key -- range samples, azimuth
-lines, raw format, bit depth, precision form and GPU name -- to the chosen options and the
-measured milliseconds of the default and the chosen set.
+lines, raw format, bit depth, precision form, GPU name and kernel revision -- to the chosen options
+and the measured milliseconds of the default and the chosen set.
 """
 from __future__ import annotations
 
@@ -21,6 +21,10 @@ import os
 from pathlib import Path
 
 from . import FocusPlan, _lib
+
+# Revision of the kernels and the planner's cost model, part of the cache key: shapes timed on other kernels are
+# not served.  Raise it whenever a kernel's shapes or their relative times change.
+REVISION = 2
 
 # range FFT lengths with compile-time-scheduled kernels (k_range_compress_ct)
 CT_LENGTHS = (768, 1024, 1536, 2048, 3072, 4096, 6144, 8192)
@@ -37,7 +41,7 @@ def shape_key(scene, precision: int = 0) -> str:
     import torch
     dev = torch.cuda.get_device_name() if torch.cuda.is_available() else "host"
     return (f"{scene.range_size}x{scene.azimuth_size}:{scene.raw_format}:{scene.bits}bit:"
-            f"{'split' if precision else 'fp32'}:{dev}")
+            f"{'split' if precision else 'fp32'}:{dev}:r{REVISION}")
 
 
 def _time_options(scene, raw_d, out_d, lib, opts: dict, runs: int) -> float | None:
@@ -68,10 +72,10 @@ def _time_options(scene, raw_d, out_d, lib, opts: dict, runs: int) -> float | No
         plan.close()
 
 
-def _n2_candidates(az_pad: int, count: int = 4) -> list[int]:
-    divs = [d for d in range(16, 257) if az_pad % d == 0]
-    root = math.sqrt(az_pad)
-    divs.sort(key=lambda d: abs(math.log(d / root)))
+def _n2_candidates(az_pad: int, planned: int, count: int = 4) -> list[int]:
+    """The admissible azimuth splits nearest to the planner's own (itself not among them)."""
+    divs = [d for d in range(16, 257) if az_pad % d == 0 and d != planned]
+    divs.sort(key=lambda d: abs(math.log(d / planned)))
     return sorted(divs[:count])
 
 
@@ -113,7 +117,7 @@ def tune(scene, raw_d, lib=None, precision: int = 0, cache=None, runs: int = 4, 
                 best, best_ms = trial, ms
 
     if not quick:
-        sweep("az_n2", [d for d in _n2_candidates(dims["az_pad"]) if d != dims["n2"]])
+        sweep("az_n2", _n2_candidates(dims["az_pad"], dims["n2"]))
     sweep("az_tile_width", [w for w in (64, 62, 60, 58, 56, 52, 48) if w != dims["az_tile_width"]])
     sweep("strided_tile_width", [w for w in (16, 32) if w != dims["strided_tile_width"]])
     if not quick:
