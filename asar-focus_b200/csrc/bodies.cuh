@@ -184,6 +184,34 @@ struct StatsRowsInPlace {
     }
 };
 
+// What a ring slot takes of line y: the bytes [b0, b1) of the samples under columns [x_lo, x_hi) (none: b0 =
+// b1), b0 at slot offset `lead`.  The 16-byte units [c0, c1) (none: c1 <= c0) move by a bulk copy,
+// from the boundary before the first byte to the one after the last; at the two ends of the raw buffer, where
+// that would leave it, a unit less, and the bytes it would have brought by plain loads.
+struct StatsSlotCopy {
+    const uint8_t *b0, *b1, *c0, *c1;
+    int lead;
+    int sample0;  // slot offset of the line's sample 0 (may lie before the slot)
+    ASARF_HD ASARF_INLINE StatsSlotCopy(const RawStatsArgs& a, int y, int off, int x_lo, int x_hi) {
+        const int i0 = x_lo > off ? x_lo - off : 0, i1 = x_hi - off < a.spl ? x_hi - off : a.spl;
+        const uint8_t* row = a.raw + static_cast<long long>(y) * a.line_bytes;
+        b0 = row + 2ll * i0;
+        b1 = i1 > i0 ? row + 2ll * i1 : b0;
+        lead = static_cast<int>(reinterpret_cast<uintptr_t>(b0) & 15);
+        sample0 = lead - 2 * i0;
+        c0 = b0 - lead;
+        c1 = b1 + (static_cast<int>(-reinterpret_cast<uintptr_t>(b1)) & 15);
+        if (c0 < a.raw) c0 += 16;
+        if (c1 > a.raw + static_cast<long long>(a.na - 1) * a.line_bytes + 2ll * a.spl) c1 -= 16;
+        if (b0 == b1) c1 = c0;
+    }
+    // the odd bytes, to slot offsets
+    ASARF_HD ASARF_INLINE void plain(unsigned char* slot) const {
+        for (const uint8_t* p = b0; p < c0 && p < b1; ++p) slot[lead + (p - b0)] = *p;
+        for (const uint8_t* p = c1 > b0 ? c1 : b0; p < b1; ++p) slot[lead + (p - b0)] = *p;
+    }
+};
+
 // Host side: work units and grid width of the statistics kernel for this raw buffer.
 inline int raw_stats_grid_x(RawStatsArgs& a, const void* raw) {
     a.gpb = (a.dc_step + 3) / 4 + 1;  // aligned groups a block's columns touch

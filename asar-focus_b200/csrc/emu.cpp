@@ -30,16 +30,79 @@ bool g_fail_finalize = false;
 bool g_capturing = false;
 }  // namespace
 
-int backend_raw_stats(const RawStatsArgs& a, int gx, int gy, void*) {
-    if (g_capturing) return ASARF_OK;
+// The lines of a statistics block in slots as the device's ring holds them (all batches at once), filled by the
+// same copies; a copy that leaves the raw buffer or its slot, or is misaligned, is an error.
+struct StatsRowsSlots {
+    static constexpr bool kCollective = true;
+    static constexpr int kMargin = 0;
+    const StatsBatches& bt;
+    std::vector<float4> ring;  // 16-byte aligned
+    std::vector<int> sample0;
+    bool ok = true;
+    unsigned char* slot(int k, int u) {
+        return reinterpret_cast<unsigned char*>(ring.data()) + (static_cast<size_t>(k) * kStatsBatch + u) * kStatsSlotBytes;
+    }
+    StatsRowsSlots(const RawStatsArgs& a, const RawStatsSmem& sm, const StatsBatches& b)
+        : bt(b), ring(static_cast<size_t>(b.count) * kStatsBatch * kStatsSlotBytes / sizeof(float4)),
+          sample0(static_cast<size_t>(b.count) * kStatsBatch) {
+        std::memset(ring.data(), 0xEE, ring.size() * sizeof(float4));  // nothing may count on what a copy leaves out
+        const uint8_t* end = a.raw + static_cast<long long>(a.na - 1) * a.line_bytes + 2ll * a.spl;
+        for (int k = 0; k < b.count; ++k) {
+            int yg, ye;
+            b.lines(k, &yg, &ye);
+            for (int y = yg; y < ye; ++y) {
+                const StatsSlotCopy c(a, y, sm.off[y - b.ys], sm.x_lo, sm.x_hi);
+                unsigned char* base = slot(k, y - yg);
+                ok = ok && c.lead + (c.b1 - c.b0) <= kStatsSlotBytes;
+                if (ok) c.plain(base);
+                if (c.c0 < c.c1) {
+                    const long long to = c.lead + (c.c0 - c.b0), n = c.c1 - c.c0;
+                    ok = ok && c.c0 >= a.raw && c.c1 <= end && to >= 0 && to + n <= kStatsSlotBytes && n % 16 == 0 &&
+                         (reinterpret_cast<uintptr_t>(c.c0) & 15) == 0 && (reinterpret_cast<uintptr_t>(base + to) & 15) == 0;
+                    if (ok) std::memcpy(base + to, c.c0, static_cast<size_t>(n));
+                }
+                sample0[static_cast<size_t>(k) * kStatsBatch + (y - yg)] = c.sample0;
+            }
+        }
+    }
+    void begin(int) const {}
+    void end(int) const {}
+    const uint8_t* row(int k, int u, int) const {
+        return reinterpret_cast<const unsigned char*>(ring.data()) +
+               (static_cast<size_t>(k) * kStatsBatch + u) * kStatsSlotBytes + sample0[static_cast<size_t>(k) * kStatsBatch + u];
+    }
+};
+
+// staged: unaligned lines through the slots (the planned path); in place otherwise.
+static int emu_raw_stats(const RawStatsArgs& a, int gx, int gy, bool staged) {
     RawStatsSmem sm;
+    const FastDiv dgpb = make_fastdiv(static_cast<unsigned int>(a.gpb));
     for (int by = 0; by < gy; ++by)
         for (int bx = 0; bx < gx; ++bx) {
             const StatsBatches bt = raw_stats_begin(a, by, 0, 1, &sm);
-            if (a.aligned) raw_stats_body<true>(a, StatsRowsInPlace<true>{a}, bt, bx, 0, 1, &sm);
-            else raw_stats_body<false>(a, StatsRowsInPlace<false>{a}, bt, bx, 0, 1, &sm);
+            if (a.aligned) {
+                raw_stats_body<true>(a, StatsRowsInPlace<true>{a}, bt, bx, 0, 1, &sm);
+            } else if (!staged) {
+                raw_stats_body<false>(a, StatsRowsInPlace<false>{a}, bt, bx, 0, 1, &sm);
+            } else {
+                sm.x_lo = 0x3fffffff;
+                sm.x_hi = 0;
+                for (int c = 0; c < kStatsCols; ++c) {
+                    const StatsUnit un(a, dgpb, bx * kStatsCols + c);
+                    if (!un.colmask) continue;
+                    sm.x_lo = un.x0 < sm.x_lo ? un.x0 : sm.x_lo;
+                    sm.x_hi = un.x0 + 4 > sm.x_hi ? un.x0 + 4 : sm.x_hi;
+                }
+                const StatsRowsSlots rows(a, sm, bt);
+                if (!rows.ok) return set_error(ASARF_ERR_INVALID, "statistics slots: a copy out of bounds");
+                raw_stats_body<false>(a, rows, bt, bx, 0, 1, &sm);
+            }
         }
     return ASARF_OK;
+}
+
+int backend_raw_stats(const RawStatsArgs& a, int gx, int gy, void*) {
+    return g_capturing ? ASARF_OK : emu_raw_stats(a, gx, gy, true);
 }
 
 int backend_raw_stats_fbaq(const RawStatsArgs& a, int gx, int gy, void*) {
@@ -347,8 +410,7 @@ extern "C" int asarf_raw_statistics_noalloc(const uint8_t* d_raw, int32_t raw_li
     st.nblk = nblk;
     st.lines_per_cta = kStatsLinesPerBlock;
     st.acc = &g_emu_scratch.acc;
-    backend_raw_stats(st, raw_stats_grid_x(st, d_raw), (azimuth_size + st.lines_per_cta - 1) / st.lines_per_cta,
-                      nullptr);
+    emu_raw_stats(st, raw_stats_grid_x(st, d_raw), (azimuth_size + st.lines_per_cta - 1) / st.lines_per_cta, false);
     FinalizeArgs fin{};
     fin.acc = &g_emu_scratch.acc;
     fin.state = &g_emu_scratch.state;

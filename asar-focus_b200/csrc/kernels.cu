@@ -44,30 +44,15 @@ struct StatsRowsStaged {
         const uint8_t* src = nullptr;
         unsigned char* dst = nullptr;
         if (lane < kStatsBatch && y < ye) {
-            const int off = sm->off[y - bt.ys];
-            const int i0 = max(sm->x_lo - off, 0), i1 = min(sm->x_hi - off, a.spl);
-            if (i0 < i1) {
-                const uint8_t* row = a.raw + static_cast<long long>(y) * a.line_bytes;
-                const uint8_t *b0 = row + 2ll * i0, *b1 = row + 2ll * i1;
-                const int lead = static_cast<int>(reinterpret_cast<uintptr_t>(b0) & 15);
-                const int tail = static_cast<int>(-reinterpret_cast<uintptr_t>(b1) & 15);
-                const uint8_t *c0 = b0 - lead, *c1 = b1 + tail;
-                unsigned char* base = ring + slot * kStatsSlotBytes;
-                if (c0 < a.raw) {
-                    c0 += 16;
-                    for (const uint8_t* p = b0; p < c0 && p < b1; ++p) base[lead + (p - b0)] = *p;
-                }
-                if (c1 > a.raw + static_cast<long long>(a.na - 1) * a.line_bytes + 2ll * a.spl) {
-                    c1 -= 16;
-                    for (const uint8_t* p = c1 > b0 ? c1 : b0; p < b1; ++p) base[lead + (p - b0)] = *p;
-                }
-                if (c0 < c1) {
-                    bytes = static_cast<uint32_t>(c1 - c0);
-                    src = c0;
-                    dst = base + lead + (c0 - b0);
-                }
-                sm->sample0[slot] = slot * kStatsSlotBytes + lead - 2 * i0;
+            const StatsSlotCopy c(a, y, sm->off[y - bt.ys], sm->x_lo, sm->x_hi);
+            unsigned char* base = ring + slot * kStatsSlotBytes;
+            c.plain(base);
+            if (c.c0 < c.c1) {
+                bytes = static_cast<uint32_t>(c.c1 - c.c0);
+                src = c.c0;
+                dst = base + c.lead + (c.c0 - c.b0);
             }
+            sm->sample0[slot] = slot * kStatsSlotBytes + c.sample0;
         }
         const uint32_t total = __reduce_add_sync(0xffffffffu, bytes);
         if (lane == 0) mbar_expect_tx(&sm->full[stage], total);
