@@ -115,8 +115,8 @@ ASARF_HD inline bool polyfit_qr(const double* x, const double* y, int m, int deg
 constexpr int kStatsCols = 256;
 constexpr int kStatsBatch = 8;
 constexpr int kStatsMaxLines = 256;
-// lines per block of the statistics kernel (measured on the 28000- and 30000-line scenes:
-// 64 -> 0.203, 128 -> 0.170, 192 -> 0.155, 256 -> 0.171 ms)
+// lines per block of the statistics kernel, with the whole-wave rule below (28000, 30000, 60000 lines of 5616
+// samples: 128 -> 114, 135, 250 us; 160 -> 114, 116, 231; 192 -> 114, 115, 213; 256 -> 127, 125, 220)
 constexpr int kStatsLinesPerBlock = 192;
 constexpr int kStatsBlocksPerSm = 3;  // resident blocks of k_raw_stats (its launch bounds)
 
@@ -1242,7 +1242,7 @@ constexpr int kRcmcNodes = 4096;
 constexpr int kRcmcRowFloats = 32;                   // per node: (w, w') of taps 1 .. 14, padded to 128 bytes
 constexpr int kRcmcBufFloats = 2 * (kRcmcTaps - 2);  // a warp's copy of one node
 constexpr float kRcmcMaxStep = 5e-4f;
-constexpr int kRowSlow = -1, kRowSkip = -2;          // other codes: rcmc_row_code
+constexpr int kRowSlow = -1, kRowSkip = -2;          // other codes: rcmc_row
 
 // Weights of tap i = 1 .. 14 at fraction dl = n / kRcmcNodes - 1/2 and their derivatives, as the
 // quotients v_i / sum v of v_i = dl (-1)^i W_i / (dl + 8 - i) (v_8 = W_8: finite at dl = 0).
@@ -1499,7 +1499,8 @@ struct RowRec {
 
 // Record of the row at bin frequency bf.  Code of a uniform row: table node (from bit 12), wrap + 1
 // (bits 8-9: the filter's frequency is bf - dc_off - wrap PRF), walk (bits 0-7).  All tests are
-// written so that a NaN takes the slow path.
+// written so that a NaN extreme takes the slow path.  (The device's extremes leave out the columns whose own
+// constants are NaN: those columns come out NaN whichever path their rows take.)
 ASARF_HD ASARF_INLINE RowRec rcmc_row(const AzRdArgs& a, const RowSpan& sp, float bf) {
     RowRec r{bf, 0.0f, kRowSlow};
     const float half = a.half_prf;
@@ -1551,7 +1552,7 @@ ASARF_HD ASARF_INLINE int az_rd_used_columns(const AzRdArgs& a, const RowSpan& s
 
 // Shared-memory tables after the tile: the columns' constants (xt) and their extremes (two warps'),
 // and in the same memory, once every lane holds its columns' constants, the 16 warps' weight buffers;
-// absolute-phase factors (xt, only when asked for); the rows' records (n2).
+// the columns' centroids (xt); absolute-phase factors (xt, only when asked for); the rows' records (n2).
 ASARF_HD ASARF_INLINE int az_rd_cols_bytes(int xt) {
     const int cols = static_cast<int>(sizeof(ColUse)) * xt + 2 * static_cast<int>(sizeof(RowSpan)) + 16;
     const int bufs = 16 * kRcmcBufFloats * static_cast<int>(sizeof(float));
@@ -1708,12 +1709,13 @@ inline int rcmc_right_halo(double max_walk) { return kRcmcTaps / 2 - 1 + static_
 // room for two resident blocks per SM (2 x 512 threads at 64 registers fill the register file;
 // 228 KB of shared memory per SM, 1 KB reserved per block).  With one block per SM the
 // block-wide barriers of the FFT stages leave the SM idle (measured 2.63 -> 1.92 ms at n2 = 168).
-// Where the halo leaves no such width of at least 16, 16; less than that only to fit a block at all.
+// Where the halo leaves no such width of at least 16, 16; 14 where only that fits a block at all (the row
+// records and column tables take up to 3 KB more than the 16 columns they come with leave).
 constexpr size_t kAzRdTwoBlockSmem = 228 * 1024 / 2 - 1024 - 128;
 inline int az_rd_tile_width(int n2, int hl, int hr, bool absolute_phase, size_t limit) {
     int xt = 64;
     while (xt > 16 && az_rd_smem(n2, xt + hl + hr, xt, absolute_phase) > kAzRdTwoBlockSmem) xt -= 2;
-    while (xt > 8 && az_rd_smem(n2, xt + hl + hr, xt, absolute_phase) > limit) xt -= 2;
+    while (xt > 14 && az_rd_smem(n2, xt + hl + hr, xt, absolute_phase) > limit) xt -= 2;
     return xt;
 }
 
@@ -1857,7 +1859,7 @@ ASARF_HD ASARF_INLINE void az_rd_body(const AzRdArgs& a, int tile, int k1, int t
 }
 
 // ----------------------------------------------------------------------------- level-0 packets
-// Word `w` (0 .. 3) of the 16 bytes that start `sh` bytes into the 32 bytes (lo, hi).
+// The 16 bytes that start `sh` bytes (at most 15) into the 32 bytes (lo, hi).
 ASARF_HD ASARF_INLINE uint4 shift_bytes(const uint4& lo, const uint4& hi, unsigned int sh) {
     const unsigned int bits = 8u * (sh & 3u);
     const bool two = (sh & 8u) != 0, one = (sh & 4u) != 0;
@@ -1938,7 +1940,7 @@ ASARF_HD ASARF_INLINE void ers_unpack_line(const ErsUnpackArgs& a, int y, int ti
 // little-endian host), the blocks, zeros up to record_bytes.  SWST and PRI codes are the source
 // packet's.  The packet's data field header length (29) and mode ID (0x54) are checked as the
 // reference checks them (:470-484); a block length beyond the record sets kErrL0Length and the
-// record keeps only what fits.  Block y: the record's 16-byte aligned interior moves by whole
+// record keeps only what fits.  A warp takes the record: its 16-byte aligned interior moves by whole
 // units, what lies before and after it (records have any size and any alignment) by bytes.
 ASARF_HD ASARF_INLINE void asar_unpack_line(const AsarUnpackArgs& a, int y, int tid, int nthr) {
     const uint8_t* pk = a.mdsr + ASARF_LDG(a.src + y);

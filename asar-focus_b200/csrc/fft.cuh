@@ -378,39 +378,6 @@ ASARF_HD ASARF_INLINE void fft_stage(float2* s, int n, int S, const FastDiv& sdi
     }
 }
 
-// Inverse transform in decimation-in-frequency form: small inverse DFT, then multiply output
-// q by conj(W_M^{j q}).  Natural-order input, digit-reversed output (same map as the forward).
-template <int R>
-ASARF_HD ASARF_INLINE void fft_stage_dif_inv(float2* s, int n, int S, const FastDiv& sdiv, int ncol, const FastDiv& cdiv,
-                                             int ldc, const float2* __restrict__ tw, int tid, int nthr) {
-    const int M = S * R;
-    const int items = (n / R) * ncol;
-    const int tw_step = n / M;
-    for (int t = tid; t < items; t += nthr) {
-        const int bj = ncol == 1 ? t : static_cast<int>(fdiv_u(t, cdiv));
-        const int c = t - bj * ncol;
-        const int b = static_cast<int>(fdiv_u(bj, sdiv));
-        const int j = bj - b * S;
-        float2* p = s + (b * M + j) * ldc + c;
-        const int st = S * ldc;
-        float2 v[R];
-#pragma unroll
-        for (int m = 0; m < R; ++m) v[m] = p[m * st];
-        dft<R, true>(v);
-        if (j != 0) {
-            const float2 w1 = ASARF_LDG(tw + j * tw_step);
-            float2 w = w1;
-#pragma unroll
-            for (int q = 1; q < R; ++q) {
-                v[q] = cmulc(v[q], w);
-                w = cmul(w, w1);
-            }
-        }
-#pragma unroll
-        for (int m = 0; m < R; ++m) p[m * st] = v[m];
-    }
-}
-
 // ----------------------------------------------------------------------------- column pairs
 // The same stages over PAIRS of adjacent columns: one 16-byte shared-memory access moves
 // both columns' samples and one twiddle set serves both butterflies.  Needs ldc even, the
@@ -588,14 +555,13 @@ ASARF_HD ASARF_INLINE void fft_stage_pair_w_dispatch(int R, float2* s, int n, in
 #undef ASARF_PAIR
 }
 
-// Column-pair stages take the prime-power radices: a larger composite radix holds twice its
+// Column-pair stages take radices up to 9: a larger composite radix holds twice its
 // length in registers per column pair, which lifts the azimuth kernels from 64 to 128
 // registers per thread and halves their resident CTAs (measured slower despite fewer passes).
-// NINE adds radix 9 (two radix-3 DFTs in registers, 36 values per column pair: 71 registers
-// in the strided kernel, whose occupancy shared memory limits anyway) for plans that merge
-// factors 3 * 3; it is compiled only where such plans run, since every extra case costs the
-// other kernels registers.  PTW selects the packed twiddle products: the strided kernel uses them,
-// the range-Doppler block for radix <= 5 schedules only (az_rd_packed_twiddles).
+// Radix 9 (two radix-3 DFTs in registers, 36 values per column pair: 71 registers) only in the strided
+// kernel, whose occupancy shared memory limits anyway; the range-Doppler block's stages (64
+// registers) stop at 8.  The strided kernel takes the packed twiddle products (PTW), the range-Doppler
+// block for radix <= 5 schedules only (az_rd_packed_twiddles).
 template <bool INV, bool TW_FIRST, int NPAIR, int LDC, int PRE>
 ASARF_HD ASARF_INLINE void fft_stage_pair_dispatch(int R, float2* s, int n, int S, const FastDiv& sdiv,
                                                    const float2* __restrict__ tw, int tid, int nthr,
@@ -745,23 +711,6 @@ ASARF_HD ASARF_INLINE void fft_inverse(const FftPlan& p, float2* s, int ncol, in
     const FastDiv cdiv = make_fastdiv(static_cast<unsigned int>(ncol));
     for (int i = p.nst - 1; i >= 0; --i) {
         fft_stage_dispatch<true>(p.radix[i], s, p.n, p.span[i], p.sdiv[i], ncol, cdiv, ldc, p.tw, tid, nthr);
-        ASARF_SYNC();
-    }
-}
-
-// Inverse transform, natural-order input, digit-reversed output, unscaled.
-ASARF_HD ASARF_INLINE void fft_inverse_dif(const FftPlan& p, float2* s, int ncol, int ldc, int tid, int nthr) {
-    const FastDiv cdiv = make_fastdiv(static_cast<unsigned int>(ncol));
-    for (int i = 0; i < p.nst; ++i) {
-        const FastDiv& sd = p.sdiv[i];
-        switch (p.radix[i]) {
-            case 2: fft_stage_dif_inv<2>(s, p.n, p.span[i], sd, ncol, cdiv, ldc, p.tw, tid, nthr); break;
-            case 3: fft_stage_dif_inv<3>(s, p.n, p.span[i], sd, ncol, cdiv, ldc, p.tw, tid, nthr); break;
-            case 4: fft_stage_dif_inv<4>(s, p.n, p.span[i], sd, ncol, cdiv, ldc, p.tw, tid, nthr); break;
-            case 5: fft_stage_dif_inv<5>(s, p.n, p.span[i], sd, ncol, cdiv, ldc, p.tw, tid, nthr); break;
-            case 7: fft_stage_dif_inv<7>(s, p.n, p.span[i], sd, ncol, cdiv, ldc, p.tw, tid, nthr); break;
-            default: fft_stage_dif_inv<8>(s, p.n, p.span[i], sd, ncol, cdiv, ldc, p.tw, tid, nthr); break;
-        }
         ASARF_SYNC();
     }
 }

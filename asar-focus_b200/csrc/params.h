@@ -94,7 +94,7 @@ struct RawStatsArgs {
     int dc_step, nblk;
     int lines_per_cta;    // at most kStatsMaxLines
     int aligned;          // raw base and line stride 8-byte aligned
-    int gpb;              // 4-column groups per Doppler block: ceil(dc_step / 4)
+    int gpb;              // 4-column groups a Doppler block may touch: ceil(dc_step / 4) + 1
     StatAccum* acc;
     // ASAR FBAQ4 records (k_raw_stats_fbaq): FP64 partial sums of each 32-column tile
     const double* lut_i;  // [256 block ids][16 raw codes], the float tables' values
@@ -163,7 +163,7 @@ struct AzStridedArgs {
     int nb;               // adjacent b (tiles side by side) per block: 1, 2, 4 or 8
     int valid_rows;       // forward: rows at or beyond this are zero
     const FocusState* state;  // inverse: rows outside the results window are not stored
-    float scale;          // inverse: 1 / N as the reference multiplies
+    float scale;          // inverse: 1 / N less the transforms' gain (azimuth_scale)
     int inverse;
     int use_tma;          // tile loaded by TMA (device only)
     int n1_box;           // rows per TMA box (n1 split into n1 / n1_box boxes of <= 256 rows)
