@@ -1233,9 +1233,10 @@ ASARF_HD ASARF_INLINE float2 az_abs_phase(const AzRdArgs& a, const ColParams& cp
 // the sinc's centre), about 1e-8 over a scene, below the 1e-6 the reference's fraction is rounded
 // to.  Every branch-deciding quantity keeps the reference's float32 value: a row is taken as
 // uniform only when the extremes over its columns prove that each of them decides alike, and any
-// other row goes sample by sample (rcmc_mf_sample).  The block is bound by instruction issue and
+// other row goes sample by sample (rcmc_mf_samples).  The block is bound by instruction issue and
 // shared-memory wavefronts: on the ERS 5616 x 8990 cut 360 -> 296 million warp instructions, 28000
-// lines 1462 -> 1320 us, ASAR IM 30000 lines 1606 -> 1450 us.  (With one column per lane and the
+// lines 1462 -> 1320 us, ASAR IM 30000 lines 1606 -> 1450 us (and 272 million, 1241 and 1415 us since the slow
+// rows hold their constants).  (With one column per lane and the
 // table's weights summed as sum w d + (dl - node) sum w' d, 345 million instructions and 15 % more
 // wavefronts, it took 1537 us; weights read straight from the table 1549 us.)
 constexpr int kRcmcNodes = 4096;
