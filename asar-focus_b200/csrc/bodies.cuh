@@ -2434,15 +2434,13 @@ ASARF_HD ASARF_INLINE void zero_nan_item(float2* img, long long i) {
 
 // Moment partials for RawDataCorrection / CalcMean / CalcStdDev
 // (sar/iq_correction.cu:40-138, cuda_util/device_padded_image.cu:156-257): block `blk` sums
-// rows [blk*rpb, ...) in double, NaN samples skipped; deterministic in-block tree.  The data
-// columns' sums are taken about the block's first finite pixel, which the partial states: the
-// deviations then come from one pass whatever the level (about zero, a channel of one
-// non-dyadic value or a mean of 1e6 beside a deviation of 0.3 cancelled to NaN or to a wrong value).
-// With the shift one of the n samples, its distance D from the mean is in the variance as D^2 / n at
-// least, so the cancellation left costs n ulps of FP64 at most.
-ASARF_HD ASARF_INLINE void img_moments_add(double acc[6], float2 v, float2 about) {
+// rows [blk*rpb, ...) in double, NaN samples skipped; deterministic in-block tree.  ABOUT: the data
+// columns' sums are taken about (about_i, about_q) in place of zero.
+template <bool ABOUT>
+ASARF_HD ASARF_INLINE void img_moments_add(const ImgMomentsArgs& a, double acc[6], float2 v) {
     if (is_nan_f(v.x) || is_nan_f(v.y)) return;
-    const double i = static_cast<double>(v.x) - about.x, q = static_cast<double>(v.y) - about.y;
+    double i = v.x, q = v.y;
+    if (ABOUT) i -= a.about_i, q -= a.about_q;
     acc[0] += 1.0;
     acc[1] += i;
     acc[2] += q;
@@ -2450,51 +2448,23 @@ ASARF_HD ASARF_INLINE void img_moments_add(double acc[6], float2 v, float2 about
     acc[4] += q * q;
     acc[5] += i * q;
 }
-
-// First finite data pixel of rows [y0, y1) in row order, 0 when there is none.  One step in nearly
-// every block: threads look at nthr consecutive pixels at a time.
-ASARF_HD ASARF_INLINE float2 img_moments_about(const ImgMomentsArgs& a, int y0, int y1, int tid, int nthr, int* first) {
-    for (int y = y0; y < y1; ++y) {
-        const float2* row = a.img + static_cast<long long>(y) * a.x_stride;
-        for (int x0 = 0; x0 < a.x_size; x0 += nthr) {
-            const int x = x0 + tid;
-            const float2 v = x < a.x_size ? row[x] : make_float2(qnan_f(), qnan_f());
-            const bool ok = v.x - v.x == 0.0f && v.y - v.y == 0.0f;
-#if defined(__CUDA_ARCH__)
-            if (tid == 0) *first = nthr;
-            __syncthreads();
-            if (ok) atomicMin(first, tid);
-            __syncthreads();
-            const int at = *first;
-            __syncthreads();
-            if (at < nthr) return row[x0 + at];
-#else
-            (void)first;
-            if (ok) return v;
-#endif
-        }
-    }
-    return make_float2(0.0f, 0.0f);
-}
-
+template <bool ABOUT>
 ASARF_HD ASARF_INLINE void img_moments_body(const ImgMomentsArgs& a, int blk, int tid, int nthr, double* red) {
     double data[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, pad[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     const int y0 = blk * a.rows_per_block;
     const int y1 = (y0 + a.rows_per_block < a.y_size) ? y0 + a.rows_per_block : a.y_size;
-    const float2 about = img_moments_about(a, y0, y1, tid, nthr, reinterpret_cast<int*>(red));
-    const float2 zero = make_float2(0.0f, 0.0f);
     for (int y = y0; y < y1; ++y) {
         const float2* row = a.img + static_cast<long long>(y) * a.x_stride;
         int x = tid;
         for (; x + 3 * nthr < a.x_size; x += 4 * nthr) {  // four loads in flight
             const float2 v0 = row[x], v1 = row[x + nthr], v2 = row[x + 2 * nthr], v3 = row[x + 3 * nthr];
-            img_moments_add(data, v0, about);
-            img_moments_add(data, v1, about);
-            img_moments_add(data, v2, about);
-            img_moments_add(data, v3, about);
+            img_moments_add<ABOUT>(a, data, v0);
+            img_moments_add<ABOUT>(a, data, v1);
+            img_moments_add<ABOUT>(a, data, v2);
+            img_moments_add<ABOUT>(a, data, v3);
         }
-        for (; x < a.x_size; x += nthr) img_moments_add(data, row[x], about);
-        for (; x < a.x_stride; x += nthr) img_moments_add(pad, row[x], zero);
+        for (; x < a.x_size; x += nthr) img_moments_add<ABOUT>(a, data, row[x]);
+        for (; x < a.x_stride; x += nthr) img_moments_add<false>(a, pad, row[x]);
     }
     for (int k = 0; k < 6; ++k) red[k * nthr + tid] = data[k], red[(6 + k) * nthr + tid] = pad[k];
     ASARF_SYNC();
@@ -2507,9 +2477,7 @@ ASARF_HD ASARF_INLINE void img_moments_body(const ImgMomentsArgs& a, int blk, in
         ASARF_SYNC();
     }
 #endif
-    double* out = a.partial + static_cast<long long>(blk) * kImgMoments;
-    for (int k = tid; k < 12; k += nthr) out[k] = red[k * nthr];
-    if (tid == 0) out[12] = about.x, out[13] = about.y;
+    for (int k = tid; k < 12; k += nthr) a.partial[blk * 12 + k] = red[k * nthr];
 }
 
 // CorrectDCBias + ApplyGainCorrection + ApplyPhaseCorrection (sar/iq_correction.cu:140-178)

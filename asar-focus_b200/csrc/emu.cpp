@@ -268,7 +268,10 @@ int backend_decode_fbaq(const DecodeFbaqArgs& a, void*) {
 
 int backend_img_moments(const ImgMomentsArgs& a, int blocks, void*) {
     std::vector<double> red(12);
-    for (int b = 0; b < blocks; ++b) img_moments_body(a, b, 0, 1, red.data());
+    for (int b = 0; b < blocks; ++b) {
+        if (a.about) img_moments_body<true>(a, b, 0, 1, red.data());
+        else img_moments_body<false>(a, b, 0, 1, red.data());
+    }
     return ASARF_OK;
 }
 int backend_iq_apply(const IqApplyArgs& a, long long n, void*) {

@@ -260,9 +260,10 @@ __global__ void __launch_bounds__(256) k_zero_nans(float2* img, long long n) {
     for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += step) zero_nan_item(img, i);
 }
 
+template <bool ABOUT>
 __global__ void __launch_bounds__(256) k_img_moments(ImgMomentsArgs a) {
     __shared__ double red[12 * 256];
-    img_moments_body(a, blockIdx.x, threadIdx.x, 256, red);
+    img_moments_body<ABOUT>(a, blockIdx.x, threadIdx.x, 256, red);
 }
 
 __global__ void __launch_bounds__(kAcccCols) k_accc(AcccArgs a) {
@@ -459,7 +460,8 @@ int backend_decode_fbaq(const DecodeFbaqArgs& a, void* stream) {
     return check_launch("decode_fbaq");
 }
 int backend_img_moments(const ImgMomentsArgs& a, int blocks, void* stream) {
-    k_img_moments<<<blocks, 256, 0, S(stream)>>>(a);
+    if (a.about) k_img_moments<true><<<blocks, 256, 0, S(stream)>>>(a);
+    else k_img_moments<false><<<blocks, 256, 0, S(stream)>>>(a);
     return check_launch("img_moments");
 }
 int backend_iq_apply(const IqApplyArgs& a, long long n, void* stream) {

@@ -352,13 +352,13 @@ struct DecodeFbaqArgs {
 // NaN-aware moment partials of rows [row0, row0 + rows) per block: data region x < x_size
 // and padding region x_size <= x < x_stride, 12 doubles per block:
 // n, sI, sQ, sII, sQQ, sIQ (data) then the same six for the padding.
-// Partials of an image block: six moments of the data columns about a pixel, six of the padding, the pixel.
-constexpr int kImgMoments = 14;
 struct ImgMomentsArgs {
     const float2* img;
     int x_size, y_size, x_stride;
     int rows_per_block;
-    double* partial;    // [blocks][kImgMoments]
+    int about;          // 1: the data columns' sums about (about_i, about_q)
+    double about_i, about_q;
+    double* partial;    // [blocks][12]: n and the sums of I, Q, I^2, Q^2, I Q of the data columns, then the padding's
 };
 
 struct IqApplyArgs {

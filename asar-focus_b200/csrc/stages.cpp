@@ -43,20 +43,14 @@ struct Scratch {
 
 int nomem() { return set_error(ASARF_ERR_NOMEM, "device allocation failed"); }
 
-// NaN-aware moments of the data block, about the value (i, q), and of the padding columns.
-struct ImageMoments {
-    double i = 0.0, q = 0.0;
-    double data[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // n and the sums of I, Q, I^2, Q^2, I Q
-    double pad[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-};
-
-// The blocks' sums (each about a pixel of its own), moved to the first block's that holds a sample and
-// added on the host in a fixed order.
-int image_moments(const float2* img, int x_size, int y_size, int x_stride, ImageMoments* out, void* stream) {
+// NaN-aware moments of the data block and of the padding columns, summed on the host in a
+// fixed order; about (optional): the value the data block's sums are taken about.
+int image_moments(const float2* img, int x_size, int y_size, int x_stride, const double* about, double out[12],
+                  void* stream) {
     const int rpb = 8;
     const int blocks = (y_size + rpb - 1) / rpb;
     Scratch part(stream);
-    part.add(sizeof(double) * kImgMoments * static_cast<size_t>(blocks));
+    part.add(sizeof(double) * 12 * static_cast<size_t>(blocks));
     if (!part.alloc()) return nomem();
     ImgMomentsArgs a{};
     a.img = img;
@@ -64,29 +58,18 @@ int image_moments(const float2* img, int x_size, int y_size, int x_stride, Image
     a.y_size = y_size;
     a.x_stride = x_stride;
     a.rows_per_block = rpb;
+    if (about) a.about = 1, a.about_i = about[0], a.about_q = about[1];
     a.partial = part.as<double>(0);
     int rc = backend_img_moments(a, blocks, stream);
     if (rc) return rc;
-    std::vector<double> h(kImgMoments * static_cast<size_t>(blocks));
+    std::vector<double> h(12 * static_cast<size_t>(blocks));
     rc = mem_d2h(h.data(), part.p, sizeof(double) * h.size(), stream);
     if (rc) return rc;
     rc = stream_sync(stream);
     if (rc) return rc;
-    for (int b = 0; b < blocks; ++b) {
-        const double* v = &h[kImgMoments * static_cast<size_t>(b)];
-        const double n = v[0];
-        if (n > 0.0) {
-            if (out->data[0] == 0.0) out->i = v[12], out->q = v[13];
-            const double di = v[12] - out->i, dq = v[13] - out->q;
-            out->data[0] += n;
-            out->data[1] += v[1] + n * di;
-            out->data[2] += v[2] + n * dq;
-            out->data[3] += v[3] + 2.0 * di * v[1] + n * di * di;
-            out->data[4] += v[4] + 2.0 * dq * v[2] + n * dq * dq;
-            out->data[5] += v[5] + dq * v[1] + di * v[2] + n * di * dq;
-        }
-        for (int k = 0; k < 6; ++k) out->pad[k] += v[6 + k];
-    }
+    for (int k = 0; k < 12; ++k) out[k] = 0.0;
+    for (int b = 0; b < blocks; ++b)
+        for (int k = 0; k < 12; ++k) out[k] += h[static_cast<size_t>(b) * 12 + k];
     return ASARF_OK;
 }
 
@@ -180,28 +163,34 @@ int asarf_raw_data_correction(void* d_img, int32_t x_size, int32_t y_size, int32
     if (!d_img || !results || x_size <= 0 || y_size <= 0 || x_stride < x_size || y_stride < y_size)
         return set_error(ASARF_ERR_INVALID, "raw_data_correction: bad arguments");
     float2* img = static_cast<float2*>(d_img);
-    ImageMoments m;
-    int rc = image_moments(img, x_size, y_size, x_stride, &m, stream);
+    double m[12];
+    int rc = image_moments(img, x_size, y_size, x_stride, nullptr, m, stream);
     if (rc) return rc;
     const double total = n_total_samples > 0 ? static_cast<double>(n_total_samples) : static_cast<double>(x_size) * y_size;
     const float totf = static_cast<float>(total);
     // CalcMean: float(double sum) / float(total)
-    const float dc_i = static_cast<float>(m.data[1] + m.data[0] * m.i) / totf;
-    const float dc_q = static_cast<float>(m.data[2] + m.data[0] * m.q) / totf;
-    // sums over x < XStride after the DC step, both regions (closed forms of the FP64 moments; a sum of
-    // squares that is zero may round to just below it)
-    auto sq = [](const double* s, int s1, int s2, double d) {
-        const double v = s[s2] - 2.0 * d * s[s1] + s[0] * d * d;
-        return v < 0.0 ? 0.0 : v;
-    };
-    auto cross = [](const double* s, double di, double dq) { return s[5] - dq * s[1] - di * s[2] + s[0] * di * dq; };
-    const double di = dc_i, dq = dc_q, ei = di - m.i, eq = dq - m.q;  // the mean, and from m's value
-    const double cii = sq(m.data, 1, 3, ei), cqq = sq(m.data, 2, 4, eq);
+    const float dc_i = static_cast<float>(m[1]) / totf;
+    const float dc_q = static_cast<float>(m[2]) / totf;
+    // sums over x < XStride after the DC step, both regions (closed forms of the FP64 moments)
+    const double di = dc_i, dq = dc_q;
+    auto sq = [&](int o, int s1, int s2, double d) { return m[o + s2] - 2.0 * d * m[o + s1] + m[o] * d * d; };
+    auto cross = [&](int o) { return m[o + 5] - dq * m[o + 1] - di * m[o + 2] + m[o] * di * dq; };
+    double cii = sq(0, 1, 3, di), cqq = sq(0, 2, 4, dq), ciq = cross(0);
+    // The closed form loses S2 / c of the FP64 sums' digits: where a channel's spread is that small beside its level
+    // (a dead channel; never a raw signal), the sums are taken again about the mean itself.
+    constexpr double kCancels = 1e-4;
+    if (cii <= kCancels * m[3] || cqq <= kCancels * m[4]) {
+        const double about[2] = {di, dq};
+        double c[12];
+        rc = image_moments(img, x_size, y_size, x_stride, about, c, stream);
+        if (rc) return rc;
+        cii = c[3], cqq = c[4], ciq = c[5];
+    }
     const float std_i = std::sqrt(static_cast<float>(cii) / totf);
     const float std_q = std::sqrt(static_cast<float>(cqq) / totf);
-    const double i1sq = cii + sq(m.pad, 1, 3, di);
-    const double q1sq = cqq + sq(m.pad, 2, 4, dq);
-    const double i1q1 = cross(m.data, ei, eq) + cross(m.pad, di, dq);
+    const double i1sq = cii + sq(6, 1, 3, di);
+    const double q1sq = cqq + sq(6, 2, 4, dq);
+    const double i1q1 = ciq + cross(6);
     const double gain = std::sqrt(i1sq / q1sq);
     const float gf = static_cast<float>(gain);
     const double delta = (i1q1 / gf) / (i1sq / (static_cast<double>(gf) * gf));

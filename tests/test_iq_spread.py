@@ -5,8 +5,8 @@ the first pixel, a total that counts more samples than were filled.
 The reference value is sqrt(sum (v - dc)^2 / total) in FP64 about the mean that the call itself
 reports, so a dead channel gives |v - dc|, at most an ulp of the level.  The call forms the sum in FP64
 and rounds it, the quotient and the root to float32: three roundings of at most 2^-24 each, halved by the
-root for the first two, so 1.2e-7; the sums themselves are taken about an image value and lose less than
-n * 2^-53 * 10 relative (n = 120000 pixels: 1.4e-10).  2e-7 covers both.
+root for the first two, so 1.2e-7; the FP64 sums lose at most 1e4 times their own rounding (1e-14 of
+120000 pixels), 1e-10, before they are taken again about the mean.  2e-7 covers both.
 """
 from __future__ import annotations
 
